@@ -374,16 +374,16 @@ __global__ void __launch_bounds__(256) k_adj_ph(DevTables T, const double *__res
   const unsigned long long u = p.rows;
   const unsigned x1 = (unsigned)(u & 0xFFFF), y1 = (unsigned)((u >> 16) & 0xFFFF);
   const unsigned x2 = (unsigned)((u >> 32) & 0xFFFF), y2 = (unsigned)(u >> 48);
-  const int rl = T.cc_rlen[p.qx];
-  double *W = WCCb + T.wcc_off[p.qx];
+  const int q1 = p.q & 0xFFFF, q2 = p.q >> 16, rl = T.cc_rlen[q1];
+  double *W = WCCb + T.wcc_off[q1], *W2 = WCCb + T.wcc_off[q2];  // the two blocks have one size
   const double a = dflip(z, hL < 0), c = -dflip(z, hR < 0);
   if (x1 != 0xFFFFu && y1 != 0xFFFFu) {
     atomicAdd(W + x1 + (long)y1 * rl, a);
     atomicAdd(W + y1 + (long)x1 * rl, c);
   }
   if (x2 != 0xFFFFu && y2 != 0xFFFFu) {
-    atomicAdd(W + x2 + (long)y2 * rl, dflip(a, p.nph));
-    atomicAdd(W + y2 + (long)x2 * rl, dflip(c, p.nph));
+    atomicAdd(W2 + x2 + (long)y2 * rl, dflip(a, p.nph));
+    atomicAdd(W2 + y2 + (long)x2 * rl, dflip(c, p.nph));
   }
 }
 

@@ -450,11 +450,11 @@ int imsrg_gpu_basis_info(const imsrg_basis_t *b, imsrg_basis_info_t *info) {
   info->nparts = b->P;
   info->nblocks = b->nblocks;
   info->jtotal_max = b->jtm;
-  info->ccblocks = b->ccblocks;
+  info->ccblocks = b->ccgroups;
   info->nfull = b->nfull;
   info->neq = b->neq;
-  info->cc_total = b->cc_total;
-  info->wcc_total = b->wcc_total;
+  info->cc_total = b->cc_total_ref;
+  info->wcc_total = b->wcc_total_ref;
   return IMSRG_OK;
 }
 

@@ -75,7 +75,7 @@ struct DevTables {
   const unsigned *pre_el;
   const unsigned long long *pre_terms;
   int n_pre_warps;
-  const int *ccf_order;    // cross-coupled elements (bits 0-23), with their block in bits 24-30 if ccf_packed
+  const int *ccf_order;    // cross-coupled elements (bits 0-23), with their exponent group in bits 24-30 if ccf_packed
   int n_ccf;
   int ccf_packed;
   // Gather lists of the Pandya transform: element e of every CC block is
@@ -121,12 +121,14 @@ struct __align__(16) Asm2PreWarp {
 // channel: the kernel forms
 //   Z = herm_L (W(x1,y1) + e W(x2,y2)) - herm_R (e W(y2,x2) + W(y1,x1))
 // from four cross-coupled rows (16 bits each in `rows`: x1, y1, x2, y2;
-// 0xFFFF = absent) of WCC block qx, e = (-1)^((ja+jb+jc+jd)/2).  The
+// 0xFFFF = absent), x1 and y1 of WCC block q & 0xFFFF, x2 and y2 of block
+// q >> 16 (the same block at equal isospins, its pair otherwise), e =
+// (-1)^((ja+jb+jc+jd)/2).  The
 // reference's four products per J' become sum_J' {6j} Z(J') per element, with
 // the inside channel's (-1)^n2(J) applied after the sum.
 struct __align__(16) PhTerm {
   unsigned long long rows;
-  int qx;
+  int q;
   int nph;  // the exponent of e
 };
 
@@ -244,7 +246,7 @@ struct Profiler {
 
 struct imsrg_basis {
   // host copies
-  int norb, A, P, nblocks, jtm, ccblocks;
+  int norb, A, P, nblocks, jtm, ccblocks, ccgroups;
   std::vector<int> nn, ll, jj, itzp, con;
   std::vector<int> holes, parts;  // 0-based orbit ids
   std::vector<int> npp, nph, nhh; // per block
@@ -252,9 +254,11 @@ struct imsrg_basis {
   std::vector<int> gam_n1, gam_n2;
   std::vector<std::vector<int>> qn;  // [q*3+c] pair list (0-based, 2 ints per pair)
   std::vector<int> cc_rlen, cc_nph, cc_J2;
+  std::vector<int> cc_group;         // the reference's (J', |Tz|, parity) block of each cross-coupled block
   std::vector<int> pairrow;          // [(a * norb + b) * (jtm + 1) + J2 / 2] row of pair a <= b in its block
   std::vector<long> cc_off, wcc_off;
   long nfull = 0, neq = 0, cc_total = 0, wcc_total = 0;
+  long cc_total_ref = 0, wcc_total_ref = 0;  // the same in the reference's blocks (zeros between them included)
   long off_fhh = 1, off_fph = 0, off_fpp = 0;
 
   // device

@@ -279,14 +279,15 @@ __global__ void __launch_bounds__(256) k_ph_inputs(DevTables T, const double *__
   const unsigned long long u = p.rows;
   const unsigned x1 = (unsigned)(u & 0xFFFF), y1 = (unsigned)((u >> 16) & 0xFFFF);
   const unsigned x2 = (unsigned)((u >> 32) & 0xFFFF), y2 = (unsigned)(u >> 48);
-  const int rl = T.cc_rlen[p.qx];
+  const int q1 = p.q & 0xFFFF, q2 = p.q >> 16, rl = T.cc_rlen[q1];  // both blocks have one size and scale
   if (exps) {
-    const long long *W = reinterpret_cast<const long long *>(WCC) + T.wcc_off[p.qx];
-    const long long w2 = wcc_at_int(W, rl, x2, y2), w3 = wcc_at_int(W, rl, y2, x2);
+    const long long *W = reinterpret_cast<const long long *>(WCC) + T.wcc_off[q1];
+    const long long *V = reinterpret_cast<const long long *>(WCC) + T.wcc_off[q2];
+    const long long w2 = wcc_at_int(V, rl, x2, y2), w3 = wcc_at_int(V, rl, y2, x2);
     const long long a = wcc_at_int(W, rl, x1, y1) + (p.nph ? -w2 : w2);
     const long long c = (p.nph ? -w3 : w3) + wcc_at_int(W, rl, y1, x1);
     const long long z = (hL < 0 ? -a : a) - (hR < 0 ? -c : c);
-    const int2 g = ccg[p.qx];
+    const int2 g = ccg[q1];
     const int k = (exps[g.x] - 1022) + (exps[g.y] - 1022) - kshift;
     // z 2^k: add k to the exponent field on the integer pipe when the result
     // stays normal (exactly ldexp's value), else ldexp
@@ -302,9 +303,9 @@ __global__ void __launch_bounds__(256) k_ph_inputs(DevTables T, const double *__
     Z[t] = d;
     return;
   }
-  const double *W = WCC + T.wcc_off[p.qx];
-  const double a = wcc_at(W, rl, x1, y1) + dflip(wcc_at(W, rl, x2, y2), p.nph);
-  const double c = dflip(wcc_at(W, rl, y2, x2), p.nph) + wcc_at(W, rl, y1, x1);
+  const double *W = WCC + T.wcc_off[q1], *V = WCC + T.wcc_off[q2];
+  const double a = wcc_at(W, rl, x1, y1) + dflip(wcc_at(V, rl, x2, y2), p.nph);
+  const double c = dflip(wcc_at(V, rl, y2, x2), p.nph) + wcc_at(W, rl, y1, x1);
   Z[t] = dflip(a, hL < 0) - dflip(c, hR < 0);
 }
 

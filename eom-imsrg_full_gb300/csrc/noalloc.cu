@@ -60,7 +60,9 @@ extern "C" int imsrg_gpu_commutator_noalloc(imsrg_basis_t *b, const double *d_L,
   if ((herm_L != 1 && herm_L != -1) || (herm_R != 1 && herm_R != -1)) return IMSRG_ERR_INVALID;
   if (overlaps(d_RES, d_L, b->nfull) || overlaps(d_RES, d_R, b->nfull)) return IMSRG_ERR_INVALID;
   long ne0p = round_up(imsrg::asm2_ctas(b));
-  long need = 2 * round_up(b->nfull) + 2 * round_up(b->cc_total) + round_up(b->wcc_total) + round_up(b->T.n_ph) + ne0p;
+  // the limit of the documented sizes (imsrg_basis_info_t), at least what is used
+  long need = 2 * round_up(b->nfull) + 2 * round_up(b->cc_total_ref) + round_up(b->wcc_total_ref) +
+              round_up(b->T.n_ph) + ne0p;
   if (need > IMSRG_NOALLOC_SCRATCH_DOUBLES) return IMSRG_ERR_TOO_LARGE;
   int dev = -1;
   cudaError_t e = cudaGetDevice(&dev);

@@ -896,7 +896,8 @@ int ozaki_prepare(imsrg_basis *b) {
   if (major != 10) return IMSRG_ERR_INVALID;  // tcgen05 needs a Blackwell data-center part
 
   // matrices: L and R arrays per (2J,Tz,parity) block (one exponent group per
-  // block), LCC and RCC per cross-coupled block (one group each)
+  // block), LCC and RCC per cross-coupled block (one group each per block of the
+  // reference)
   std::map<std::pair<int, long>, int> mat_of;  // (src, off) -> matrix index
   std::vector<OzChunk> &chunks = pl->chunks;
   int ngroups = 0;
@@ -929,10 +930,15 @@ int ozaki_prepare(imsrg_basis *b) {
   pl->group_lo[2] = ngroups;
   pl->chunk_lo[2] = (int)chunks.size();
   for (int src = 2; src < 4; src++)
-    for (int q1 = 0; q1 < b->ccblocks; q1++) {
-      long len = (long)b->cc_rlen[q1] * b->cc_nph[q1];
-      int g = add_group(src, b->cc_off[q1], len);
-      add_matrix(src, g, b->cc_off[q1], b->cc_rlen[q1], b->cc_nph[q1]);
+    for (int q0 = 0; q0 < b->ccblocks;) {  // the blocks of one group are neighbours
+      int q1 = q0;
+      long len = 0;
+      while (q1 < b->ccblocks && b->cc_group[q1] == b->cc_group[q0]) {
+        len += (long)b->cc_rlen[q1] * b->cc_nph[q1];
+        q1++;
+      }
+      int g = add_group(src, b->cc_off[q0], len);
+      for (; q0 < q1; q0++) add_matrix(src, g, b->cc_off[q0], b->cc_rlen[q0], b->cc_nph[q0]);
     }
   pl->ngroups = ngroups;
   pl->nchunks = (int)chunks.size();
@@ -1151,7 +1157,7 @@ int ozaki_prepare(imsrg_basis *b) {
   IMSRG_TRY(up(pl->maps.data(), pl->maps.size() * sizeof(CUtensorMap), (void **)&pl->d_maps));
   std::vector<int2> ccg(b->ccblocks);
   for (int q1 = 0; q1 < b->ccblocks; q1++)
-    ccg[q1] = make_int2(pl->group_lo[2] + q1, pl->group_lo[2] + b->ccblocks + q1);
+    ccg[q1] = make_int2(pl->group_lo[2] + b->cc_group[q1], pl->group_lo[2] + b->ccgroups + b->cc_group[q1]);
   IMSRG_TRY(up(ccg.data(), ccg.size() * sizeof(int2), (void **)&pl->d_ccgroups));
   IMSRG_CUDA_TRY(cudaMalloc((void **)&pl->d_exps, std::max(pl->ngroups, 1) * sizeof(int)));
   IMSRG_CUDA_TRY(cudaMalloc((void **)&pl->d_err, sizeof(int)));
@@ -1182,7 +1188,7 @@ int ozaki_cc_exponents(imsrg_basis *b, cudaStream_t st, int **exps, int *gL, int
   if (g1 > g0) IMSRG_CUDA_TRY(cudaMemsetAsync(pl->d_exps + g0, 0, (g1 - g0) * sizeof(int), st));
   *exps = pl->d_exps;
   *gL = g0;
-  *gR = g0 + b->ccblocks;
+  *gR = g0 + b->ccgroups;
   return IMSRG_OK;
 }
 

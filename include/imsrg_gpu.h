@@ -79,11 +79,11 @@ typedef struct {
   int norb, nholes, nparts;
   int nblocks;       /* (Jtotal_max + 1) * 6 */
   int jtotal_max;    /* maxval(jj) */
-  int ccblocks;      /* (Jtotal_max + 1) * 4 */
+  int ccblocks;      /* (Jtotal_max + 1) * 4: the reference's cross-coupled blocks */
   long nfull;        /* doubles in the flat layout */
   long neq;          /* doubles in the packed (vectorize) layout */
-  long cc_total;     /* doubles of one cross-coupled operator (all CCX) */
-  long wcc_total;    /* doubles of the WCC workspace */
+  long cc_total;     /* doubles of one cross-coupled operator (all CCX) in those blocks */
+  long wcc_total;    /* doubles of all rlen x rlen products WCC of those blocks */
 } imsrg_basis_info_t;
 
 /* --- basis (replaces read_sp_basis/find_holes + allocate_blocks +

@@ -39,7 +39,7 @@
 #include <cstring>
 #include <vector>
 
-#include "device.cuh"
+#include "gemm_fp64.cuh"
 
 namespace imsrg {
 
@@ -48,9 +48,8 @@ namespace {
 // ---------------------------------------------------------------------------
 // Grouped FP64 products of the adjoint: C += sum_t alpha_t op(A_t) op(B_t),
 // each term with its own contraction length (the transposed ladder products
-// of one output array read different intermediates).  64 x 64 tiles laid out
-// as the forward's k_gemm_fp64: warp w owns columns 8w .. 8w + 7 and skips
-// its products when they lie past N; a short last K chunk runs only its k.
+// of one output array read different intermediates), in the forward's tiles
+// (gemm_fp64.cuh).
 // ---------------------------------------------------------------------------
 struct AdjTerm {
   int a_src, b_src, ta, tb;
@@ -64,7 +63,7 @@ constexpr int kAdjTerms = 6;
 struct AdjProb {
   int M, N, nterms, c_dst;
   long c_off;
-  int ldc, tile0, tiles_m, tiles;
+  int ldc;
   AdjTerm t[kAdjTerms];
 };
 
@@ -75,94 +74,20 @@ struct AdjOps {
   double *dst[2];
 };
 
-constexpr int BM = 64, BN = 64, BK = 16;
-
-__global__ void __launch_bounds__(256) k_gemm_adj(const AdjProb *__restrict__ probs, int nprobs, AdjOps ops, int hL,
-                                                  int hR) {
-  __shared__ double As[BK][BM + 1];
-  __shared__ double Bs[BK][BN + 1];
-  const int tile = blockIdx.x;
-  int lo = 0, hi = nprobs;
-  while (lo < hi) {
-    const int mid = (lo + hi) >> 1;
-    if (probs[mid].tile0 <= tile) lo = mid + 1;
-    else hi = mid;
-  }
-  const AdjProb &P = probs[lo - 1];
-  const int lt = tile - P.tile0;
-  const int m0 = (lt % P.tiles_m) * BM, n0 = (lt / P.tiles_m) * BN;
-  const int tid = threadIdx.x, tx = tid & 15, ty = tid >> 4;
-  const bool live = n0 + 8 * (tid >> 5) < P.N;  // warp-uniform: the warp's eight columns 4 ty + j
-  double acc[4][4];
-#pragma unroll
-  for (int i = 0; i < 4; i++)
-#pragma unroll
-    for (int j = 0; j < 4; j++) acc[i][j] = 0.0;
-  for (int it = 0; it < P.nterms; it++) {
-    const AdjTerm &Tm = P.t[it];
-    const double *A = ops.src[Tm.a_src] + Tm.a_off;
-    const double *B = ops.src[Tm.b_src] + Tm.b_off;
-    const double alpha = Tm.coef * (Tm.use_hl ? hL : 1) * (Tm.use_hr ? hR : 1);
-    double part[4][4];
-#pragma unroll
-    for (int i = 0; i < 4; i++)
-#pragma unroll
-      for (int j = 0; j < 4; j++) part[i][j] = 0.0;
-    for (int k0 = 0; k0 < Tm.K; k0 += BK) {
-#pragma unroll
-      for (int l = 0; l < 4; l++) {
-        int m, k;
-        if (!Tm.ta) { m = tid & 63; k = (tid >> 6) + 4 * l; }
-        else { k = tid & 15; m = (tid >> 4) + 16 * l; }
-        const int gm = m0 + m, gk = k0 + k;
-        double v = 0.0;
-        if (gm < P.M && gk < Tm.K) v = Tm.ta ? A[gk + (long)gm * Tm.lda] : A[gm + (long)gk * Tm.lda];
-        As[k][m] = v;
-      }
-#pragma unroll
-      for (int l = 0; l < 4; l++) {
-        int n, k;
-        if (!Tm.tb) { k = tid & 15; n = (tid >> 4) + 16 * l; }
-        else { n = tid & 63; k = (tid >> 6) + 4 * l; }
-        const int gn = n0 + n, gk = k0 + k;
-        double v = 0.0;
-        if (gn < P.N && gk < Tm.K) v = Tm.tb ? B[gn + (long)gk * Tm.ldb] : B[gk + (long)gn * Tm.ldb];
-        Bs[k][n] = v;
-      }
-      __syncthreads();
-      const int kn = live ? min(BK, Tm.K - k0) : 0;
-#pragma unroll
-      for (int k = 0; k < BK; k++) {
-        if (k < kn) {
-          double a[4], bv[4];
-#pragma unroll
-          for (int i = 0; i < 4; i++) a[i] = As[k][tx + 16 * i];
-#pragma unroll
-          for (int j = 0; j < 4; j++) bv[j] = Bs[k][4 * ty + j];
-#pragma unroll
-          for (int i = 0; i < 4; i++)
-#pragma unroll
-            for (int j = 0; j < 4; j++) part[i][j] = fma(a[i], bv[j], part[i][j]);
-        }
-      }
-      __syncthreads();
-    }
-#pragma unroll
-    for (int i = 0; i < 4; i++)
-#pragma unroll
-      for (int j = 0; j < 4; j++) acc[i][j] += alpha * part[i][j];
-  }
-  double *Cp = ops.dst[P.c_dst] + P.c_off;
-#pragma unroll
-  for (int j = 0; j < 4; j++) {
-    const int gn = n0 + 4 * ty + j;
-    if (gn >= P.N) continue;
-#pragma unroll
-    for (int i = 0; i < 4; i++) {
-      const int gm = m0 + tx + 16 * i;
-      if (gm < P.M) Cp[gm + (long)gn * P.ldc] += acc[i][j];
-    }
-  }
+__global__ void __launch_bounds__(GT_THREADS, GT_CTAS) k_gemm_adj(const AdjProb *__restrict__ probs,
+                                                         const GemmTile *__restrict__ tiles, AdjOps ops, int hL,
+                                                         int hR) {
+  const GemmTile t = tiles[blockIdx.x];
+  const AdjProb &P = probs[t.prob];
+  gemm_cta_tile<true>(
+      t,
+      [&](int it, auto add) {
+        const AdjTerm &m = P.t[it];
+        add(ops.src[m.a_src] + m.a_off, m.ta ? (long)m.lda : 1L, m.ta ? 1L : (long)m.lda, ops.src[m.b_src] + m.b_off,
+            m.tb ? (long)m.ldb : 1L, m.tb ? 1L : (long)m.ldb, m.K,
+            (m.coef < 0) ^ (m.use_hl && hL < 0) ^ (m.use_hr && hR < 0));  // coefficients are +-1
+      },
+      P.nterms, P.M, P.N, ops.dst[P.c_dst] + P.c_off, P.ldc);
 }
 
 // ---------------------------------------------------------------------------
@@ -432,7 +357,8 @@ struct AdjState {
   double *w1b = nullptr, *w2b = nullptr, *rccb = nullptr, *wccb = nullptr, *zb = nullptr;
   double *monob = nullptr, *part = nullptr, *dot = nullptr, *h_dot = nullptr;
   AdjProb *d_probs = nullptr;
-  int nprobs = 0, ntiles = 0;
+  GemmTile *d_tiles = nullptr;
+  int ntiles = 0;
 };
 
 namespace {
@@ -519,13 +445,6 @@ std::vector<AdjProb> adjoint_problems(const imsrg_basis *b) {
     const int r = b->cc_rlen[q1], nb = b->cc_nph[q1];
     add(r, nb, AD_RCC, b->cc_off[q1], r, {aterm(AS_WCC, b->wcc_off[q1], r, 1, AS_LCC, b->cc_off[q1], r, 0, r, 1.0)});
   }
-  int tiles = 0;
-  for (AdjProb &p : out) {
-    p.tiles_m = (p.M + BM - 1) / BM;
-    p.tiles = p.tiles_m * ((p.N + BN - 1) / BN);
-    p.tile0 = tiles;
-    tiles += p.tiles;
-  }
   return out;
 }
 
@@ -545,15 +464,22 @@ int adjoint_prepare(imsrg_basis *b) {
   IMSRG_TRY(adj_alloc(b, 1, &a->dot));
   IMSRG_CUDA_TRY(cudaMallocHost((void **)&a->h_dot, sizeof(double)));
   std::vector<AdjProb> probs = adjoint_problems(b);
-  a->nprobs = (int)probs.size();
-  a->ntiles = probs.empty() ? 0 : probs.back().tile0 + probs.back().tiles;
-  if (a->nprobs) {
-    void *p = nullptr;
-    IMSRG_CUDA_TRY(cudaMalloc(&p, probs.size() * sizeof(AdjProb)));
-    b->dev_allocs.push_back(p);
-    a->d_probs = (AdjProb *)p;
-    IMSRG_CUDA_TRY(cudaMemcpy(a->d_probs, probs.data(), probs.size() * sizeof(AdjProb), cudaMemcpyHostToDevice));
+  std::vector<GemmShape> shapes;
+  for (const AdjProb &p : probs) {
+    long k = 0;
+    for (int t = 0; t < p.nterms; t++) k += p.t[t].K;
+    shapes.push_back({p.M, p.N, k, 0});
   }
+  gemm_split(shapes, b->num_sms);
+  const std::vector<GemmTile> tiles = gemm_tiles(shapes);
+  a->ntiles = (int)tiles.size();
+  auto up = [&](const void *h, size_t bytes, void **d) -> int {
+    IMSRG_CUDA_TRY(cudaMalloc(d, std::max<size_t>(bytes, 16)));
+    b->dev_allocs.push_back(*d);
+    return cuda_status(cudaMemcpy(*d, h, bytes, cudaMemcpyHostToDevice));
+  };
+  IMSRG_TRY(up(probs.data(), probs.size() * sizeof(AdjProb), (void **)&a->d_probs));
+  IMSRG_TRY(up(tiles.data(), tiles.size() * sizeof(GemmTile), (void **)&a->d_tiles));
   return IMSRG_OK;
 }
 
@@ -602,7 +528,7 @@ int commutator_adjoint_dev(imsrg_basis *b, const double *X, int hX, const double
     ops.src[AS_LCC] = b->lcc;
     ops.dst[AD_Y] = Yb;
     ops.dst[AD_RCC] = a->rccb;
-    k_gemm_adj<<<a->ntiles, 256, 0, st>>>(a->d_probs, a->nprobs, ops, hL, hR);
+    k_gemm_adj<<<a->ntiles, GT_THREADS, 0, st>>>(a->d_probs, a->d_tiles, ops, hL, hR);
   }
   if (b->cc_total > 0)
     k_adj_cc<<<(unsigned)((b->cc_total + 255) / 256), 256, 0, st>>>(b->T, a->rccb, hR, Yb);

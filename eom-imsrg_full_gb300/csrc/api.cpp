@@ -729,8 +729,7 @@ struct imsrg_batch {
   // merged FP64 product lists, one per operand set (graphs replay them)
   struct Fp64List {
     std::vector<const void *> key;
-    imsrg::GemmProb *d_probs;
-    int nprobs, ntiles;
+    imsrg::GemmMerged g;
   };
   std::vector<Fp64List> fp64;
 };
@@ -740,7 +739,7 @@ namespace {
 void batch_release(imsrg_batch *bt) {
   imsrg::batch_flow_free(bt->flow);
   bt->flow = nullptr;
-  for (imsrg_batch::Fp64List &l : bt->fp64) cudaFree(l.d_probs);
+  for (imsrg_batch::Fp64List &l : bt->fp64) l.g.release();
   bt->fp64.clear();
   for (imsrg_batch::Graph &g : bt->graphs) cudaGraphExecDestroy(g.exec);
   bt->graphs.clear();
@@ -769,8 +768,8 @@ int batch_fp64_list(imsrg_batch *bt, imsrg_op_t *const *L, imsrg_op_t *const *R,
       *out = &l;
       return IMSRG_OK;
     }
-  imsrg_batch::Fp64List l{key, nullptr, 0, 0};
-  IMSRG_TRY(imsrg::gemm_fp64_merged(bt->bases.data(), n, dl.data(), dr.data(), &l.d_probs, &l.nprobs, &l.ntiles));
+  imsrg_batch::Fp64List l{key, {}};
+  IMSRG_TRY(imsrg::gemm_fp64_merged(bt->bases.data(), n, dl.data(), dr.data(), &l.g));
   bt->fp64.push_back(l);
   *out = &bt->fp64.back();
   return IMSRG_OK;
@@ -800,8 +799,7 @@ int batch_sequence(imsrg_batch *bt, imsrg_op_t *const *L, imsrg_op_t *const *R, 
   if (oz) {
     IMSRG_TRY(imsrg::ozaki_batch_mma(bt->oz, bt->st, L[0]->herm, R[0]->herm));
   } else {
-    IMSRG_TRY(imsrg::launch_gemm_fp64_merged(fl->d_probs, fl->nprobs, fl->ntiles, L[0]->herm, R[0]->herm, nullptr,
-                                             bt->st));
+    IMSRG_TRY(imsrg::launch_gemm_fp64_merged(fl->g, L[0]->herm, R[0]->herm, nullptr, bt->st));
   }
   for (imsrg_basis *b : bt->bases) b->launches++;
   IMSRG_CUDA_TRY(cudaEventRecord(bt->ev_mma, bt->st));

@@ -385,25 +385,8 @@ int build_basis(imsrg_basis *b) {
     pb.add(r, r, nb, SRC_WCC, b->wcc_off[q1], r,
            {term(SRC_LCC, b->cc_off[q1], r, 0, SRC_RCC, b->cc_off[q1], r, 1, 1.0)});
   }
-  // FP64 tiles: 64 x 64, or 256 x 8 for the problems whose output has at
-  // most eight columns (the hole-pair-wide ladder products), which a 64-wide
-  // tile would mostly pad
-  int tiles = 0;
-  for (GemmProb &p : pb.probs) {
-    p.shape = p.N <= 8 ? 1 : 0;
-    if (p.shape == 1) {
-      p.tiles_m = (p.M + 255) / 256;
-      p.tiles = p.tiles_m;
-    } else {
-      p.tiles_m = (p.M + 63) / 64;
-      p.tiles = p.tiles_m * ((p.N + 63) / 64);
-    }
-    p.tile0 = tiles;
-    tiles += p.tiles;
-  }
   b->probs = pb.probs;
   b->nprobs = (int)pb.probs.size();
-  b->ntiles = tiles;
 
   // norm chunks (mat_frob_norm weights: fph and non-square gam count twice)
   std::vector<NormChunk> chunks;
@@ -923,9 +906,15 @@ int build_basis(imsrg_basis *b) {
   IMSRG_TRY(dev_upload(b, b->holes, &T.hole_orb));
   IMSRG_TRY(dev_upload(b, b->parts, &T.part_orb));
   T.n_ph_pairs = (int)ph_pairs.size() / 2;
+  gemm_fp64_plan(b->probs, b->num_sms);
+  const std::vector<GemmTile> tiles = gemm_fp64_tiles(b->probs);
+  b->ntiles = (int)tiles.size();
   const GemmProb *dp = nullptr;
   IMSRG_TRY(dev_upload(b, b->probs, &dp));
   b->d_probs = (GemmProb *)dp;
+  const GemmTile *dt = nullptr;
+  IMSRG_TRY(dev_upload(b, tiles, &dt));
+  b->d_tiles = (GemmTile *)dt;
   const NormChunk *dc = nullptr;
   IMSRG_TRY(dev_upload(b, chunks, &dc));
   b->d_chunks = (NormChunk *)dc;

@@ -440,8 +440,7 @@ struct BatchFlowGraph {
   FlowDev *d_state = nullptr, *h_state = nullptr;
   int *d_go = nullptr, *d_flow = nullptr, *d_act = nullptr, *h_flow = nullptr;
   cudaGraphConditionalHandle *d_h = nullptr;  // IF handles: 3n of the step, 2n per series body
-  GemmProb *d_fp64 = nullptr;                 // FP64: the merged product list of [G_i, X0_i]
-  int fp64_nprobs = 0, fp64_ntiles = 0;
+  GemmMerged fp64;                            // FP64: the merged product list of [G_i, X0_i]
   cudaGraph_t graph = nullptr;
   cudaGraphExec_t exec = nullptr;
 };
@@ -456,7 +455,7 @@ void batch_flow_free(void *p) {
   cudaFree(f->d_flow);
   cudaFree(f->d_act);
   cudaFree(f->d_h);
-  cudaFree(f->d_fp64);
+  f->fp64.release();
   if (f->h_state) cudaFreeHost(f->h_state);
   if (f->h_flow) cudaFreeHost(f->h_flow);
   delete f;
@@ -478,7 +477,7 @@ int build_batch_graph(BatchFlowGraph *f, imsrg_basis *const *bases, void *oz, cu
       Lp[i] = G[i]->d;
       Rp[i] = X0[i]->d;
     }
-    IMSRG_TRY(gemm_fp64_merged(bases, n, Lp.data(), Rp.data(), &f->d_fp64, &f->fp64_nprobs, &f->fp64_ntiles));
+    IMSRG_TRY(gemm_fp64_merged(bases, n, Lp.data(), Rp.data(), &f->fp64));
   }
   cudaGraph_t g = nullptr;
   IMSRG_CUDA_TRY(cudaGraphCreate(&g, 0));
@@ -548,7 +547,7 @@ int build_batch_graph(BatchFlowGraph *f, imsrg_basis *const *bases, void *oz, cu
     std::vector<cudaGraphNode_t> mfr;
     IMSRG_TRY(capture_st(st, body, fronts, [&]() -> int {
       if (ozp) return ozaki_batch_mma(oz, st, -1, hX, f->d_act);
-      return launch_gemm_fp64_merged(f->d_fp64, f->fp64_nprobs, f->fp64_ntiles, -1, hX, f->d_act, st);
+      return launch_gemm_fp64_merged(f->fp64, -1, hX, f->d_act, st);
     }, &mfr));
     for (int i = 0; i < n; i++) {
       imsrg_basis *b = bases[i];

@@ -172,12 +172,14 @@ struct GemmProb {
   int c_dst;
   long c_off;
   int ldc;
-  int tile0;    // first tile id of this problem
-  int tiles_m;  // tiles along M
-  int tiles;    // tiles of this problem
-  int shape;    // FP64 tile: 0 = 64 x 64, 1 = 256 x 8 (problems with N <= 8)
+  int split;      // the FP64 tiles split K over a CTA's warps (gemm_fp64.cuh)
   double *c_abs;  // merged lists of several bases: the output itself
   int inst;       // merged lists: the basis the problem belongs to
+};
+
+// One CTA of a grouped FP64 product: outputs from (m0, n0) of a problem.
+struct __align__(16) GemmTile {
+  int prob, m0, n0, split;
 };
 
 struct Operands {
@@ -299,6 +301,7 @@ struct imsrg_basis {
   int partials_len = 0;
   // grouped GEMM problems
   imsrg::GemmProb *d_probs = nullptr;
+  imsrg::GemmTile *d_tiles = nullptr;
   int nprobs = 0, ntiles = 0;
   std::vector<imsrg::GemmProb> probs;
   // norm chunks
@@ -370,13 +373,26 @@ int launch_cc_forward(imsrg_basis *b, const double *L, int hL, const double *R, 
                       int gL = 0, int gR = 0, int sides = 3, cudaStream_t st = nullptr);
 int launch_gemm_fp64(imsrg_basis *b, const double *L, int hL, const double *R, int hR);
 // The FP64 products of several bases (operators L[i], R[i] of bases[i]) as one
-// problem list with absolute pointers, uploaded to *d_probs (cudaFree it).
+// problem list with absolute pointers, and its tiles.
+struct GemmMerged {
+  GemmProb *d_probs = nullptr;
+  GemmTile *d_tiles = nullptr;
+  int ntiles = 0;
+  void release() {
+    cudaFree(d_probs);
+    cudaFree(d_tiles);
+    d_probs = nullptr;
+    d_tiles = nullptr;
+  }
+};
 int gemm_fp64_merged(imsrg_basis *const *bases, int n, const double *const *L, const double *const *R,
-                     GemmProb **d_probs, int *nprobs, int *ntiles);
+                     GemmMerged *out);
+// which problems of a list split K, and the list's tiles, longest first
+void gemm_fp64_plan(std::vector<GemmProb> &probs, int num_sms);
+std::vector<GemmTile> gemm_fp64_tiles(const std::vector<GemmProb> &probs);
 // one launch of a merged list; act (optional, one int per basis): only the
 // bases with act[i] != 0 take part
-int launch_gemm_fp64_merged(const GemmProb *d_probs, int nprobs, int ntiles, int hL, int hR, const int *act,
-                            cudaStream_t st);
+int launch_gemm_fp64_merged(const GemmMerged &g, int hL, int hR, const int *act, cudaStream_t st);
 // the two-body assembly: the recoupling inputs of 222_ph, then the elements
 // [w0, w1) of the signature work order or of the order by output range, on
 // top of launch_asm2_122's part in RES

@@ -21,7 +21,7 @@
 //                      L and R
 // No float atomics: every reduction has a fixed order, so results are
 // bit-reproducible run to run.
-#include "device.cuh"
+#include "gemm_fp64.cuh"
 
 namespace imsrg {
 
@@ -76,178 +76,28 @@ __global__ void __launch_bounds__(256) k_cc_forward(DevTables T, const double *_
 }
 
 // ---------------------------------------------------------------------------
-// 2. Grouped FP64 GEMM: C = sum_t alpha_t op(A_t) op(B_t), one problem
-//    list, tiles of 64 x 64 (4 x 4 outputs per thread: rows tx + 16 i,
-//    columns 4 ty + j, so warp w owns columns 8w .. 8w + 7 and skips the
-//    products when they all lie past N) or, for outputs of at most eight
-//    columns, 256 x 8 (one row of eight outputs per thread; warps whose rows
-//    all lie past M skip the products).  A last K chunk shorter than BK runs
-//    only its valid k.
+// 2. Grouped FP64 products: C = sum_t alpha_t op(A_t) op(B_t), one CTA per tile
+//    of the list (gemm_fp64.cuh).  ABS: a merged list of several bases (absolute
+//    pointers, tiles of bases with act[inst] == 0 skipped).
 // ---------------------------------------------------------------------------
-constexpr int BM = 64, BN = 64, BK = 16;
-constexpr int TBM = 256, TBN = 8, TBK = 8;
-
 template <bool ABS>
-__device__ __forceinline__ void gemm_thin_tile(const GemmProb &P, int lt, const Operands &ops, int hL, int hR) {
-  __shared__ double As[TBK][TBM];
-  __shared__ double Bs[TBK][TBN];
-  const int tid = threadIdx.x;
-  const int m0 = lt * TBM;
-  const bool live = m0 + (tid & ~31) < P.M;  // warp-uniform
-  double acc[TBN];
-#pragma unroll
-  for (int j = 0; j < TBN; j++) acc[j] = 0.0;
-  for (int it = 0; it < P.nterms; it++) {
-    const GemmTerm &Tm = P.t[it];
-    const double *A = ABS ? Tm.a_abs : ops.src[Tm.a_src] + Tm.a_off;
-    const double *B = ABS ? Tm.b_abs : ops.src[Tm.b_src] + Tm.b_off;
-    const double alpha = Tm.coef * (Tm.use_hl ? hL : 1) * (Tm.use_hr ? hR : 1);
-    double part[TBN];
-#pragma unroll
-    for (int j = 0; j < TBN; j++) part[j] = 0.0;
-    for (int k0 = 0; k0 < P.K; k0 += TBK) {
-#pragma unroll
-      for (int l = 0; l < TBK; l++) {
-        const int idx = l * TBM + tid;
-        int m, k;
-        if (!Tm.ta) { m = idx % TBM; k = idx / TBM; }
-        else { k = idx % TBK; m = idx / TBK; }
-        const int gm = m0 + m, gk = k0 + k;
-        double v = 0.0;
-        if (gm < P.M && gk < P.K) v = Tm.ta ? A[gk + (long)gm * Tm.lda] : A[gm + (long)gk * Tm.lda];
-        As[k][m] = v;
-      }
-      if (tid < TBK * TBN) {
-        int n, k;
-        if (!Tm.tb) { k = tid % TBK; n = tid / TBK; }
-        else { n = tid % TBN; k = tid / TBN; }
-        const int gk = k0 + k;
-        double v = 0.0;
-        if (n < P.N && gk < P.K) v = Tm.tb ? B[n + (long)gk * Tm.ldb] : B[gk + (long)n * Tm.ldb];
-        Bs[k][n] = v;
-      }
-      __syncthreads();
-      if (live) {
-        const int kn = min(TBK, P.K - k0);
-#pragma unroll
-        for (int k = 0; k < TBK; k++) {
-          if (k < kn) {
-            const double a = As[k][tid];
-#pragma unroll
-            for (int j = 0; j < TBN; j++) part[j] = fma(a, Bs[k][j], part[j]);
-          }
-        }
-      }
-      __syncthreads();
-    }
-#pragma unroll
-    for (int j = 0; j < TBN; j++) acc[j] += alpha * part[j];
-  }
-  const int gm = m0 + tid;
-  if (gm >= P.M) return;
-  double *Cp = ABS ? P.c_abs : ops.dst[P.c_dst] + P.c_off;
-#pragma unroll
-  for (int j = 0; j < TBN; j++)
-    if (j < P.N) Cp[gm + (long)j * P.ldc] = acc[j];
-}
-
-// ABS: a merged list of several bases (absolute pointers, tiles of bases
-// with act[inst] == 0 skipped)
-template <bool ABS>
-__global__ void __launch_bounds__(256) k_gemm_fp64(const GemmProb *__restrict__ probs, int nprobs, Operands ops,
-                                                   int hL, int hR, const int *__restrict__ act) {
-  __shared__ double As[BK][BM + 1];
-  __shared__ double Bs[BK][BN + 1];
-  int tile = blockIdx.x;
-  // find problem: last p with tile0 <= tile
-  int lo = 0, hi = nprobs;
-  while (lo < hi) {
-    int mid = (lo + hi) >> 1;
-    if (probs[mid].tile0 <= tile) lo = mid + 1;
-    else hi = mid;
-  }
-  const GemmProb &P = probs[lo - 1];
+__global__ void __launch_bounds__(GT_THREADS, GT_CTAS) k_gemm_fp64(const GemmProb *__restrict__ probs,
+                                                          const GemmTile *__restrict__ tiles, Operands ops, int hL,
+                                                          int hR, const int *__restrict__ act) {
+  const GemmTile t = tiles[blockIdx.x];
+  const GemmProb &P = probs[t.prob];
   if (ABS && act && !act[P.inst]) return;  // block-uniform
-  int lt = tile - P.tile0;
-  if (P.shape == 1) {  // block-uniform
-    gemm_thin_tile<ABS>(P, lt, ops, hL, hR);
-    return;
-  }
-  int m0 = (lt % P.tiles_m) * BM, n0 = (lt / P.tiles_m) * BN;
-  int tid = threadIdx.x, tx = tid & 15, ty = tid >> 4;
-  const bool live = n0 + 8 * (tid >> 5) < P.N;  // warp-uniform: the warp's eight columns
-  double acc[4][4];
-#pragma unroll
-  for (int i = 0; i < 4; i++)
-#pragma unroll
-    for (int j = 0; j < 4; j++) acc[i][j] = 0.0;
-  for (int it = 0; it < P.nterms; it++) {
-    const GemmTerm &Tm = P.t[it];
-    const double *A = ABS ? Tm.a_abs : ops.src[Tm.a_src] + Tm.a_off;
-    const double *B = ABS ? Tm.b_abs : ops.src[Tm.b_src] + Tm.b_off;
-    double alpha = Tm.coef * (Tm.use_hl ? hL : 1) * (Tm.use_hr ? hR : 1);
-    double part[4][4];
-#pragma unroll
-    for (int i = 0; i < 4; i++)
-#pragma unroll
-      for (int j = 0; j < 4; j++) part[i][j] = 0.0;
-    for (int k0 = 0; k0 < P.K; k0 += BK) {
-      // A tile: op(A)(m, k), m in [m0, m0+64), k in [k0, k0+16)
-#pragma unroll
-      for (int l = 0; l < 4; l++) {
-        int m, k;
-        if (!Tm.ta) { m = tid & 63; k = (tid >> 6) + 4 * l; }
-        else { k = tid & 15; m = (tid >> 4) + 16 * l; }
-        int gm = m0 + m, gk = k0 + k;
-        double v = 0.0;
-        if (gm < P.M && gk < P.K) v = Tm.ta ? A[gk + (long)gm * Tm.lda] : A[gm + (long)gk * Tm.lda];
-        As[k][m] = v;
-      }
-      // B tile: op(B)(k, n)
-#pragma unroll
-      for (int l = 0; l < 4; l++) {
-        int n, k;
-        if (!Tm.tb) { k = tid & 15; n = (tid >> 4) + 16 * l; }
-        else { n = tid & 63; k = (tid >> 6) + 4 * l; }
-        int gn = n0 + n, gk = k0 + k;
-        double v = 0.0;
-        if (gn < P.N && gk < P.K) v = Tm.tb ? B[gn + (long)gk * Tm.ldb] : B[gk + (long)gn * Tm.ldb];
-        Bs[k][n] = v;
-      }
-      __syncthreads();
-      const int kn = live ? min(BK, P.K - k0) : 0;
-#pragma unroll
-      for (int k = 0; k < BK; k++) {
-        if (k < kn) {
-          double a[4], bv[4];
-#pragma unroll
-          for (int i = 0; i < 4; i++) a[i] = As[k][tx + 16 * i];
-#pragma unroll
-          for (int j = 0; j < 4; j++) bv[j] = Bs[k][4 * ty + j];
-#pragma unroll
-          for (int i = 0; i < 4; i++)
-#pragma unroll
-            for (int j = 0; j < 4; j++) part[i][j] = fma(a[i], bv[j], part[i][j]);
-        }
-      }
-      __syncthreads();
-    }
-#pragma unroll
-    for (int i = 0; i < 4; i++)
-#pragma unroll
-      for (int j = 0; j < 4; j++) acc[i][j] += alpha * part[i][j];
-  }
-  double *Cp = ABS ? P.c_abs : ops.dst[P.c_dst] + P.c_off;
-#pragma unroll
-  for (int j = 0; j < 4; j++) {
-    int gn = n0 + 4 * ty + j;
-    if (gn >= P.N) continue;
-#pragma unroll
-    for (int i = 0; i < 4; i++) {
-      int gm = m0 + tx + 16 * i;
-      if (gm < P.M) Cp[gm + (long)gn * P.ldc] = acc[i][j];
-    }
-  }
+  double *C = ABS ? P.c_abs : ops.dst[P.c_dst] + P.c_off;
+  gemm_cta_tile<false>(
+      t,
+      [&](int it, auto add) {
+        const GemmTerm &m = P.t[it];
+        const double *A = ABS ? m.a_abs : ops.src[m.a_src] + m.a_off;
+        const double *B = ABS ? m.b_abs : ops.src[m.b_src] + m.b_off;
+        add(A, m.ta ? (long)m.lda : 1L, m.ta ? 1L : (long)m.lda, B, m.tb ? (long)m.ldb : 1L, m.tb ? 1L : (long)m.ldb,
+            P.K, (m.coef < 0) ^ (m.use_hl && hL < 0) ^ (m.use_hr && hR < 0));  // coefficients are +-1
+      },
+      P.nterms, P.M, P.N, C, P.ldc);
 }
 
 // ---------------------------------------------------------------------------
@@ -691,15 +541,29 @@ int launch_gemm_fp64(imsrg_basis *b, const double *L, int hL, const double *R, i
   ops.dst[SRC_W2] = b->w2;
   ops.dst[SRC_WCC] = b->wcc;
   ProfScope ps(b, IMSRG_KERNEL_GEMM_FP64);
-  k_gemm_fp64<false><<<b->ntiles, 256, 0, b->stream>>>(b->d_probs, b->nprobs, ops, hL, hR, nullptr);
+  k_gemm_fp64<false><<<b->ntiles, GT_THREADS, 0, b->stream>>>(b->d_probs, b->d_tiles, ops, hL, hR, nullptr);
   b->launches++;
   return cuda_status(cudaGetLastError());
 }
 
+void gemm_fp64_plan(std::vector<GemmProb> &probs, int num_sms) {
+  std::vector<GemmShape> sh;
+  for (const GemmProb &p : probs) sh.push_back({p.M, p.N, (long)p.K * p.nterms, 0});
+  gemm_split(sh, num_sms);
+  for (size_t i = 0; i < probs.size(); i++) probs[i].split = sh[i].split;
+}
+
+std::vector<GemmTile> gemm_fp64_tiles(const std::vector<GemmProb> &probs) {
+  std::vector<GemmShape> sh;
+  for (const GemmProb &p : probs) sh.push_back({p.M, p.N, (long)p.K * p.nterms, p.split});
+  return gemm_tiles(sh);
+}
+
+// Every problem keeps its own basis's K split, so a merged launch gives the
+// bits of the single ones.
 int gemm_fp64_merged(imsrg_basis *const *bases, int n, const double *const *L, const double *const *R,
-                     GemmProb **d_probs, int *nprobs, int *ntiles) {
+                     GemmMerged *out) {
   std::vector<GemmProb> all;
-  int tiles = 0;
   for (int i = 0; i < n; i++) {
     imsrg_basis *b = bases[i];
     const double *src[7] = {L[i], R[i], b->w1, b->w2, b->lcc, b->rcc, b->wcc};
@@ -711,25 +575,30 @@ int gemm_fp64_merged(imsrg_basis *const *bases, int n, const double *const *L, c
       }
       p.c_abs = dst[p.c_dst] + p.c_off;
       p.inst = i;
-      p.tile0 = tiles;
-      tiles += p.tiles;
       all.push_back(p);
     }
   }
-  *d_probs = nullptr;
-  *nprobs = (int)all.size();
-  *ntiles = tiles;
-  if (all.empty()) return IMSRG_OK;
-  IMSRG_CUDA_TRY(cudaMalloc((void **)d_probs, all.size() * sizeof(GemmProb)));
-  IMSRG_CUDA_TRY(cudaMemcpy(*d_probs, all.data(), all.size() * sizeof(GemmProb), cudaMemcpyHostToDevice));
+  *out = GemmMerged();
+  const std::vector<GemmTile> tiles = gemm_fp64_tiles(all);
+  if (tiles.empty()) return IMSRG_OK;
+  auto up = [](const void *h, size_t bytes, void **d) -> int {
+    IMSRG_CUDA_TRY(cudaMalloc(d, bytes));
+    return cuda_status(cudaMemcpy(*d, h, bytes, cudaMemcpyHostToDevice));
+  };
+  int s = up(all.data(), all.size() * sizeof(GemmProb), (void **)&out->d_probs);
+  if (s == IMSRG_OK) s = up(tiles.data(), tiles.size() * sizeof(GemmTile), (void **)&out->d_tiles);
+  if (s != IMSRG_OK) {
+    out->release();
+    return s;
+  }
+  out->ntiles = (int)tiles.size();
   return IMSRG_OK;
 }
 
-int launch_gemm_fp64_merged(const GemmProb *d_probs, int nprobs, int ntiles, int hL, int hR, const int *act,
-                            cudaStream_t st) {
-  if (ntiles == 0) return IMSRG_OK;
+int launch_gemm_fp64_merged(const GemmMerged &g, int hL, int hR, const int *act, cudaStream_t st) {
+  if (g.ntiles == 0) return IMSRG_OK;
   Operands ops{};
-  k_gemm_fp64<true><<<ntiles, 256, 0, st>>>(d_probs, nprobs, ops, hL, hR, act);
+  k_gemm_fp64<true><<<g.ntiles, GT_THREADS, 0, st>>>(g.d_probs, g.d_tiles, ops, hL, hR, act);
   return cuda_status(cudaGetLastError());
 }
 
@@ -809,7 +678,7 @@ int launch_commutator_fp64_ws(imsrg_basis *b, const Workspace &ws, const double 
     ops.dst[SRC_W1] = ws.w1;
     ops.dst[SRC_W2] = ws.w2;
     ops.dst[SRC_WCC] = ws.wcc;
-    k_gemm_fp64<false><<<b->ntiles, 256, 0, st>>>(b->d_probs, b->nprobs, ops, hL, hR, nullptr);
+    k_gemm_fp64<false><<<b->ntiles, GT_THREADS, 0, st>>>(b->d_probs, b->d_tiles, ops, hL, hR, nullptr);
     b->launches++;
   }
   if (b->T.n_ph > 0) {

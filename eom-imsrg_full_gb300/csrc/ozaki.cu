@@ -112,12 +112,10 @@ struct OzMatrix {
   int group;       // exponent group
   long off;        // element offset in the source buffer
   int n1, n2;      // column-major shape
-  long img_r;      // byte offset of the R image (rows n1, K = n2), -1 when no problem reads it
-  long img_c;      // byte offset of the C image (rows n2, K = n1), -1 when no problem reads it
+  int unit_r;      // first 256-byte unit of the R image (rows n1, K = n2), -1 when no problem reads it
+  int unit_c;      // first unit of the C image (rows n2, K = n1), -1 when no problem reads it
   int rg_r, rg_c;  // row groups (of 8 rows) of each image
-  long plane_r, plane_c;  // bytes per digit plane
-  int np_r, np_c;         // digit planes stored (S)
-  int line_r0, line_c0;   // first line of this matrix in the R / C slicing grids
+  int line_r0, line_c0;  // first line of this matrix in the R / C slicing grids
 };
 
 // A contiguous chunk of one exponent group's elements.
@@ -127,29 +125,29 @@ struct OzChunk {
   int len;
 };
 
-struct OzTerm {
-  const uint8_t *a_img, *b_img;
-  long a_plane, b_plane;
-  int a_rg, b_rg;
-  int a_map, b_map;  // tensor maps of the A and B images (index into the plan's maps)
-  int neg, use_hl, use_hr;
-};
-
-struct OzProb {
-  int M, N, K, ksteps, nterms;
-  // The (term, K step) sequence of a tile, term-major, runs in chunks of
-  // kchunk steps, each into a fresh accumulator set: a chunk's FP32 level sums
-  // stay exact integers (kchunk TK 5 2^12 < 2^24) and the epilogue adds the
-  // chunks' int64 level sums exactly before the one conversion.
+// One 128 x TN output tile, everything its roles need in one contiguous record
+// (each role loads the next record while it works on this one; following
+// schedule -> problem -> term -> tensor map pointers cost every tile about four
+// dependent memory latencies: 46.4 us for the product launch at emax = 6, five
+// digits, 38.1 with records and one tensor map per box).  The (term, K step) sequence, term-major, runs
+// in chunks of kchunk steps, each into a fresh accumulator set: a chunk's FP32
+// level sums stay exact integers (kchunk TK 5 2^12 < 2^24) and the epilogue adds
+// the chunks' int64 level sums exactly before the one conversion.
+struct __align__(16) OzTile {
+  int ay[2], by[2];    // per term: unit of the tile's first A / B row group at K step 0
+  int arg[2], brg[2];  // units per K step
+  int ksteps, flags;   // flags: see kTile*
   int kchunk, nchunks;
-  OzTerm t[2];
-  double *C;
-  int ldc;
-  int gA, gB;
-  int tiles_m, tile0, tiles;
-  int raw;   // store the exact int64 level sum v (result = v 2^k) instead of FP64: the WCC products
-  int inst;  // instance (basis) of a merged batch plan; its tiles run only while act[inst] (0 alone)
+  int rows, cols;      // outputs of the problem from this tile's origin on
+  int ldc, inst;       // inst: instance (basis) of a merged batch plan; runs only while act[inst]
+  int gA, gB;          // exponent groups of A and B
+  int map, pad;        // the A tensor map; the B map follows it
+  double *C;           // the tile's origin
+  long pad2;
 };
+static_assert(sizeof(OzTile) == 96, "record of six 16-byte loads");
+constexpr int kTileTwoTerms = 1, kTileRaw = 2;  // raw: store the exact int64 level sum v (result = v 2^k): WCC
+constexpr int kTileNeg = 4, kTileHL = 8, kTileHR = 16, kTileTermShift = 3;  // term 1's signs at << kTileTermShift
 
 // Cost models of the CTA schedule tried by the autotuner (weights of K steps,
 // of the epilogue's live outputs in 64ths of a tile, and a per-tile
@@ -167,37 +165,36 @@ constexpr SchedModel kSchedModels[kNumSchedModels] = {{16, 1, 16}, {4, 0, 1}, {3
 struct OzPlan {
   int S = OZ_SMAX;  // digits per operand
   int chunk_steps = kOzChunkSteps;  // K steps per accumulator chunk (<= kOzChunkSteps)
-  bool chunked = false;             // some problem runs in more than one chunk
+  bool chunked = false;             // some tile runs in more than one chunk
   std::vector<OzMatrix> mats;
   std::vector<OzChunk> chunks;
-  std::vector<OzProb> probs;
   OzMatrix *d_mats = nullptr;
   OzChunk *d_chunks = nullptr;
-  OzProb *d_probs = nullptr;
-  int2 *d_sched = nullptr;     // (problem, tile within the problem), grouped by CTA
-  int *d_sched_off = nullptr;  // [grid + 1] start of each CTA's list
+  OzTile *d_tiles = nullptr;   // grouped by CTA
+  int *d_sched_off = nullptr;  // [grid + 1] start of each CTA's tiles
   int *d_exps = nullptr;       // per group: max biased exponent (e = value - 1022)
   int *d_err = nullptr;
-  uint8_t *img[4] = {nullptr, nullptr, nullptr, nullptr};
-  long img_bytes[4] = {0, 0, 0, 0};
-  int nmats = 0, ngroups = 0, nchunks = 0, nprobs = 0, ntiles = 0;
-  int lines_r = 0, lines_c = 0;
-  // The operands fall in three parts that are sliced separately (and
-  // concurrently): part 0 = L, part 1 = R (both available at once), part 2 =
-  // LCC and RCC (after the Pandya transform).  Groups, chunks and image lines
-  // are numbered part by part; part k owns [x_lo[k], x_lo[k + 1]).
+  // All digit images in one buffer of S planes, each `units` 256-byte units (8
+  // rows x 16 K, two core matrices): one tensor map per box shape serves every
+  // problem, so no tile waits for a descriptor fetch.
+  uint8_t *img = nullptr;
+  long units = 0;
+  int nmats = 0, ngroups = 0, nchunks = 0;
+  // The operands fall in three parts that can be sliced separately: part 0 = L,
+  // part 1 = R (both available at once), part 2 = LCC and RCC (after the Pandya
+  // transform).  Groups, chunks and image lines are numbered part by part; part
+  // k owns [x_lo[k], x_lo[k + 1]).
   int group_lo[4] = {0, 0, 0, 0}, chunk_lo[4] = {0, 0, 0, 0}, linec_lo[4] = {0, 0, 0, 0}, liner_lo[4] = {0, 0, 0, 0};
-  int *d_blk_mat = nullptr;  // slicing grids: matrix of each CTA's first line
+  uint16_t *d_mat_c = nullptr, *d_mat_r = nullptr;  // matrix of each C / R image line
   int2 *d_ccgroups = nullptr;  // [ccblocks]: exponent groups of LCC and RCC block q1
-  int cblocks[3] = {0, 0, 0}, rblocks[3] = {0, 0, 0}, blk_off[3] = {0, 0, 0};
   int grid = 0;
   int tune_choice = 0;                   // the schedule model the autotuner kept
   double tune_us[kNumSchedModels] = {};  // its timings of each model
   bool tuned = false;
+  std::vector<OzTile> tiles;                // in problem order
   std::vector<int> tile_ksteps, tile_live;  // per tile: K steps x terms, live outputs / 64
-  std::vector<int2> tile_slot;
-  std::vector<CUtensorMap> maps;     // TMA maps of the digit images, by role (see map_of)
-  CUtensorMap *d_maps = nullptr;
+  CUtensorMap *d_maps = nullptr;            // A box, B box
+  CUtensorMap maps[2];
   bool ok = false;
 };
 
@@ -259,6 +256,8 @@ __device__ __forceinline__ void tma_load_3d(void *sdst, const CUtensorMap *map, 
       "l"(reinterpret_cast<uint64_t>(map)), "r"(0), "r"(y), "r"(z), "r"(smem_u32(bar))
       : "memory");
 }
+
+__device__ __forceinline__ void prefetch_l1(const void *p) { asm volatile("prefetch.global.L1 [%0];" ::"l"(p)); }
 
 __device__ __forceinline__ uint64_t smem_desc(uint32_t saddr, uint32_t lbo, uint32_t sbo) {
   uint64_t d = 0;
@@ -438,14 +437,16 @@ __device__ __forceinline__ void digits(double x, int e, int *d) {
 // Threads of the first cblocks CTAs write C-image lines [c_lo, c_hi) (8
 // consecutive rows of one column: one 16-byte row of a C core matrix per digit
 // plane); the other CTAs write R-image lines [r_lo, r_hi) (8 consecutive
-// columns of one row).  blk_mat[b] is the matrix of CTA b's first line.  Padding lines of the images are never
-// written and stay zero.
+// columns of one row).  mat_c / mat_r: the matrix of each line (a walk over the
+// matrices from each CTA's first one took 26 us at emax = 2, where a CTA's lines
+// span dozens).  Padding lines of the images are never written and stay zero.
 template <int S>
-__global__ void __launch_bounds__(SLICE_THREADS) k_oz_slice(const OzMatrix *__restrict__ mats, int nmats,
-                                                  const int *__restrict__ blk_mat, int cblocks, int c_lo, int c_hi,
-                                                  int r_lo, int r_hi, const double *L, const double *R, const double *LCC,
-                                                  const double *RCC, const int *exps, uint8_t *imgL, uint8_t *imgR,
-                                                  uint8_t *imgLCC, uint8_t *imgRCC) {
+__global__ void __launch_bounds__(SLICE_THREADS) k_oz_slice(const OzMatrix *__restrict__ mats,
+                                                            const uint16_t *__restrict__ mat_c,
+                                                            const uint16_t *__restrict__ mat_r, int cblocks, int c_lo,
+                                                            int c_hi, int r_lo, int r_hi, const double *L,
+                                                            const double *R, const double *LCC, const double *RCC,
+                                                            const int *exps, uint8_t *img, long plane) {
   // BF16 bit patterns of the digits -128..128 (exact), built once per CTA
   __shared__ uint32_t tab[257];
   for (int i = threadIdx.x; i < 257; i += blockDim.x) {
@@ -456,15 +457,11 @@ __global__ void __launch_bounds__(SLICE_THREADS) k_oz_slice(const OzMatrix *__re
   const bool cimg = (int)blockIdx.x < cblocks;
   const int t = (cimg ? c_lo : r_lo) + ((int)blockIdx.x - (cimg ? 0 : cblocks)) * blockDim.x + threadIdx.x;
   if (t >= (cimg ? c_hi : r_hi)) return;
-  int mi = blk_mat[blockIdx.x];
-  while (mi + 1 < nmats && (cimg ? mats[mi + 1].line_c0 : mats[mi + 1].line_r0) <= t) mi++;
-  const OzMatrix &m = mats[mi];
+  const OzMatrix &m = mats[cimg ? mat_c[t] : mat_r[t]];
   const double *src = (m.src == 0 ? L : m.src == 1 ? R : m.src == 2 ? LCC : RCC) + m.off;
-  uint8_t *img = m.src == 0 ? imgL : m.src == 1 ? imgR : m.src == 2 ? imgLCC : imgRCC;
   const int e = exps[m.group] - 1022;
   double x[8];
   long off;
-  long plane;
   if (cimg) {
     const int RG = (m.n1 + 7) >> 3;
     const int l = t - m.line_c0;
@@ -474,8 +471,7 @@ __global__ void __launch_bounds__(SLICE_THREADS) k_oz_slice(const OzMatrix *__re
       const int r = rg * 8 + i;
       x[i] = r < m.n1 ? src[r + (long)c * m.n1] : 0.0;
     }
-    off = m.img_c + ((long)((rg >> 1) * m.rg_c + (c >> 3)) * 2 + (rg & 1)) * 128 + (c & 7) * 16;
-    plane = m.plane_c;
+    off = (long)m.unit_c * 256 + ((long)((rg >> 1) * m.rg_c + (c >> 3)) * 2 + (rg & 1)) * 128 + (c & 7) * 16;
   } else {
     const int l = t - m.line_r0;
     const int r = l % m.n1, cg = l / m.n1;
@@ -484,8 +480,7 @@ __global__ void __launch_bounds__(SLICE_THREADS) k_oz_slice(const OzMatrix *__re
       const int c = cg * 8 + j;
       x[j] = c < m.n2 ? src[r + (long)c * m.n1] : 0.0;
     }
-    off = m.img_r + ((long)((cg >> 1) * m.rg_r + (r >> 3)) * 2 + (cg & 1)) * 128 + (r & 7) * 16;
-    plane = m.plane_r;
+    off = (long)m.unit_r * 256 + ((long)((cg >> 1) * m.rg_r + (r >> 3)) * 2 + (cg & 1)) * 128 + (r & 7) * 16;
   }
   uint32_t h[8][S];  // BF16 bits of each digit
 #pragma unroll
@@ -509,11 +504,10 @@ __global__ void __launch_bounds__(SLICE_THREADS) k_oz_slice(const OzMatrix *__re
 // 3. tensor-core products and exact recombination
 // ---------------------------------------------------------------------------
 
-// CH: the plan has contractions in several chunks (see OzProb); without any,
+// CH: the plan has contractions in several chunks (see OzTile); without any,
 // the chunk bookkeeping folds away at compile time.
 template <int S, bool CH>
-__global__ void __launch_bounds__(oz_threads(S), 1) k_oz_mma(const OzProb *__restrict__ probs, int nprobs,
-                                                          const int2 *__restrict__ sched,
+__global__ void __launch_bounds__(oz_threads(S), 1) k_oz_mma(const OzTile *__restrict__ tiles,
                                                           const int *__restrict__ sched_off,
                                                           const int *__restrict__ exps, int hL, int hR, int *err,
                                                           const CUtensorMap *__restrict__ maps,
@@ -557,19 +551,19 @@ __global__ void __launch_bounds__(oz_threads(S), 1) k_oz_mma(const OzProb *__res
   const uint32_t tmem = *tmem_slot;
 
   if (warp == 0) {
-    if (lane == 0) {
+    if (lane == 0 && t_begin < t_end) {
       // producer: digit planes of A and B for every K step
       int stage = 0;
       uint32_t phase = 0;
+      OzTile next = tiles[t_begin];
       for (int ti = t_begin; ti < t_end && !*abort_flag; ti++) {
-        const int2 slot = sched[ti];
-        const OzProb &P = probs[slot.x];
-        if (P.ksteps == 0 || (act && !act[P.inst])) continue;
-        const int lt = slot.y;
-        int tm = lt % P.tiles_m, tn = lt / P.tiles_m;
-        for (int it = 0; it < P.nterms; it++) {
-          const OzTerm &T = P.t[it];
-          const CUtensorMap *amap = maps + T.a_map, *bmap = maps + T.b_map;
+        const OzTile P = next;
+        if (ti + 1 < t_end) next = tiles[ti + 1];
+        if (act && !act[P.inst]) continue;
+        const CUtensorMap *amap = maps + P.map, *bmap = amap + 1;
+        for (int it = 0; it <= (P.flags & kTileTwoTerms); it++) {
+          int ay = it ? P.ay[1] : P.ay[0], by = it ? P.by[1] : P.by[0];
+          const int arg = it ? P.arg[1] : P.arg[0], brg = it ? P.brg[1] : P.brg[0];
           for (int kk = 0; kk < P.ksteps; kk++) {  // the chunks only regroup these steps
             if (!mbar_wait(&empty[stage], phase ^ 1, abort_flag)) {
               atomicExch(err, 1);
@@ -577,13 +571,15 @@ __global__ void __launch_bounds__(oz_threads(S), 1) k_oz_mma(const OzProb *__res
               break;
             }
             // two whole boxes: the row groups past the tile's operand rows
-            // (next K step's rows, or zeros past the image) only reach
+            // (other rows of the buffer, or zeros past its end) only reach
             // accumulator rows and columns that are never stored
             mbar_expect_tx(&full[stage], STAGE_BYTES);
             uint8_t *sa = smem + stage * STAGE_BYTES;
             uint8_t *sb = sa + S * A_SLICE_BYTES;
-            tma_load_3d(sa, amap, kk * T.a_rg + tm * (TM / 8), 0, &full[stage]);
-            tma_load_3d(sb, bmap, kk * T.b_rg + tn * (TN / 8), 0, &full[stage]);
+            tma_load_3d(sa, amap, ay, 0, &full[stage]);
+            tma_load_3d(sb, bmap, by, 0, &full[stage]);
+            ay += arg;
+            by += brg;
             if (++stage == STAGES) {
               stage = 0;
               phase ^= 1;
@@ -594,23 +590,26 @@ __global__ void __launch_bounds__(oz_threads(S), 1) k_oz_mma(const OzProb *__res
       }
     }
   } else if (warp == 1) {
-    if (lane == 0) {
+    if (lane == 0 && t_begin < t_end) {
       // MMA issuer: alternates between the two accumulator sets so the next
       // tile's products overlap the epilogue of the previous one
       int stage = 0, nt = 0;
       uint32_t phase = 0;
+      const uint64_t desc0 = smem_desc(smem_u32(smem), 128, 256);
+      OzTile next = tiles[t_begin];
       for (int ti = t_begin; ti < t_end && !*abort_flag; ti++) {
-        const OzProb &P = probs[sched[ti].x];
-        if (P.ksteps == 0 || (act && !act[P.inst])) continue;
-        const uint64_t desc0 = smem_desc(smem_u32(smem), 128, 256);
+        const OzTile P = next;
+        if (ti + 1 < t_end) next = tiles[ti + 1];
+        if (act && !act[P.inst]) continue;
+        const int nterms = 1 + (P.flags & kTileTwoTerms);
         const int kchunk = CH ? P.kchunk : 0x40000000;
-        int left = 0;                          // steps left in the current chunk
-        int total = P.nterms * P.ksteps;       // steps left in the tile
+        int left = 0;                      // steps left in the current chunk
+        int total = nterms * P.ksteps;     // steps left in the tile
         uint32_t dbase = 0;
         bool first = true;  // first K step of a chunk overwrites the accumulators
-        for (int it = 0; it < P.nterms && !*abort_flag; it++) {
-          const OzTerm &T = P.t[it];
-          int neg = T.neg ^ (T.use_hl & (hL < 0)) ^ (T.use_hr & (hR < 0));
+        for (int it = 0; it < nterms && !*abort_flag; it++) {
+          const int f = P.flags >> (it * kTileTermShift);
+          const int neg = ((f & kTileNeg) != 0) ^ ((f & kTileHL) && hL < 0) ^ ((f & kTileHR) && hR < 0);
           uint32_t idesc[S];  // A plane s: width (S - s) TN
 #pragma unroll
           for (int s = 0; s < S; s++) idesc[s] = idesc_bf16(TM, (S - s) * TN, neg);
@@ -664,31 +663,19 @@ __global__ void __launch_bounds__(oz_threads(S), 1) k_oz_mma(const OzProb *__res
     // epilogue warps 2..: TMEM lane quadrant = warp % 4 (the lanes a warp
     // may read), 16-column chunk = (warp - 2) / 4
     const int quad = warp & 3, chunk = (warp - 2) >> 2;
-    const int row = quad * 32 + lane;
+    const int row = quad * 32 + lane, n0 = 16 * chunk;
     int nt = 0;
     for (int ti = t_begin; ti < t_end; ti++) {
-      const int2 slot = sched[ti];
-      const OzProb &P = probs[slot.x];
+      const OzTile &P = tiles[ti];
+      if (ti + 1 < t_end) prefetch_l1(&tiles[ti + 1].ksteps);  // its registers are better spent on the accumulators
       if (act && !act[P.inst]) continue;  // an instance whose series has stopped: its outputs stay
-      const int lt = slot.y;
-      // problem fields in registers: the stores below could alias the problem
-      // table as far as the compiler knows, which would force a reload per column
-      const int Mp = P.M, Np = P.N, ldc = P.ldc, ksteps = P.ksteps, gA = P.gA, gB = P.gB;
-      const int nch = CH ? P.nchunks : 1, raw = P.raw;
-      const int tiles_m = P.tiles_m;
-      double *const Cbase = P.C;
-      const int m0 = (lt % tiles_m) * TM;
-      const int m = m0 + row;
-      const int n0 = (lt / tiles_m) * TN + 16 * chunk;
-      const bool row_ok = m < Mp;
-      double *crow = Cbase + m;
-      if (ksteps == 0) {
-        if (row_ok)
-          for (int c = 0; c < 16 && n0 + c < Np; c++) crow[(long)(n0 + c) * ldc] = 0.0;
-        continue;
-      }
+      const int Mp = P.rows, Np = P.cols, ldc = P.ldc;
+      const int nch = CH ? P.nchunks : 1, raw = P.flags & kTileRaw;
+      const int k = (exps[P.gA] - 1022) + (exps[P.gB] - 1022) - 7 * LMAX;  // result = v * 2^k
+      const bool row_ok = row < Mp;
+      double *crow = P.C + row;
       // warp-uniform: a piece entirely past M or N is neither read nor converted
-      const bool live = m0 + quad * 32 < Mp && n0 < Np;
+      const bool live = quad * 32 < Mp && n0 < Np;
       // A tile in several chunks adds the chunks' exact level sums in the
       // output's own 8-byte slots (each thread owns its elements), as int64,
       // until the last chunk converts
@@ -721,7 +708,6 @@ __global__ void __launch_bounds__(oz_threads(S), 1) k_oz_mma(const OzProb *__res
         // operations)
 #define OZ_LEVEL_SUM(c) oz_level_sum<S>(acc, c)
         if (nch == 1 && !raw) {
-          const int k = (exps[gA] - 1022) + (exps[gB] - 1022) - 7 * LMAX;  // result = v * 2^k
 #pragma unroll
           for (int c = 0; c < 16; c++) {
             const double d = oz_scale(oz_level_value<S>(acc, c), k);
@@ -743,7 +729,6 @@ __global__ void __launch_bounds__(oz_threads(S), 1) k_oz_mma(const OzProb *__res
             }
           }
           if (ch < nch - 1 || !row_ok) continue;
-          const int k = (exps[gA] - 1022) + (exps[gB] - 1022) - 7 * LMAX;
           for (int c = 0; c < 16 && n0 + c < Np; c++) crow[(long)(n0 + c) * ldc] = oz_scale(crow[(long)(n0 + c) * ldc], k);
         } else {
           // WCC keeps the exact level sum as an integer (the 222_ph recoupling
@@ -760,7 +745,6 @@ __global__ void __launch_bounds__(oz_threads(S), 1) k_oz_mma(const OzProb *__res
           }
           if (raw || ch < nch - 1 || !row_ok) continue;
           // the last chunk of a long FP64 contraction: convert the summed integers
-          const int k = (exps[gA] - 1022) + (exps[gB] - 1022) - 7 * LMAX;
           for (int c = 0; c < 16 && n0 + c < Np; c++)
             crow[(long)(n0 + c) * ldc] = oz_scale((double)irow[(long)(n0 + c) * ldc], k);
         }
@@ -779,12 +763,10 @@ __global__ void __launch_bounds__(oz_threads(S), 1) k_oz_mma(const OzProb *__res
 
 OzPlan *plan_of(imsrg_basis *b) { return (OzPlan *)b->ozaki; }
 
-void launch_mma(int S, bool chunked, int grid, cudaStream_t st, const OzProb *probs, int nprobs, const int2 *sched,
-                const int *sched_off, const int *exps, int hL, int hR, int *err, const CUtensorMap *maps,
-                const int *act = nullptr) {
-#define OZ_LAUNCH(SS, CC)                                                                                    \
-  k_oz_mma<SS, CC><<<grid, oz_threads(SS), oz_mma_smem(SS), st>>>(probs, nprobs, sched, sched_off, exps, hL, hR, err, \
-                                                              maps, act)
+void launch_mma(int S, bool chunked, int grid, cudaStream_t st, const OzTile *tiles, const int *sched_off,
+                const int *exps, int hL, int hR, int *err, const CUtensorMap *maps, const int *act = nullptr) {
+#define OZ_LAUNCH(SS, CC) \
+  k_oz_mma<SS, CC><<<grid, oz_threads(SS), oz_mma_smem(SS), st>>>(tiles, sched_off, exps, hL, hR, err, maps, act)
   switch (S) {
     case 4: if (chunked) OZ_LAUNCH(4, true); else OZ_LAUNCH(4, false); break;
     case 5: if (chunked) OZ_LAUNCH(5, true); else OZ_LAUNCH(5, false); break;
@@ -798,8 +780,8 @@ void launch_mma(int S, bool chunked, int grid, cudaStream_t st, const OzProb *pr
 // CTA schedule: longest-processing-time-first assignment of tiles to the
 // persistent CTAs under the cost model cost = kw * (K steps x terms) + ew *
 // (live outputs / 64) + base.
-void build_sched(const OzPlan *pl, const SchedModel &md, std::vector<int2> &sched, std::vector<int> &sched_off) {
-  const int tiles = (int)pl->tile_slot.size();
+void build_sched(const OzPlan *pl, const SchedModel &md, std::vector<OzTile> &sched, std::vector<int> &sched_off) {
+  const int tiles = (int)pl->tiles.size();
   std::vector<long> cost(tiles);
   for (int i = 0; i < tiles; i++)
     cost[i] = (long)md.kw * pl->tile_ksteps[i] + (long)md.ew * pl->tile_live[i] + md.base;
@@ -817,16 +799,16 @@ void build_sched(const OzPlan *pl, const SchedModel &md, std::vector<int2> &sche
   sched_off.assign(pl->grid + 1, 0);
   for (int c = 0; c < pl->grid; c++) {
     sched_off[c] = (int)sched.size();
-    for (int t : lists[c]) sched.push_back(pl->tile_slot[t]);
+    for (int t : lists[c]) sched.push_back(pl->tiles[t]);
   }
   sched_off[pl->grid] = (int)sched.size();
 }
 
 int use_model(imsrg_basis *b, OzPlan *pl, int c) {
-  std::vector<int2> sched;
+  std::vector<OzTile> sched;
   std::vector<int> sched_off;
   build_sched(pl, kSchedModels[c], sched, sched_off);
-  IMSRG_CUDA_TRY(cudaMemcpyAsync(pl->d_sched, sched.data(), sched.size() * sizeof(int2), cudaMemcpyHostToDevice,
+  IMSRG_CUDA_TRY(cudaMemcpyAsync(pl->d_tiles, sched.data(), sched.size() * sizeof(OzTile), cudaMemcpyHostToDevice,
                                  b->stream));
   IMSRG_CUDA_TRY(cudaMemcpyAsync(pl->d_sched_off, sched_off.data(), sched_off.size() * sizeof(int),
                                  cudaMemcpyHostToDevice, b->stream));
@@ -846,8 +828,8 @@ int autotune(imsrg_basis *b, OzPlan *pl, int hL, int hR) {
   IMSRG_CUDA_TRY(cudaEventCreate(&e1));
   auto launch_timed = [&](float *ms) -> int {
     IMSRG_CUDA_TRY(cudaEventRecord(e0, b->stream));
-    launch_mma(pl->S, pl->chunked, pl->grid, b->stream, pl->d_probs, pl->nprobs, pl->d_sched, pl->d_sched_off, pl->d_exps, hL, hR,
-               pl->d_err, pl->d_maps);
+    launch_mma(pl->S, pl->chunked, pl->grid, b->stream, pl->d_tiles, pl->d_sched_off, pl->d_exps, hL, hR, pl->d_err,
+               pl->d_maps);
     b->launches++;
     IMSRG_CUDA_TRY(cudaEventRecord(e1, b->stream));
     IMSRG_CUDA_TRY(cudaEventSynchronize(e1));
@@ -914,7 +896,7 @@ int ozaki_prepare(imsrg_basis *b) {
     m.off = off;
     m.n1 = n1;
     m.n2 = n2;
-    m.img_r = m.img_c = -1;
+    m.unit_r = m.unit_c = -1;
     mat_of[{src, off}] = (int)pl->mats.size();
     pl->mats.push_back(m);
   };
@@ -946,13 +928,11 @@ int ozaki_prepare(imsrg_basis *b) {
   pl->chunk_lo[3] = (int)chunks.size();
 
   // which images each matrix needs: op(A) = X reads X's R image, X^T its C
-  // image; op(B) = Y reads Y's C image, Y^T its R image.  An image read as a B
-  // operand also carries the scaled tail planes.
+  // image; op(B) = Y reads Y's C image, Y^T its R image
   auto img_of = [&](int gsrc) -> int {
     return gsrc == SRC_L ? 0 : gsrc == SRC_R ? 1 : gsrc == SRC_LCC ? 2 : gsrc == SRC_RCC ? 3 : -1;
   };
-  std::vector<int> role_r(pl->mats.size(), 0), role_c(pl->mats.size(), 0);  // 0 unused, 1 B, 2 A
-  std::vector<int> b_role_r(pl->mats.size(), 0), b_role_c(pl->mats.size(), 0);  // read as a B operand
+  std::vector<char> role_r(pl->mats.size(), 0), role_c(pl->mats.size(), 0);
   for (const GemmProb &gp : b->probs) {
     if (gp.K <= 0) continue;
     for (int it = 0; it < gp.nterms; it++) {
@@ -961,37 +941,34 @@ int ozaki_prepare(imsrg_basis *b) {
       if (sa < 0 || sb < 0) return IMSRG_ERR_INVALID;
       auto ia = mat_of.find({sa, t.a_off}), ib = mat_of.find({sb, t.b_off});
       if (ia == mat_of.end() || ib == mat_of.end()) return IMSRG_ERR_INVALID;
-      (t.ta ? role_c : role_r)[ia->second] = 2;
-      int &rb = (t.tb ? role_r : role_c)[ib->second];
-      rb = std::max(rb, 1);
-      (t.tb ? b_role_r : b_role_c)[ib->second] = 1;
+      (t.ta ? role_c : role_r)[ia->second] = 1;
+      (t.tb ? role_r : role_c)[ib->second] = 1;
     }
   }
-  long imgb[4] = {0, 0, 0, 0};
+  long units = 0;
   int lines_r = 0, lines_c = 0;
+  std::vector<uint16_t> mat_r, mat_c;  // matrix of each image line
+  if (pl->mats.size() > 0xFFFF) return IMSRG_ERR_TOO_LARGE;
   for (size_t i = 0; i < pl->mats.size(); i++) {
     OzMatrix &m = pl->mats[i];
     m.line_r0 = lines_r;
     m.line_c0 = lines_c;
     if (role_r[i]) {
       m.rg_r = (m.n1 + 7) / 8;
-      m.plane_r = (long)m.rg_r * ((m.n2 + 15) / 16) * 256;
-      m.np_r = pl->S;
-      m.img_r = imgb[m.src];
-      imgb[m.src] += m.np_r * m.plane_r;
+      m.unit_r = (int)units;
+      units += (long)m.rg_r * ((m.n2 + 15) / 16);
       lines_r += ((m.n2 + 7) / 8) * m.n1;
     }
     if (role_c[i]) {
       m.rg_c = (m.n2 + 7) / 8;
-      m.plane_c = (long)m.rg_c * ((m.n1 + 15) / 16) * 256;
-      m.np_c = pl->S;
-      m.img_c = imgb[m.src];
-      imgb[m.src] += m.np_c * m.plane_c;
+      m.unit_c = (int)units;
+      units += (long)m.rg_c * ((m.n1 + 15) / 16);
       lines_c += ((m.n1 + 7) / 8) * m.n2;
     }
+    mat_r.resize(lines_r, (uint16_t)i);
+    mat_c.resize(lines_c, (uint16_t)i);
   }
-  pl->lines_r = lines_r;
-  pl->lines_c = lines_c;
+  if (units >= (1L << 30)) return IMSRG_ERR_TOO_LARGE;
   // first lines of each part (matrices are ordered L, R, then LCC and RCC)
   for (int part = 0; part < 3; part++) {
     pl->linec_lo[part] = lines_c;
@@ -1005,38 +982,18 @@ int ozaki_prepare(imsrg_basis *b) {
   }
   pl->linec_lo[3] = lines_c;
   pl->liner_lo[3] = lines_r;
-  // per part: the matrix of each CTA's first line (C lines, then R lines)
-  std::vector<int> blk_mat;
-  for (int part = 0; part < 3; part++) {
-    const int c_lo = pl->linec_lo[part], c_hi = pl->linec_lo[part + 1];
-    const int r_lo = pl->liner_lo[part], r_hi = pl->liner_lo[part + 1];
-    pl->cblocks[part] = (c_hi - c_lo + SLICE_THREADS - 1) / SLICE_THREADS;
-    pl->rblocks[part] = (r_hi - r_lo + SLICE_THREADS - 1) / SLICE_THREADS;
-    pl->blk_off[part] = (int)blk_mat.size();
-    for (int cimg = 1; cimg >= 0; cimg--) {
-      const int nb = cimg ? pl->cblocks[part] : pl->rblocks[part];
-      const int lo = cimg ? c_lo : r_lo;
-      int mi = 0;
-      auto l0 = [&](int k) { return cimg ? pl->mats[k].line_c0 : pl->mats[k].line_r0; };
-      for (int bk = 0; bk < nb; bk++) {
-        const int t0 = lo + bk * SLICE_THREADS;
-        while (mi + 1 < (int)pl->mats.size() && l0(mi + 1) <= t0) mi++;
-        blk_mat.push_back(mi);
-      }
-    }
-  }
-  for (int s = 0; s < 4; s++) {
-    pl->img_bytes[s] = std::max<long>(imgb[s], 256);
+  pl->units = std::max<long>(units, 1);
+  {
     void *p = nullptr;
-    IMSRG_CUDA_TRY(cudaMalloc(&p, pl->img_bytes[s]));
-    IMSRG_CUDA_TRY(cudaMemset(p, 0, pl->img_bytes[s]));  // padding stays zero
-    pl->img[s] = (uint8_t *)p;
+    const size_t bytes = (size_t)pl->S * pl->units * 256;
+    IMSRG_CUDA_TRY(cudaMalloc(&p, bytes));
+    IMSRG_CUDA_TRY(cudaMemset(p, 0, bytes));  // padding stays zero
+    pl->img = (uint8_t *)p;
   }
 
-  // TMA maps of the images, one per (image, role): a digit image is planes x
-  // (K steps x row groups) x 256-byte core-matrix rows; an A tile is the box
-  // 16 row groups x 6 planes, a B tile 8 row groups x 15 planes.  The encoder
-  // is the driver's cuTensorMapEncodeTiled, reached through the runtime.
+  // TMA maps of the image buffer, S planes of 256-byte core-matrix rows: an A
+  // box is 16 row groups (128 rows) of every plane, a B box TN / 8.  The
+  // encoder is the driver's cuTensorMapEncodeTiled, reached through the runtime.
   static PFN_cuTensorMapEncodeTiled_v12000 encode = nullptr;
   if (!encode) {
     void *fn = nullptr;
@@ -1047,98 +1004,73 @@ int ozaki_prepare(imsrg_basis *b) {
       return IMSRG_ERR_CUDA;
     encode = (PFN_cuTensorMapEncodeTiled_v12000)fn;
   }
-  std::map<std::pair<const uint8_t *, int>, int> map_index;
-  auto map_of = [&](const uint8_t *img, long plane, int np, int brole, int *idx) -> int {
-    auto it = map_index.find({img, brole});
-    if (it != map_index.end()) {
-      *idx = it->second;
-      return IMSRG_OK;
-    }
-    const cuuint32_t box_planes = pl->S;
-    if (plane <= 0 || plane % 256 || (long)np < (long)box_planes) return IMSRG_ERR_INVALID;
-    CUtensorMap m;
-    const cuuint64_t gdim[3] = {32, (cuuint64_t)(plane / 256), (cuuint64_t)np};
-    const cuuint64_t gstride[2] = {256, (cuuint64_t)plane};
-    const cuuint32_t box[3] = {32, (cuuint32_t)(brole ? oz_tn(pl->S) / 8 : TM / 8), box_planes};
+  for (int brole = 0; brole < 2; brole++) {
+    const cuuint64_t gdim[3] = {32, (cuuint64_t)pl->units, (cuuint64_t)pl->S};
+    const cuuint64_t gstride[2] = {256, (cuuint64_t)pl->units * 256};
+    const cuuint32_t box[3] = {32, (cuuint32_t)(brole ? oz_tn(pl->S) / 8 : TM / 8), (cuuint32_t)pl->S};
     const cuuint32_t estride[3] = {1, 1, 1};
-    if (encode(&m, CU_TENSOR_MAP_DATA_TYPE_UINT64, 3, (void *)img, gdim, gstride, box, estride,
+    if (encode(&pl->maps[brole], CU_TENSOR_MAP_DATA_TYPE_UINT64, 3, (void *)pl->img, gdim, gstride, box, estride,
                CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
                CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) != CUDA_SUCCESS)
       return IMSRG_ERR_INVALID;
-    *idx = (int)pl->maps.size();
-    pl->maps.push_back(m);
-    map_index[{img, brole}] = *idx;
-    return IMSRG_OK;
-  };
+  }
 
-  // problems: the FP64 grouped-GEMM list mapped onto images
-  int tiles = 0;
+  // tiles: the FP64 grouped-GEMM list mapped onto images.  Products with an
+  // empty contraction have none: their outputs are the zeros that W1, W2 and
+  // WCC were allocated with, which nothing else writes.
   std::vector<int> &tile_ksteps = pl->tile_ksteps, &tile_live = pl->tile_live;
-  std::vector<int2> &tile_slot = pl->tile_slot;  // (problem, tile within the problem) of each tile
+  const int TN = oz_tn(pl->S);
   for (const GemmProb &gp : b->probs) {
-    OzProb p{};
-    p.M = gp.M;
-    p.N = gp.N;
-    p.K = gp.K;
+    if (gp.K <= 0) continue;
+    OzTile p{};
     p.ksteps = (gp.K + TK - 1) / TK;
-    p.nterms = gp.nterms;
     double *dst = gp.c_dst == SRC_W1 ? b->w1 : gp.c_dst == SRC_W2 ? b->w2 : b->wcc;
-    p.C = dst + gp.c_off;
-    p.raw = gp.c_dst == SRC_WCC && !oz_fp64_class(pl->S);
+    if (gp.c_dst == SRC_WCC && !oz_fp64_class(pl->S)) p.flags |= kTileRaw;
+    if (gp.nterms > 1) p.flags |= kTileTwoTerms;
     p.ldc = gp.ldc;
     for (int it = 0; it < gp.nterms; it++) {
       const GemmTerm &t = gp.t[it];
-      OzTerm &o = p.t[it];
-      if (p.K > 0) {
-        const OzMatrix &A = pl->mats[mat_of[{img_of(t.a_src), t.a_off}]];
-        const OzMatrix &B = pl->mats[mat_of[{img_of(t.b_src), t.b_off}]];
-        o.a_img = pl->img[A.src] + (t.ta ? A.img_c : A.img_r);
-        o.a_plane = t.ta ? A.plane_c : A.plane_r;
-        o.a_rg = t.ta ? A.rg_c : A.rg_r;
-        o.b_img = pl->img[B.src] + (t.tb ? B.img_r : B.img_c);
-        o.b_plane = t.tb ? B.plane_r : B.plane_c;
-        o.b_rg = t.tb ? B.rg_r : B.rg_c;
-        IMSRG_TRY(map_of(o.a_img, o.a_plane, t.ta ? A.np_c : A.np_r, 0, &o.a_map));
-        IMSRG_TRY(map_of(o.b_img, o.b_plane, t.tb ? B.np_r : B.np_c, 1, &o.b_map));
-        if (it == 0) {
-          p.gA = A.group;
-          p.gB = B.group;
-        }
+      const OzMatrix &A = pl->mats[mat_of[{img_of(t.a_src), t.a_off}]];
+      const OzMatrix &B = pl->mats[mat_of[{img_of(t.b_src), t.b_off}]];
+      p.ay[it] = t.ta ? A.unit_c : A.unit_r;
+      p.arg[it] = t.ta ? A.rg_c : A.rg_r;
+      p.by[it] = t.tb ? B.unit_r : B.unit_c;
+      p.brg[it] = t.tb ? B.rg_r : B.rg_c;
+      if (it == 0) {
+        p.gA = A.group;
+        p.gB = B.group;
       }
-      o.neg = t.coef < 0;
-      o.use_hl = t.use_hl;
-      o.use_hr = t.use_hr;
+      p.flags |= ((t.coef < 0 ? kTileNeg : 0) | (t.use_hl ? kTileHL : 0) | (t.use_hr ? kTileHR : 0))
+                 << (it * kTileTermShift);
     }
     // exactness bound of the FP32 level accumulators (levels 2..4 are exact
     // integers while their sums stay below 2^24; each of their products adds
     // at most 5 x 2^12 per element): a chunk holds at most kOzChunkSteps steps of
     // TK, and longer contractions run in several chunks
-    {
-      const int steps = p.nterms * p.ksteps;
-      const int lim = std::min(oz_chunk_steps(pl->S), std::max(1, pl->chunk_steps));
-      p.kchunk = std::max(1, std::min(steps, lim));
-      p.nchunks = steps > 0 ? (steps + p.kchunk - 1) / p.kchunk : 0;
-      if (p.nchunks > 1) pl->chunked = true;
-    }
-    const int TN = oz_tn(pl->S);
-    p.tiles_m = (p.M + TM - 1) / TM;
-    p.tiles = p.tiles_m * ((p.N + TN - 1) / TN);
-    p.tile0 = tiles;
-    tiles += p.tiles;
-    for (int k = 0; k < p.tiles; k++) {
-      const int live_m = std::min(TM, p.M - (k % p.tiles_m) * TM), live_n = std::min(TN, p.N - (k / p.tiles_m) * TN);
-      tile_ksteps.push_back(p.nterms * p.ksteps);
-      tile_live.push_back((64 * live_m * live_n) / (TM * TN));
-      tile_slot.push_back(make_int2((int)pl->probs.size(), k));
-    }
-    pl->probs.push_back(p);
+    const int steps = gp.nterms * p.ksteps;
+    const int lim = std::min(oz_chunk_steps(pl->S), std::max(1, pl->chunk_steps));
+    p.kchunk = std::max(1, std::min(steps, lim));
+    p.nchunks = (steps + p.kchunk - 1) / p.kchunk;
+    if (p.nchunks > 1) pl->chunked = true;
+    for (int n0 = 0; n0 < gp.N; n0 += TN)
+      for (int m0 = 0; m0 < gp.M; m0 += TM) {
+        OzTile q = p;
+        for (int it = 0; it < gp.nterms; it++) {
+          q.ay[it] += m0 / 8;
+          q.by[it] += n0 / 8;
+        }
+        q.rows = gp.M - m0;
+        q.cols = gp.N - n0;
+        q.C = dst + gp.c_off + m0 + (long)n0 * gp.ldc;
+        tile_ksteps.push_back(steps);
+        tile_live.push_back((64 * std::min(TM, q.rows) * std::min(TN, q.cols)) / (TM * TN));
+        pl->tiles.push_back(q);
+      }
   }
   pl->nmats = (int)pl->mats.size();
-  pl->nprobs = (int)pl->probs.size();
-  pl->ntiles = tiles;
-  pl->grid = std::min(nsm, std::max(tiles, 1));
+  pl->grid = std::min(nsm, std::max((int)pl->tiles.size(), 1));
 
-  std::vector<int2> sched;
+  std::vector<OzTile> sched;
   std::vector<int> sched_off;
   build_sched(pl, kSchedModels[0], sched, sched_off);
 
@@ -1149,12 +1081,12 @@ int ozaki_prepare(imsrg_basis *b) {
   };
   IMSRG_TRY(up(pl->mats.data(), pl->mats.size() * sizeof(OzMatrix), (void **)&pl->d_mats));
   IMSRG_TRY(up(chunks.data(), chunks.size() * sizeof(OzChunk), (void **)&pl->d_chunks));
-  IMSRG_TRY(up(pl->probs.data(), pl->probs.size() * sizeof(OzProb), (void **)&pl->d_probs));
-  IMSRG_TRY(up(sched.data(), sched.size() * sizeof(int2), (void **)&pl->d_sched));
+  IMSRG_TRY(up(sched.data(), sched.size() * sizeof(OzTile), (void **)&pl->d_tiles));
   IMSRG_TRY(up(sched_off.data(), sched_off.size() * sizeof(int), (void **)&pl->d_sched_off));
-  IMSRG_TRY(up(blk_mat.data(), blk_mat.size() * sizeof(int), (void **)&pl->d_blk_mat));
+  IMSRG_TRY(up(mat_c.data(), mat_c.size() * sizeof(uint16_t), (void **)&pl->d_mat_c));
+  IMSRG_TRY(up(mat_r.data(), mat_r.size() * sizeof(uint16_t), (void **)&pl->d_mat_r));
   // (cudaMalloc memory is 256-byte aligned: the 64-byte alignment of a tensor map holds)
-  IMSRG_TRY(up(pl->maps.data(), pl->maps.size() * sizeof(CUtensorMap), (void **)&pl->d_maps));
+  IMSRG_TRY(up(pl->maps, sizeof(pl->maps), (void **)&pl->d_maps));
   std::vector<int2> ccg(b->ccblocks);
   for (int q1 = 0; q1 < b->ccblocks; q1++)
     ccg[q1] = make_int2(pl->group_lo[2] + b->cc_group[q1], pl->group_lo[2] + b->ccgroups + b->cc_group[q1]);
@@ -1204,12 +1136,15 @@ int ozaki_slice(imsrg_basis *b, const double *L, const double *R, int part, cuda
     k_oz_exponents<<<k1 - k0, 256, 0, st>>>(pl->d_chunks + k0, L, R, b->lcc, b->rcc, pl->d_exps);
     b->launches++;
   }
-  const int nblk = pl->cblocks[part] + pl->rblocks[part];
+  const int c_lo = pl->linec_lo[part], c_hi = pl->linec_lo[part + 1];
+  const int r_lo = pl->liner_lo[part], r_hi = pl->liner_lo[part + 1];
+  const int cblocks = (c_hi - c_lo + SLICE_THREADS - 1) / SLICE_THREADS;
+  const int nblk = cblocks + (r_hi - r_lo + SLICE_THREADS - 1) / SLICE_THREADS;
   if (nblk) {
-    (pl->S == 4 ? k_oz_slice<4> : pl->S == 5 ? k_oz_slice<5> : pl->S == 6 ? k_oz_slice<6> : pl->S == 7 ? k_oz_slice<7> : k_oz_slice<8>)<<<nblk, SLICE_THREADS, 0, st>>>(pl->d_mats, pl->nmats, pl->d_blk_mat + pl->blk_off[part], pl->cblocks[part],
-                                     pl->linec_lo[part], pl->linec_lo[part + 1], pl->liner_lo[part],
-                                     pl->liner_lo[part + 1], L, R, b->lcc, b->rcc, pl->d_exps, pl->img[0],
-                                     pl->img[1], pl->img[2], pl->img[3]);
+    auto *kernel = pl->S == 4 ? k_oz_slice<4> : pl->S == 5 ? k_oz_slice<5> : pl->S == 6 ? k_oz_slice<6> :
+                   pl->S == 7 ? k_oz_slice<7> : k_oz_slice<8>;
+    kernel<<<nblk, SLICE_THREADS, 0, st>>>(pl->d_mats, pl->d_mat_c, pl->d_mat_r, cblocks, c_lo, c_hi, r_lo, r_hi, L, R,
+                                           b->lcc, b->rcc, pl->d_exps, pl->img, pl->units * 256);
     b->launches++;
   }
   return cuda_status(cudaGetLastError());
@@ -1224,8 +1159,8 @@ int ozaki_mma(imsrg_basis *b, int hL, int hR) {
     if (cs == cudaStreamCaptureStatusNone) IMSRG_TRY(autotune(b, pl, hL, hR));
   }
   ProfScope ps(b, IMSRG_KERNEL_OZAKI_MMA);
-  launch_mma(pl->S, pl->chunked, pl->grid, b->stream, pl->d_probs, pl->nprobs, pl->d_sched, pl->d_sched_off, pl->d_exps, hL, hR,
-             pl->d_err, pl->d_maps);
+  launch_mma(pl->S, pl->chunked, pl->grid, b->stream, pl->d_tiles, pl->d_sched_off, pl->d_exps, hL, hR, pl->d_err,
+             pl->d_maps);
   b->launches++;
   return cuda_status(cudaGetLastError());
 }
@@ -1304,15 +1239,13 @@ namespace {
 struct OzBatch {
   std::vector<OzPlan *> plans;
   std::vector<int> exps_base;
-  OzProb *d_probs = nullptr;
-  int nprobs = 0, grid = 0, ngroups = 0;
-  bool chunked = false;  // some merged problem runs in more than one chunk
-  int2 *d_sched = nullptr;
+  int grid = 0, ngroups = 0;
+  bool chunked = false;  // some merged tile runs in more than one chunk
+  OzTile *d_tiles = nullptr;
   int *d_sched_off = nullptr, *d_exps = nullptr, *d_err = nullptr;
   CUtensorMap *d_maps = nullptr;
   ~OzBatch() {
-    cudaFree(d_probs);
-    cudaFree(d_sched);
+    cudaFree(d_tiles);
     cudaFree(d_sched_off);
     cudaFree(d_exps);
     cudaFree(d_err);
@@ -1330,7 +1263,6 @@ int ozaki_batch_create(imsrg_basis *const *bases, int n, void **out) {
     return s;
   };
   OzPlan all;  // the merged tile list, for build_sched
-  std::vector<OzProb> probs;
   std::vector<CUtensorMap> maps;
   int model = -1;
   for (int i = 0; i < n; i++) {
@@ -1342,24 +1274,17 @@ int ozaki_batch_create(imsrg_basis *const *bases, int n, void **out) {
     bt->chunked = bt->chunked || pl->chunked;
     if (pl->S != bt->plans[0]->S) return fail(IMSRG_ERR_INVALID);  // one digit count per merged launch
     bt->exps_base.push_back(bt->ngroups);
-    const int p0 = (int)probs.size(), m0 = (int)maps.size();
-    for (const OzProb &p : pl->probs) {
-      OzProb q = p;
+    for (size_t k = 0; k < pl->tiles.size(); k++) {
+      OzTile q = pl->tiles[k];
       q.inst = i;
       q.gA += bt->ngroups;
       q.gB += bt->ngroups;
-      for (int t = 0; t < q.nterms; t++) {
-        q.t[t].a_map += m0;
-        q.t[t].b_map += m0;
-      }
-      probs.push_back(q);
-    }
-    for (size_t k = 0; k < pl->tile_slot.size(); k++) {
+      q.map += (int)maps.size();
+      all.tiles.push_back(q);
       all.tile_ksteps.push_back(pl->tile_ksteps[k]);
       all.tile_live.push_back(pl->tile_live[k]);
-      all.tile_slot.push_back(make_int2(pl->tile_slot[k].x + p0, pl->tile_slot[k].y));
     }
-    maps.insert(maps.end(), pl->maps.begin(), pl->maps.end());
+    maps.insert(maps.end(), pl->maps, pl->maps + 2);
     bt->ngroups += pl->ngroups;
     // the bases' own tuned cost model when they agree, else the one usually chosen
     const int m = pl->tuned ? pl->tune_choice : 1;
@@ -1367,20 +1292,18 @@ int ozaki_batch_create(imsrg_basis *const *bases, int n, void **out) {
   }
   int nsm = 0;
   IMSRG_CUDA_TRY(cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, bases[0]->device));
-  all.grid = std::min(nsm, std::max((int)all.tile_slot.size(), 1));
-  std::vector<int2> sched;
+  all.grid = std::min(nsm, std::max((int)all.tiles.size(), 1));
+  std::vector<OzTile> sched;
   std::vector<int> sched_off;
   build_sched(&all, kSchedModels[model < 0 ? 1 : model], sched, sched_off);
   bt->grid = all.grid;
-  bt->nprobs = (int)probs.size();
   auto up = [&](const void *h, size_t bytes, void **d) -> int {
     IMSRG_CUDA_TRY(cudaMalloc(d, std::max<size_t>(bytes, 16)));
     if (bytes) IMSRG_CUDA_TRY(cudaMemcpy(*d, h, bytes, cudaMemcpyHostToDevice));
     return IMSRG_OK;
   };
   int s = IMSRG_OK;
-  if (s == IMSRG_OK) s = up(probs.data(), probs.size() * sizeof(OzProb), (void **)&bt->d_probs);
-  if (s == IMSRG_OK) s = up(sched.data(), sched.size() * sizeof(int2), (void **)&bt->d_sched);
+  if (s == IMSRG_OK) s = up(sched.data(), sched.size() * sizeof(OzTile), (void **)&bt->d_tiles);
   if (s == IMSRG_OK) s = up(sched_off.data(), sched_off.size() * sizeof(int), (void **)&bt->d_sched_off);
   // (cudaMalloc memory is 256-byte aligned: the 64-byte alignment of a tensor map holds)
   if (s == IMSRG_OK) s = up(maps.data(), maps.size() * sizeof(CUtensorMap), (void **)&bt->d_maps);
@@ -1399,8 +1322,8 @@ int ozaki_batch_mma(void *batch, cudaStream_t st, int hL, int hR, const int *act
     if (bt->plans[i]->ngroups > 0)
       IMSRG_CUDA_TRY(cudaMemcpyAsync(bt->d_exps + bt->exps_base[i], bt->plans[i]->d_exps,
                                      bt->plans[i]->ngroups * sizeof(int), cudaMemcpyDeviceToDevice, st));
-  launch_mma(bt->plans[0]->S, bt->chunked, bt->grid, st, bt->d_probs, bt->nprobs, bt->d_sched, bt->d_sched_off,
-             bt->d_exps, hL, hR, bt->d_err, bt->d_maps, act);
+  launch_mma(bt->plans[0]->S, bt->chunked, bt->grid, st, bt->d_tiles, bt->d_sched_off, bt->d_exps, hL, hR, bt->d_err,
+             bt->d_maps, act);
   return cuda_status(cudaGetLastError());
 }
 
@@ -1422,13 +1345,13 @@ void ozaki_batch_free(void *batch) { delete (OzBatch *)batch; }
 void ozaki_free(imsrg_basis *b) {
   OzPlan *pl = plan_of(b);
   if (!pl) return;
-  for (int s = 0; s < 4; s++) cudaFree(pl->img[s]);
+  cudaFree(pl->img);
   cudaFree(pl->d_mats);
   cudaFree(pl->d_chunks);
-  cudaFree(pl->d_probs);
-  cudaFree(pl->d_sched);
+  cudaFree(pl->d_tiles);
   cudaFree(pl->d_sched_off);
-  cudaFree(pl->d_blk_mat);
+  cudaFree(pl->d_mat_c);
+  cudaFree(pl->d_mat_r);
   cudaFree(pl->d_ccgroups);
   cudaFree(pl->d_exps);
   cudaFree(pl->d_maps);

@@ -31,3 +31,24 @@ def test_fp64_products(gpu_lib, oracle_mod, emax, nucleus):
     gpu_lib.commutator_adjoint(L, gpu_lib.Operator(B, 1, Cb), 1, Yb)
     scale = float(np.dot(np.abs(Cb), np.abs(ref))) + 1.0
     assert abs(float(np.dot(Cb, ref)) - float(np.dot(Yb.download(), Rh))) <= 1e-12 * scale
+
+
+@pytest.mark.parametrize("emax,nucleus", [(1, "4He"), (3, "16O"), (5, "4He")])
+@pytest.mark.parametrize("digits", [4, 5, 6, 7, 8])
+def test_split_products(gpu_lib, oracle_mod, emax, nucleus, digits):
+    """The split engine's tiles and digit images at the same ragged sizes.  The
+    dropped levels and the digit rounding are below 2^-(7 S) (S + 2) K max|A|
+    max|B| per product; with |elements| <= 5, K <= 200 and results of some
+    hundreds that is 2^-(7 S) 200 of the result's scale, plus the FP64 bar."""
+    from imsrg_gpu.layout import Layout, ho_basis
+    from imsrg_gpu.synth import random_operator
+    bas = ho_basis(emax, nucleus)
+    lay = Layout(**bas)
+    B = gpu_lib.Basis.from_dict(bas)
+    B.set_split_digits(digits)
+    Lh, Rh = random_operator(lay, -1, 25, 1), random_operator(lay, 1, 26, 2)
+    ref = oracle_mod.Oracle(**bas).commutator(Lh, -1, Rh, 1)
+    L, R, RES = gpu_lib.Operator(B, -1, Lh), gpu_lib.Operator(B, 1, Rh), gpu_lib.Operator(B, 1)
+    for _ in range(2):  # the autotuning call, then the graph
+        gpu_lib.commutator(L, R, RES, precision="ozaki")
+        assert rel_err(RES.download(), ref) <= 200.0 * 2.0 ** (-7 * digits) + 1e-10

@@ -8,22 +8,23 @@
 // built here by transposing every piece of the forward kernels
 // (kernels_comm.cu) on the same host-built gather lists, one kernel per
 // piece, in the reverse order of the forward data flow:
-//   1. two-body assembly^T: the ladder epilogue of 222_pp_hh hands Cbar to
-//      W1bar / W2bar, the 222_ph recoupling to Zbar, the commutator_122
-//      insertions to Ybar (two- and one-body), the 220 energy to Ybar's pphh;
-//   2. one-body assembly^T: commutator_111 / 121 to Ybar, 221 to W1bar/W2bar;
-//   3. 110^T: the energy's particle-hole sum to Ybar's fph;
-//   4. recoupling inputs^T: Zbar to WCCbar;
-//   5. every dense product transposed as one grouped FP64 launch: the twelve
+//   1. k_adj_prep, everything that needs only X and Cbar: the ladder epilogue
+//      of 222_pp_hh hands Cbar to W1bar / W2bar and to the commutator_122
+//      sums' weights, the 222_ph recoupling to Zbar, LCC is X's Pandya transform;
+//   2. k_adj_122: the commutator_122 insertions to Ybar (two- and one-body, on
+//      transposed gather lists) and the recoupling inputs^T, Zbar to WCCbar;
+//   3. k_adj_one: one-body assembly^T (commutator_111 / 121 to Ybar, 221 to
+//      W1bar / W2bar) and the energy's 110 and 220 terms;
+//   4. every dense product transposed as one grouped FP64 launch: the twelve
 //      ladder products of each block into Ybar's two-body arrays, and
 //      RCCbar = WCCbar^T LCC per cross-coupled block;
-//   6. Pandya transform^T (calculate_cross_coupled, cross_coupled.f90:
+//   5. Pandya transform^T (calculate_cross_coupled, cross_coupled.f90:
 //      1190-1300): RCCbar back to Ybar.
 // The adjoint with respect to X follows from antisymmetry, [X, Y] = -[Y, X]:
 //     d<Cbar, [X, Y]> / dX = -(the adjoint above with the roles swapped).
-// The gather lists become scatters, added with FP64 atomics: the adjoint's
-// results agree run to run to rounding, not bit for bit (the forward
-// commutator stays atomic-free and bit-reproducible).
+// The one-body, recoupling and Pandya lists become scatters, added with FP64
+// atomics: the adjoint's results agree run to run to rounding, not bit for bit
+// (the forward commutator stays atomic-free and bit-reproducible).
 //
 // The flow's adjoint (imsrg_gpu_magnus_decouple_adjoint) records one Magnus
 // flow (the host-driven sequence of magnus_decouple, IMSRG_MAGNUS.f90:15-128,
@@ -91,81 +92,194 @@ __global__ void __launch_bounds__(GT_THREADS, GT_CTAS) k_gemm_adj(const AdjProb 
 }
 
 // ---------------------------------------------------------------------------
-// 1. Two-body assembly^T, one thread per element head (k_assemble_2body's
-//    sequence read backwards).  Forward, per head:
+// 1 and 2. Two-body assembly^T (k_assemble_2body's sequence read backwards).
+// Forward, per element e with mirror em:
 //      t0 = s122 * nd;  t1 = diag ? -t0 (herm(RES) < 0) : t0;
 //      t2 = t1 + W1[e] - W2[e] - [square] (+-)(W1[em] - W2[em]) + sm;
 //      RES[e] = diag ? +-t2 : t2;  RES[em] = herm(RES) t2 (square, off-diagonal)
+// The commutator_122 sums s122 = sum fL vR + fR vL are transposed on lists of
+// their own, one per two-body element of Y and one per one-body element, so
+// nothing scatters: as scatters, five million atomics fell on a few hundred
+// one-body elements (324 us at emax = 6, 39 us at emax = 4; k_adj_122 takes 55
+// and 15 us with the recoupling inputs^T in it, which took 23 and 5).  Work
+// that depends on the same inputs shares a launch, by CTA range: five launches
+// instead of seven and six memsets (emax = 4: 119 -> 63 us, emax = 6: 850 -> 567).
 // ---------------------------------------------------------------------------
-__global__ void __launch_bounds__(128) k_adj_asm2(DevTables T, const double *__restrict__ X, int hL, int hR,
-                                                  const double *__restrict__ Cb, int hRES, int with220,
-                                                  double *Yb, double *W1b, double *W2b, double *Zb) {
-  const long w = (long)blockIdx.x * blockDim.x + threadIdx.x;
-  if (w >= T.n_asm2) return;
-  const Asm2Head h = T.asm2_head[w];
-  const unsigned meta = h.meta;
-  const int nL = hL < 0, nR = hR < 0, nres = hRES < 0, npm = (hL * hR) < 0;
-  const bool diag = (meta >> 20) & 1, square = (meta >> 21) & 1;
-  const long e = h.e, em = h.em;
-  double tb = diag ? dflip(Cb[e], nres) : Cb[e];
-  if (square && !diag) tb += dflip(Cb[em], nres);
-  // ladder epilogue of 222_pp_hh (each W index belongs to one head)
-  if (square) {
-    const double m = dflip(tb, npm);
-    if (diag) {
-      W1b[e] += tb - m;
-      W2b[e] += m - tb;
-    } else {
-      W1b[e] += tb;
-      W2b[e] -= tb;
-      W1b[em] -= m;
-      W2b[em] += m;
+
+// Gather lists of the transposed sums (host-built from the forward's).
+struct AdjLists {
+  const int *mir;             // per two-body flat index from off_2b: partner (bits 0-27), 28 upper or diagonal, 29
+                              // diagonal, 30 square array
+  const int4 *quad;           // per orbit quadruple: first head, heads, first Z, inside Zs
+  const Asm2Head *qhead;      // heads in quadruple order
+  const int *zquad;           // quadruple of each Z
+  const Asm2PreWarp *v_warp;  // two-body targets: 32 to a warp, n entries each (as DevTables::pre_warp)
+  const int *v_el;            // target, -1 pads
+  const unsigned long long *v_terms;  // bits 0-27 element e, 28-47 one-body f, 48 sign, 51 V transposed, 52 f transposed
+  int n_v_warps;
+  const unsigned long long *f_terms;  // one-body targets: bits 0-27 element e, 28-55 V, 56 sign, 57-58 sqrt(2)
+                                      // factors, 59 V transposed, 60 f transposed
+  const int2 *f_chunk;        // first entry and entries of each chunk
+  int n_f_chunks;
+  const int4 *f_target;       // one-body flat index, first chunk, chunks
+  int n_f_targets;
+};
+constexpr int ADJ_THREADS = 256, ADJ_F_CHUNK = 2048, ADJ_ZERO = 2048;
+
+// d(t2) of the element whose stored index is e (upper or diagonal) from Cbar
+__device__ __forceinline__ double adj_tb(const double *__restrict__ Cb, long e, long em, bool square, int nres) {
+  if (!square) return Cb[e];
+  return e == em ? dflip(Cb[e], nres) : Cb[e] + dflip(Cb[em], nres);
+}
+
+// CTAs [0, n0): W1bar, W2bar = -W1bar and the 122 weights U, by flat index;
+// [n0, n1): Zbar; [n1, n2): LCC; the rest zero WCCbar, RCCbar and Ybar's E0 and
+// one-body part.
+__global__ void __launch_bounds__(ADJ_THREADS) k_adj_prep(DevTables T, AdjLists A, const double *__restrict__ X,
+                                                          int hL, int hR, const double *__restrict__ Cb, int hRES,
+                                                          long off_2b, int n0, int n1, int n2, double *W1b,
+                                                          double *W2b, double *U, double *Zb, double *LCC,
+                                                          double *WCCb, double *RCCb, double *Yb) {
+  const int nres = hRES < 0;
+  int blk = blockIdx.x;
+  if (blk < n0) {
+    const long i = off_2b + (long)blk * ADJ_THREADS + threadIdx.x;
+    if (i >= T.nfull) return;
+    const int m = A.mir[i - off_2b];
+    const long p = m & 0x0FFFFFFF;
+    const bool upper = (m >> 28) & 1, diag = (m >> 29) & 1, square = (m >> 30) & 1;
+    const int npm = (hL * hR) < 0;
+    const double tb = upper ? adj_tb(Cb, i, p, square, nres) : adj_tb(Cb, p, i, square, nres);
+    double w = tb;
+    if (diag) w = tb - dflip(tb, npm);
+    else if (!upper) w = -dflip(tb, npm);
+    W1b[i] = w;
+    W2b[i] = -w;
+    double u = diag ? dflip(tb, nres) : tb;
+    const int nd = T.vsq[i];  // identical orbit pairs
+    if (nd) u = u * (nd == 1 ? 0.7071067811865476 : 0.5);
+    U[i] = u;
+    return;
+  }
+  if (blk < n1) {
+    const long t = (long)(blk - n0) * ADJ_THREADS + threadIdx.x;
+    if (t >= T.n_ph) return;
+    const int4 q = A.quad[A.zquad[t]];
+    const int k = (int)t - q.z;
+    double z = 0.0;
+    for (int h = q.x; h < q.x + q.y; h++) {
+      const Asm2Head H = A.qhead[h];
+      const int nd = (H.meta >> 18) & 3;
+      double s = adj_tb(Cb, H.e, H.em, (H.meta >> 21) & 1, nres);
+      if (nd) s = s * (nd == 1 ? .70710678118 : .70710678118 * .70710678118);
+      if (k < q.w) z = fma(dflip(s, (H.meta >> 16) & 1), T.six[H.six1 + k], z);
+      else z = fma(s, T.six[H.six2 + k - q.w], z);
     }
-  } else {
-    W1b[e] += tb;
-    W2b[e] -= tb;
+    Zb[t] = z;
+    return;
   }
-  const int nd = (meta >> 18) & 3;
-  // 222_ph recoupling: sm = c (+-sum_J' {6j} Z_in + sum_J' {6j} Z_out)
-  if ((meta >> 15) & 1) {
-    const int n_in = (meta >> 5) & 31, n_out = (meta >> 10) & 31;
-    const double c = nd ? (nd == 1 ? .70710678118 : .70710678118 * .70710678118) : 1.0;
-    const double s2 = tb * c, s1 = dflip(s2, (meta >> 16) & 1);
-    const double *six1 = T.six + h.six1, *six2 = T.six + h.six2;
-    double *z = Zb + h.zs;
-    for (int k = 0; k < n_in; k++) atomicAdd(z + k, s1 * six1[k]);
-    for (int k = 0; k < n_out; k++) atomicAdd(z + n_in + k, s2 * six2[k]);
+  if (blk < n2) {
+    const long t = (long)(blk - n1) * ADJ_THREADS + threadIdx.x;
+    if (t >= T.cc_total) return;
+    const int v = T.ccf_order[t];
+    const long e = T.ccf_packed ? (v & 0xFFFFFF) : v;
+    double s = 0.0;
+    for (int k = T.cct_start[e]; k < T.cct_start[e + 1]; k++) {
+      const int ix = T.cct_idx[k];
+      s = fma(T.cct_coef[k], dflip(X[ix & 0x7fffffff], ((unsigned)ix >> 31) & (hL < 0)), s);
+    }
+    LCC[e] = s;
+    return;
   }
-  // commutator_122: s122 = sum fL vR + fR vL over the element's terms, where
-  // (L, R) = (X, Y) and only the Y factors vary
-  double u = diag ? dflip(tb, nres) : tb;
-  if (nd) u = u * (nd == 1 ? 0.7071067811865476 : 0.5);
-  const unsigned long long *tm = T.asm2_terms + h.start;
-  const int n122 = meta & 31;
-  for (int k = 0; k < n122; k++) {
-    const unsigned long long v = tm[k];
-    const long vi = (long)(v & 0xFFFFFFFull), fi = (long)((v >> 28) & 0xFFFFFull);
-    const int sg = (int)(v >> 48) & 1, nsq = (int)(v >> 49) & 3, tr = (int)(v >> 51) & 1, ftr = (int)(v >> 52) & 1;
-    const double c = nsq ? (nsq == 1 ? IMSRG_SQRT2 : 2.0000000000000004) : 1.0;
-    const double fL = dflip(X[fi], (ftr & nL) ^ sg);
-    const double vL = dflip(X[vi], tr & nL) * c;
-    atomicAdd(Yb + vi, dflip(u * fL * c, tr & nR));
-    atomicAdd(Yb + fi, dflip(u * vL, (ftr & nR) ^ sg ^ 1));
+  const long z0 = (long)(blk - n2) * ADJ_ZERO, nz = T.wcc_total + T.cc_total + off_2b;
+  for (long i = z0 + threadIdx.x; i < min(z0 + ADJ_ZERO, nz); i += ADJ_THREADS) {
+    if (i < T.wcc_total) WCCb[i] = 0.0;
+    else if (i < T.wcc_total + T.cc_total) RCCb[i - T.wcc_total] = 0.0;
+    else Yb[i - T.wcc_total - T.cc_total] = 0.0;
   }
-  // commutator_220 (E0 = ... - 2 herm_R sum (2J+1) L_pphh R_pphh)
-  if (with220 && ((meta >> 22) & 1)) atomicAdd(Yb + e, -2.0 * hR * (h.J2 + 1.0) * Cb[0] * X[e]);
+}
+
+// Recoupling inputs^T: Z = herm_L (W(x1,y1) + e W(x2,y2)) - herm_R (e W(y2,x2) + W(y1,x1))
+__device__ __forceinline__ void adj_ph(const DevTables &T, const double *__restrict__ Zb, int hL, int hR, double *WCCb,
+                                       long t) {
+  if (t >= T.n_ph) return;
+  const double z = Zb[t];
+  if (z == 0.0) return;
+  const PhTerm p = T.ph_terms[t];
+  const unsigned long long u = p.rows;
+  const unsigned x1 = (unsigned)(u & 0xFFFF), y1 = (unsigned)((u >> 16) & 0xFFFF);
+  const unsigned x2 = (unsigned)((u >> 32) & 0xFFFF), y2 = (unsigned)(u >> 48);
+  const int q1 = p.q & 0xFFFF, q2 = p.q >> 16, rl = T.cc_rlen[q1];
+  double *W = WCCb + T.wcc_off[q1], *W2 = WCCb + T.wcc_off[q2];  // the two blocks have one size
+  const double a = dflip(z, hL < 0), c = -dflip(z, hR < 0);
+  if (x1 != 0xFFFFu && y1 != 0xFFFFu) {
+    atomicAdd(W + x1 + (long)y1 * rl, a);
+    atomicAdd(W + y1 + (long)x1 * rl, c);
+  }
+  if (x2 != 0xFFFFu && y2 != 0xFFFFu) {
+    atomicAdd(W2 + x2 + (long)y2 * rl, dflip(a, p.nph));
+    atomicAdd(W2 + y2 + (long)x2 * rl, dflip(c, p.nph));
+  }
+}
+
+// CTAs [0, n0): the partial sum of one chunk of a one-body target's list;
+// [n0, n1): two-body targets, a warp per 32 (sets Ybar there); the rest: the
+// recoupling inputs^T.
+__global__ void __launch_bounds__(ADJ_THREADS) k_adj_122(DevTables T, AdjLists A, const double *__restrict__ X, int hL,
+                                                         int hR, const double *__restrict__ U,
+                                                         const double *__restrict__ Zb, int n0, int n1, double *fpart,
+                                                         double *WCCb, double *Yb) {
+  __shared__ double sh[32];
+  const int nL = hL < 0, nR = hR < 0;
+  const int blk = blockIdx.x;
+  if (blk < n0) {
+    const int2 c = A.f_chunk[blk];
+    double s = 0.0;
+    for (int k = threadIdx.x; k < c.y; k += ADJ_THREADS) {
+      const unsigned long long u = A.f_terms[(long)c.x + k];
+      const long e = (long)(u & 0xFFFFFFFull), vi = (long)((u >> 28) & 0xFFFFFFFull);
+      const int sg = (int)(u >> 56) & 1, nsq = (int)(u >> 57) & 3, tr = (int)(u >> 59) & 1, ftr = (int)(u >> 60) & 1;
+      double v = X[vi];
+      if (nsq) v = v * (nsq == 1 ? IMSRG_SQRT2 : 2.0000000000000004);
+      s = fma(dflip(U[e], (tr & nL) ^ (ftr & nR) ^ sg ^ 1), v, s);
+    }
+    s = block_sum_ops(s, sh);
+    if (threadIdx.x == 0) fpart[blk] = s;
+    return;
+  }
+  if (blk < n1) {
+    const int g = (blk - n0) * (ADJ_THREADS / 32) + (int)(threadIdx.x >> 5), lane = threadIdx.x & 31;
+    if (g >= A.n_v_warps) return;
+    const int vi = A.v_el[(long)g * 32 + lane];
+    if (vi < 0) return;  // padding
+    const Asm2PreWarp W = A.v_warp[g];
+    const unsigned long long *tm = A.v_terms + W.base + lane;
+    double s = 0.0;
+    for (int k = 0; k < W.n122; k++) {
+      const unsigned long long u = tm[k * 32];
+      if (u >> 63) break;  // the lane's list has ended
+      const long e = (long)(u & 0xFFFFFFFull), fi = (long)((u >> 28) & 0xFFFFFull);
+      const int sg = (int)(u >> 48) & 1, tr = (int)(u >> 51) & 1, ftr = (int)(u >> 52) & 1;
+      s = fma(dflip(U[e], (tr & nR) ^ (ftr & nL) ^ sg), X[fi], s);
+    }
+    const int nsq = T.vsq[vi];
+    if (nsq) s = s * (nsq == 1 ? IMSRG_SQRT2 : 2.0000000000000004);
+    Yb[vi] = s;
+    return;
+  }
+  adj_ph(T, Zb, hL, hR, WCCb, (long)(blk - n1) * ADJ_THREADS + threadIdx.x);
 }
 
 // ---------------------------------------------------------------------------
-// 2. One-body assembly^T over k_assemble_1body's work split (an allowed
+// 3. One-body assembly^T over k_assemble_1body's work split (an allowed
 //    upper-triangle element per CTA, every other element per warp).  Forward:
 //      x = c0 v0 + c1 v1 + c2 v2 + c3 v3 + [allowed] (rj v4 + c5 v5)
 //    with v0..v3 the commutator_111 dot products, v4 the 121 sums, v5 the 221
 //    sums; RES[p, q] = x and, for allowed square elements, RES[q, p] = herm x.
 // ---------------------------------------------------------------------------
-__global__ void __launch_bounds__(128) k_adj_1body(DevTables T, const double *X, int hL, int hR,
-                                                   const double *__restrict__ Cb, int hRES, double *Yb,
-                                                   double *W1b, double *W2b) {
+__device__ __forceinline__ void adj_1body(const DevTables &T, const double *X, int hL, int hR,
+                                          const double *__restrict__ Cb, int hRES, double *Yb, double *W1b,
+                                          double *W2b) {
   const int A = T.A, P = T.P;
   const double *Lhh = X + T.off_fhh, *Lph = X + T.off_fph, *Lpp = X + T.off_fpp;
   double *Rhh = Yb + T.off_fhh, *Rph = Yb + T.off_fph, *Rpp = Yb + T.off_fpp;
@@ -279,40 +393,38 @@ __global__ void __launch_bounds__(128) k_adj_1body(DevTables T, const double *X,
   }
 }
 
-// 3. commutator_110^T: E0 += sum_ai (2j_i+1) (L_ai R_ai herm_L - R_ai L_ai herm_R)
-__global__ void k_adj_e0(DevTables T, const double *__restrict__ X, int hL, int hR, const double *__restrict__ Cb,
-                         double *Yb) {
-  const int k = blockIdx.x * blockDim.x + threadIdx.x;
-  if (k >= T.P * T.A) return;
-  const int ji = T.orb[T.hole_orb[k / T.P]].x;
-  atomicAdd(Yb + T.off_fph + k, Cb[0] * (double)(hL - hR) * (ji + 1) * X[T.off_fph + k]);
-}
-
-// 4. Recoupling inputs^T: Z = herm_L (W(x1,y1) + e W(x2,y2)) - herm_R (e W(y2,x2) + W(y1,x1))
-__global__ void __launch_bounds__(256) k_adj_ph(DevTables T, const double *__restrict__ Zb, int hL, int hR,
-                                                double *WCCb) {
-  const long t = (long)blockIdx.x * blockDim.x + threadIdx.x;
-  if (t >= T.n_ph) return;
-  const double z = Zb[t];
-  if (z == 0.0) return;
-  const PhTerm p = T.ph_terms[t];
-  const unsigned long long u = p.rows;
-  const unsigned x1 = (unsigned)(u & 0xFFFF), y1 = (unsigned)((u >> 16) & 0xFFFF);
-  const unsigned x2 = (unsigned)((u >> 32) & 0xFFFF), y2 = (unsigned)(u >> 48);
-  const int q1 = p.q & 0xFFFF, q2 = p.q >> 16, rl = T.cc_rlen[q1];
-  double *W = WCCb + T.wcc_off[q1], *W2 = WCCb + T.wcc_off[q2];  // the two blocks have one size
-  const double a = dflip(z, hL < 0), c = -dflip(z, hR < 0);
-  if (x1 != 0xFFFFu && y1 != 0xFFFFu) {
-    atomicAdd(W + x1 + (long)y1 * rl, a);
-    atomicAdd(W + y1 + (long)x1 * rl, c);
-  }
-  if (x2 != 0xFFFFu && y2 != 0xFFFFu) {
-    atomicAdd(W2 + x2 + (long)y2 * rl, dflip(a, p.nph));
-    atomicAdd(W2 + y2 + (long)x2 * rl, dflip(c, p.nph));
+// CTAs [0, n0): the one-body assembly^T; [n0, n1): the one-body targets of the
+// commutator_122 lists, their chunks in order; [n1, n2): commutator_110^T, E0 +=
+// sum_ai (2j_i+1) (L_ai R_ai herm_L - R_ai L_ai herm_R); the rest, a CTA per (2J,
+// Tz, pi) block: commutator_220^T, E0 -= 2 herm_R (2J+1) L_pphh R_pphh.
+__global__ void __launch_bounds__(128) k_adj_one(DevTables T, AdjLists A, const double *X, int hL, int hR,
+                                                 const double *__restrict__ Cb, int hRES,
+                                                 const double *__restrict__ fpart, int n0, int n1, int n2, double *Yb,
+                                                 double *W1b, double *W2b) {
+  const int blk = blockIdx.x;
+  if (blk < n0) {
+    adj_1body(T, X, hL, hR, Cb, hRES, Yb, W1b, W2b);
+  } else if (blk < n1) {
+    const int t = (blk - n0) * 128 + threadIdx.x;
+    if (t >= A.n_f_targets) return;
+    const int4 f = A.f_target[t];
+    double s = 0.0;
+    for (int k = f.y; k < f.y + f.z; k++) s += fpart[k];
+    atomicAdd(Yb + f.x, s);
+  } else if (blk < n2) {
+    const int k = (blk - n1) * 128 + threadIdx.x;
+    if (k >= T.P * T.A) return;
+    const int ji = T.orb[T.hole_orb[k / T.P]].x;
+    atomicAdd(Yb + T.off_fph + k, Cb[0] * (double)(hL - hR) * (ji + 1) * X[T.off_fph + k]);
+  } else {
+    const int q = blk - n2, n = T.gam_n1[q * 6 + 2] * T.gam_n2[q * 6 + 2];
+    const long o = T.gam_off[q * 6 + 2];
+    for (int k = threadIdx.x; k < n; k += 128)
+      atomicAdd(Yb + o + k, -2.0 * hR * (T.blk_J2[q] + 1.0) * Cb[0] * X[o + k]);
   }
 }
 
-// 6. Pandya transform^T: RCC[e] = sum_k coef_k (herm_R if transposed) R[idx_k]
+// 5. Pandya transform^T: RCC[e] = sum_k coef_k (herm_R if transposed) R[idx_k]
 __global__ void __launch_bounds__(256) k_adj_cc(DevTables T, const double *__restrict__ RCCb, int hR, double *Yb) {
   const long e = (long)blockIdx.x * blockDim.x + threadIdx.x;
   if (e >= T.cc_total) return;
@@ -354,7 +466,9 @@ __global__ void k_dot_final(const double *__restrict__ part, double *out) {
 
 // Per-basis state of the adjoint (allocated on first use).
 struct AdjState {
-  double *w1b = nullptr, *w2b = nullptr, *rccb = nullptr, *wccb = nullptr, *zb = nullptr;
+  double *w1b = nullptr, *w2b = nullptr, *rccb = nullptr, *wccb = nullptr, *zb = nullptr, *u = nullptr;
+  double *fpart = nullptr;
+  AdjLists lists{};
   double *monob = nullptr, *part = nullptr, *dot = nullptr, *h_dot = nullptr;
   AdjProb *d_probs = nullptr;
   GemmTile *d_tiles = nullptr;
@@ -450,6 +564,123 @@ std::vector<AdjProb> adjoint_problems(const imsrg_basis *b) {
 
 }  // namespace
 
+namespace {
+
+template <typename V>
+int adj_upload(imsrg_basis *b, const std::vector<V> &h, const V **out) {
+  void *p = nullptr;
+  IMSRG_CUDA_TRY(cudaMalloc(&p, std::max<size_t>(h.size() * sizeof(V), 16)));
+  b->dev_allocs.push_back(p);
+  if (!h.empty()) IMSRG_CUDA_TRY(cudaMemcpy(p, h.data(), h.size() * sizeof(V), cudaMemcpyHostToDevice));
+  *out = (const V *)p;
+  return IMSRG_OK;
+}
+
+// The transposed lists, from the forward's heads and commutator_122 terms.
+int adj_lists(imsrg_basis *b, AdjState *a) {
+  const DevTables &T = b->T;
+  AdjLists &A = a->lists;
+  std::vector<Asm2Head> heads(T.n_asm2);
+  if (T.n_asm2)
+    IMSRG_CUDA_TRY(cudaMemcpy(heads.data(), T.asm2_head, heads.size() * sizeof(Asm2Head), cudaMemcpyDeviceToHost));
+  // by flat index: the entries of one target then run along matrix columns
+  std::sort(heads.begin(), heads.end(), [](const Asm2Head &x, const Asm2Head &y) { return x.e < y.e; });
+  long nt = 0;
+  for (const Asm2Head &h : heads) nt = std::max(nt, (long)h.start + (long)(h.meta & 31));
+  std::vector<unsigned long long> terms(nt);
+  if (nt) IMSRG_CUDA_TRY(cudaMemcpy(terms.data(), T.asm2_terms, nt * 8, cudaMemcpyDeviceToHost));
+  const long off = b->off_2b, n2 = b->nfull - off;
+  // partner of every element
+  std::vector<int> mir(n2, 0);
+  for (const Asm2Head &h : heads) {
+    const bool diag = (h.meta >> 20) & 1, square = (h.meta >> 21) & 1;
+    mir[h.e - off] = (square ? h.em : h.e) | 1 << 28 | (diag ? 1 << 29 : 0) | (square ? 1 << 30 : 0);
+    if (square && !diag) mir[h.em - off] = h.e | 1 << 30;
+  }
+  // heads by quadruple (the elements that share recoupling inputs)
+  std::vector<Asm2Head> qhead;
+  for (const Asm2Head &h : heads)
+    if (((h.meta >> 15) & 1) && ((h.meta >> 5) & 1023)) qhead.push_back(h);
+  std::stable_sort(qhead.begin(), qhead.end(), [](const Asm2Head &x, const Asm2Head &y) { return x.zs < y.zs; });
+  std::vector<int4> quad;
+  std::vector<int> zquad(T.n_ph, 0);
+  for (size_t h = 0; h < qhead.size(); h++) {
+    const int n_in = (qhead[h].meta >> 5) & 31, n_out = (qhead[h].meta >> 10) & 31;
+    if (h == 0 || qhead[h].zs != qhead[h - 1].zs) {
+      quad.push_back(make_int4((int)h, 0, qhead[h].zs, n_in));
+      for (int k = 0; k < n_in + n_out; k++) zquad[qhead[h].zs + k] = (int)quad.size() - 1;
+    }
+    quad.back().y++;
+  }
+  // commutator_122 terms by two-body element of Y (grouped by count, 32 to a
+  // warp) and by one-body element (chunks)
+  std::vector<int> vn(n2, 0), fn(off, 0);
+  for (const Asm2Head &h : heads)
+    for (int k = 0; k < (int)(h.meta & 31); k++) {
+      const unsigned long long u = terms[h.start + k];
+      vn[(long)(u & 0xFFFFFFFull) - off]++;
+      fn[(u >> 28) & 0xFFFFFull]++;
+    }
+  std::vector<int> order(n2);
+  for (long i = 0; i < n2; i++) order[i] = (int)i;
+  std::stable_sort(order.begin(), order.end(), [&](int x, int y) { return vn[x] > vn[y]; });
+  std::vector<Asm2PreWarp> vw;
+  std::vector<int> ve;
+  std::vector<long> vpos(n2);  // next entry of each target
+  long nv = 0;
+  for (long g = 0; g < n2; g += 32) {
+    const int n = vn[order[g]];  // the warp's longest list; shorter ones end early
+    vw.push_back({nv, n, 0});
+    for (long l = 0; l < 32; l++) {
+      ve.push_back(g + l < n2 ? (int)(order[g + l] + off) : -1);
+      if (g + l < n2) vpos[order[g + l]] = nv + l;
+    }
+    nv += 32L * n;
+  }
+  std::vector<unsigned long long> vt(nv, ~0ull);  // padding: bit 63
+  std::vector<long> fpos(off);
+  std::vector<int2> chunk;
+  std::vector<int4> target;
+  long nf = 0;
+  for (long f = 0; f < off; f++) {
+    fpos[f] = nf;
+    if (!fn[f]) continue;
+    target.push_back(make_int4((int)f, (int)chunk.size(), 0, 0));
+    for (int k = 0; k < fn[f]; k += ADJ_F_CHUNK) {
+      chunk.push_back(make_int2((int)(nf + k), std::min(ADJ_F_CHUNK, fn[f] - k)));
+      target.back().z++;
+    }
+    nf += fn[f];
+  }
+  if (nf >= (1L << 31)) return IMSRG_ERR_TOO_LARGE;
+  std::vector<unsigned long long> ft(nf);
+  for (const Asm2Head &h : heads)
+    for (int k = 0; k < (int)(h.meta & 31); k++) {
+      const unsigned long long u = terms[h.start + k];
+      const unsigned long long v = u & 0xFFFFFFFull, f = (u >> 28) & 0xFFFFFull, e = (unsigned long long)h.e;
+      vt[vpos[(long)v - off]] = (u & ~0xFFFFFFFull) | e;
+      vpos[(long)v - off] += 32;
+      ft[fpos[f]++] = e | v << 28 | ((u >> 48) & 1) << 56 | ((u >> 49) & 3) << 57 | ((u >> 51) & 1) << 59 |
+                      ((u >> 52) & 1) << 60;
+    }
+  A.n_v_warps = (int)vw.size();
+  A.n_f_chunks = (int)chunk.size();
+  A.n_f_targets = (int)target.size();
+  IMSRG_TRY(adj_upload(b, mir, &A.mir));
+  IMSRG_TRY(adj_upload(b, quad, &A.quad));
+  IMSRG_TRY(adj_upload(b, qhead, &A.qhead));
+  IMSRG_TRY(adj_upload(b, zquad, &A.zquad));
+  IMSRG_TRY(adj_upload(b, vw, &A.v_warp));
+  IMSRG_TRY(adj_upload(b, ve, &A.v_el));
+  IMSRG_TRY(adj_upload(b, vt, &A.v_terms));
+  IMSRG_TRY(adj_upload(b, ft, &A.f_terms));
+  IMSRG_TRY(adj_upload(b, chunk, &A.f_chunk));
+  IMSRG_TRY(adj_upload(b, target, &A.f_target));
+  return IMSRG_OK;
+}
+
+}  // namespace
+
 int adjoint_prepare(imsrg_basis *b) {
   if (b->adjoint) return IMSRG_OK;
   AdjState *a = new AdjState();
@@ -459,6 +690,9 @@ int adjoint_prepare(imsrg_basis *b) {
   IMSRG_TRY(adj_alloc(b, b->cc_total, &a->rccb));
   IMSRG_TRY(adj_alloc(b, b->wcc_total, &a->wccb));
   IMSRG_TRY(adj_alloc(b, b->T.n_ph, &a->zb));
+  IMSRG_TRY(adj_lists(b, a));
+  IMSRG_TRY(adj_alloc(b, b->nfull, &a->u));
+  IMSRG_TRY(adj_alloc(b, a->lists.n_f_chunks, &a->fpart));
   IMSRG_TRY(adj_alloc(b, (long)b->norb * b->norb, &a->monob));
   IMSRG_TRY(adj_alloc(b, DOT_CTAS, &a->part));
   IMSRG_TRY(adj_alloc(b, 1, &a->dot));
@@ -499,26 +733,27 @@ int commutator_adjoint_dev(imsrg_basis *b, const double *X, int hX, const double
   AdjState *a = adj_of(b);
   cudaStream_t st = b->stream;
   const int hL = hX, hR = hY, hRES = -hX * hY;
-  const size_t nf = b->nfull * sizeof(double);
-  IMSRG_CUDA_TRY(cudaMemsetAsync(Yb, 0, nf, st));
-  IMSRG_CUDA_TRY(cudaMemsetAsync(a->w1b, 0, nf, st));
-  IMSRG_CUDA_TRY(cudaMemsetAsync(a->w2b, 0, nf, st));
-  if (b->T.n_ph) IMSRG_CUDA_TRY(cudaMemsetAsync(a->zb, 0, b->T.n_ph * sizeof(double), st));
-  if (b->cc_total) IMSRG_CUDA_TRY(cudaMemsetAsync(a->rccb, 0, b->cc_total * sizeof(double), st));
-  if (b->wcc_total) IMSRG_CUDA_TRY(cudaMemsetAsync(a->wccb, 0, b->wcc_total * sizeof(double), st));
-  // LCC = Pandya transform of X (the fixed factor of RCCbar = WCCbar^T LCC)
-  IMSRG_TRY(launch_cc_forward(b, X, hX, X, hX, nullptr, 0, 0, 1, st));
+  const DevTables &T = b->T;
+  const AdjLists &A = a->lists;
   ProfScope ps(b, IMSRG_KERNEL_OPS, st);
-  const int with220 = with_e0 && hL * hR == -1;
-  if (b->T.n_asm2 > 0)
-    k_adj_asm2<<<(unsigned)((b->T.n_asm2 + 127) / 128), 128, 0, st>>>(b->T, X, hL, hR, Cb, hRES, with220, Yb,
-                                                                       a->w1b, a->w2b, a->zb);
-  const int grid1 = b->T.n_asm1_heavy + (b->T.n_asm1_light + 3) / 4;
-  if (grid1 > 0) k_adj_1body<<<grid1, 128, 0, st>>>(b->T, X, hL, hR, Cb, hRES, Yb, a->w1b, a->w2b);
-  if (with_e0 && b->P * b->A > 0)
-    k_adj_e0<<<(b->P * b->A + 255) / 256, 256, 0, st>>>(b->T, X, hL, hR, Cb, Yb);
-  if (b->T.n_ph > 0)
-    k_adj_ph<<<(unsigned)((b->T.n_ph + 255) / 256), 256, 0, st>>>(b->T, a->zb, hL, hR, a->wccb);
+  auto ctas = [](long n, long per) { return (int)((n + per - 1) / per); };
+  {
+    const int n0 = ctas(b->nfull - b->off_2b, ADJ_THREADS), n1 = n0 + ctas(T.n_ph, ADJ_THREADS),
+              n2 = n1 + ctas(b->cc_total, ADJ_THREADS),
+              n3 = n2 + ctas(b->wcc_total + b->cc_total + b->off_2b, ADJ_ZERO);
+    k_adj_prep<<<n3, ADJ_THREADS, 0, st>>>(T, A, X, hL, hR, Cb, hRES, b->off_2b, n0, n1, n2, a->w1b, a->w2b, a->u,
+                                            a->zb, b->lcc, a->wccb, a->rccb, Yb);
+  }
+  {
+    const int n0 = A.n_f_chunks, n1 = n0 + ctas(A.n_v_warps, ADJ_THREADS / 32), n2 = n1 + ctas(T.n_ph, ADJ_THREADS);
+    if (n2) k_adj_122<<<n2, ADJ_THREADS, 0, st>>>(T, A, X, hL, hR, a->u, a->zb, n0, n1, a->fpart, a->wccb, Yb);
+  }
+  {
+    const int n0 = T.n_asm1_heavy + (T.n_asm1_light + 3) / 4, n1 = n0 + ctas(A.n_f_targets, 128),
+              n2 = n1 + (with_e0 ? ctas((long)b->P * b->A, 128) : 0),
+              n3 = n2 + (with_e0 && hL * hR == -1 ? b->nblocks : 0);
+    if (n3) k_adj_one<<<n3, 128, 0, st>>>(T, A, X, hL, hR, Cb, hRES, a->fpart, n0, n1, n2, Yb, a->w1b, a->w2b);
+  }
   if (a->ntiles > 0) {
     AdjOps ops{};
     ops.src[AS_X] = X;
@@ -532,7 +767,7 @@ int commutator_adjoint_dev(imsrg_basis *b, const double *X, int hX, const double
   }
   if (b->cc_total > 0)
     k_adj_cc<<<(unsigned)((b->cc_total + 255) / 256), 256, 0, st>>>(b->T, a->rccb, hR, Yb);
-  b->launches += 6;
+  b->launches += 5;
   return cuda_status(cudaGetLastError());
 }
 

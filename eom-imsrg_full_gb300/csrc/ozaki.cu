@@ -29,7 +29,7 @@
 //      sets of S x TN columns) so the epilogue warps read one tile
 //      (tcgen05.ld), combine its levels in int64 and write FP64 while the
 //      next tile's products run.  Each CTA takes a host-built list of
-//      (problem, tile) slots, longest first under a cost model that an
+//      tiles, spread by longest processing time under a cost model that an
 //      autotuner picks by timing the kernel when the plan is built.
 //
 // Exactness: the level sums of levels 2..4 are bounded by 5 * 2^12 per
@@ -91,20 +91,36 @@ constexpr int A_SLICE_BYTES = TM * TK * 2;   // 4096
 __host__ __device__ constexpr int oz_b_slice_bytes(int S) { return oz_tn(S) * TK * 2; }
 __host__ __device__ constexpr int oz_stage_bytes(int S) { return S * (A_SLICE_BYTES + oz_b_slice_bytes(S)); }
 __host__ __device__ constexpr int oz_stages(int S) { return S >= 8 ? 5 : STAGES; }
-__host__ __device__ constexpr int oz_mma_smem(int S) { return oz_stages(S) * oz_stage_bytes(S) + 1024 + 256; }
+// tile records kept in shared memory (the rest of a longer list is read from
+// global memory), in what the stages leave of 227 KB
+constexpr int kRecBytes = 96;
+__host__ __device__ constexpr int oz_rec_cap(int S) {
+  const int room = (227 * 1024 - oz_stages(S) * oz_stage_bytes(S) - 1024 - 256) / kRecBytes;
+  return room < 256 ? room : 256;
+}
+__host__ __device__ constexpr int oz_mma_smem(int S) {
+  return oz_stages(S) * oz_stage_bytes(S) + 1024 + 256 + oz_rec_cap(S) * kRecBytes;
+}
 // K steps per accumulator chunk (see kOzChunkSteps and oz_fp64_class)
 __host__ __device__ constexpr int oz_chunk_steps(int S) {
   return oz_fp64_class(S) ? (16777216 - 1) / (TK * (S + 2) * 4096) : kOzChunkSteps;
 }
 constexpr int TMEM_COLS = 512;
 constexpr int ACC_BUF_COLS = 256;  // accumulator set b (double-buffered) starts at column 256 b
-// epilogue warps: one per (TMEM lane quadrant, 16-column chunk of the tile)
-__host__ __device__ constexpr int oz_epi_warps(int S) { return 4 * (oz_tn(S) / 16); }
+// epilogue warps: one per (TMEM lane quadrant, quarter of the tile's columns).
+// Sixteen: the conversions' latencies need four warps per scheduler (eight
+// warps of twice the columns: 32.5 us for the product launch at emax = 6, five
+// digits, against 27.4; 92 against 63 with eight digits).
+__host__ __device__ constexpr int oz_ec(int S) { return oz_tn(S) / 4; }
+__host__ __device__ constexpr int oz_epi_warps(int S) { return 16; }
 // warp 0 producer, 1 MMA issuer, then the epilogue warps
 __host__ __device__ constexpr int oz_threads(int S) { return 32 * (2 + oz_epi_warps(S)); }
 static_assert(OZ_SMAX * 32 <= ACC_BUF_COLS && 4 * 64 <= ACC_BUF_COLS, "level accumulators of a set");
-static_assert(oz_mma_smem(6) <= 227 * 1024 && oz_mma_smem(7) <= 227 * 1024 && oz_mma_smem(8) <= 227 * 1024,
-              "stages");
+static_assert(oz_rec_cap(4) > 0 && oz_rec_cap(6) > 0 && oz_rec_cap(7) > 0 && oz_rec_cap(8) > 0, "stages");
+// A boxes of 16, 32, 64 and 128 rows: a tile loads no more rows of A than the
+// smallest that covers its own (kinds 0 .. 3); one B box
+constexpr int kABoxes = 4, kMaps = kABoxes + 1;
+__host__ __device__ constexpr int oz_abox_groups(int kind) { return 2 << kind; }
 constexpr unsigned long long WAIT_NS = 2000000000ull;
 
 struct OzMatrix {
@@ -125,11 +141,11 @@ struct OzChunk {
   int len;
 };
 
-// One 128 x TN output tile, everything its roles need in one contiguous record
-// (each role loads the next record while it works on this one; following
-// schedule -> problem -> term -> tensor map pointers cost every tile about four
-// dependent memory latencies: 46.4 us for the product launch at emax = 6, five
-// digits, 38.1 with records and one tensor map per box).  The (term, K step) sequence, term-major, runs
+// One 128 x TN output tile, everything its roles need in one contiguous record;
+// a CTA copies its records into shared memory first (following schedule ->
+// problem -> term -> tensor map pointers cost every tile about four dependent
+// memory latencies: 46.4 us for the product launch at emax = 6, five digits,
+// 38.1 with records).  The (term, K step) sequence, term-major, runs
 // in chunks of kchunk steps, each into a fresh accumulator set: a chunk's FP32
 // level sums stay exact integers (kchunk TK 5 2^12 < 2^24) and the epilogue adds
 // the chunks' int64 level sums exactly before the one conversion.
@@ -141,11 +157,11 @@ struct __align__(16) OzTile {
   int rows, cols;      // outputs of the problem from this tile's origin on
   int ldc, inst;       // inst: instance (basis) of a merged batch plan; runs only while act[inst]
   int gA, gB;          // exponent groups of A and B
-  int map, pad;        // the A tensor map; the B map follows it
+  int map, abox;       // first tensor map of the instance (see kMaps), A box kind
   double *C;           // the tile's origin
   long pad2;
 };
-static_assert(sizeof(OzTile) == 96, "record of six 16-byte loads");
+static_assert(sizeof(OzTile) == kRecBytes, "record of six 16-byte loads");
 constexpr int kTileTwoTerms = 1, kTileRaw = 2;  // raw: store the exact int64 level sum v (result = v 2^k): WCC
 constexpr int kTileNeg = 4, kTileHL = 8, kTileHR = 16, kTileTermShift = 3;  // term 1's signs at << kTileTermShift
 
@@ -193,8 +209,8 @@ struct OzPlan {
   bool tuned = false;
   std::vector<OzTile> tiles;                // in problem order
   std::vector<int> tile_ksteps, tile_live;  // per tile: K steps x terms, live outputs / 64
-  CUtensorMap *d_maps = nullptr;            // A box, B box
-  CUtensorMap maps[2];
+  CUtensorMap *d_maps = nullptr;            // A boxes, B box
+  CUtensorMap maps[kMaps];
   bool ok = false;
 };
 
@@ -237,10 +253,10 @@ __device__ __forceinline__ bool mbar_wait(uint64_t *bar, uint32_t parity, volati
         : "r"(addr), "r"(parity)
         : "memory");
     if (done) return true;
-    if ((it & 255) == 0) {
+    if ((it & 63) == 63) {  // (the timer is slow to read: not on a wait that is about to succeed)
       if (*abort_flag) return false;
       unsigned long long t = gtimer();
-      if (it == 0) t0 = t;
+      if (it == 63) t0 = t;
       else if (t - t0 > WAIT_NS) return false;
     }
   }
@@ -257,8 +273,6 @@ __device__ __forceinline__ void tma_load_3d(void *sdst, const CUtensorMap *map, 
       : "memory");
 }
 
-__device__ __forceinline__ void prefetch_l1(const void *p) { asm volatile("prefetch.global.L1 [%0];" ::"l"(p)); }
-
 __device__ __forceinline__ uint64_t smem_desc(uint32_t saddr, uint32_t lbo, uint32_t sbo) {
   uint64_t d = 0;
   d |= (uint64_t)((saddr & 0x3FFFF) >> 4);
@@ -266,6 +280,19 @@ __device__ __forceinline__ uint64_t smem_desc(uint32_t saddr, uint32_t lbo, uint
   d |= (uint64_t)((sbo >> 4) & 0x3FFF) << 32;
   d |= (uint64_t)1 << 46;  // descriptor version for tcgen05
   return d;                // base offset 0, no swizzle
+}
+
+__device__ __forceinline__ uint64_t desc_of(uint32_t lo, uint32_t hi) { return (uint64_t)hi << 32 | lo; }
+
+// true in one lane of the (converged) warp
+__device__ __forceinline__ bool elect_one() {
+  uint32_t p;
+  asm volatile(
+      "{\n\t.reg .pred q;\n\t"
+      "elect.sync _|q, 0xffffffff;\n\t"
+      "selp.u32 %0, 1, 0, q;\n\t}"
+      : "=r"(p));
+  return p != 0;
 }
 
 // kind::f16 instruction descriptor: D F32, A and B BF16, both K-major.
@@ -291,7 +318,13 @@ __device__ __forceinline__ void mma_commit(uint64_t *bar) {
 __device__ __forceinline__ void tc_fence_before() { asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory"); }
 __device__ __forceinline__ void tc_fence_after() { asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory"); }
 
-__device__ __forceinline__ void tmem_ld16(uint32_t taddr, uint32_t *r) {
+__device__ __forceinline__ void tmem_ld(uint32_t taddr, uint32_t (&r)[8]) {
+  asm volatile("tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];"
+               : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7])
+               : "r"(taddr));
+}
+
+__device__ __forceinline__ void tmem_ld(uint32_t taddr, uint32_t (&r)[16]) {
   asm volatile(
       "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15}, [%16];"
       : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]),
@@ -305,7 +338,7 @@ __device__ __forceinline__ void tmem_ld_wait() { asm volatile("tcgen05.wait::ld.
 // combined exactly in int64, in units of level S + 1 (32-bit conversions: the
 // conversion pipe, where a 64-bit one would take the FP64 pipe).
 template <int S>
-__device__ __forceinline__ long long oz_level_sum(const uint32_t (&acc)[S][16], int c) {
+__device__ __forceinline__ long long oz_level_sum(const uint32_t (&acc)[S][oz_ec(S)], int c) {
   long long v = 0;
 #pragma unroll
   for (int l = 0; l < S; l++) v += (long long)__float2int_rn(__uint_as_float(acc[l][c])) << (7 * (S - 1 - l));
@@ -317,7 +350,7 @@ __device__ __forceinline__ long long oz_level_sum(const uint32_t (&acc)[S][16], 
 // levels at least 2^28 apart and the rest, each exact in int64 and below
 // 2^53) converted exactly and added with one rounding.
 template <int S>
-__device__ __forceinline__ double oz_level_value(const uint32_t (&acc)[S][16], int c) {
+__device__ __forceinline__ double oz_level_value(const uint32_t (&acc)[S][oz_ec(S)], int c) {
   if constexpr (S <= 6) {
     return (double)oz_level_sum<S>(acc, c);
   } else {
@@ -521,9 +554,14 @@ __global__ void __launch_bounds__(oz_threads(S), 1) k_oz_mma(const OzTile *__res
   uint64_t *acc_empty = acc_full + 2;    // [2]
   uint32_t *tmem_slot = (uint32_t *)(acc_empty + 2);
   volatile int *abort_flag = (volatile int *)(tmem_slot + 1);
+  OzTile *srec = (OzTile *)(smem + STAGES * STAGE_BYTES + 256);
+  constexpr int REC_CAP = oz_rec_cap(S);
   int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   // this CTA's tiles (longest first, assigned on the host)
   const int t_begin = sched_off[blockIdx.x], t_end = sched_off[blockIdx.x + 1];
+  for (int i = threadIdx.x; i < min(t_end - t_begin, REC_CAP) * (kRecBytes / 16); i += oz_threads(S))
+    reinterpret_cast<uint4 *>(srec)[i] = __ldg(reinterpret_cast<const uint4 *>(tiles + t_begin) + i);
+  auto record = [&](int ti) -> const OzTile & { return ti - t_begin < REC_CAP ? srec[ti - t_begin] : tiles[ti]; };
 
   if (threadIdx.x == 0) {
     for (int s = 0; s < STAGES; s++) {
@@ -551,29 +589,30 @@ __global__ void __launch_bounds__(oz_threads(S), 1) k_oz_mma(const OzTile *__res
   const uint32_t tmem = *tmem_slot;
 
   if (warp == 0) {
-    if (lane == 0 && t_begin < t_end) {
+    if (lane == 0) {
       // producer: digit planes of A and B for every K step
       int stage = 0;
       uint32_t phase = 0;
-      OzTile next = tiles[t_begin];
       for (int ti = t_begin; ti < t_end && !*abort_flag; ti++) {
-        const OzTile P = next;
-        if (ti + 1 < t_end) next = tiles[ti + 1];
+        const OzTile &P = record(ti);
         if (act && !act[P.inst]) continue;
-        const CUtensorMap *amap = maps + P.map, *bmap = amap + 1;
+        const CUtensorMap *amap = maps + P.map + P.abox, *bmap = maps + P.map + kABoxes;
+        const uint32_t bytes = (uint32_t)(S * (oz_abox_groups(P.abox) * 256 + oz_b_slice_bytes(S)));
         for (int it = 0; it <= (P.flags & kTileTwoTerms); it++) {
           int ay = it ? P.ay[1] : P.ay[0], by = it ? P.by[1] : P.by[0];
           const int arg = it ? P.arg[1] : P.arg[0], brg = it ? P.brg[1] : P.brg[0];
-          for (int kk = 0; kk < P.ksteps; kk++) {  // the chunks only regroup these steps
+          const int ksteps = P.ksteps;
+          for (int kk = 0; kk < ksteps; kk++) {  // the chunks only regroup these steps
             if (!mbar_wait(&empty[stage], phase ^ 1, abort_flag)) {
               atomicExch(err, 1);
               *abort_flag = 1;
               break;
             }
             // two whole boxes: the row groups past the tile's operand rows
-            // (other rows of the buffer, or zeros past its end) only reach
-            // accumulator rows and columns that are never stored
-            mbar_expect_tx(&full[stage], STAGE_BYTES);
+            // (other rows of the buffer, zeros past its end, or what a longer
+            // box left in the stage) only reach accumulator rows and columns
+            // that are never stored
+            mbar_expect_tx(&full[stage], bytes);
             uint8_t *sa = smem + stage * STAGE_BYTES;
             uint8_t *sb = sa + S * A_SLICE_BYTES;
             tma_load_3d(sa, amap, ay, 0, &full[stage]);
@@ -590,84 +629,92 @@ __global__ void __launch_bounds__(oz_threads(S), 1) k_oz_mma(const OzTile *__res
       }
     }
   } else if (warp == 1) {
-    if (lane == 0 && t_begin < t_end) {
-      // MMA issuer: alternates between the two accumulator sets so the next
-      // tile's products overlap the epilogue of the previous one
-      int stage = 0, nt = 0;
-      uint32_t phase = 0;
-      const uint64_t desc0 = smem_desc(smem_u32(smem), 128, 256);
-      OzTile next = tiles[t_begin];
-      for (int ti = t_begin; ti < t_end && !*abort_flag; ti++) {
-        const OzTile P = next;
-        if (ti + 1 < t_end) next = tiles[ti + 1];
-        if (act && !act[P.inst]) continue;
-        const int nterms = 1 + (P.flags & kTileTwoTerms);
-        const int kchunk = CH ? P.kchunk : 0x40000000;
-        int left = 0;                      // steps left in the current chunk
-        int total = nterms * P.ksteps;     // steps left in the tile
-        uint32_t dbase = 0;
-        bool first = true;  // first K step of a chunk overwrites the accumulators
-        for (int it = 0; it < nterms && !*abort_flag; it++) {
-          const int f = P.flags >> (it * kTileTermShift);
-          const int neg = ((f & kTileNeg) != 0) ^ ((f & kTileHL) && hL < 0) ^ ((f & kTileHR) && hR < 0);
-          uint32_t idesc[S];  // A plane s: width (S - s) TN
-#pragma unroll
-          for (int s = 0; s < S; s++) idesc[s] = idesc_bf16(TM, (S - s) * TN, neg);
-          for (int kk = 0; kk < P.ksteps; kk++) {
-            if (left == 0) {  // a chunk starts: take the next accumulator set
-              const int buf = nt & 1;
-              const uint32_t use = (uint32_t)(nt >> 1);
-              nt++;
-              if (!mbar_wait(&acc_empty[buf], (use & 1) ^ 1, abort_flag)) {
-                atomicExch(err, 2);
-                *abort_flag = 1;
-                break;
-              }
-              tc_fence_after();
-              dbase = tmem + (uint32_t)(buf * ACC_BUF_COLS);
-              first = true;
-              left = kchunk;
-            }
-            if (!mbar_wait(&full[stage], phase, abort_flag)) {
-              atomicExch(err, 3);
-              *abort_flag = 1;
+    // MMA issuer: alternates between the two accumulator sets so the next
+    // tile's products overlap the epilogue of the previous one.  The whole warp
+    // walks the tiles and waits; one elected lane issues.  (With the walk inside
+    // `if (lane == 0)` a K step of five digits took about 670 cycles whatever its
+    // boxes, by clock64 stamps, the issue itself and not the tensor pipe setting
+    // the pace; now about 370 of the tensor pipe's 240: 37.5 -> 32.5 us for the
+    // launch at emax = 6.)
+    const bool leader = elect_one();
+    int stage = 0, nt = 0;
+    uint32_t phase = 0;
+    const uint32_t desc_lo = (uint32_t)smem_desc(smem_u32(smem), 128, 256);
+    const uint32_t desc_hi = (uint32_t)(smem_desc(smem_u32(smem), 128, 256) >> 32);
+    bool ok = true;
+    for (int ti = t_begin; ti < t_end && ok; ti++) {
+      const OzTile &P = record(ti);
+      if (act && !act[P.inst]) continue;
+      const uint32_t aplane = (uint32_t)(oz_abox_groups(P.abox) * 256 >> 4);  // descriptor units per A plane
+      const int ksteps = P.ksteps, flags = P.flags;
+      const int nterms = 1 + (flags & kTileTwoTerms);
+      const int kchunk = CH ? P.kchunk : 0x40000000;
+      int left = 0;                  // steps left in the current chunk
+      int total = nterms * ksteps;   // steps left in the tile
+      uint32_t dbase = 0;
+      bool first = true;  // first K step of a chunk overwrites the accumulators
+      for (int it = 0; it < nterms && ok; it++) {
+        const int f = flags >> (it * kTileTermShift);
+        const int neg = ((f & kTileNeg) != 0) ^ ((f & kTileHL) && hL < 0) ^ ((f & kTileHR) && hR < 0);
+        const uint32_t sign = (uint32_t)neg << 13;
+        for (int kk = 0; kk < ksteps; kk++) {
+          if (left == 0) {  // a chunk starts: take the next accumulator set
+            const int buf = nt & 1;
+            const uint32_t use = (uint32_t)(nt >> 1);
+            nt++;
+            ok = mbar_wait(&acc_empty[buf], (use & 1) ^ 1, abort_flag);
+            if (!ok) {
+              if (leader) atomicExch(err, 2);
               break;
             }
-            tc_fence_after();
-            // descriptor start-address fields advance in 16-byte units
-            const uint64_t da = desc0 + (uint64_t)((stage * STAGE_BYTES) >> 4);
-            const uint64_t db = da + (uint64_t)((S * A_SLICE_BYTES) >> 4);
-            // A plane s (0-based) times B planes 0 .. S - 1 - s (side by side
-            // in the stage) is one MMA into the accumulators of levels s + 2
-            // .. S + 1 (side by side in TMEM).  The first K step of a chunk
-            // overwrites: plane 0's MMA covers every accumulator.
+            dbase = tmem + (uint32_t)(buf * ACC_BUF_COLS);
+            first = true;
+            left = kchunk;
+          }
+          ok = mbar_wait(&full[stage], phase, abort_flag);
+          if (!ok) {
+            if (leader) atomicExch(err, 3);
+            break;
+          }
+          tc_fence_after();
+          // descriptor start-address fields advance in 16-byte units
+          const uint32_t da = desc_lo + (uint32_t)((stage * STAGE_BYTES) >> 4);
+          const uint32_t db = da + (uint32_t)((S * A_SLICE_BYTES) >> 4);
+          // A plane s (0-based) times B planes 0 .. S - 1 - s (side by side
+          // in the stage) is one MMA into the accumulators of levels s + 2
+          // .. S + 1 (side by side in TMEM).  The first K step of a chunk
+          // overwrites: plane 0's MMA covers every accumulator.
+          // a chunk ends with this step: its accumulator set goes to the epilogue
+          --left;
+          --total;
+          if (leader) {
 #pragma unroll
             for (int s = 0; s < S; s++)
-              mma_bf16(dbase + (uint32_t)(s * TN), da + (uint64_t)(s * (A_SLICE_BYTES >> 4)), db, idesc[s],
-                       (first && s == 0) ? 0 : 1);
-            first = false;
+              mma_bf16(dbase + (uint32_t)(s * TN), desc_of(da + s * aplane, desc_hi), desc_of(db, desc_hi),
+                       idesc_bf16(TM, (S - s) * TN, 0) | sign, (first && s == 0) ? 0 : 1);
             mma_commit(&empty[stage]);
-            if (++stage == STAGES) {
-              stage = 0;
-              phase ^= 1;
-            }
-            // a chunk ends: its accumulator set goes to the epilogue
-            --left;
-            --total;
             if (left == 0 || total == 0) mma_commit(&acc_full[(nt - 1) & 1]);
+          }
+          __syncwarp();
+          first = false;
+          if (++stage == STAGES) {
+            stage = 0;
+            phase ^= 1;
           }
         }
       }
     }
+    if (!ok && leader) *abort_flag = 1;
   } else {
     // epilogue warps 2..: TMEM lane quadrant = warp % 4 (the lanes a warp
-    // may read), 16-column chunk = (warp - 2) / 4
+    // may read), column chunk = (warp - 2) / 4
     const int quad = warp & 3, chunk = (warp - 2) >> 2;
-    const int row = quad * 32 + lane, n0 = 16 * chunk;
+    const int row = quad * 32 + lane;
+    constexpr int EC = oz_ec(S);
+    const int n0 = EC * chunk;
     int nt = 0;
     for (int ti = t_begin; ti < t_end; ti++) {
-      const OzTile &P = tiles[ti];
-      if (ti + 1 < t_end) prefetch_l1(&tiles[ti + 1].ksteps);  // its registers are better spent on the accumulators
+      const OzTile &P = record(ti);
       if (act && !act[P.inst]) continue;  // an instance whose series has stopped: its outputs stay
       const int Mp = P.rows, Np = P.cols, ldc = P.ldc;
       const int nch = CH ? P.nchunks : 1, raw = P.flags & kTileRaw;
@@ -690,12 +737,11 @@ __global__ void __launch_bounds__(oz_threads(S), 1) k_oz_mma(const OzTile *__res
           break;
         }
         tc_fence_after();
-        uint32_t acc[S][16];
+        uint32_t acc[S][EC];
         if (live) {
 #pragma unroll
           for (int l = 0; l < S; l++)
-            tmem_ld16(tmem + ((uint32_t)(quad * 32) << 16) + (uint32_t)(buf * ACC_BUF_COLS + l * TN + 16 * chunk),
-                      acc[l]);
+            tmem_ld(tmem + ((uint32_t)(quad * 32) << 16) + (uint32_t)(buf * ACC_BUF_COLS + l * TN + n0), acc[l]);
         }
         tmem_ld_wait();
         // the accumulators are in registers: hand the TMEM set back to the MMA issuer
@@ -709,10 +755,11 @@ __global__ void __launch_bounds__(oz_threads(S), 1) k_oz_mma(const OzTile *__res
 #define OZ_LEVEL_SUM(c) oz_level_sum<S>(acc, c)
         if (nch == 1 && !raw) {
 #pragma unroll
-          for (int c = 0; c < 16; c++) {
-            const double d = oz_scale(oz_level_value<S>(acc, c), k);
+          for (int c = 0; c < EC; c++) {
             const int n = n0 + c;
-            if (row_ok && n < Np) crow[(long)n * ldc] = d;
+            if (n >= Np) break;  // warp-uniform: thin products convert only their own columns
+            const double d = oz_scale(oz_level_value<S>(acc, c), k);
+            if (row_ok) crow[(long)n * ldc] = d;
           }
           continue;
         }
@@ -720,32 +767,34 @@ __global__ void __launch_bounds__(oz_threads(S), 1) k_oz_mma(const OzTile *__res
           // a long contraction at seven or eight digits adds its chunks in
           // FP64 in the output's own slots, then scales once
 #pragma unroll
-          for (int c = 0; c < 16; c++) {
-            double v = oz_level_value<S>(acc, c);
+          for (int c = 0; c < EC; c++) {
             const int n = n0 + c;
-            if (row_ok && n < Np) {
+            if (n >= Np) break;
+            double v = oz_level_value<S>(acc, c);
+            if (row_ok) {
               if (ch > 0) v += crow[(long)n * ldc];
               crow[(long)n * ldc] = v;
             }
           }
           if (ch < nch - 1 || !row_ok) continue;
-          for (int c = 0; c < 16 && n0 + c < Np; c++) crow[(long)(n0 + c) * ldc] = oz_scale(crow[(long)(n0 + c) * ldc], k);
+          for (int c = 0; c < EC && n0 + c < Np; c++) crow[(long)(n0 + c) * ldc] = oz_scale(crow[(long)(n0 + c) * ldc], k);
         } else {
           // WCC keeps the exact level sum as an integer (the 222_ph recoupling
           // combines four entries of one block, which share 2^k, before its one
           // conversion to FP64); a long contraction adds its chunks there
 #pragma unroll
-          for (int c = 0; c < 16; c++) {
-            long long v = OZ_LEVEL_SUM(c);
+          for (int c = 0; c < EC; c++) {
             const int n = n0 + c;
-            if (row_ok && n < Np) {
+            if (n >= Np) break;
+            long long v = OZ_LEVEL_SUM(c);
+            if (row_ok) {
               if (ch > 0) v += irow[(long)n * ldc];
               irow[(long)n * ldc] = v;
             }
           }
           if (raw || ch < nch - 1 || !row_ok) continue;
           // the last chunk of a long FP64 contraction: convert the summed integers
-          for (int c = 0; c < 16 && n0 + c < Np; c++)
+          for (int c = 0; c < EC && n0 + c < Np; c++)
             crow[(long)(n0 + c) * ldc] = oz_scale((double)irow[(long)(n0 + c) * ldc], k);
         }
 #undef OZ_LEVEL_SUM
@@ -779,7 +828,11 @@ void launch_mma(int S, bool chunked, int grid, cudaStream_t st, const OzTile *ti
 
 // CTA schedule: longest-processing-time-first assignment of tiles to the
 // persistent CTAs under the cost model cost = kw * (K steps x terms) + ew *
-// (live outputs / 64) + base.
+// (live outputs / 64) + base.  A CTA runs its tiles shortest first: the
+// epilogues of the short tiles, which cost more than their products, then
+// overlap the products that follow instead of queueing at the end (emax = 6,
+// five digits: 26.0 us, longest first 27.4, long and short in turn 26.6; eight
+// digits 59, 65, 64).
 void build_sched(const OzPlan *pl, const SchedModel &md, std::vector<OzTile> &sched, std::vector<int> &sched_off) {
   const int tiles = (int)pl->tiles.size();
   std::vector<long> cost(tiles);
@@ -799,7 +852,7 @@ void build_sched(const OzPlan *pl, const SchedModel &md, std::vector<OzTile> &sc
   sched_off.assign(pl->grid + 1, 0);
   for (int c = 0; c < pl->grid; c++) {
     sched_off[c] = (int)sched.size();
-    for (int t : lists[c]) sched.push_back(pl->tiles[t]);
+    for (size_t i = lists[c].size(); i-- > 0;) sched.push_back(pl->tiles[lists[c][i]]);
   }
   sched_off[pl->grid] = (int)sched.size();
 }
@@ -991,9 +1044,9 @@ int ozaki_prepare(imsrg_basis *b) {
     pl->img = (uint8_t *)p;
   }
 
-  // TMA maps of the image buffer, S planes of 256-byte core-matrix rows: an A
-  // box is 16 row groups (128 rows) of every plane, a B box TN / 8.  The
-  // encoder is the driver's cuTensorMapEncodeTiled, reached through the runtime.
+  // TMA maps of the image buffer, S planes of 256-byte core-matrix rows: the A
+  // boxes are 2 to 16 row groups (16 to 128 rows) of every plane, the B box TN /
+  // 8.  The encoder is the driver's cuTensorMapEncodeTiled, reached through the runtime.
   static PFN_cuTensorMapEncodeTiled_v12000 encode = nullptr;
   if (!encode) {
     void *fn = nullptr;
@@ -1004,12 +1057,12 @@ int ozaki_prepare(imsrg_basis *b) {
       return IMSRG_ERR_CUDA;
     encode = (PFN_cuTensorMapEncodeTiled_v12000)fn;
   }
-  for (int brole = 0; brole < 2; brole++) {
+  for (int m = 0; m < kMaps; m++) {
     const cuuint64_t gdim[3] = {32, (cuuint64_t)pl->units, (cuuint64_t)pl->S};
     const cuuint64_t gstride[2] = {256, (cuuint64_t)pl->units * 256};
-    const cuuint32_t box[3] = {32, (cuuint32_t)(brole ? oz_tn(pl->S) / 8 : TM / 8), (cuuint32_t)pl->S};
+    const cuuint32_t box[3] = {32, (cuuint32_t)(m == kABoxes ? oz_tn(pl->S) / 8 : oz_abox_groups(m)), (cuuint32_t)pl->S};
     const cuuint32_t estride[3] = {1, 1, 1};
-    if (encode(&pl->maps[brole], CU_TENSOR_MAP_DATA_TYPE_UINT64, 3, (void *)pl->img, gdim, gstride, box, estride,
+    if (encode(&pl->maps[m], CU_TENSOR_MAP_DATA_TYPE_UINT64, 3, (void *)pl->img, gdim, gstride, box, estride,
                CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
                CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) != CUDA_SUCCESS)
       return IMSRG_ERR_INVALID;
@@ -1060,6 +1113,7 @@ int ozaki_prepare(imsrg_basis *b) {
           q.by[it] += n0 / 8;
         }
         q.rows = gp.M - m0;
+        while (q.abox < kABoxes - 1 && 8 * oz_abox_groups(q.abox) < std::min(TM, q.rows)) q.abox++;
         q.cols = gp.N - n0;
         q.C = dst + gp.c_off + m0 + (long)n0 * gp.ldc;
         tile_ksteps.push_back(steps);
@@ -1284,7 +1338,7 @@ int ozaki_batch_create(imsrg_basis *const *bases, int n, void **out) {
       all.tile_ksteps.push_back(pl->tile_ksteps[k]);
       all.tile_live.push_back(pl->tile_live[k]);
     }
-    maps.insert(maps.end(), pl->maps, pl->maps + 2);
+    maps.insert(maps.end(), pl->maps, pl->maps + kMaps);
     bt->ngroups += pl->ngroups;
     // the bases' own tuned cost model when they agree, else the one usually chosen
     const int m = pl->tuned ? pl->tune_choice : 1;

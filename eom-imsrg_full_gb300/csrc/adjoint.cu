@@ -133,13 +133,13 @@ __device__ __forceinline__ double adj_tb(const double *__restrict__ Cb, long e, 
 }
 
 // CTAs [0, n0): W1bar, W2bar = -W1bar and the 122 weights U, by flat index;
-// [n0, n1): Zbar; [n1, n2): LCC; the rest zero WCCbar, RCCbar and Ybar's E0 and
-// one-body part.
+// [n0, n1): Zbar; [n1, n2): LCC; the rest zero RCCbar and Ybar's E0 and one-body
+// part.
 __global__ void __launch_bounds__(ADJ_THREADS) k_adj_prep(DevTables T, AdjLists A, const double *__restrict__ X,
                                                           int hL, int hR, const double *__restrict__ Cb, int hRES,
                                                           long off_2b, int n0, int n1, int n2, double *W1b,
                                                           double *W2b, double *U, double *Zb, double *LCC,
-                                                          double *WCCb, double *RCCb, double *Yb) {
+                                                          double *RCCb, double *Yb) {
   const int nres = hRES < 0;
   int blk = blockIdx.x;
   if (blk < n0) {
@@ -172,8 +172,9 @@ __global__ void __launch_bounds__(ADJ_THREADS) k_adj_prep(DevTables T, AdjLists 
       const int nd = (H.meta >> 18) & 3;
       double s = adj_tb(Cb, H.e, H.em, (H.meta >> 21) & 1, nres);
       if (nd) s = s * (nd == 1 ? .70710678118 : .70710678118 * .70710678118);
+      const bool shared = (H.meta >> 23) & 1;  // the outside channel reads the inside Z
       if (k < q.w) z = fma(dflip(s, (H.meta >> 16) & 1), T.six[H.six1 + k], z);
-      else z = fma(s, T.six[H.six2 + k - q.w], z);
+      if (shared || k >= q.w) z = fma(dflip(s, (H.meta >> 24) & 1), T.six[H.six2 + (shared ? k : k - q.w)], z);
     }
     Zb[t] = z;
     return;
@@ -191,35 +192,56 @@ __global__ void __launch_bounds__(ADJ_THREADS) k_adj_prep(DevTables T, AdjLists 
     LCC[e] = s;
     return;
   }
-  const long z0 = (long)(blk - n2) * ADJ_ZERO, nz = T.wcc_total + T.cc_total + off_2b;
+  const long z0 = (long)(blk - n2) * ADJ_ZERO, nz = T.cc_total + off_2b;
   for (long i = z0 + threadIdx.x; i < min(z0 + ADJ_ZERO, nz); i += ADJ_THREADS) {
-    if (i < T.wcc_total) WCCb[i] = 0.0;
-    else if (i < T.wcc_total + T.cc_total) RCCb[i - T.wcc_total] = 0.0;
-    else Yb[i - T.wcc_total - T.cc_total] = 0.0;
+    if (i < T.cc_total) RCCb[i] = 0.0;
+    else Yb[i - T.cc_total] = 0.0;
   }
 }
 
-// Recoupling inputs^T: Z = herm_L (W(x1,y1) + e W(x2,y2)) - herm_R (e W(y2,x2) + W(y1,x1))
+// Recoupling inputs^T, a quarter of a patch of a block's (x, y) plane
+// (k_ph_patches): every entry of WCCbar belongs to one (x, y) of the patches, as
+// W(x,y), W(y',x'), W(x',y') or W(y,x), or as several of them at once, so the
+// patches write the whole plane, zeros included, without atomics.
 __device__ __forceinline__ void adj_ph(const DevTables &T, const double *__restrict__ Zb, int hL, int hR, double *WCCb,
-                                       long t) {
-  if (t >= T.n_ph) return;
-  const double z = Zb[t];
-  if (z == 0.0) return;
-  const PhTerm p = T.ph_terms[t];
-  const unsigned long long u = p.rows;
-  const unsigned x1 = (unsigned)(u & 0xFFFF), y1 = (unsigned)((u >> 16) & 0xFFFF);
-  const unsigned x2 = (unsigned)((u >> 32) & 0xFFFF), y2 = (unsigned)(u >> 48);
-  const int q1 = p.q & 0xFFFF, q2 = p.q >> 16, rl = T.cc_rlen[q1];
-  double *W = WCCb + T.wcc_off[q1], *W2 = WCCb + T.wcc_off[q2];  // the two blocks have one size
-  const double a = dflip(z, hL < 0), c = -dflip(z, hR < 0);
-  if (x1 != 0xFFFFu && y1 != 0xFFFFu) {
-    atomicAdd(W + x1 + (long)y1 * rl, a);
-    atomicAdd(W + y1 + (long)x1 * rl, c);
+                                       int quarter) {
+  const PhPatch &p = T.ph_patch[quarter >> 2];
+  const int lane = threadIdx.x & 31, ty = (threadIdx.x >> 5) + (quarter & 3) * 8, rl = p.rlen;
+  const int x = p.x0 + lane, y = p.y0 + ty;
+  // only the form that the patches hold
+  if (x >= p.half || y >= rl || (y >= p.half ? y - p.half : y) < x) return;
+  double *W = WCCb + p.w, *V = WCCb + p.v;
+  const bool one = p.w == p.v;
+  const unsigned char *ph = T.cc_rowph + p.row0;
+  const int nph = __ldg(ph + x) ^ __ldg(ph + y), xr = ph_rev(p, x), yr = ph_rev(p, y);
+  double z = 0.0;
+  for (int l = 0; l < p.layers; l++) {
+    const unsigned u = __ldg(T.ph_slots + ((long)p.table + l) * 1024 + ty * 32 + lane);
+    if ((u & kPhSlot) != kPhNone) z += dflip(Zb[u & kPhSlot], ((u & kPhFlip) != 0) ^ ((u & kPhSwap) && hL * hR > 0));
   }
-  if (x2 != 0xFFFFu && y2 != 0xFFFFu) {
-    atomicAdd(W2 + x2 + (long)y2 * rl, dflip(a, p.nph));
-    atomicAdd(W2 + y2 + (long)x2 * rl, dflip(c, p.nph));
+  const double c1 = dflip(z, hL < 0), c4 = -dflip(z, hR < 0);  // W(x, y), W(y, x)
+  const double c2 = dflip(c1, nph), c3 = dflip(c4, nph);       // W(y', x'), W(x', y')
+  double v1 = c1, v2 = c2, v3 = c3, v4 = c4;
+  if (x == y) {
+    v1 += c4;
+    v4 = v1;
+    v2 += c3;
+    v3 = v2;
   }
+  if (one && x == yr) {
+    const double t1 = v1 + v2, t3 = v3 + v4;
+    v1 = v2 = t1;
+    v3 = v4 = t3;
+  }
+  if (one && x == xr && y == yr && x != y) {
+    const double t1 = v1 + v3, t2 = v2 + v4;
+    v1 = v3 = t1;
+    v2 = v4 = t2;
+  }
+  W[x + (long)y * rl] = v1;
+  V[xr + (long)yr * rl] = v3;
+  V[yr + (long)xr * rl] = v2;
+  W[y + (long)x * rl] = v4;
 }
 
 // CTAs [0, n0): the partial sum of one chunk of a one-body target's list;
@@ -267,7 +289,7 @@ __global__ void __launch_bounds__(ADJ_THREADS) k_adj_122(DevTables T, AdjLists A
     Yb[vi] = s;
     return;
   }
-  adj_ph(T, Zb, hL, hR, WCCb, (long)(blk - n1) * ADJ_THREADS + threadIdx.x);
+  adj_ph(T, Zb, hL, hR, WCCb, blk - n1);
 }
 
 // ---------------------------------------------------------------------------
@@ -605,7 +627,7 @@ int adj_lists(imsrg_basis *b, AdjState *a) {
   std::vector<int4> quad;
   std::vector<int> zquad(T.n_ph, 0);
   for (size_t h = 0; h < qhead.size(); h++) {
-    const int n_in = (qhead[h].meta >> 5) & 31, n_out = (qhead[h].meta >> 10) & 31;
+    const int n_in = (qhead[h].meta >> 5) & 31, n_out = (qhead[h].meta >> 23) & 1 ? 0 : (qhead[h].meta >> 10) & 31;
     if (h == 0 || qhead[h].zs != qhead[h - 1].zs) {
       quad.push_back(make_int4((int)h, 0, qhead[h].zs, n_in));
       for (int k = 0; k < n_in + n_out; k++) zquad[qhead[h].zs + k] = (int)quad.size() - 1;
@@ -740,12 +762,12 @@ int commutator_adjoint_dev(imsrg_basis *b, const double *X, int hX, const double
   {
     const int n0 = ctas(b->nfull - b->off_2b, ADJ_THREADS), n1 = n0 + ctas(T.n_ph, ADJ_THREADS),
               n2 = n1 + ctas(b->cc_total, ADJ_THREADS),
-              n3 = n2 + ctas(b->wcc_total + b->cc_total + b->off_2b, ADJ_ZERO);
+              n3 = n2 + ctas(b->cc_total + b->off_2b, ADJ_ZERO);
     k_adj_prep<<<n3, ADJ_THREADS, 0, st>>>(T, A, X, hL, hR, Cb, hRES, b->off_2b, n0, n1, n2, a->w1b, a->w2b, a->u,
-                                            a->zb, b->lcc, a->wccb, a->rccb, Yb);
+                                            a->zb, b->lcc, a->rccb, Yb);
   }
   {
-    const int n0 = A.n_f_chunks, n1 = n0 + ctas(A.n_v_warps, ADJ_THREADS / 32), n2 = n1 + ctas(T.n_ph, ADJ_THREADS);
+    const int n0 = A.n_f_chunks, n1 = n0 + ctas(A.n_v_warps, ADJ_THREADS / 32), n2 = n1 + 4 * T.n_ph_patches;
     if (n2) k_adj_122<<<n2, ADJ_THREADS, 0, st>>>(T, A, X, hL, hR, a->u, a->zb, n0, n1, a->fpart, a->wccb, Yb);
   }
   {

@@ -270,6 +270,7 @@ int build_basis(imsrg_basis *b) {
   b->wcc_off.assign(b->ccblocks, 0);
   // block of the pairs (i, j) with tz_j - tz_i = 2 d in the reference's block q1
   std::vector<int> cc_sub((size_t)ccref * 3, -1);
+  std::vector<int> cc_half(b->ccblocks, 0);  // first reversed pair of a Tz = 0 block
   std::vector<int> cc_row((size_t)b->ccblocks * N * N, -1);
   std::vector<int> cc_rowpair, cc_rowstart(b->ccblocks), cc_colpair, cc_colstart(b->ccblocks);
   long coff = 0, woff = 0;
@@ -295,6 +296,7 @@ int build_basis(imsrg_basis *b) {
       if (TZ == 0) {
         add_rows(1, false);
         add_rows(0, false);
+        cc_half[qs] = (int)rows.size();
         add_rows(1, true);
       } else {
         add_rows(2, d < 0);
@@ -525,7 +527,7 @@ int build_basis(imsrg_basis *b) {
   };
 
   // --- two-body assembly: work order, gather lists and the recoupling inputs
-  // shared by the elements of one orbit quadruple (see Asm2Head, PhTerm)
+  // shared by the elements of one orbit quadruple (see Asm2Head, PhPatch)
   {
     auto jpcount = [&](int lo, int hi) { return hi >= lo ? (hi - lo) / 2 + 1 : 0; };
     static const int c1tab[6] = {0, 0, 0, 1, 2, 1}, c2tab[6] = {0, 1, 2, 1, 2, 2};
@@ -568,7 +570,14 @@ int build_basis(imsrg_basis *b) {
           }
       }
     std::vector<Asm2Head> heads;
-    std::vector<PhTerm> zt;
+    // recoupling inputs: (block, x, y) in canonical form and their place in Z
+    struct ZTerm {
+      int block, x, y;
+      unsigned slot;
+    };
+    std::vector<ZTerm> zt;
+    std::vector<PhTerm> zl;
+    bool rows_ok = true;
     std::vector<unsigned long long> terms;
     std::vector<std::pair<long, int>> items;      // (signature, head)
     std::vector<std::pair<long, int>> items_out;  // (output range << 40 | signature, head)
@@ -582,7 +591,40 @@ int build_basis(imsrg_basis *b) {
       }
       b->asm2_addr[kOutChunks] = b->nfull;
     }
-    auto row16 = [](int r) -> unsigned long long { return r < 0 ? 0xFFFFull : (unsigned long long)r; };
+    // Of the four forms of Z(x1, y1) (see PhPatch) the one in the first block of a
+    // pair, with x no reversed pair and before y
+    auto ph_term = [&](int q1, int q2, int x1, int y1, int x2, int y2, int nph, int slot) {
+      if (x1 < 0 || y1 < 0 || x2 < 0 || y2 < 0) rows_ok = false;
+      bool bar = false, swap = false;
+      if (q1 == q2) {
+        const int half = cc_half[q1];
+        auto base = [&](int r) { return r >= half ? r - half : r; };
+        if (base(x1) > base(y1)) {
+          std::swap(x1, y1);
+          std::swap(x2, y2);
+          swap = true;
+        }
+        if (x1 >= half) {  // (x, y) -> (x', y')
+          x1 = y2;
+          y1 = x2;
+          bar = true;
+          swap = !swap;
+        }
+      } else {
+        if (q1 > q2) {
+          q1 = q2;
+          x1 = x2;
+          y1 = y2;
+          bar = true;
+        }
+        if (x1 > y1) {
+          std::swap(x1, y1);
+          swap = true;
+        }
+      }
+      zt.push_back({q1, x1, y1, (unsigned)slot | (bar && nph ? kPhFlip : 0u) | (swap ? kPhSwap : 0u)});
+    };
+    int n_z = 0;
     for (unsigned long long key : qorder) {
       const std::vector<El> &els = qmap[key];
       const int g = (int)(key & 7);
@@ -596,7 +638,10 @@ int build_basis(imsrg_basis *b) {
       const bool valid = std::abs(b->itzp[l] - b->itzp[j]) == Tz1 * 2 && ((b->ll[l] + b->ll[j]) & 1) == PAR1 &&
                          std::abs(b->itzp[k] - b->itzp[j]) == Tz2 * 2 && ((b->ll[k] + b->ll[j]) & 1) == PAR2;
       const int nph = ((ji + jjv + jk + jl) >> 1) & 1;
-      const int zs = (int)zt.size();
+      const int zs = n_z;
+      // with identical orbits the two channels' inputs are the same ones (x, y) or,
+      // for i == j, the reversed pairs (y', x'), which gives a factor e
+      const bool one_channel = i == j || k == l;
       const int jmin1 = std::max(std::abs(jjv - jl), std::abs(ji - jk)), jmax1 = std::min(jjv + jl, ji + jk);
       const int jmin2 = std::max(std::abs(ji - jl), std::abs(jjv - jk)), jmax2 = std::min(ji + jl, jjv + jk);
       int n_in = 0, n_out = 0;
@@ -606,14 +651,17 @@ int build_basis(imsrg_basis *b) {
         auto add_ph = [&](int q1, int u, int v) {
           const int d = (b->itzp[i] - b->itzp[u]) / 2;
           const int qx = cc_sub[(size_t)q1 * 3 + 1 + d], q2 = cc_sub[(size_t)q1 * 3 + 1 - d];
-          zt.push_back({row16(ccr(qx, u, i)) | (row16(ccr(qx, j, v)) << 16) | (row16(ccr(q2, v, j)) << 32) |
-                            (row16(ccr(q2, i, u)) << 48),
-                        qx | (q2 << 16), nph});
+          const int x1 = ccr(qx, u, i), y1 = ccr(qx, j, v), x2 = ccr(q2, v, j), y2 = ccr(q2, i, u);
+          const long o1 = b->wcc_off[qx], o2 = b->wcc_off[q2], rl = b->cc_rlen[qx];
+          auto at = [](long k, int bits) { return ((unsigned)k & 0x0FFFFFFFu) | (unsigned)(bits & 15) << 28; };
+          zl.push_back(make_uint4(at(o1 + x1 + y1 * rl, nph), at(o2 + x2 + y2 * rl, q1), at(o2 + y2 + x2 * rl, q1 >> 4),
+                                  at(o1 + y1 + x1 * rl, q1 >> 8)));
+          ph_term(qx, q2, x1, y1, x2, y2, nph, n_z++);
         };
         for (int JP = jmin1; JP <= jmax1; JP += 2, n_in++)
           add_ph(JP / 2 + Tz1 * (JTM + 1) + 2 * PAR1 * (JTM + 1), k, l);
         for (int JP = jmin2; JP <= jmax2; JP += 2, n_out++)
-          add_ph(JP / 2 + Tz2 * (JTM + 1) + 2 * PAR2 * (JTM + 1), l, k);
+          if (!one_channel) add_ph(JP / 2 + Tz2 * (JTM + 1) + 2 * PAR2 * (JTM + 1), l, k);
       }
       const int nd = (i == j) + (k == l);
       for (const El &el : els) {
@@ -659,7 +707,8 @@ int build_basis(imsrg_basis *b) {
         const int n2par = (((jl + jk + J2) >> 1) + 1) & 1;
         h.meta = (unsigned)n122 | ((unsigned)n_in << 5) | ((unsigned)n_out << 10) | ((unsigned)valid << 15) |
                  ((unsigned)n2par << 16) | ((unsigned)nd << 18) | ((unsigned)(sq[g] && el.IX == el.JX) << 20) |
-                 ((unsigned)sq[g] << 21) | ((unsigned)(g == 2) << 22);
+                 ((unsigned)sq[g] << 21) | ((unsigned)(g == 2) << 22) | ((unsigned)one_channel << 23) |
+                 ((unsigned)(i == j && k != l && nph) << 24);
         // warps run elements of one loop-trip signature; in the order by
         // output range, within the range of the element's lower write
         const long lo = el.em >= 0 ? std::min(el.e, el.em) : el.e;
@@ -689,7 +738,10 @@ int build_basis(imsrg_basis *b) {
                                        [](const std::pair<long, int> &x, long key) { return x.first < key; }) -
                       items_out.begin();
     T.n_asm2 = (int)ordered.size();
-    T.n_ph = (int)zt.size();
+    if (!rows_ok || (long)n_z >= (long)kPhNone) return rows_ok ? IMSRG_ERR_TOO_LARGE : IMSRG_ERR_INVALID;
+    T.n_ph = n_z;
+    T.ph_terms = nullptr;
+    if (T.n_asm2 <= kPhList && b->wcc_total < (1L << 28) && b->ccgroups < 4096) IMSRG_TRY(dev_upload(b, zl, &T.ph_terms));
     {  // the commutator_122 sums by term count, 32 elements to a warp (see DevTables::pre_warp)
       std::vector<std::vector<int>> by_n(32);
       for (size_t h = 0; h < heads.size(); h++) by_n[heads[h].meta & 31].push_back((int)h);
@@ -720,7 +772,49 @@ int build_basis(imsrg_basis *b) {
     IMSRG_TRY(dev_upload(b, ordered, &T.asm2_head));
     IMSRG_TRY(dev_upload(b, ordered_out, &T.asm2_head_out));
     IMSRG_TRY(dev_upload(b, terms, &T.asm2_terms));
-    IMSRG_TRY(dev_upload(b, zt, &T.ph_terms));
+    {  // the dense patches: every canonical (x, y), so that the adjoint can write the whole plane
+      std::vector<PhPatch> patches;
+      std::map<std::pair<int, std::pair<int, int>>, int> patch_of;  // (block, (y, x) in patches)
+      for (int q1 = 0; q1 < b->ccgroups; q1++) {
+        const int *sub = &cc_sub[(size_t)q1 * 3];  // isospin differences -1, 0, 1
+        const bool tz0 = sub[1] >= 0;
+        const int q = tz0 ? sub[1] : sub[2], pair = tz0 ? sub[1] : sub[0];
+        const int r = b->cc_rlen[q], half = tz0 ? cc_half[q] : r;
+        if (b->cc_rlen[pair] != r) return IMSRG_ERR_INVALID;
+        for (int y0 = 0; y0 < r; y0 += 32)
+          for (int x0 = 0; x0 < half; x0 += 32) {
+            bool any = false;  // some row's pair, in either order, not before x0
+            for (int y = y0; y < std::min(y0 + 32, r); y++) any = any || (y >= half ? y - half : y) >= x0;
+            if (!any) continue;
+            patch_of[{q, {y0 / 32, x0 / 32}}] = (int)patches.size();
+            PhPatch p{b->wcc_off[q], b->wcc_off[pair], r, r - half, half, cc_rowstart[q], q1, x0, y0, 0, 0, {0, 0, 0}};
+            patches.push_back(p);
+          }
+      }
+      std::vector<std::vector<std::vector<unsigned>>> tables(patches.size());
+      for (const ZTerm &z : zt) {
+        auto it = patch_of.find({z.block, {z.y / 32, z.x / 32}});
+        if (it == patch_of.end()) return IMSRG_ERR_INVALID;
+        std::vector<std::vector<unsigned>> &ls = tables[it->second];
+        const int at = (z.y & 31) * 32 + (z.x & 31);
+        size_t l = 0;
+        while (l < ls.size() && ls[l][at] != kPhNone) l++;
+        if (l == ls.size()) ls.push_back(std::vector<unsigned>(1024, kPhNone));
+        ls[l][at] = z.slot;
+      }
+      std::vector<unsigned> slots;
+      for (size_t k = 0; k < patches.size(); k++) {
+        patches[k].table = (int)(slots.size() / 1024);
+        patches[k].layers = (int)tables[k].size();
+        for (const std::vector<unsigned> &l : tables[k]) slots.insert(slots.end(), l.begin(), l.end());
+      }
+      std::vector<unsigned char> rowph;
+      for (int rp : cc_rowpair) rowph.push_back(((b->jj[rp >> 16] + b->jj[rp & 0xffff]) >> 1) & 1);
+      T.n_ph_patches = (int)patches.size();
+      IMSRG_TRY(dev_upload(b, patches, &T.ph_patch));
+      IMSRG_TRY(dev_upload(b, slots, &T.ph_slots));
+      IMSRG_TRY(dev_upload(b, rowph, &T.cc_rowph));
+    }
     IMSRG_TRY(dev_upload(b, vsq, &T.vsq));
 
     std::vector<std::pair<long, int>> cit;

@@ -114,6 +114,11 @@ __device__ __forceinline__ double sixj_w(const DevTables &T, int j1, int j2, int
   return T.six_w[sixj_index(T, j1, j2, J3, j4, j5, J6)];
 }
 
+// the reversed pair's row in the block of the reversed pairs
+__device__ __forceinline__ int ph_rev(const PhPatch &B, int r) {
+  return r < B.n_u ? r + B.half : r < B.half ? r : r - B.half;
+}
+
 __device__ __forceinline__ double warp_sum(double v) {
 #pragma unroll
   for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);

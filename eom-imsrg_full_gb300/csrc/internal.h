@@ -52,8 +52,8 @@ struct DevTables {
   // Two-body elements (upper triangles only): asm2_head[w] is the w-th
   // element of the work order, its commutator_122 terms asm2_terms[head.start
   // ..]; the 222_ph recoupling inputs Z (one per orbit quadruple, channel and
-  // J', shared by the quadruple's elements of every J) come from the ph_terms
-  // list (see Asm2Head, PhTerm).  asm2_head_out holds the same heads grouped
+  // J', shared by the quadruple's elements of every J) are formed patch by patch
+  // (see Asm2Head, PhPatch).  asm2_head_out holds the same heads grouped
   // by output range first (imsrg_basis::asm2_el), for copies of RES to the
   // host that run beside the assembly.
   const struct Asm2Head *asm2_head, *asm2_head_out;
@@ -63,8 +63,12 @@ struct DevTables {
   const unsigned char *vsq;
   const unsigned long long *asm2_terms;
   int n_asm2;
-  const struct PhTerm *ph_terms;
-  int n_ph;
+  int n_ph;                // recoupling inputs Z
+  const struct PhPatch *ph_patch;
+  const unsigned *ph_slots;
+  const uint4 *ph_terms;   // PhTerm, small bases (kPhList), else null
+  const unsigned char *cc_rowph;  // per cross-coupled row (a, b): (ja + jb) / 2 odd
+  int n_ph_patches;
   // The commutator_122 sums again, for the kernel that runs them ahead of the
   // products (k_asm2_122): warp g takes elements pre_el[32 g .. 32 g + 32),
   // all with pre_warp[g].n122 terms; term k of its lane l is
@@ -116,21 +120,33 @@ struct __align__(16) Asm2PreWarp {
   int pad;
 };
 
-// One J'-term of the inverse Pandya recoupling of commutator_222_ph
-// (commutators.f90:855-910) for an orbit quadruple (a,b,c,d) and one exchange
-// channel: the kernel forms
-//   Z = herm_L (W(x1,y1) + e W(x2,y2)) - herm_R (e W(y2,x2) + W(y1,x1))
-// from four cross-coupled rows (16 bits each in `rows`: x1, y1, x2, y2;
-// 0xFFFF = absent), x1 and y1 of WCC block q & 0xFFFF, x2 and y2 of block
-// q >> 16 (the same block at equal isospins, its pair otherwise), e =
-// (-1)^((ja+jb+jc+jd)/2).  The
+// The recoupling inputs of commutator_222_ph (commutators.f90:855-910): for an
+// orbit quadruple (a,b,c,d), an exchange channel and J',
+//   Z = herm_L (W(x,y) + e W(y',x')) - herm_R (e W(x',y') + W(y,x))
+// with x, y two rows of one WCC block, x', y' the reversed pairs (in the same
+// block at equal isospins, else in its pair) and e = (-1)^((ja+jb+jc+jd)/2).  The
 // reference's four products per J' become sum_J' {6j} Z(J') per element, with
-// the inside channel's (-1)^n2(J) applied after the sum.
-struct __align__(16) PhTerm {
-  unsigned long long rows;
-  int q;
-  int nph;  // the exponent of e
+// the inside channel's (-1)^n2(J) applied after the sum.  Z(x,y) = e Z(y',x') =
+// -herm_L herm_R Z(y,x), and those forms read the same four entries, so the
+// inputs of a block are one dense part of its (x,y) plane: PhPatch is a 32 x 32
+// patch of it, whose entries name the places in Z (if any) that take them.
+struct __align__(16) PhPatch {
+  long w, v;        // offsets of the block's W and of the one with the reversed pairs
+  int rlen;
+  int n_u, half;    // rows [0, n_u) reversed are [half, ..), rows [n_u, half) their own reversals
+  int row0;         // the block's first row in DevTables::cc_rowph
+  int group;        // its exponent group (imsrg_basis::cc_group)
+  int x0, y0;
+  int layers;       // tables of 1024 slot entries, entry 32 (y - y0) + (x - x0); the first at ph_slots[1024 table]
+  int table, pad[3];
 };
+// The same input by its place in Z, for small bases (kPhList): the places of
+// W(x,y), W(y',x'), W(x',y') and W(y,x) in WCC (28 bits each; no block table to
+// look up first), the exponent of e in bit 28 of the first and the exponent
+// group in bits 28-31 of the other three, low bits first.
+using PhTerm = uint4;
+constexpr unsigned kPhNone = 0x3FFFFFFFu, kPhSlot = 0x3FFFFFFFu;  // slot entry: place in Z,
+constexpr unsigned kPhFlip = 1u << 30, kPhSwap = 1u << 31;        // its sign, and that of -herm_L herm_R
 
 // One two-body element of the assembly kernel with its operator-independent
 // gather list, resolved once per basis on the host: n122 commutator_122
@@ -139,8 +155,9 @@ struct __align__(16) PhTerm {
 // sign (leg sign x pair-reordering phase), bits 49-50 number of sqrt(2)
 // factors, bit 51 V read transposed, bit 52 f read transposed (each transposed
 // read takes the operator's herm).  Its recoupling reads Z[zs .. zs + n_in)
-// (inside channel) and Z[zs + n_in .. + n_out) (outside) against consecutive
-// 6j-table entries from six1 and six2.
+// (inside channel) and Z[zs + n_in .. + n_out) (outside; the inside ones again
+// where a == b or c == d makes the channels one) against consecutive 6j-table
+// entries from six1 and six2.
 struct __align__(16) Asm2Head {
   int e;       // flat index of the element
   int em;      // flat index of its mirror (JX, IX) in a square array, else -1 (== e on the diagonal)
@@ -150,7 +167,7 @@ struct __align__(16) Asm2Head {
   int six2;
   unsigned meta;  // bits 0-4 n122, 5-9 n_in, 10-14 n_out, 15 recoupling applies,
                   // 16 inside phase n2, 18-19 identical orbit pairs, 20 diagonal,
-                  // 21 square array, 22 pphh array
+                  // 21 square array, 22 pphh array, 23 outside channel reads the inside Z, 24 times -1
   int J2;
 };
 
@@ -397,6 +414,13 @@ int launch_gemm_fp64_merged(const GemmMerged &g, int hL, int hR, const int *act,
 // [w0, w1) of the signature work order or of the order by output range, on
 // top of launch_asm2_122's part in RES
 int launch_ph_inputs(imsrg_basis *b, int hL, int hR, int precision);
+// Bases of at most this many two-body elements form the recoupling inputs one
+// thread per input, in the order of Z, larger ones patch by patch.  The line:
+// below it the inputs' latency counts and few patches fill the GPU badly, above
+// it the four WCC reads of an input (per input against patches: emax 2 / 4 FP64
+// commutators 19.1 / 39.7 us against 20.1 / 41.0, emax 5 / 6 split 52.8 / 115.0
+// against 47.3 / 111.5).
+constexpr long kPhList = 65536;
 // commutator_122 part of every two-body element into RES on stream st (the
 // assembly after the products adds the rest)
 int launch_asm2_122(imsrg_basis *b, const double *L, int hL, const double *R, int hR, double *RES, int hRES,
@@ -462,10 +486,10 @@ int ozaki_check_error(imsrg_basis *b);  // IMSRG_ERR_TIMEOUT if a bounded device
 int synchronize_checked(imsrg_basis *b);
 bool ozaki_tuned(imsrg_basis *b);       // the CTA schedule has been autotuned
 // After a split-precision product WCC holds exact int64 level sums v with
-// WCC = v 2^k, k = (exps[g.x] - 1022) + (exps[g.y] - 1022) - kshift for the
-// groups g = ccgroups[q1] of cross-coupled block q1 (kshift = 7 (S + 1) for S
-// digits: 49 with six, 42 with five).
-int ozaki_wcc_scale(imsrg_basis *b, const int **exps, const int2 **ccgroups, int *kshift);
+// WCC = v 2^k, k = (exps[gL + g] - 1022) + (exps[gR + g] - 1022) - kshift for the
+// group g of the cross-coupled block (kshift = 7 (S + 1) for S digits: 49 with
+// six, 42 with five).
+int ozaki_wcc_scale(imsrg_basis *b, const int **exps, int *gL, int *gR, int *kshift);
 int ozaki_schedule_info(imsrg_basis *b, int *choice, int *ncand, double *us, int max);
 int ozaki_set_schedule(imsrg_basis *b, int model);  // pin one cost model, no timing
 void ozaki_free(imsrg_basis *b);

@@ -103,60 +103,82 @@ __global__ void __launch_bounds__(GT_THREADS, GT_CTAS) k_gemm_fp64(const GemmPro
 // ---------------------------------------------------------------------------
 // 3. Two-body assembly from the per-element gather lists (see Asm2Head).
 // ---------------------------------------------------------------------------
-// Cross-coupled W(r, c) of one WCC block, zero where a row is absent (not
-// reached for number-conserving blocks; the guard keeps the read in bounds).
-__device__ __forceinline__ double wcc_at(const double *W, int rlen, unsigned r, unsigned c) {
-  if (r == 0xFFFFu || c == 0xFFFFu) return 0.0;
-  return W[r + (long)c * rlen];
+// Z from its four entries (see PhPatch): FP64, or the split engine's exact int64
+// level sums (WCC = v 2^k), combined exactly before one conversion.
+template <bool INT>
+__device__ __forceinline__ double ph_combine(double w1, double w2, double w3, double w4, int nph, int hL, int hR,
+                                             int k) {
+  if (!INT) {
+    const double a = w1 + dflip(w2, nph), c = dflip(w3, nph) + w4;
+    return dflip(a, hL < 0) - dflip(c, hR < 0);
+  }
+  const long long i2 = __double_as_longlong(w2), i3 = __double_as_longlong(w3);
+  const long long a = __double_as_longlong(w1) + (nph ? -i2 : i2);
+  const long long c = (nph ? -i3 : i3) + __double_as_longlong(w4);
+  const long long z = (hL < 0 ? -a : a) - (hR < 0 ? -c : c);
+  // z 2^k: add k to the exponent field on the integer pipe when the result
+  // stays normal (exactly ldexp's value), else ldexp
+  double d = (double)z;
+  unsigned long long bits = (unsigned long long)__double_as_longlong(d);
+  const int E = (int)((bits >> 52) & 0x7FF);
+  if (E != 0 && E + k > 0 && E + k < 2047) {
+    bits += (unsigned long long)(long long)k << 52;
+    d = __longlong_as_double((long long)bits);
+  } else if (E != 0) {
+    d = ldexp(d, k);
+  }
+  return d;
 }
 
-__device__ __forceinline__ long long wcc_at_int(const long long *W, int rlen, unsigned r, unsigned c) {
-  if (r == 0xFFFFu || c == 0xFFFFu) return 0;
-  return W[r + (long)c * rlen];
+// Recoupling inputs Z of commutator_222_ph, large bases: four CTAs per 32 x 32
+// patch of a block's (x, y) plane, an input per thread (see PhPatch).  W(x, y)
+// and W(x', y') are read along their columns; W(y, x) and W(y', x') across
+// theirs, the CTA's eight rows sharing sectors; each value goes to its place in
+// Z.  What bounds it: the latency of the reads, now independent of one another
+// once the patch is known, and then their sectors (3.5 million at emax = 6
+// against 6.3 million of one thread per input in the order of Z).
+template <bool INT>
+__global__ void __launch_bounds__(256) k_ph_patches(DevTables T, const double *__restrict__ WCC, int hL, int hR,
+                                                    const int *__restrict__ exps, int gL, int gR, int kshift,
+                                                    double *__restrict__ Z) {
+  const PhPatch &p = T.ph_patch[blockIdx.x >> 2];
+  const int layers = p.layers;
+  if (layers == 0) return;
+  const int lane = threadIdx.x & 31, ty = (threadIdx.x >> 5) + (blockIdx.x & 3) * 8, rl = p.rlen;
+  const double *W = WCC + p.w, *V = WCC + p.v;
+  const unsigned *slots = T.ph_slots + (long)p.table * 1024 + ty * 32 + lane;
+  const unsigned char *ph = T.cc_rowph + p.row0;
+  const int x = p.x0 + lane, y = p.y0 + ty;
+  if (x >= rl || y >= rl) return;
+  const int xr = ph_rev(p, x), yr = ph_rev(p, y);
+  unsigned u = __ldg(slots);
+  const double w1 = W[x + (long)y * rl], w2 = V[yr + (long)xr * rl], w3 = V[xr + (long)yr * rl],
+               w4 = W[y + (long)x * rl];
+  const int nph = __ldg(ph + x) ^ __ldg(ph + y);
+  const int k = INT ? (exps[gL + p.group] - 1022) + (exps[gR + p.group] - 1022) - kshift : 0;
+  const double d = ph_combine<INT>(w1, w2, w3, w4, nph, hL, hR, k);
+  for (int l = 0;;) {
+    if ((u & kPhSlot) != kPhNone) Z[u & kPhSlot] = dflip(d, ((u & kPhFlip) != 0) ^ ((u & kPhSwap) && hL * hR > 0));
+    if (++l == layers) break;
+    u = __ldg(slots + l * 1024);
+  }
 }
 
-// Recoupling inputs Z of commutator_222_ph, one thread per PhTerm.  With
-// exps == nullptr WCC holds FP64 (the FP64 path); otherwise it holds the
-// split engine's exact int64 level sums, WCC = v 2^k per cross-coupled block
-// (k = both block exponents - kshift, kshift = 7 x the highest level kept),
-// and the four entries are combined exactly in int64 before one conversion.
-__global__ void __launch_bounds__(256) k_ph_inputs(DevTables T, const double *__restrict__ WCC, int hL, int hR,
-                                                   const int *__restrict__ exps, const int2 *__restrict__ ccg,
-                                                   int kshift, double *__restrict__ Z) {
-  const long t = (long)blockIdx.x * blockDim.x + threadIdx.x;
+// The same for small bases, one thread per input in the order of Z.
+template <bool INT>
+__global__ void __launch_bounds__(256) k_ph_list(DevTables T, const double *__restrict__ WCC, int hL, int hR,
+                                                 const int *__restrict__ exps, int gL, int gR, int kshift,
+                                                 double *__restrict__ Z) {
+  const int t = blockIdx.x * blockDim.x + threadIdx.x;
   if (t >= T.n_ph) return;
   const PhTerm p = T.ph_terms[t];
-  const unsigned long long u = p.rows;
-  const unsigned x1 = (unsigned)(u & 0xFFFF), y1 = (unsigned)((u >> 16) & 0xFFFF);
-  const unsigned x2 = (unsigned)((u >> 32) & 0xFFFF), y2 = (unsigned)(u >> 48);
-  const int q1 = p.q & 0xFFFF, q2 = p.q >> 16, rl = T.cc_rlen[q1];  // both blocks have one size and scale
-  if (exps) {
-    const long long *W = reinterpret_cast<const long long *>(WCC) + T.wcc_off[q1];
-    const long long *V = reinterpret_cast<const long long *>(WCC) + T.wcc_off[q2];
-    const long long w2 = wcc_at_int(V, rl, x2, y2), w3 = wcc_at_int(V, rl, y2, x2);
-    const long long a = wcc_at_int(W, rl, x1, y1) + (p.nph ? -w2 : w2);
-    const long long c = (p.nph ? -w3 : w3) + wcc_at_int(W, rl, y1, x1);
-    const long long z = (hL < 0 ? -a : a) - (hR < 0 ? -c : c);
-    const int2 g = ccg[q1];
-    const int k = (exps[g.x] - 1022) + (exps[g.y] - 1022) - kshift;
-    // z 2^k: add k to the exponent field on the integer pipe when the result
-    // stays normal (exactly ldexp's value), else ldexp
-    double d = (double)z;
-    unsigned long long bits = (unsigned long long)__double_as_longlong(d);
-    const int E = (int)((bits >> 52) & 0x7FF);
-    if (E != 0 && E + k > 0 && E + k < 2047) {
-      bits += (unsigned long long)(long long)k << 52;
-      d = __longlong_as_double((long long)bits);
-    } else if (E != 0) {
-      d = ldexp(d, k);
-    }
-    Z[t] = d;
-    return;
+  const unsigned m = 0x0FFFFFFFu;
+  int k = 0;
+  if (INT) {
+    const int g = p.y >> 28 | (p.z >> 28) << 4 | (p.w >> 28) << 8;
+    k = (exps[gL + g] - 1022) + (exps[gR + g] - 1022) - kshift;
   }
-  const double *W = WCC + T.wcc_off[q1], *V = WCC + T.wcc_off[q2];
-  const double a = wcc_at(W, rl, x1, y1) + dflip(wcc_at(V, rl, x2, y2), p.nph);
-  const double c = dflip(wcc_at(V, rl, y2, x2), p.nph) + wcc_at(W, rl, y1, x1);
-  Z[t] = dflip(a, hL < 0) - dflip(c, hR < 0);
+  Z[t] = ph_combine<INT>(WCC[p.x & m], WCC[p.y & m], WCC[p.z & m], WCC[p.w & m], (p.x >> 28) & 1, hL, hR, k);
 }
 
 // E0 = commutator_110 + commutator_220 (commutators.f90:10-33, 399-432) by one
@@ -292,10 +314,11 @@ __global__ void __launch_bounds__(ASM2_THREADS) k_assemble_2body(DevTables T, co
     if ((meta >> 15) & 1) {
       const int n_in = (meta >> 5) & 31, n_out = (meta >> 10) & 31;
       const double *z = Z + h.zs, *s1 = T.six + h.six1, *s2 = T.six + h.six2;
+      const double *zo = (meta >> 23) & 1 ? z : z + n_in;
       double a1 = 0.0, a2 = 0.0;
       for (int k = 0; k < n_in; k++) a1 = fma(s1[k], z[k], a1);
-      for (int k = 0; k < n_out; k++) a2 = fma(s2[k], z[n_in + k], a2);
-      double sm = dflip(a1, (meta >> 16) & 1) + a2;
+      for (int k = 0; k < n_out; k++) a2 = fma(s2[k], zo[k], a2);
+      double sm = dflip(a1, (meta >> 16) & 1) + dflip(a2, (meta >> 24) & 1);
       // the reference's truncated 1/sqrt(2) literal for identical orbits
       if (nd) sm = sm * (nd == 1 ? .70710678118 : .70710678118 * .70710678118);
       t = t + sm;
@@ -602,17 +625,26 @@ int launch_gemm_fp64_merged(const GemmMerged &g, int hL, int hR, const int *act,
   return cuda_status(cudaGetLastError());
 }
 
+// exps == nullptr: WCC holds FP64 (the FP64 path and the split engine's FP64
+// class), else the split engine's int64 level sums
+static int ph_inputs(imsrg_basis *b, const double *WCC, int hL, int hR, const int *exps, int gL, int gR, int kshift,
+                     double *Z, cudaStream_t st) {
+  if (b->T.n_ph == 0) return IMSRG_OK;
+  if (b->T.ph_terms)
+    (exps ? k_ph_list<true> : k_ph_list<false>)<<<(b->T.n_ph + 255) / 256, 256, 0, st>>>(b->T, WCC, hL, hR, exps, gL,
+                                                                                         gR, kshift, Z);
+  else
+    (exps ? k_ph_patches<true> : k_ph_patches<false>)<<<4 * b->T.n_ph_patches, 256, 0, st>>>(b->T, WCC, hL, hR, exps,
+                                                                                            gL, gR, kshift, Z);
+  b->launches++;
+  return cuda_status(cudaGetLastError());
+}
+
 int launch_ph_inputs(imsrg_basis *b, int hL, int hR, int precision) {
   const int *exps = nullptr;
-  const int2 *ccg = nullptr;
-  int kshift = 0;
-  if (precision == IMSRG_PREC_OZAKI) IMSRG_TRY(ozaki_wcc_scale(b, &exps, &ccg, &kshift));
-  if (b->T.n_ph > 0) {
-    k_ph_inputs<<<(unsigned)((b->T.n_ph + 255) / 256), 256, 0, b->stream>>>(b->T, b->wcc, hL, hR, exps, ccg,
-                                                                            kshift, b->zph);
-    b->launches++;
-  }
-  return cuda_status(cudaGetLastError());
+  int gL = 0, gR = 0, kshift = 0;
+  if (precision == IMSRG_PREC_OZAKI) IMSRG_TRY(ozaki_wcc_scale(b, &exps, &gL, &gR, &kshift));
+  return ph_inputs(b, b->wcc, hL, hR, exps, gL, gR, kshift, b->zph, b->stream);
 }
 
 int launch_asm2_range(imsrg_basis *b, const double *L, int hL, const double *R, int hR, double *RES, int hRES,
@@ -681,11 +713,7 @@ int launch_commutator_fp64_ws(imsrg_basis *b, const Workspace &ws, const double 
     k_gemm_fp64<false><<<b->ntiles, GT_THREADS, 0, st>>>(b->d_probs, b->d_tiles, ops, hL, hR, nullptr);
     b->launches++;
   }
-  if (b->T.n_ph > 0) {
-    k_ph_inputs<<<(unsigned)((b->T.n_ph + 255) / 256), 256, 0, st>>>(b->T, ws.wcc, hL, hR, nullptr, nullptr,
-                                                                       0, ws.zph);
-    b->launches++;
-  }
+  IMSRG_TRY(ph_inputs(b, ws.wcc, hL, hR, nullptr, 0, 0, 0, ws.zph, st));
   const long n2 = b->T.n_asm2;
   if (n2 > 0) {
     const int has220 = with_e0 && hL * hR == -1;
@@ -708,7 +736,8 @@ int launch_commutator_fp64_ws(imsrg_basis *b, const Workspace &ws, const double 
 
 int preload_commutator_fp64_ws() {
   cudaFuncAttributes a;
-  const void *fns[] = {(const void *)k_cc_forward<3>, (const void *)k_gemm_fp64<false>, (const void *)k_ph_inputs,
+  const void *fns[] = {(const void *)k_cc_forward<3>, (const void *)k_gemm_fp64<false>, (const void *)k_ph_list<false>,
+                       (const void *)k_ph_patches<false>,
                        (const void *)k_assemble_2body<false>, (const void *)k_assemble_1body, (const void *)k_energy};
   for (const void *f : fns) {
     cudaError_t e = cudaFuncGetAttributes(&a, f);

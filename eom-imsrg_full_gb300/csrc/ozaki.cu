@@ -202,7 +202,6 @@ struct OzPlan {
   // k owns [x_lo[k], x_lo[k + 1]).
   int group_lo[4] = {0, 0, 0, 0}, chunk_lo[4] = {0, 0, 0, 0}, linec_lo[4] = {0, 0, 0, 0}, liner_lo[4] = {0, 0, 0, 0};
   uint16_t *d_mat_c = nullptr, *d_mat_r = nullptr;  // matrix of each C / R image line
-  int2 *d_ccgroups = nullptr;  // [ccblocks]: exponent groups of LCC and RCC block q1
   int grid = 0;
   int tune_choice = 0;                   // the schedule model the autotuner kept
   double tune_us[kNumSchedModels] = {};  // its timings of each model
@@ -1141,10 +1140,6 @@ int ozaki_prepare(imsrg_basis *b) {
   IMSRG_TRY(up(mat_r.data(), mat_r.size() * sizeof(uint16_t), (void **)&pl->d_mat_r));
   // (cudaMalloc memory is 256-byte aligned: the 64-byte alignment of a tensor map holds)
   IMSRG_TRY(up(pl->maps, sizeof(pl->maps), (void **)&pl->d_maps));
-  std::vector<int2> ccg(b->ccblocks);
-  for (int q1 = 0; q1 < b->ccblocks; q1++)
-    ccg[q1] = make_int2(pl->group_lo[2] + b->cc_group[q1], pl->group_lo[2] + b->ccgroups + b->cc_group[q1]);
-  IMSRG_TRY(up(ccg.data(), ccg.size() * sizeof(int2), (void **)&pl->d_ccgroups));
   IMSRG_CUDA_TRY(cudaMalloc((void **)&pl->d_exps, std::max(pl->ngroups, 1) * sizeof(int)));
   IMSRG_CUDA_TRY(cudaMalloc((void **)&pl->d_err, sizeof(int)));
   IMSRG_CUDA_TRY(cudaMemset(pl->d_err, 0, sizeof(int)));
@@ -1241,12 +1236,13 @@ int synchronize_checked(imsrg_basis *b) {
   return IMSRG_OK;
 }
 
-int ozaki_wcc_scale(imsrg_basis *b, const int **exps, const int2 **ccgroups, int *kshift) {
+int ozaki_wcc_scale(imsrg_basis *b, const int **exps, int *gL, int *gR, int *kshift) {
   OzPlan *pl = plan_of(b);
   if (!pl || !pl->ok) return IMSRG_ERR_INVALID;
   // FP64-class digit counts store WCC as FP64: the recoupling inputs read it so
   *exps = oz_fp64_class(pl->S) ? nullptr : pl->d_exps;
-  *ccgroups = pl->d_ccgroups;
+  *gL = pl->group_lo[2];
+  *gR = pl->group_lo[2] + b->ccgroups;
   *kshift = 7 * (pl->S + 1);
   return IMSRG_OK;
 }
@@ -1406,7 +1402,6 @@ void ozaki_free(imsrg_basis *b) {
   cudaFree(pl->d_sched_off);
   cudaFree(pl->d_mat_c);
   cudaFree(pl->d_mat_r);
-  cudaFree(pl->d_ccgroups);
   cudaFree(pl->d_exps);
   cudaFree(pl->d_maps);
   cudaFree(pl->d_err);

@@ -1,6 +1,7 @@
 """The |Tz| = 1 cross-coupled blocks as two independent ones (proton-neutron
 and neutron-proton pairs), with different hole shells for the two isospins so
-that the halves have different column counts, one of them none at all.
+that the halves have different column counts, one of them none at all; emax = 5
+forms its recoupling inputs patch by patch, the others one by one.
 
 Tolerances: the FP64 bar max |gpu - oracle| <= 1e-10 max |oracle|; six digits
 truncate each product at 2^-42 K max|A| max|B| (K <= 200 here, operands up to
@@ -14,7 +15,7 @@ from conftest import rel_err
 pytestmark = pytest.mark.gpu
 
 
-@pytest.mark.parametrize("emax,protons,neutrons", [(2, 1, 0), (2, 0, 1), (3, 1, 2), (3, 2, 1), (4, 2, 0)])
+@pytest.mark.parametrize("emax,protons,neutrons", [(2, 1, 0), (2, 0, 1), (3, 1, 2), (3, 2, 1), (4, 2, 0), (5, 1, 2)])
 def test_unequal_hole_shells(gpu_lib, oracle_mod, emax, protons, neutrons):
     from imsrg_gpu.layout import Layout, ho_basis
     from imsrg_gpu.synth import random_operator

@@ -742,28 +742,44 @@ int build_basis(imsrg_basis *b) {
     T.n_ph = n_z;
     T.ph_terms = nullptr;
     if (T.n_asm2 <= kPhList && b->wcc_total < (1L << 28) && b->ccgroups < 4096) IMSRG_TRY(dev_upload(b, zl, &T.ph_terms));
-    {  // the commutator_122 sums by term count, 32 elements to a warp (see DevTables::pre_warp)
-      std::vector<std::vector<int>> by_n(32);
-      for (size_t h = 0; h < heads.size(); h++) by_n[heads[h].meta & 31].push_back((int)h);
+    {  // the commutator_122 sums, 32 elements to a warp (see DevTables::pre_warp)
+      // The lanes of a warp have the same term count and the same terms with a
+      // sqrt(2) factor, whose two FP64 multiplications a warp pays for one lane as
+      // for all (emax = 6, alone: 28 us for the sums, 33 grouped by count), longest
+      // first, then in storage order.
+      std::vector<std::pair<unsigned long long, int>> order;
+      for (size_t h = 0; h < heads.size(); h++) {
+        const int n = heads[h].meta & 31;
+        unsigned long long mask = 0;
+        for (int k = 0; k < n; k++) mask |= (unsigned long long)((terms[(size_t)heads[h].start + k] >> 49) & 3 ? 1 : 0) << k;
+        order.push_back({(unsigned long long)(31 - n) << 32 | mask, (int)h});
+      }
+      std::sort(order.begin(), order.end(), [&](const std::pair<unsigned long long, int> &x,
+                                                const std::pair<unsigned long long, int> &y) {
+        return x.first != y.first ? x.first < y.first : heads[x.second].e < heads[y.second].e;
+      });
       std::vector<Asm2PreWarp> pw;
       std::vector<unsigned> pe;
       std::vector<unsigned long long> pt;
-      for (int n = 0; n < 32; n++)
-        for (size_t g0 = 0; g0 < by_n[n].size(); g0 += 32) {
-          Asm2PreWarp w{(long long)pt.size(), n, 0};
-          pw.push_back(w);
-          pt.resize(pt.size() + (size_t)32 * n, 0ull);
-          for (int l = 0; l < 32; l++) {
-            if (g0 + l >= by_n[n].size()) {
-              pe.push_back(0xFFFFFFFFu);
-              continue;
-            }
-            const Asm2Head &h = heads[by_n[n][g0 + l]];
-            const unsigned nd = (h.meta >> 18) & 3, diag = (h.meta >> 20) & 1;
-            pe.push_back((unsigned)h.e | nd << 28 | diag << 30);
-            for (int k = 0; k < n; k++) pt[(size_t)w.base + (size_t)32 * k + l] = terms[(size_t)h.start + k];
+      for (size_t g0 = 0; g0 < order.size();) {
+        size_t g1 = g0;
+        while (g1 < order.size() && g1 < g0 + 32 && order[g1].first == order[g0].first) g1++;
+        const int n = 31 - (int)(order[g0].first >> 32);
+        Asm2PreWarp w{(long long)pt.size(), n, 0};
+        pw.push_back(w);
+        pt.resize(pt.size() + (size_t)32 * n, 0ull);
+        for (int l = 0; l < 32; l++) {
+          if (g0 + l >= g1) {
+            pe.push_back(0xFFFFFFFFu);
+            continue;
           }
+          const Asm2Head &h = heads[order[g0 + l].second];
+          const unsigned nd = (h.meta >> 18) & 3, diag = (h.meta >> 20) & 1;
+          pe.push_back((unsigned)h.e | nd << 28 | diag << 30);
+          for (int k = 0; k < n; k++) pt[(size_t)w.base + (size_t)32 * k + l] = terms[(size_t)h.start + k];
         }
+        g0 = g1;
+      }
       T.n_pre_warps = (int)pw.size();
       IMSRG_TRY(dev_upload(b, pw, &T.pre_warp));
       IMSRG_TRY(dev_upload(b, pe, &T.pre_el));

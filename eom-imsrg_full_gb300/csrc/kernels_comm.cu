@@ -230,19 +230,23 @@ template <int STRIDE>
 __device__ __forceinline__ double sum122(const unsigned long long *tm, int n122, const double *L, int nL,
                                          const double *R, int nR) {
   double t = 0.0;
+  unsigned long long next = n122 > 0 ? tm[0] : 0;
   for (int k = 0; k < n122; k++) {
-    const unsigned long long u = tm[k * STRIDE];
+    const unsigned long long u = next;
+    if (k + 1 < n122) next = tm[(k + 1) * STRIDE];
     const long vi = (long)(u & 0xFFFFFFFull), fi = (long)((u >> 28) & 0xFFFFFull);
     const int sg = (int)(u >> 48) & 1, nsq = (int)(u >> 49) & 3, tr = (int)(u >> 51) & 1, ftr = (int)(u >> 52) & 1;
-    double vR = dflip(R[vi], tr & nR), vL = dflip(L[vi], tr & nL);
+    // the term's four gathers, and the next term, before the branch
+    double vR = R[vi], vL = L[vi], fL = L[fi], fR = R[fi];
+    vR = dflip(vR, tr & nR);
+    vL = dflip(vL, tr & nL);
     if (nsq) {
       const double c = nsq == 1 ? IMSRG_SQRT2 : 2.0000000000000004;
       vR = vR * c;
       vL = vL * c;
     }
-    const double fL = dflip(L[fi], (ftr & nL) ^ sg), fR = dflip(R[fi], (ftr & nR) ^ sg ^ 1);
-    t = fma(fL, vR, t);
-    t = fma(fR, vL, t);
+    t = fma(dflip(fL, (ftr & nL) ^ sg), vR, t);
+    t = fma(dflip(fR, (ftr & nR) ^ sg ^ 1), vL, t);
   }
   return t;
 }
@@ -255,22 +259,28 @@ __device__ __forceinline__ double sum122(const unsigned long long *tm, int n122,
 // The arithmetic is the assembly's own, so RES is bit-identical either way.
 // (Packing the sqrt(2)-scaled (L, R) pairs first, for one 16-byte gather per
 // term, measured slower here: the pack kernel took more of the shared front
-// than it saved.)
+// than it saved.)  What bounds it: the FP64 pipe (two FMAs a term) and its
+// gathers.  It has time until the products are done, so half of the SMs' warp
+// slots are enough and the kernels before the products find the other half free:
+// with a CTA per four groups it took every slot first (emax = 6, five digits:
+// 112.4 us per commutator, 109.5 with eight CTAs per SM, 111.5 with six or
+// twelve; host call 203 -> 194, two flow steps 3440 -> 3250, FP64 493 -> 487).
+constexpr int kPreCtas = 8;
 __global__ void __launch_bounds__(ASM2_THREADS) k_asm2_122(DevTables T, const double *__restrict__ L, int hL,
                                                            const double *__restrict__ R, int hR, int hRES,
                                                            double *RES) {
-  const int g = (int)(((long)blockIdx.x * blockDim.x + threadIdx.x) >> 5), lane = threadIdx.x & 31;
-  if (g >= T.n_pre_warps) return;
-  const unsigned pe = T.pre_el[(long)g * 32 + lane];
-  if (pe >> 31) return;  // padding
-  const Asm2PreWarp W = T.pre_warp[g];
-  const unsigned long long *tm = T.pre_terms + W.base + lane;
-  const int nL = hL < 0, nR = hR < 0;
-  double t = sum122<32>(tm, W.n122, L, nL, R, nR);
-  const int nd = (pe >> 28) & 3;
-  if (nd) t = t * (nd == 1 ? 0.7071067811865476 : 0.5);
-  if ((pe >> 30) & 1) t = dflip(t, hRES < 0);
-  RES[pe & 0x0FFFFFFFu] = t;
+  const int lane = threadIdx.x & 31;
+  for (int g = (int)(((long)blockIdx.x * blockDim.x + threadIdx.x) >> 5); g < T.n_pre_warps;
+       g += (int)(gridDim.x * blockDim.x >> 5)) {
+    const unsigned pe = T.pre_el[(long)g * 32 + lane];
+    if (pe >> 31) continue;  // padding
+    const Asm2PreWarp W = T.pre_warp[g];
+    double t = sum122<32>(T.pre_terms + W.base + lane, W.n122, L, hL < 0, R, hR < 0);
+    const int nd = (pe >> 28) & 3;
+    if (nd) t = t * (nd == 1 ? 0.7071067811865476 : 0.5);
+    if ((pe >> 30) & 1) t = dflip(t, hRES < 0);
+    RES[pe & 0x0FFFFFFFu] = t;
+  }
 }
 
 // Every two-body element of RES once (upper triangles of square arrays, the
@@ -663,7 +673,8 @@ int launch_asm2_122(imsrg_basis *b, const double *L, int hL, const double *R, in
                     cudaStream_t st) {
   if (b->T.n_pre_warps == 0) return IMSRG_OK;
   ProfScope ps(b, IMSRG_KERNEL_ASSEMBLE_2BODY, st);
-  const unsigned grid = (unsigned)(((long)b->T.n_pre_warps * 32 + ASM2_THREADS - 1) / ASM2_THREADS);
+  const unsigned grid = (unsigned)std::min(((long)b->T.n_pre_warps * 32 + ASM2_THREADS - 1) / ASM2_THREADS,
+                                           (long)kPreCtas * b->num_sms);
   k_asm2_122<<<grid, ASM2_THREADS, 0, st>>>(b->T, L, hL, R, hR, hRES, RES);
   b->launches++;
   return cuda_status(cudaGetLastError());

@@ -22,7 +22,7 @@
 //      1190-1300): RCCbar back to Ybar.
 // The adjoint with respect to X follows from antisymmetry, [X, Y] = -[Y, X]:
 //     d<Cbar, [X, Y]> / dX = -(the adjoint above with the roles swapped).
-// The one-body, recoupling and Pandya lists become scatters, added with FP64
+// The one-body and Pandya lists become scatters, added with FP64
 // atomics: the adjoint's results agree run to run to rounding, not bit for bit
 // (the forward commutator stays atomic-free and bit-reproducible).
 //
@@ -104,6 +104,13 @@ __global__ void __launch_bounds__(GT_THREADS, GT_CTAS) k_gemm_adj(const AdjProb 
 // and 15 us with the recoupling inputs^T in it, which took 23 and 5).  Work
 // that depends on the same inputs shares a launch, by CTA range: five launches
 // instead of seven and six memsets (emax = 4: 119 -> 63 us, emax = 6: 850 -> 567).
+// The particle-hole part (Zbar, LCC, WCCbar, then RCCbar's product) and the rest
+// (weights, 122 sums, one-body assembly^T, then the ladder products) meet only in
+// the Pandya transform^T, so they run on two streams, each with its share of the
+// first two kernels' CTA ranges: 63.5 -> 53.5 us at emax = 4, where the chain of
+// launches is the time, and 560 -> 548 at emax = 6, where both halves want the
+// FP64 pipe (a high-priority second stream 557, three product CTAs per SM beside
+// it 552).
 // ---------------------------------------------------------------------------
 
 // Gather lists of the transposed sums (host-built from the forward's).
@@ -132,19 +139,23 @@ __device__ __forceinline__ double adj_tb(const double *__restrict__ Cb, long e, 
   return e == em ? dflip(Cb[e], nres) : Cb[e] + dflip(Cb[em], nres);
 }
 
-// CTAs [0, n0): W1bar, W2bar = -W1bar and the 122 weights U, by flat index;
-// [n0, n1): Zbar; [n1, n2): LCC; the rest zero RCCbar and Ybar's E0 and one-body
-// part.
+// CTAs (from `first` on) [0, n0): W1bar, W2bar = -W1bar and the 122 weights U, by
+// flat index, and zeros to Ybar's E0 and one-body part; [n0, n1): Zbar; [n1, n2):
+// LCC; the rest zero RCCbar.
 __global__ void __launch_bounds__(ADJ_THREADS) k_adj_prep(DevTables T, AdjLists A, const double *__restrict__ X,
                                                           int hL, int hR, const double *__restrict__ Cb, int hRES,
-                                                          long off_2b, int n0, int n1, int n2, double *W1b,
-                                                          double *W2b, double *U, double *Zb, double *LCC,
-                                                          double *RCCb, double *Yb) {
+                                                          long off_2b, int first, int n0, int n1, int n2,
+                                                          double *W1b, double *W2b, double *U, double *Zb,
+                                                          double *LCC, double *RCCb, double *Yb) {
   const int nres = hRES < 0;
-  int blk = blockIdx.x;
+  const int blk = blockIdx.x + first;
   if (blk < n0) {
-    const long i = off_2b + (long)blk * ADJ_THREADS + threadIdx.x;
+    const long i = (long)blk * ADJ_THREADS + threadIdx.x;
     if (i >= T.nfull) return;
+    if (i < off_2b) {
+      Yb[i] = 0.0;
+      return;
+    }
     const int m = A.mir[i - off_2b];
     const long p = m & 0x0FFFFFFF;
     const bool upper = (m >> 28) & 1, diag = (m >> 29) & 1, square = (m >> 30) & 1;
@@ -192,11 +203,8 @@ __global__ void __launch_bounds__(ADJ_THREADS) k_adj_prep(DevTables T, AdjLists 
     LCC[e] = s;
     return;
   }
-  const long z0 = (long)(blk - n2) * ADJ_ZERO, nz = T.cc_total + off_2b;
-  for (long i = z0 + threadIdx.x; i < min(z0 + ADJ_ZERO, nz); i += ADJ_THREADS) {
-    if (i < T.cc_total) RCCb[i] = 0.0;
-    else Yb[i - T.cc_total] = 0.0;
-  }
+  const long z0 = (long)(blk - n2) * ADJ_ZERO;
+  for (long i = z0 + threadIdx.x; i < min(z0 + ADJ_ZERO, (long)T.cc_total); i += ADJ_THREADS) RCCb[i] = 0.0;
 }
 
 // Recoupling inputs^T, a quarter of a patch of a block's (x, y) plane
@@ -244,16 +252,16 @@ __device__ __forceinline__ void adj_ph(const DevTables &T, const double *__restr
   W[y + (long)x * rl] = v4;
 }
 
-// CTAs [0, n0): the partial sum of one chunk of a one-body target's list;
-// [n0, n1): two-body targets, a warp per 32 (sets Ybar there); the rest: the
+// CTAs (from `first` on) [0, n0): the partial sum of one chunk of a one-body
+// target's list; [n0, n1): two-body targets, a warp per 32 (sets Ybar there); the rest: the
 // recoupling inputs^T.
 __global__ void __launch_bounds__(ADJ_THREADS) k_adj_122(DevTables T, AdjLists A, const double *__restrict__ X, int hL,
                                                          int hR, const double *__restrict__ U,
-                                                         const double *__restrict__ Zb, int n0, int n1, double *fpart,
-                                                         double *WCCb, double *Yb) {
+                                                         const double *__restrict__ Zb, int first, int n0, int n1,
+                                                         double *fpart, double *WCCb, double *Yb) {
   __shared__ double sh[32];
   const int nL = hL < 0, nR = hR < 0;
-  const int blk = blockIdx.x;
+  const int blk = blockIdx.x + first;
   if (blk < n0) {
     const int2 c = A.f_chunk[blk];
     double s = 0.0;
@@ -494,7 +502,9 @@ struct AdjState {
   double *monob = nullptr, *part = nullptr, *dot = nullptr, *h_dot = nullptr;
   AdjProb *d_probs = nullptr;
   GemmTile *d_tiles = nullptr;
-  int ntiles = 0;
+  int ntiles = 0, nladder = 0;  // tiles: the ladder products', then RCCbar's
+  cudaStream_t side = nullptr;  // the part without the particle-hole product
+  cudaEvent_t ev_fork = nullptr, ev_join = nullptr;
 };
 
 namespace {
@@ -727,8 +737,14 @@ int adjoint_prepare(imsrg_basis *b) {
     shapes.push_back({p.M, p.N, k, 0});
   }
   gemm_split(shapes, b->num_sms);
-  const std::vector<GemmTile> tiles = gemm_tiles(shapes);
+  std::vector<GemmTile> tiles = gemm_tiles(shapes);
   a->ntiles = (int)tiles.size();
+  a->nladder = (int)(std::stable_partition(tiles.begin(), tiles.end(), [&](const GemmTile &t) {
+                       return probs[t.prob].c_dst == AD_Y;
+                     }) - tiles.begin());
+  IMSRG_CUDA_TRY(cudaStreamCreateWithFlags(&a->side, cudaStreamNonBlocking));
+  IMSRG_CUDA_TRY(cudaEventCreateWithFlags(&a->ev_fork, cudaEventDisableTiming));
+  IMSRG_CUDA_TRY(cudaEventCreateWithFlags(&a->ev_join, cudaEventDisableTiming));
   auto up = [&](const void *h, size_t bytes, void **d) -> int {
     IMSRG_CUDA_TRY(cudaMalloc(d, std::max<size_t>(bytes, 16)));
     b->dev_allocs.push_back(*d);
@@ -743,6 +759,9 @@ void adjoint_free(imsrg_basis *b) {
   AdjState *a = adj_of(b);
   if (!a) return;
   if (a->h_dot) cudaFreeHost(a->h_dot);
+  if (a->ev_fork) cudaEventDestroy(a->ev_fork);
+  if (a->ev_join) cudaEventDestroy(a->ev_join);
+  if (a->side) cudaStreamDestroy(a->side);
   delete a;  // device buffers are in b->dev_allocs
   b->adjoint = nullptr;
 }
@@ -759,37 +778,63 @@ int commutator_adjoint_dev(imsrg_basis *b, const double *X, int hX, const double
   const AdjLists &A = a->lists;
   ProfScope ps(b, IMSRG_KERNEL_OPS, st);
   auto ctas = [](long n, long per) { return (int)((n + per - 1) / per); };
-  {
-    const int n0 = ctas(b->nfull - b->off_2b, ADJ_THREADS), n1 = n0 + ctas(T.n_ph, ADJ_THREADS),
-              n2 = n1 + ctas(b->cc_total, ADJ_THREADS),
-              n3 = n2 + ctas(b->cc_total + b->off_2b, ADJ_ZERO);
-    k_adj_prep<<<n3, ADJ_THREADS, 0, st>>>(T, A, X, hL, hR, Cb, hRES, b->off_2b, n0, n1, n2, a->w1b, a->w2b, a->u,
-                                            a->zb, b->lcc, a->rccb, Yb);
+  const bool serial = b->prof.on;
+  cudaStream_t side = serial ? st : a->side;
+  if (!serial) {
+    IMSRG_CUDA_TRY(cudaEventRecord(a->ev_fork, st));
+    IMSRG_CUDA_TRY(cudaStreamWaitEvent(side, a->ev_fork, 0));
   }
-  {
-    const int n0 = A.n_f_chunks, n1 = n0 + ctas(A.n_v_warps, ADJ_THREADS / 32), n2 = n1 + 4 * T.n_ph_patches;
-    if (n2) k_adj_122<<<n2, ADJ_THREADS, 0, st>>>(T, A, X, hL, hR, a->u, a->zb, n0, n1, a->fpart, a->wccb, Yb);
-  }
+  const int p0 = ctas(b->nfull, ADJ_THREADS), p1 = p0 + ctas(T.n_ph, ADJ_THREADS),
+            p2 = p1 + ctas(b->cc_total, ADJ_THREADS), p3 = p2 + ctas(b->cc_total, ADJ_ZERO);
+  const int v0 = A.n_f_chunks, v1 = v0 + ctas(A.n_v_warps, ADJ_THREADS / 32), v2 = v1 + 4 * T.n_ph_patches;
+  auto prep = [&](int from, int to, cudaStream_t s) {
+    if (to == from) return;
+    k_adj_prep<<<to - from, ADJ_THREADS, 0, s>>>(T, A, X, hL, hR, Cb, hRES, b->off_2b, from, p0, p1, p2, a->w1b,
+                                                 a->w2b, a->u, a->zb, b->lcc, a->rccb, Yb);
+    b->launches++;
+  };
+  auto sums = [&](int from, int to, cudaStream_t s) {
+    if (to == from) return;
+    k_adj_122<<<to - from, ADJ_THREADS, 0, s>>>(T, A, X, hL, hR, a->u, a->zb, from, v0, v1, a->fpart, a->wccb, Yb);
+    b->launches++;
+  };
+  AdjOps ops{};
+  ops.src[AS_X] = X;
+  ops.src[AS_W1] = a->w1b;
+  ops.src[AS_W2] = a->w2b;
+  ops.src[AS_WCC] = a->wccb;
+  ops.src[AS_LCC] = b->lcc;
+  ops.dst[AD_Y] = Yb;
+  ops.dst[AD_RCC] = a->rccb;
+  auto products = [&](int from, int to, cudaStream_t s) {
+    if (to == from) return;
+    k_gemm_adj<<<to - from, GT_THREADS, 0, s>>>(a->d_probs, a->d_tiles + from, ops, hL, hR);
+    b->launches++;
+  };
+  // (while kernel timing is on, one stream; the order below holds there too)
+  prep(0, p0, side);
+  prep(p0, p3, st);
+  sums(v1, v2, st);
+  products(a->nladder, a->ntiles, st);
+  sums(0, v1, side);
   {
     const int n0 = T.n_asm1_heavy + (T.n_asm1_light + 3) / 4, n1 = n0 + ctas(A.n_f_targets, 128),
               n2 = n1 + (with_e0 ? ctas((long)b->P * b->A, 128) : 0),
               n3 = n2 + (with_e0 && hL * hR == -1 ? b->nblocks : 0);
-    if (n3) k_adj_one<<<n3, 128, 0, st>>>(T, A, X, hL, hR, Cb, hRES, a->fpart, n0, n1, n2, Yb, a->w1b, a->w2b);
+    if (n3) {
+      k_adj_one<<<n3, 128, 0, side>>>(T, A, X, hL, hR, Cb, hRES, a->fpart, n0, n1, n2, Yb, a->w1b, a->w2b);
+      b->launches++;
+    }
   }
-  if (a->ntiles > 0) {
-    AdjOps ops{};
-    ops.src[AS_X] = X;
-    ops.src[AS_W1] = a->w1b;
-    ops.src[AS_W2] = a->w2b;
-    ops.src[AS_WCC] = a->wccb;
-    ops.src[AS_LCC] = b->lcc;
-    ops.dst[AD_Y] = Yb;
-    ops.dst[AD_RCC] = a->rccb;
-    k_gemm_adj<<<a->ntiles, GT_THREADS, 0, st>>>(a->d_probs, a->d_tiles, ops, hL, hR);
+  products(0, a->nladder, side);
+  if (!serial) {
+    IMSRG_CUDA_TRY(cudaEventRecord(a->ev_join, side));
+    IMSRG_CUDA_TRY(cudaStreamWaitEvent(st, a->ev_join, 0));
   }
-  if (b->cc_total > 0)
+  if (b->cc_total > 0) {
     k_adj_cc<<<(unsigned)((b->cc_total + 255) / 256), 256, 0, st>>>(b->T, a->rccb, hR, Yb);
-  b->launches += 5;
+    b->launches++;
+  }
   return cuda_status(cudaGetLastError());
 }
 

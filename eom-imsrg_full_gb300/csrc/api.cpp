@@ -124,8 +124,9 @@ int commutator_launches(imsrg_basis *b, const double *L, int hL, const double *R
   const bool direct = overlap && packed && io->Ldev && io->Rdev && io->RESdev;
   // the transform also reduces the LCC/RCC block exponents (split precision)
   int *cc_exps = nullptr, gL = 0, gR = 0;
+  if (oz && front) IMSRG_TRY(ozaki_exps_begin(b));
   if (overlap) {
-    if (oz) IMSRG_TRY(ozaki_cc_exponents(b, b->stream, &cc_exps, &gL, &gR));
+    if (oz) IMSRG_TRY(ozaki_cc_exponents(b, &cc_exps, &gL, &gR));
     if (direct) {
       // the unpack kernels of R (side2) and L read the host arrays at once
       IMSRG_CUDA_TRY(cudaEventRecord(b->ev_hostR, b->stream));
@@ -147,7 +148,7 @@ int commutator_launches(imsrg_basis *b, const double *L, int hL, const double *R
       IMSRG_CUDA_TRY(cudaMemcpyAsync(const_cast<double *>(L), io->L, bytes, cudaMemcpyHostToDevice, b->stream));
       IMSRG_CUDA_TRY(cudaStreamWaitEvent(b->side2, b->ev_hostR, 0));
     }
-    if (oz) IMSRG_TRY(ozaki_slice(b, L, R, 1, b->side2));
+    if (oz) IMSRG_TRY(ozaki_slice(b, L, R, 1, 2, b->side2));
     IMSRG_TRY(launch_cc_forward(b, L, hL, R, hR, cc_exps, gL, gR, 2, b->side2));
     IMSRG_CUDA_TRY(cudaEventRecord(b->ev_join2, b->side2));
   } else if (io && packed) {  // pageable packed host operands, one after the other
@@ -174,29 +175,28 @@ int commutator_launches(imsrg_basis *b, const double *L, int hL, const double *R
     return IMSRG_OK;
   };
   // E0 and the commutator_122 part of the two-body assembly need only L and
-  // R: E0's single CTA runs on side3 and the 122 sums on side4 from here,
-  // beside the Pandya transform, the slicing and the products.  E0 is joined at the end (after the one-body
-  // assembly, where it ran before, it finished last: the one-body kernel runs
-  // slowly beside the 3,769 CTAs of the two-body assembly), the 122 sums
-  // before the rest of the two-body assembly.
-  if (front) {
+  // R: E0's single CTA runs on side3 and the 122 sums on side4 from where
+  // ev_fork[0] is recorded, beside the Pandya transform, the slicing and the
+  // products.  E0 is joined at the end (after the one-body assembly, where it
+  // ran before, it finished last: the one-body kernel runs slowly beside the
+  // 3,769 CTAs of the two-body assembly), the 122 sums before the rest of the
+  // two-body assembly.
+  auto sums_beside = [&]() -> int {
     if (serial) {
       if (with_e0) IMSRG_TRY(launch_e0(b, L, hL, R, hR, RES, b->stream));
-      IMSRG_TRY(launch_asm2_122(b, L, hL, R, hR, RES, hRES, b->stream));
-    } else {
-      IMSRG_CUDA_TRY(cudaEventRecord(b->ev_fork[0], b->stream));
-      for (cudaStream_t s : {b->side3, b->side4}) {
-        IMSRG_CUDA_TRY(cudaStreamWaitEvent(s, b->ev_fork[0], 0));
-        if (overlap && packed) IMSRG_CUDA_TRY(cudaStreamWaitEvent(s, b->ev_rdev, 0));
-      }
-      if (with_e0) {
-        IMSRG_TRY(launch_e0(b, L, hL, R, hR, RES, b->side3));
-        IMSRG_CUDA_TRY(cudaEventRecord(b->ev_join3, b->side3));
-      }
-      IMSRG_TRY(launch_asm2_122(b, L, hL, R, hR, RES, hRES, b->side4));
-      IMSRG_CUDA_TRY(cudaEventRecord(b->ev_pre, b->side4));
+      return launch_asm2_122(b, L, hL, R, hR, RES, hRES, b->stream);
     }
-  }
+    for (cudaStream_t s : {b->side3, b->side4}) {
+      IMSRG_CUDA_TRY(cudaStreamWaitEvent(s, b->ev_fork[0], 0));
+      if (overlap && packed) IMSRG_CUDA_TRY(cudaStreamWaitEvent(s, b->ev_rdev, 0));
+    }
+    if (with_e0) {
+      IMSRG_TRY(launch_e0(b, L, hL, R, hR, RES, b->side3));
+      IMSRG_CUDA_TRY(cudaEventRecord(b->ev_join3, b->side3));
+    }
+    IMSRG_TRY(launch_asm2_122(b, L, hL, R, hR, RES, hRES, b->side4));
+    return cuda_status(cudaEventRecord(b->ev_pre, b->side4));
+  };
   const bool e0_front = (phases & kPhaseJoinE0Front) != 0;
   auto join_e0 = [&]() -> int {
     if (with_e0 && !serial) IMSRG_CUDA_TRY(cudaStreamWaitEvent(b->stream, b->ev_join3, 0));
@@ -208,11 +208,12 @@ int commutator_launches(imsrg_basis *b, const double *L, int hL, const double *R
   };
   if (overlap) {  // R's half is under way on side2; L's half once L is in
     IMSRG_TRY(fork(0));
-    if (oz) IMSRG_TRY(ozaki_slice(b, L, R, 0, side));
+    IMSRG_TRY(sums_beside());
+    if (oz) IMSRG_TRY(ozaki_slice(b, L, R, 0, 1, side));
     IMSRG_TRY(launch_cc_forward(b, L, hL, R, hR, cc_exps, gL, gR, 1));
     IMSRG_CUDA_TRY(cudaStreamWaitEvent(b->stream, b->ev_join2, 0));
     if (oz) {
-      IMSRG_TRY(ozaki_slice(b, L, R, 2, b->stream, cc_exps != nullptr));
+      IMSRG_TRY(ozaki_slice(b, L, R, 2, 3, b->stream, cc_exps != nullptr));
       IMSRG_TRY(join(0));
       IMSRG_TRY(ozaki_mma(b, hL, hR));
     } else {
@@ -220,25 +221,34 @@ int commutator_launches(imsrg_basis *b, const double *L, int hL, const double *R
       IMSRG_TRY(launch_gemm_fp64(b, L, hL, R, hR));
     }
   } else if (oz) {
-    // digit images of L and of R on the two side streams, beside the Pandya
-    // transform and the images of LCC and RCC
+    // digit images of L and R on a side stream (of R on a second one where the
+    // host's R is still in flight), beside the Pandya transform and the images
+    // of LCC and RCC.  The 122 sums come after them in launch order: a graph
+    // starts its branches in that order, and ahead of them their CTAs took the
+    // warp slots (two emax 6 flow steps: 3,400 us with the sums first, 3,285 so)
     if (front) {
+      const bool two = io && !serial;
       IMSRG_TRY(fork(0));
-      if (!serial) IMSRG_CUDA_TRY(cudaStreamWaitEvent(b->side2, b->ev_fork[0], 0));
-      IMSRG_TRY(ozaki_slice(b, L, R, 0, side));
-      IMSRG_TRY(ozaki_slice(b, L, R, 1, side2));
-      IMSRG_TRY(ozaki_cc_exponents(b, b->stream, &cc_exps, &gL, &gR));
+      if (two) IMSRG_CUDA_TRY(cudaStreamWaitEvent(b->side2, b->ev_fork[0], 0));
+      IMSRG_TRY(ozaki_slice(b, L, R, 0, two ? 1 : 2, side));
+      if (two) IMSRG_TRY(ozaki_slice(b, L, R, 1, 2, side2));
+      IMSRG_TRY(ozaki_cc_exponents(b, &cc_exps, &gL, &gR));
       IMSRG_TRY(launch_cc_forward(b, L, hL, R, hR, cc_exps, gL, gR));
-      IMSRG_TRY(ozaki_slice(b, L, R, 2, b->stream, cc_exps != nullptr));
+      IMSRG_TRY(sums_beside());
+      IMSRG_TRY(ozaki_slice(b, L, R, 2, 3, b->stream, cc_exps != nullptr));
       IMSRG_TRY(join(0));
-      if (!serial) {
+      if (two) {
         IMSRG_CUDA_TRY(cudaEventRecord(b->ev_join2, b->side2));
         IMSRG_CUDA_TRY(cudaStreamWaitEvent(b->stream, b->ev_join2, 0));
       }
     }
     if (prods) IMSRG_TRY(ozaki_mma(b, hL, hR));
   } else {
-    if (front) IMSRG_TRY(launch_cc_forward(b, L, hL, R, hR));
+    if (front) {
+      if (!serial) IMSRG_CUDA_TRY(cudaEventRecord(b->ev_fork[0], b->stream));
+      IMSRG_TRY(sums_beside());
+      IMSRG_TRY(launch_cc_forward(b, L, hL, R, hR));
+    }
     if (prods) IMSRG_TRY(launch_gemm_fp64(b, L, hL, R, hR));
   }
   if (front && e0_front) {  // phases in separate graphs: join what the front forked
@@ -246,6 +256,8 @@ int commutator_launches(imsrg_basis *b, const double *L, int hL, const double *R
     IMSRG_TRY(join_pre());
   }
   if (!back) return IMSRG_OK;
+  int *exps = nullptr, nexps = 0;  // cleared by the two-body assembly
+  if (oz) IMSRG_TRY(ozaki_exps_end(b, &exps, &nexps));
   // one-body assembly beside the two-body assembly
   IMSRG_TRY(fork(1));
   IMSRG_TRY(launch_assemble_1body(b, L, hL, R, hR, RES, hRES, side));
@@ -255,7 +267,8 @@ int commutator_launches(imsrg_basis *b, const double *L, int hL, const double *R
     IMSRG_TRY(launch_ph_inputs(b, hL, hR, precision));
     if (!e0_front) IMSRG_TRY(join_pre());
     for (int c = 0; c < kOutChunks; c++) {
-      IMSRG_TRY(launch_asm2_range(b, L, hL, R, hR, RES, hRES, b->asm2_el[c], b->asm2_el[c + 1], true));
+      IMSRG_TRY(launch_asm2_range(b, L, hL, R, hR, RES, hRES, b->asm2_el[c], b->asm2_el[c + 1], true, exps,
+                                  nexps));
       IMSRG_CUDA_TRY(cudaEventRecord(b->ev_out[c], b->stream));
       IMSRG_CUDA_TRY(cudaStreamWaitEvent(b->side2, b->ev_out[c], 0));
       const long a0 = b->asm2_addr[c], a1 = b->asm2_addr[c + 1];
@@ -276,7 +289,7 @@ int commutator_launches(imsrg_basis *b, const double *L, int hL, const double *R
     ProfScope ps(b, IMSRG_KERNEL_ASSEMBLE_2BODY);
     IMSRG_TRY(launch_ph_inputs(b, hL, hR, precision));
     if (!e0_front) IMSRG_TRY(join_pre());
-    IMSRG_TRY(launch_asm2_range(b, L, hL, R, hR, RES, hRES, 0, b->T.n_asm2, false));
+    IMSRG_TRY(launch_asm2_range(b, L, hL, R, hR, RES, hRES, 0, b->T.n_asm2, false, exps, nexps));
   }
   IMSRG_TRY(join(1));
   if (!e0_front) IMSRG_TRY(join_e0());

@@ -426,7 +426,7 @@ constexpr long kPhList = 65536;
 int launch_asm2_122(imsrg_basis *b, const double *L, int hL, const double *R, int hR, double *RES, int hRES,
                     cudaStream_t st);
 int launch_asm2_range(imsrg_basis *b, const double *L, int hL, const double *R, int hR, double *RES, int hRES,
-                      long w0, long w1, bool by_range);
+                      long w0, long w1, bool by_range, int *exps, int nexps);
 int launch_assemble_1body(imsrg_basis *b, const double *L, int hL, const double *R, int hR, double *RES, int hRES,
                           cudaStream_t st);
 // E0 of [L, R] into RES[0] on stream st (independent of the assembly kernels)
@@ -470,15 +470,19 @@ int preload_commutator_fp64_ws();
 
 // Ozaki split-precision contraction engine (ozaki.cu)
 int ozaki_prepare(imsrg_basis *b);  // plans and allocates the engine once; errors if unavailable
-// part 0: exponents and digit images of L; part 1: of R; part 2: of LCC and
+// parts [p0, p1): 0, exponents and digit images of L; 1, of R; 2, of LCC and
 // RCC (after the Pandya transform).  ozaki_mma then runs every contraction.
-// exps_ready: the part's block exponents are already in place (part 2: the
+// exps_ready: the parts' block exponents are already in place (part 2: the
 // Pandya transform reduced them, see ozaki_cc_exponents).
-int ozaki_slice(imsrg_basis *b, const double *L, const double *R, int part, cudaStream_t st,
+int ozaki_slice(imsrg_basis *b, const double *L, const double *R, int p0, int p1, cudaStream_t st,
                 bool exps_ready = false);
-// Where the Pandya transform may leave the LCC/RCC block exponents (zeroed on
-// st here): exps[gL + q1], exps[gR + q1]; *exps = nullptr if it cannot.
-int ozaki_cc_exponents(imsrg_basis *b, cudaStream_t st, int **exps, int *gL, int *gR);
+// Where the Pandya transform may leave the LCC/RCC block exponents: exps[gL +
+// q1], exps[gR + q1]; *exps = nullptr if it cannot.
+int ozaki_cc_exponents(imsrg_basis *b, int **exps, int *gL, int *gR);
+// Around a commutator's launches: exponents zero at its start; its two-body
+// assembly clears the n of them at exps.
+int ozaki_exps_begin(imsrg_basis *b);
+int ozaki_exps_end(imsrg_basis *b, int **exps, int *n);
 int ozaki_mma(imsrg_basis *b, int hL, int hR);
 int ozaki_check_error(imsrg_basis *b);  // IMSRG_ERR_TIMEOUT if a bounded device wait gave up
 // synchronise the basis stream and then check as ozaki_check_error, with one

@@ -288,7 +288,8 @@ __global__ void __launch_bounds__(ASM2_THREADS) k_asm2_122(DevTables T, const do
 // antisymmetrised ladder epilogue of 222_pp_hh (:658-764) and the 222_ph
 // recoupling sum over J' of {6j} Z(J').  Thread t takes element w0 + t of the
 // work order `heads` while below w1.  PRE: the 122 part is already in RES
-// (k_asm2_122).  has220 (the allocation-free path, w0 = 0): each CTA leaves
+// (k_asm2_122), and the split engine's nexps block exponents are cleared for the
+// next commutator (nothing reads them any more).  has220 (the allocation-free path, w0 = 0): each CTA leaves
 // its commutator_220 partial in e0p for k_energy.
 template <bool PRE>
 __global__ void __launch_bounds__(ASM2_THREADS) k_assemble_2body(DevTables T, const double *__restrict__ L, int hL,
@@ -297,8 +298,10 @@ __global__ void __launch_bounds__(ASM2_THREADS) k_assemble_2body(DevTables T, co
                                                                  const double *__restrict__ W2,
                                                                  const double *__restrict__ Z, double *RES, int hRES,
                                                                  const Asm2Head *__restrict__ heads, long w0, long w1,
-                                                                 int has220, double *e0p) {
+                                                                 int has220, double *e0p, int *exps, int nexps) {
   __shared__ double sh220[ASM2_THREADS / 32];
+  if (PRE && blockIdx.x == 0)
+    for (int i = threadIdx.x; i < nexps; i += ASM2_THREADS) exps[i] = 0;
   const long w = w0 + (long)blockIdx.x * blockDim.x + threadIdx.x;
   double e220 = 0.0;  // this element's commutator_220 term (pphh arrays only)
   if (w < w1) {
@@ -658,12 +661,12 @@ int launch_ph_inputs(imsrg_basis *b, int hL, int hR, int precision) {
 }
 
 int launch_asm2_range(imsrg_basis *b, const double *L, int hL, const double *R, int hR, double *RES, int hRES,
-                      long w0, long w1, bool by_range) {
+                      long w0, long w1, bool by_range, int *exps, int nexps) {
   const long n = w1 - w0;
   if (n > 0) {
     k_assemble_2body<true><<<(unsigned)((n + ASM2_THREADS - 1) / ASM2_THREADS), ASM2_THREADS, 0, b->stream>>>(
         b->T, L, hL, R, hR, b->w1, b->w2, b->zph, RES, hRES, by_range ? b->T.asm2_head_out : b->T.asm2_head, w0,
-        w1, 0, nullptr);
+        w1, 0, nullptr, exps, nexps);
     b->launches++;
   }
   return cuda_status(cudaGetLastError());
@@ -729,7 +732,7 @@ int launch_commutator_fp64_ws(imsrg_basis *b, const Workspace &ws, const double 
   if (n2 > 0) {
     const int has220 = with_e0 && hL * hR == -1;
     k_assemble_2body<false><<<(unsigned)((n2 + ASM2_THREADS - 1) / ASM2_THREADS), ASM2_THREADS, 0, st>>>(
-        b->T, L, hL, R, hR, ws.w1, ws.w2, ws.zph, RES, hRES, b->T.asm2_head, 0, n2, has220, ws.e0p);
+        b->T, L, hL, R, hR, ws.w1, ws.w2, ws.zph, RES, hRES, b->T.asm2_head, 0, n2, has220, ws.e0p, nullptr, 0);
     b->launches++;
   }
   const int grid1 = b->T.n_asm1_heavy + (b->T.n_asm1_light + 3) / 4;

@@ -159,7 +159,7 @@ struct __align__(16) OzTile {
   int gA, gB;          // exponent groups of A and B
   int map, abox;       // first tensor map of the instance (see kMaps), A box kind
   double *C;           // the tile's origin
-  long pad2;
+  const int *exps;     // the instance's block exponents
 };
 static_assert(sizeof(OzTile) == kRecBytes, "record of six 16-byte loads");
 constexpr int kTileTwoTerms = 1, kTileRaw = 2;  // raw: store the exact int64 level sum v (result = v 2^k): WCC
@@ -188,7 +188,8 @@ struct OzPlan {
   OzChunk *d_chunks = nullptr;
   OzTile *d_tiles = nullptr;   // grouped by CTA
   int *d_sched_off = nullptr;  // [grid + 1] start of each CTA's tiles
-  int *d_exps = nullptr;       // per group: max biased exponent (e = value - 1022)
+  int *d_exps = nullptr;       // per group: max biased exponent (e = value - 1022), zero between commutators
+  bool exps_dirty = false;     // a commutator was enqueued up to its exponents, not to its end
   int *d_err = nullptr;
   // All digit images in one buffer of S planes, each `units` 256-byte units (8
   // rows x 16 K, two core matrices): one tensor map per box shape serves every
@@ -540,8 +541,7 @@ __global__ void __launch_bounds__(SLICE_THREADS) k_oz_slice(const OzMatrix *__re
 // the chunk bookkeeping folds away at compile time.
 template <int S, bool CH>
 __global__ void __launch_bounds__(oz_threads(S), 1) k_oz_mma(const OzTile *__restrict__ tiles,
-                                                          const int *__restrict__ sched_off,
-                                                          const int *__restrict__ exps, int hL, int hR, int *err,
+                                                          const int *__restrict__ sched_off, int hL, int hR, int *err,
                                                           const CUtensorMap *__restrict__ maps,
                                                           const int *__restrict__ act) {
   extern __shared__ __align__(1024) uint8_t smem_raw[];
@@ -717,7 +717,7 @@ __global__ void __launch_bounds__(oz_threads(S), 1) k_oz_mma(const OzTile *__res
       if (act && !act[P.inst]) continue;  // an instance whose series has stopped: its outputs stay
       const int Mp = P.rows, Np = P.cols, ldc = P.ldc;
       const int nch = CH ? P.nchunks : 1, raw = P.flags & kTileRaw;
-      const int k = (exps[P.gA] - 1022) + (exps[P.gB] - 1022) - 7 * LMAX;  // result = v * 2^k
+      const int k = (P.exps[P.gA] - 1022) + (P.exps[P.gB] - 1022) - 7 * LMAX;  // result = v * 2^k
       const bool row_ok = row < Mp;
       double *crow = P.C + row;
       // warp-uniform: a piece entirely past M or N is neither read nor converted
@@ -812,9 +812,9 @@ __global__ void __launch_bounds__(oz_threads(S), 1) k_oz_mma(const OzTile *__res
 OzPlan *plan_of(imsrg_basis *b) { return (OzPlan *)b->ozaki; }
 
 void launch_mma(int S, bool chunked, int grid, cudaStream_t st, const OzTile *tiles, const int *sched_off,
-                const int *exps, int hL, int hR, int *err, const CUtensorMap *maps, const int *act = nullptr) {
+                int hL, int hR, int *err, const CUtensorMap *maps, const int *act = nullptr) {
 #define OZ_LAUNCH(SS, CC) \
-  k_oz_mma<SS, CC><<<grid, oz_threads(SS), oz_mma_smem(SS), st>>>(tiles, sched_off, exps, hL, hR, err, maps, act)
+  k_oz_mma<SS, CC><<<grid, oz_threads(SS), oz_mma_smem(SS), st>>>(tiles, sched_off, hL, hR, err, maps, act)
   switch (S) {
     case 4: if (chunked) OZ_LAUNCH(4, true); else OZ_LAUNCH(4, false); break;
     case 5: if (chunked) OZ_LAUNCH(5, true); else OZ_LAUNCH(5, false); break;
@@ -880,8 +880,7 @@ int autotune(imsrg_basis *b, OzPlan *pl, int hL, int hR) {
   IMSRG_CUDA_TRY(cudaEventCreate(&e1));
   auto launch_timed = [&](float *ms) -> int {
     IMSRG_CUDA_TRY(cudaEventRecord(e0, b->stream));
-    launch_mma(pl->S, pl->chunked, pl->grid, b->stream, pl->d_tiles, pl->d_sched_off, pl->d_exps, hL, hR, pl->d_err,
-               pl->d_maps);
+    launch_mma(pl->S, pl->chunked, pl->grid, b->stream, pl->d_tiles, pl->d_sched_off, hL, hR, pl->d_err, pl->d_maps);
     b->launches++;
     IMSRG_CUDA_TRY(cudaEventRecord(e1, b->stream));
     IMSRG_CUDA_TRY(cudaEventSynchronize(e1));
@@ -1067,6 +1066,9 @@ int ozaki_prepare(imsrg_basis *b) {
       return IMSRG_ERR_INVALID;
   }
 
+  IMSRG_CUDA_TRY(cudaMalloc((void **)&pl->d_exps, std::max(pl->ngroups, 1) * sizeof(int)));
+  IMSRG_CUDA_TRY(cudaMemset(pl->d_exps, 0, std::max(pl->ngroups, 1) * sizeof(int)));
+
   // tiles: the FP64 grouped-GEMM list mapped onto images.  Products with an
   // empty contraction have none: their outputs are the zeros that W1, W2 and
   // WCC were allocated with, which nothing else writes.
@@ -1080,6 +1082,7 @@ int ozaki_prepare(imsrg_basis *b) {
     if (gp.c_dst == SRC_WCC && !oz_fp64_class(pl->S)) p.flags |= kTileRaw;
     if (gp.nterms > 1) p.flags |= kTileTwoTerms;
     p.ldc = gp.ldc;
+    p.exps = pl->d_exps;
     for (int it = 0; it < gp.nterms; it++) {
       const GemmTerm &t = gp.t[it];
       const OzMatrix &A = pl->mats[mat_of[{img_of(t.a_src), t.a_off}]];
@@ -1140,7 +1143,6 @@ int ozaki_prepare(imsrg_basis *b) {
   IMSRG_TRY(up(mat_r.data(), mat_r.size() * sizeof(uint16_t), (void **)&pl->d_mat_r));
   // (cudaMalloc memory is 256-byte aligned: the 64-byte alignment of a tensor map holds)
   IMSRG_TRY(up(pl->maps, sizeof(pl->maps), (void **)&pl->d_maps));
-  IMSRG_CUDA_TRY(cudaMalloc((void **)&pl->d_exps, std::max(pl->ngroups, 1) * sizeof(int)));
   IMSRG_CUDA_TRY(cudaMalloc((void **)&pl->d_err, sizeof(int)));
   IMSRG_CUDA_TRY(cudaMemset(pl->d_err, 0, sizeof(int)));
   {
@@ -1161,32 +1163,52 @@ int ozaki_prepare(imsrg_basis *b) {
   return IMSRG_OK;
 }
 
-int ozaki_cc_exponents(imsrg_basis *b, cudaStream_t st, int **exps, int *gL, int *gR) {
+// The block exponents are maxima, taken atomically from zero.  The two-body
+// assembly, the last launch of a commutator on its stream and after every
+// reader of them, leaves them zero for the next one (a memset ahead of each
+// part cost three graph nodes, one of them in the chain to the products).
+// ozaki_exps_begin clears them all where a commutator has not come to its end.
+int ozaki_exps_begin(imsrg_basis *b) {
+  OzPlan *pl = plan_of(b);
+  if (!pl || !pl->ok) return IMSRG_ERR_INVALID;
+  if (pl->exps_dirty)
+    IMSRG_CUDA_TRY(cudaMemsetAsync(pl->d_exps, 0, std::max(pl->ngroups, 1) * sizeof(int), b->stream));
+  pl->exps_dirty = true;
+  return IMSRG_OK;
+}
+
+int ozaki_exps_end(imsrg_basis *b, int **exps, int *n) {
+  OzPlan *pl = plan_of(b);
+  if (!pl || !pl->ok) return IMSRG_ERR_INVALID;
+  *exps = pl->d_exps;
+  *n = pl->ngroups;
+  pl->exps_dirty = false;
+  return IMSRG_OK;
+}
+
+int ozaki_cc_exponents(imsrg_basis *b, int **exps, int *gL, int *gR) {
   OzPlan *pl = plan_of(b);
   *exps = nullptr;
   if (!pl || !pl->ok || !b->T.ccf_packed) return IMSRG_OK;
-  const int g0 = pl->group_lo[2], g1 = pl->group_lo[3];
-  if (g1 > g0) IMSRG_CUDA_TRY(cudaMemsetAsync(pl->d_exps + g0, 0, (g1 - g0) * sizeof(int), st));
+  const int g0 = pl->group_lo[2];
   *exps = pl->d_exps;
   *gL = g0;
   *gR = g0 + b->ccgroups;
   return IMSRG_OK;
 }
 
-int ozaki_slice(imsrg_basis *b, const double *L, const double *R, int part, cudaStream_t st, bool exps_ready) {
+int ozaki_slice(imsrg_basis *b, const double *L, const double *R, int p0, int p1, cudaStream_t st, bool exps_ready) {
   OzPlan *pl = plan_of(b);
   if (!pl) return IMSRG_ERR_INVALID;
   ProfScope ps(b, IMSRG_KERNEL_OZAKI_SLICE, st);
-  if (part < 0 || part > 2) return IMSRG_ERR_INVALID;
-  const int g0 = pl->group_lo[part], g1 = pl->group_lo[part + 1];
-  const int k0 = pl->chunk_lo[part], k1 = pl->chunk_lo[part + 1];
-  if (g1 > g0 && !exps_ready) IMSRG_CUDA_TRY(cudaMemsetAsync(pl->d_exps + g0, 0, (g1 - g0) * sizeof(int), st));
+  if (p0 < 0 || p1 > 3 || p0 >= p1) return IMSRG_ERR_INVALID;
+  const int k0 = pl->chunk_lo[p0], k1 = pl->chunk_lo[p1];
   if (k1 > k0 && !exps_ready) {
     k_oz_exponents<<<k1 - k0, 256, 0, st>>>(pl->d_chunks + k0, L, R, b->lcc, b->rcc, pl->d_exps);
     b->launches++;
   }
-  const int c_lo = pl->linec_lo[part], c_hi = pl->linec_lo[part + 1];
-  const int r_lo = pl->liner_lo[part], r_hi = pl->liner_lo[part + 1];
+  const int c_lo = pl->linec_lo[p0], c_hi = pl->linec_lo[p1];
+  const int r_lo = pl->liner_lo[p0], r_hi = pl->liner_lo[p1];
   const int cblocks = (c_hi - c_lo + SLICE_THREADS - 1) / SLICE_THREADS;
   const int nblk = cblocks + (r_hi - r_lo + SLICE_THREADS - 1) / SLICE_THREADS;
   if (nblk) {
@@ -1208,8 +1230,7 @@ int ozaki_mma(imsrg_basis *b, int hL, int hR) {
     if (cs == cudaStreamCaptureStatusNone) IMSRG_TRY(autotune(b, pl, hL, hR));
   }
   ProfScope ps(b, IMSRG_KERNEL_OZAKI_MMA);
-  launch_mma(pl->S, pl->chunked, pl->grid, b->stream, pl->d_tiles, pl->d_sched_off, pl->d_exps, hL, hR, pl->d_err,
-             pl->d_maps);
+  launch_mma(pl->S, pl->chunked, pl->grid, b->stream, pl->d_tiles, pl->d_sched_off, hL, hR, pl->d_err, pl->d_maps);
   b->launches++;
   return cuda_status(cudaGetLastError());
 }
@@ -1279,25 +1300,22 @@ int ozaki_schedule_info(imsrg_basis *b, int *choice, int *ncand, double *us, int
 
 // ---------------------------------------------------------------------------
 // One persistent launch for the products of several bases.  Every problem
-// keeps its own output pointer; its exponent groups and tensor maps are
-// renumbered into merged arrays, and the tiles of all bases are assigned
-// longest first over one grid.  Each basis's slicing still writes its own
-// exponents; ozaki_batch_mma gathers them (one small copy per basis) before
-// the launch.  Tiles compute exactly as in a basis's own launch, so results
+// keeps its own output and exponent pointers (a copy of each basis's exponents
+// into a merged array, twelve graph nodes in a row, took 20 us of a batch of
+// twelve); its tensor maps are renumbered into a merged array, and the tiles of
+// all bases are assigned longest first over one grid.  Tiles compute exactly as in a basis's own launch, so results
 // are bit-identical.
 namespace {
 struct OzBatch {
   std::vector<OzPlan *> plans;
-  std::vector<int> exps_base;
-  int grid = 0, ngroups = 0;
+  int grid = 0;
   bool chunked = false;  // some merged tile runs in more than one chunk
   OzTile *d_tiles = nullptr;
-  int *d_sched_off = nullptr, *d_exps = nullptr, *d_err = nullptr;
+  int *d_sched_off = nullptr, *d_err = nullptr;
   CUtensorMap *d_maps = nullptr;
   ~OzBatch() {
     cudaFree(d_tiles);
     cudaFree(d_sched_off);
-    cudaFree(d_exps);
     cudaFree(d_err);
     cudaFree(d_maps);
   }
@@ -1323,19 +1341,15 @@ int ozaki_batch_create(imsrg_basis *const *bases, int n, void **out) {
     bt->plans.push_back(pl);
     bt->chunked = bt->chunked || pl->chunked;
     if (pl->S != bt->plans[0]->S) return fail(IMSRG_ERR_INVALID);  // one digit count per merged launch
-    bt->exps_base.push_back(bt->ngroups);
     for (size_t k = 0; k < pl->tiles.size(); k++) {
       OzTile q = pl->tiles[k];
       q.inst = i;
-      q.gA += bt->ngroups;
-      q.gB += bt->ngroups;
       q.map += (int)maps.size();
       all.tiles.push_back(q);
       all.tile_ksteps.push_back(pl->tile_ksteps[k]);
       all.tile_live.push_back(pl->tile_live[k]);
     }
     maps.insert(maps.end(), pl->maps, pl->maps + kMaps);
-    bt->ngroups += pl->ngroups;
     // the bases' own tuned cost model when they agree, else the one usually chosen
     const int m = pl->tuned ? pl->tune_choice : 1;
     model = (model < 0 || model == m) ? m : 1;
@@ -1357,7 +1371,6 @@ int ozaki_batch_create(imsrg_basis *const *bases, int n, void **out) {
   if (s == IMSRG_OK) s = up(sched_off.data(), sched_off.size() * sizeof(int), (void **)&bt->d_sched_off);
   // (cudaMalloc memory is 256-byte aligned: the 64-byte alignment of a tensor map holds)
   if (s == IMSRG_OK) s = up(maps.data(), maps.size() * sizeof(CUtensorMap), (void **)&bt->d_maps);
-  if (s == IMSRG_OK) s = cuda_status(cudaMalloc((void **)&bt->d_exps, std::max(bt->ngroups, 1) * sizeof(int)));
   const int zero = 0;
   if (s == IMSRG_OK) s = up(&zero, sizeof(int), (void **)&bt->d_err);
   if (s != IMSRG_OK) return fail(s);
@@ -1368,12 +1381,8 @@ int ozaki_batch_create(imsrg_basis *const *bases, int n, void **out) {
 int ozaki_batch_mma(void *batch, cudaStream_t st, int hL, int hR, const int *act) {
   OzBatch *bt = (OzBatch *)batch;
   if (!bt) return IMSRG_ERR_INVALID;
-  for (size_t i = 0; i < bt->plans.size(); i++)
-    if (bt->plans[i]->ngroups > 0)
-      IMSRG_CUDA_TRY(cudaMemcpyAsync(bt->d_exps + bt->exps_base[i], bt->plans[i]->d_exps,
-                                     bt->plans[i]->ngroups * sizeof(int), cudaMemcpyDeviceToDevice, st));
-  launch_mma(bt->plans[0]->S, bt->chunked, bt->grid, st, bt->d_tiles, bt->d_sched_off, bt->d_exps, hL, hR, bt->d_err,
-             bt->d_maps, act);
+  launch_mma(bt->plans[0]->S, bt->chunked, bt->grid, st, bt->d_tiles, bt->d_sched_off, hL, hR, bt->d_err, bt->d_maps,
+             act);
   return cuda_status(cudaGetLastError());
 }
 

@@ -225,28 +225,44 @@ __device__ void energy_block(const DevTables &T, const double *L, int hL, const 
 }
 
 // commutator_122 (commutators.f90:283-396) of one element: f_L V_R - f_R V_L
-// over its leg terms (term k at tm[k * STRIDE])
-template <int STRIDE>
+// over its leg terms (term k at tm[k * STRIDE]), U terms in flight: their gathers
+// and the next U terms are loaded before the first is used
+template <int STRIDE, int U>
 __device__ __forceinline__ double sum122(const unsigned long long *tm, int n122, const double *L, int nL,
                                          const double *R, int nR) {
   double t = 0.0;
-  unsigned long long next = n122 > 0 ? tm[0] : 0;
-  for (int k = 0; k < n122; k++) {
-    const unsigned long long u = next;
-    if (k + 1 < n122) next = tm[(k + 1) * STRIDE];
-    const long vi = (long)(u & 0xFFFFFFFull), fi = (long)((u >> 28) & 0xFFFFFull);
-    const int sg = (int)(u >> 48) & 1, nsq = (int)(u >> 49) & 3, tr = (int)(u >> 51) & 1, ftr = (int)(u >> 52) & 1;
-    // the term's four gathers, and the next term, before the branch
-    double vR = R[vi], vL = L[vi], fL = L[fi], fR = R[fi];
-    vR = dflip(vR, tr & nR);
-    vL = dflip(vL, tr & nL);
-    if (nsq) {
-      const double c = nsq == 1 ? IMSRG_SQRT2 : 2.0000000000000004;
-      vR = vR * c;
-      vL = vL * c;
+  unsigned long long next[U];
+#pragma unroll
+  for (int i = 0; i < U; i++) next[i] = i < n122 ? tm[i * STRIDE] : 0;
+  for (int k = 0; k < n122; k += U) {
+    unsigned long long u[U];
+    double vR[U], vL[U], fL[U], fR[U];
+#pragma unroll
+    for (int i = 0; i < U; i++) {
+      u[i] = next[i];
+      if (k + U + i < n122) next[i] = tm[(k + U + i) * STRIDE];
+      if (i == 0 || k + i < n122) {
+        const long vi = (long)(u[i] & 0xFFFFFFFull), fi = (long)((u[i] >> 28) & 0xFFFFFull);
+        vR[i] = R[vi];
+        vL[i] = L[vi];
+        fL[i] = L[fi];
+        fR[i] = R[fi];
+      }
     }
-    t = fma(dflip(fL, (ftr & nL) ^ sg), vR, t);
-    t = fma(dflip(fR, (ftr & nR) ^ sg ^ 1), vL, t);
+#pragma unroll
+    for (int i = 0; i < U; i++) {
+      if (i > 0 && k + i >= n122) break;
+      const int sg = (int)(u[i] >> 48) & 1, nsq = (int)(u[i] >> 49) & 3, tr = (int)(u[i] >> 51) & 1,
+                ftr = (int)(u[i] >> 52) & 1;
+      double a = dflip(vR[i], tr & nR), b = dflip(vL[i], tr & nL);
+      if (nsq) {
+        const double c = nsq == 1 ? IMSRG_SQRT2 : 2.0000000000000004;
+        a = a * c;
+        b = b * c;
+      }
+      t = fma(dflip(fL[i], (ftr & nL) ^ sg), a, t);
+      t = fma(dflip(fR[i], (ftr & nR) ^ sg ^ 1), b, t);
+    }
   }
   return t;
 }
@@ -265,6 +281,9 @@ __device__ __forceinline__ double sum122(const unsigned long long *tm, int n122,
 // with a CTA per four groups it took every slot first (emax = 6, five digits:
 // 112.4 us per commutator, 109.5 with eight CTAs per SM, 111.5 with six or
 // twelve; host call 203 -> 194, two flow steps 3440 -> 3250, FP64 493 -> 487).
+// They gate the products all the same, whose CTAs each want a whole SM (four
+// CTAs per SM 122 us, two 147), with loads as their longest stall: two terms in
+// flight take 108.4 to 106.1 us, three or four 108.8 and 111.2.
 constexpr int kPreCtas = 8;
 __global__ void __launch_bounds__(ASM2_THREADS) k_asm2_122(DevTables T, const double *__restrict__ L, int hL,
                                                            const double *__restrict__ R, int hR, int hRES,
@@ -275,7 +294,7 @@ __global__ void __launch_bounds__(ASM2_THREADS) k_asm2_122(DevTables T, const do
     const unsigned pe = T.pre_el[(long)g * 32 + lane];
     if (pe >> 31) continue;  // padding
     const Asm2PreWarp W = T.pre_warp[g];
-    double t = sum122<32>(T.pre_terms + W.base + lane, W.n122, L, hL < 0, R, hR < 0);
+    double t = sum122<32, 2>(T.pre_terms + W.base + lane, W.n122, L, hL < 0, R, hR < 0);
     const int nd = (pe >> 28) & 3;
     if (nd) t = t * (nd == 1 ? 0.7071067811865476 : 0.5);
     if ((pe >> 30) & 1) t = dflip(t, hRES < 0);
@@ -316,7 +335,7 @@ __global__ void __launch_bounds__(ASM2_THREADS) k_assemble_2body(DevTables T, co
     if (PRE) {
       t = RES[e];
     } else {
-      t = sum122<1>(tm, meta & 31, L, nL, R, nR);
+      t = sum122<1, 1>(tm, meta & 31, L, nL, R, nR);
       // / sqrt(1 + delta_ab) / sqrt(1 + delta_cd)
       if (nd) t = t * (nd == 1 ? 0.7071067811865476 : 0.5);
       if (diag) t = dflip(t, nres);

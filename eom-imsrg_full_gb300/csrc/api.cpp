@@ -109,6 +109,7 @@ int commutator_launches(imsrg_basis *b, const double *L, int hL, const double *R
   // While kernel timing is on, every launch goes to the basis stream in the
   // same order, so each kernel class's event pair times that kernel alone.
   const bool serial = b->prof.on;
+  b->pdl = phases == kPhaseAll;
   cudaStream_t side = serial ? b->stream : b->side, side2 = serial ? b->stream : b->side2;
   const size_t bytes = (size_t)b->nfull * sizeof(double);
   const bool oz = precision == IMSRG_PREC_OZAKI;

@@ -11,6 +11,34 @@
 
 namespace imsrg {
 
+// Programmatic dependent launches.  A kernel launched with launch_after may
+// start when every CTA of the kernel before it on the stream has called
+// pdl_go() or ended; all its threads call pdl_wait() before they touch what
+// earlier work wrote (or write what it reads), which waits for that kernel's
+// end.  Only tables that never change are read ahead of it.  A kernel without
+// pdl_go() lets its successor start as it ends.  on: else an ordinary launch.
+// In a single commutator the launch gaps of the chain are what it gives: emax 2
+// 22.6 -> 22.1 us split, 16.5 -> 16.0 FP64; emax 6 FP64 483 -> 479; Magnus steps
+// emax 4 1,766 -> 1,737, emax 6 3,256 -> 3,173.  Batches keep ordinary launches:
+// their many chains fill the gaps (twelve commutators: no difference).
+__device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+__device__ __forceinline__ void pdl_go() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+
+template <typename... P, typename... A>
+cudaError_t launch_after(bool on, void (*kernel)(P...), unsigned grid, unsigned block, size_t smem, cudaStream_t st, A... args) {
+  cudaLaunchAttribute at{};
+  at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  at.val.programmaticStreamSerializationAllowed = 1;
+  cudaLaunchConfig_t c{};
+  c.gridDim = dim3(grid);
+  c.blockDim = dim3(block);
+  c.dynamicSmemBytes = smem;
+  c.stream = st;
+  c.attrs = &at;
+  c.numAttrs = on ? 1 : 0;
+  return cudaLaunchKernelEx(&c, kernel, static_cast<P>(args)...);
+}
+
 __device__ __forceinline__ bool dtri(int j1, int j2, int J) { return J <= j1 + j2 && J >= abs(j1 - j2); }
 __device__ __forceinline__ double m1pow(int e) { return (e & 1) ? -1.0 : 1.0; }
 

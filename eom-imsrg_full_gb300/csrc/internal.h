@@ -324,6 +324,7 @@ struct imsrg_basis {
   // norm chunks
   imsrg::NormChunk *d_chunks = nullptr;
   int nchunks = 0;
+  bool pdl = true;  // the launches of the commutator being enqueued overlap (launch_after)
   // packed layout map: packed index k -> flat index, and mirrored flat index (or -1)
   long *d_pack_src = nullptr, *d_pack_mirror = nullptr;
   // staging buffer (pinned) for Fortran-style uploads/downloads

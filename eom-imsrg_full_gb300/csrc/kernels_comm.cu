@@ -41,6 +41,7 @@ __global__ void __launch_bounds__(256) k_cc_forward(DevTables T, const double *_
                                                     const double *__restrict__ R, int hR, double *LCC, double *RCC,
                                                     int *exps, int gL, int gR) {
   const long t = (long)blockIdx.x * blockDim.x + threadIdx.x;
+  pdl_go();
   int q1 = -1, xL = 0, xR = 0;
   if (t < T.cc_total) {
     const int v = T.ccf_order[t];  // elements grouped by term count
@@ -86,6 +87,8 @@ __global__ void __launch_bounds__(GT_THREADS, GT_CTAS) k_gemm_fp64(const GemmPro
                                                           int hR, const int *__restrict__ act) {
   const GemmTile t = tiles[blockIdx.x];
   const GemmProb &P = probs[t.prob];
+  pdl_go();
+  pdl_wait();
   if (ABS && act && !act[P.inst]) return;  // block-uniform
   double *C = ABS ? P.c_abs : ops.dst[P.c_dst] + P.c_off;
   gemm_cta_tile<false>(
@@ -143,8 +146,10 @@ __global__ void __launch_bounds__(256) k_ph_patches(DevTables T, const double *_
                                                     double *__restrict__ Z) {
   const PhPatch &p = T.ph_patch[blockIdx.x >> 2];
   const int layers = p.layers;
-  if (layers == 0) return;
   const int lane = threadIdx.x & 31, ty = (threadIdx.x >> 5) + (blockIdx.x & 3) * 8, rl = p.rlen;
+  pdl_go();
+  pdl_wait();
+  if (layers == 0) return;
   const double *W = WCC + p.w, *V = WCC + p.v;
   const unsigned *slots = T.ph_slots + (long)p.table * 1024 + ty * 32 + lane;
   const unsigned char *ph = T.cc_rowph + p.row0;
@@ -170,9 +175,11 @@ __global__ void __launch_bounds__(256) k_ph_list(DevTables T, const double *__re
                                                  const int *__restrict__ exps, int gL, int gR, int kshift,
                                                  double *__restrict__ Z) {
   const int t = blockIdx.x * blockDim.x + threadIdx.x;
-  if (t >= T.n_ph) return;
-  const PhTerm p = T.ph_terms[t];
+  const PhTerm p = t < T.n_ph ? T.ph_terms[t] : PhTerm{};
   const unsigned m = 0x0FFFFFFFu;
+  pdl_go();
+  pdl_wait();
+  if (t >= T.n_ph) return;
   int k = 0;
   if (INT) {
     const int g = p.y >> 28 | (p.z >> 28) << 4 | (p.w >> 28) << 8;
@@ -319,12 +326,14 @@ __global__ void __launch_bounds__(ASM2_THREADS) k_assemble_2body(DevTables T, co
                                                                  const Asm2Head *__restrict__ heads, long w0, long w1,
                                                                  int has220, double *e0p, int *exps, int nexps) {
   __shared__ double sh220[ASM2_THREADS / 32];
+  const long w = w0 + (long)blockIdx.x * blockDim.x + threadIdx.x;
+  const Asm2Head h = w < w1 ? heads[w] : Asm2Head{};
+  pdl_go();
+  pdl_wait();
   if (PRE && blockIdx.x == 0)
     for (int i = threadIdx.x; i < nexps; i += ASM2_THREADS) exps[i] = 0;
-  const long w = w0 + (long)blockIdx.x * blockDim.x + threadIdx.x;
   double e220 = 0.0;  // this element's commutator_220 term (pphh arrays only)
   if (w < w1) {
-    const Asm2Head h = heads[w];
     const unsigned long long *tm = T.asm2_terms + h.start;
     const unsigned meta = h.meta;
     const int nL = hL < 0, nR = hR < 0, nres = hRES < 0, npm = (hL * hR) < 0;
@@ -596,9 +605,9 @@ int launch_gemm_fp64(imsrg_basis *b, const double *L, int hL, const double *R, i
   ops.dst[SRC_W2] = b->w2;
   ops.dst[SRC_WCC] = b->wcc;
   ProfScope ps(b, IMSRG_KERNEL_GEMM_FP64);
-  k_gemm_fp64<false><<<b->ntiles, GT_THREADS, 0, b->stream>>>(b->d_probs, b->d_tiles, ops, hL, hR, nullptr);
   b->launches++;
-  return cuda_status(cudaGetLastError());
+  return cuda_status(launch_after(b->pdl, k_gemm_fp64<false>, b->ntiles, GT_THREADS, 0, b->stream, b->d_probs, b->d_tiles, ops,
+                                  hL, hR, nullptr));
 }
 
 void gemm_fp64_plan(std::vector<GemmProb> &probs, int num_sms) {
@@ -662,14 +671,11 @@ int launch_gemm_fp64_merged(const GemmMerged &g, int hL, int hR, const int *act,
 static int ph_inputs(imsrg_basis *b, const double *WCC, int hL, int hR, const int *exps, int gL, int gR, int kshift,
                      double *Z, cudaStream_t st) {
   if (b->T.n_ph == 0) return IMSRG_OK;
-  if (b->T.ph_terms)
-    (exps ? k_ph_list<true> : k_ph_list<false>)<<<(b->T.n_ph + 255) / 256, 256, 0, st>>>(b->T, WCC, hL, hR, exps, gL,
-                                                                                         gR, kshift, Z);
-  else
-    (exps ? k_ph_patches<true> : k_ph_patches<false>)<<<4 * b->T.n_ph_patches, 256, 0, st>>>(b->T, WCC, hL, hR, exps,
-                                                                                            gL, gR, kshift, Z);
+  auto *kernel = b->T.ph_terms ? (exps ? k_ph_list<true> : k_ph_list<false>)
+                               : (exps ? k_ph_patches<true> : k_ph_patches<false>);
+  const unsigned grid = b->T.ph_terms ? (b->T.n_ph + 255) / 256 : 4 * b->T.n_ph_patches;
   b->launches++;
-  return cuda_status(cudaGetLastError());
+  return cuda_status(launch_after(b->pdl, kernel, grid, 256, 0, st, b->T, WCC, hL, hR, exps, gL, gR, kshift, Z));
 }
 
 int launch_ph_inputs(imsrg_basis *b, int hL, int hR, int precision) {
@@ -683,9 +689,9 @@ int launch_asm2_range(imsrg_basis *b, const double *L, int hL, const double *R, 
                       long w0, long w1, bool by_range, int *exps, int nexps) {
   const long n = w1 - w0;
   if (n > 0) {
-    k_assemble_2body<true><<<(unsigned)((n + ASM2_THREADS - 1) / ASM2_THREADS), ASM2_THREADS, 0, b->stream>>>(
-        b->T, L, hL, R, hR, b->w1, b->w2, b->zph, RES, hRES, by_range ? b->T.asm2_head_out : b->T.asm2_head, w0,
-        w1, 0, nullptr, exps, nexps);
+    IMSRG_CUDA_TRY(launch_after(b->pdl, k_assemble_2body<true>, (unsigned)((n + ASM2_THREADS - 1) / ASM2_THREADS),
+                                ASM2_THREADS, 0, b->stream, b->T, L, hL, R, hR, b->w1, b->w2, b->zph, RES, hRES,
+                                by_range ? b->T.asm2_head_out : b->T.asm2_head, w0, w1, 0, nullptr, exps, nexps));
     b->launches++;
   }
   return cuda_status(cudaGetLastError());

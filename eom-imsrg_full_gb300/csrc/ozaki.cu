@@ -385,6 +385,7 @@ __device__ __forceinline__ double oz_scale(double d, int k) {
 __global__ void __launch_bounds__(256) k_oz_exponents(const OzChunk *chunks, const double *L, const double *R,
                                                       const double *LCC, const double *RCC, int *exps) {
   __shared__ int sh[8];
+  pdl_go();  // (the slicing's digit table does not wait)
   OzChunk c = chunks[blockIdx.x];
   const double *src = (c.src == 0 ? L : c.src == 1 ? R : c.src == 2 ? LCC : RCC) + c.off;
   // chunks hold at most 4 x 256 elements: four independent loads per thread
@@ -487,6 +488,7 @@ __global__ void __launch_bounds__(SLICE_THREADS) k_oz_slice(const OzMatrix *__re
     tab[i] = *reinterpret_cast<uint16_t *>(&h);
   }
   __syncthreads();
+  pdl_wait();
   const bool cimg = (int)blockIdx.x < cblocks;
   const int t = (cimg ? c_lo : r_lo) + ((int)blockIdx.x - (cimg ? 0 : cblocks)) * blockDim.x + threadIdx.x;
   if (t >= (cimg ? c_hi : r_hi)) return;
@@ -586,6 +588,12 @@ __global__ void __launch_bounds__(oz_threads(S), 1) k_oz_mma(const OzTile *__res
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem = *tmem_slot;
+  // The barriers, TMEM and tile records above are set up while the slicing ends.
+  // The slicing kernel does not call pdl_go(): these CTAs would sit on whole SMs
+  // that the 122 sums need.  Nor does this one: the recoupling inputs would take
+  // the warp slots ahead of the one-body assembly, whose heavy elements then come
+  // last (emax 4 commutator 31 -> 41 us, emax 6 105.3 -> 108.7, even from here).
+  pdl_wait();
 
   if (warp == 0) {
     if (lane == 0) {
@@ -811,10 +819,11 @@ __global__ void __launch_bounds__(oz_threads(S), 1) k_oz_mma(const OzTile *__res
 
 OzPlan *plan_of(imsrg_basis *b) { return (OzPlan *)b->ozaki; }
 
-void launch_mma(int S, bool chunked, int grid, cudaStream_t st, const OzTile *tiles, const int *sched_off,
+int launch_mma(bool pdl, int S, bool chunked, int grid, cudaStream_t st, const OzTile *tiles, const int *sched_off,
                 int hL, int hR, int *err, const CUtensorMap *maps, const int *act = nullptr) {
 #define OZ_LAUNCH(SS, CC) \
-  k_oz_mma<SS, CC><<<grid, oz_threads(SS), oz_mma_smem(SS), st>>>(tiles, sched_off, hL, hR, err, maps, act)
+  return cuda_status(launch_after(pdl, k_oz_mma<SS, CC>, grid, oz_threads(SS), oz_mma_smem(SS), st, tiles, sched_off, hL, \
+                                  hR, err, maps, act))
   switch (S) {
     case 4: if (chunked) OZ_LAUNCH(4, true); else OZ_LAUNCH(4, false); break;
     case 5: if (chunked) OZ_LAUNCH(5, true); else OZ_LAUNCH(5, false); break;
@@ -880,7 +889,8 @@ int autotune(imsrg_basis *b, OzPlan *pl, int hL, int hR) {
   IMSRG_CUDA_TRY(cudaEventCreate(&e1));
   auto launch_timed = [&](float *ms) -> int {
     IMSRG_CUDA_TRY(cudaEventRecord(e0, b->stream));
-    launch_mma(pl->S, pl->chunked, pl->grid, b->stream, pl->d_tiles, pl->d_sched_off, hL, hR, pl->d_err, pl->d_maps);
+    IMSRG_TRY(launch_mma(false, pl->S, pl->chunked, pl->grid, b->stream, pl->d_tiles, pl->d_sched_off, hL, hR, pl->d_err,
+                         pl->d_maps));
     b->launches++;
     IMSRG_CUDA_TRY(cudaEventRecord(e1, b->stream));
     IMSRG_CUDA_TRY(cudaEventSynchronize(e1));
@@ -1214,8 +1224,8 @@ int ozaki_slice(imsrg_basis *b, const double *L, const double *R, int p0, int p1
   if (nblk) {
     auto *kernel = pl->S == 4 ? k_oz_slice<4> : pl->S == 5 ? k_oz_slice<5> : pl->S == 6 ? k_oz_slice<6> :
                    pl->S == 7 ? k_oz_slice<7> : k_oz_slice<8>;
-    kernel<<<nblk, SLICE_THREADS, 0, st>>>(pl->d_mats, pl->d_mat_c, pl->d_mat_r, cblocks, c_lo, c_hi, r_lo, r_hi, L, R,
-                                           b->lcc, b->rcc, pl->d_exps, pl->img, pl->units * 256);
+    IMSRG_CUDA_TRY(launch_after(b->pdl, kernel, nblk, SLICE_THREADS, 0, st, pl->d_mats, pl->d_mat_c, pl->d_mat_r, cblocks, c_lo,
+                                c_hi, r_lo, r_hi, L, R, b->lcc, b->rcc, pl->d_exps, pl->img, pl->units * 256));
     b->launches++;
   }
   return cuda_status(cudaGetLastError());
@@ -1230,9 +1240,9 @@ int ozaki_mma(imsrg_basis *b, int hL, int hR) {
     if (cs == cudaStreamCaptureStatusNone) IMSRG_TRY(autotune(b, pl, hL, hR));
   }
   ProfScope ps(b, IMSRG_KERNEL_OZAKI_MMA);
-  launch_mma(pl->S, pl->chunked, pl->grid, b->stream, pl->d_tiles, pl->d_sched_off, hL, hR, pl->d_err, pl->d_maps);
   b->launches++;
-  return cuda_status(cudaGetLastError());
+  return launch_mma(b->pdl, pl->S, pl->chunked, pl->grid, b->stream, pl->d_tiles, pl->d_sched_off, hL, hR, pl->d_err,
+                    pl->d_maps);
 }
 
 int ozaki_check_error(imsrg_basis *b) {
@@ -1381,9 +1391,8 @@ int ozaki_batch_create(imsrg_basis *const *bases, int n, void **out) {
 int ozaki_batch_mma(void *batch, cudaStream_t st, int hL, int hR, const int *act) {
   OzBatch *bt = (OzBatch *)batch;
   if (!bt) return IMSRG_ERR_INVALID;
-  launch_mma(bt->plans[0]->S, bt->chunked, bt->grid, st, bt->d_tiles, bt->d_sched_off, hL, hR, bt->d_err, bt->d_maps,
-             act);
-  return cuda_status(cudaGetLastError());
+  return launch_mma(false, bt->plans[0]->S, bt->chunked, bt->grid, st, bt->d_tiles, bt->d_sched_off, hL, hR, bt->d_err,
+                    bt->d_maps, act);
 }
 
 int ozaki_batch_error(void *batch, cudaStream_t st) {

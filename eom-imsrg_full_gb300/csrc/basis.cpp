@@ -1051,9 +1051,12 @@ int build_basis(imsrg_basis *b) {
   b->mono = (double *)p;
   IMSRG_TRY(dev_alloc(b, 64 * sizeof(double), &p));
   b->scal = (double *)p;
-  b->partials_len = std::max(std::max(b->nchunks, b->nblocks), asm2_ctas(b)) + 64;
+  b->partials_len = std::max(std::max(2 * b->nchunks, b->nblocks), asm2_ctas(b)) + 64;
   IMSRG_TRY(dev_alloc(b, b->partials_len * sizeof(double), &p));
   b->partials = (double *)p;
+  IMSRG_TRY(dev_alloc(b, sizeof(unsigned), &p));
+  b->d_count = (unsigned *)p;
+  IMSRG_CUDA_TRY(cudaMemset(b->d_count, 0, sizeof(unsigned)));
   IMSRG_TRY(dev_alloc(b, std::max(b->nfull, b->neq) * sizeof(double), &p));
   b->d_stage = (double *)p;
   IMSRG_CUDA_TRY(cudaMallocHost(&b->h_scal, 64 * sizeof(double)));

@@ -171,4 +171,58 @@ __device__ __forceinline__ double block_sum_ops(double v, double *sh) {
   return r;
 }
 
+// a ax + b bx with its roundings spelled out, shared by every kernel that
+// updates a series sum, so the host-driven and graph-captured flows agree bit
+// for bit whatever the compiler would contract
+__device__ __forceinline__ double axpby_elem(double a, double ax, double b, double bx) {
+  return __fma_rn(b, bx, __dmul_rn(a, ax));
+}
+
+// true in every thread of the CTA that is the last of its grid to get here, with
+// the others' writes visible; *count is zero before and after
+__device__ __forceinline__ bool last_cta(unsigned *count) {
+  __shared__ bool last;
+  __threadfence();
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    last = atomicAdd(count, 1u) == gridDim.x - 1;
+    if (last) *count = 0;
+  }
+  __syncthreads();
+  if (last) __threadfence();
+  return last;
+}
+
+// The sum of n partials by one CTA, in thread 0 (read past L1: other CTAs may
+// have written them in the same launch).  One order for every caller.
+__device__ __forceinline__ double sum_partials(const double *partials, int n) {
+  __shared__ double sh[32];
+  double s = 0.0;
+  for (int i = threadIdx.x; i < n; i += blockDim.x) s += __ldcg(partials + i);
+  return block_sum_ops(s, sh);
+}
+
+// A series term's bookkeeping in one pass over the new term B: C += bx B, X0 = B
+// (the next term's operand, when X0 is set) and the CTA's mat_frob_norm partial
+// of B, in k_norm_partial's order (so the norm has its bits).  E0 (index 0) lies
+// outside the norm chunks and is updated by one thread.
+__device__ __forceinline__ void series_chunk(double *C, const double *__restrict__ B, double bx, double *X0,
+                                             const NormChunk &c, double *partials) {
+  __shared__ double sh[32];
+  double s = 0.0;
+  for (int i = threadIdx.x; i < c.len; i += blockDim.x) {
+    const long k = c.start + i;
+    const double x = B[k];
+    C[k] = axpby_elem(C[k], 1.0, x, bx);
+    if (X0) X0[k] = x;
+    s = fma(x, x, s);
+  }
+  if (blockIdx.x == 0 && threadIdx.x == 0) {
+    C[0] = axpby_elem(C[0], 1.0, B[0], bx);
+    if (X0) X0[0] = B[0];
+  }
+  s = block_sum_ops(s, sh);
+  if (threadIdx.x == 0) partials[blockIdx.x] = s * c.weight;
+}
+
 }  // namespace imsrg

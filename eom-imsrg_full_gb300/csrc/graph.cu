@@ -20,6 +20,7 @@
 // own workspace and streams) launch their step graphs back to back on their
 // own streams, so their kernels overlap on the device; each instance's
 // results equal its unbatched flow bit for bit.
+#include <algorithm>
 #include <cmath>
 #include <vector>
 
@@ -115,30 +116,70 @@ __device__ unsigned bch_next_go(FlowDev *F) {
   return go;
 }
 
-__global__ void k_magnus_init(FlowDev *F, cudaGraphConditionalHandle h) {
-  cudaGraphSetConditional(h, magnus_init_go(F));
-}
+// The kernels of the step graph each do what their neighbours in the chain would
+// otherwise wait for: nothing here is large, a link of the chain costs about two
+// microseconds, and a step had seventeen beside its commutators and one more per
+// series term (three emax 4 steps 1,759 -> 1,702 us, two emax 6 steps 3,207 ->
+// 3,155).
 
-__global__ void k_bch_init(FlowDev *F, cudaGraphConditionalHandle h, double ds) {
-  cudaGraphSetConditional(h, bch_init_go(F, ds));
-}
-
-// A series term's norm from its partials (k_final_sum's order, so the same
-// bits) and the series' stop test in one launch.
-template <bool MAGNUS>
-__global__ void __launch_bounds__(256) k_norm_next(const double *partials, int n, FlowDev *F,
-                                                   cudaGraphConditionalHandle h) {
+// MAGNUS_EXPAND set-up: X0 = DG (and X1's E0 slot, which with_e0 = 0 keeps), the
+// norms of DG and Omega by the last CTA, the series' first test.
+__global__ void __launch_bounds__(256) k_magnus_begin(const double *__restrict__ DG, const double *__restrict__ G,
+                                                      double *X0, double *X1, const NormChunk *chunks,
+                                                      double *partials, FlowDev *F, unsigned *count,
+                                                      cudaGraphConditionalHandle h) {
   __shared__ double sh[32];
-  double s = 0.0;
-  for (int i = threadIdx.x; i < n; i += blockDim.x) s += partials[i];
+  const NormChunk c = chunks[blockIdx.x];
+  double s = 0.0, g = 0.0;
+  for (int i = threadIdx.x; i < c.len; i += blockDim.x) {
+    const double x = DG[c.start + i], y = G[c.start + i];
+    X0[c.start + i] = x;
+    s = fma(x, x, s);
+    g = fma(y, y, g);
+  }
+  if (blockIdx.x == 0 && threadIdx.x == 0) X0[0] = X1[0] = DG[0];
   s = block_sum_ops(s, sh);
+  g = block_sum_ops(g, sh);
+  if (threadIdx.x == 0) {
+    partials[blockIdx.x] = s * c.weight;
+    partials[gridDim.x + blockIdx.x] = g * c.weight;
+  }
+  if (!last_cta(count)) return;
+  s = sum_partials(partials, gridDim.x);
+  g = sum_partials(partials + gridDim.x, gridDim.x);
+  if (threadIdx.x == 0) {
+    F->adv[1] = sqrt(s);
+    F->fullnorm = sqrt(g);
+    cudaGraphSetConditional(h, magnus_init_go(F));
+  }
+}
+
+// euler_step and the BCH_EXPAND set-up: Omega += ds DG, HS = X0 = H0.
+__global__ void __launch_bounds__(256) k_bch_begin(double *G, const double *__restrict__ DG, double ds,
+                                                   const double *__restrict__ H0, double *HS, double *X0, long n,
+                                                   FlowDev *F, cudaGraphConditionalHandle h) {
+  if (blockIdx.x == 0 && threadIdx.x == 0) cudaGraphSetConditional(h, bch_init_go(F, ds));
+  const long stride = (long)gridDim.x * blockDim.x;
+  for (long i = (long)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += stride) {
+    G[i] = axpby_elem(G[i], 1.0, DG[i], ds);
+    HS[i] = X0[i] = H0[i];
+  }
+}
+
+// A series term: the sum's update (series_chunk), then its norm and the series'
+// stop test by the last CTA (which rewrites the coefficient that every CTA has read).
+template <bool MAGNUS>
+__global__ void __launch_bounds__(256) k_series_next(double *C, const double *__restrict__ B, double *X0,
+                                                     const NormChunk *chunks, double *partials, FlowDev *F,
+                                                     unsigned *count, cudaGraphConditionalHandle h) {
+  series_chunk(C, B, MAGNUS ? F->cof : F->coef, X0, chunks[blockIdx.x], partials);
+  if (!last_cta(count)) return;
+  const double s = sum_partials(partials, gridDim.x);
   if (threadIdx.x == 0) {
     F->nrm = sqrt(s);
     cudaGraphSetConditional(h, MAGNUS ? magnus_next_go(F) : bch_next_go(F));
   }
 }
-
-__global__ void k_step_end(FlowDev *F, const double *HS) { F->e0 = HS[0]; }
 
 }  // namespace
 
@@ -194,7 +235,6 @@ int add_while(cudaGraph_t g, const std::vector<cudaGraphNode_t> &deps, cudaGraph
 int build_step_graph(imsrg_basis *b, FlowGraph *fg, imsrg_op *HS, imsrg_op *G, imsrg_op *H0, imsrg_op *DG,
                      imsrg_op *X0, imsrg_op *X1, int precision, double ds) {
   FlowDev *F = fg->d_state;
-  const long nb = b->nfull * (long)sizeof(double);
   cudaGraph_t g = nullptr;
   IMSRG_CUDA_TRY(cudaGraphCreate(&g, 0));
   fg->graph = g;
@@ -202,13 +242,9 @@ int build_step_graph(imsrg_basis *b, FlowGraph *fg, imsrg_op *HS, imsrg_op *G, i
   IMSRG_CUDA_TRY(cudaGraphConditionalHandleCreate(&hM, g, 0, 0));
   IMSRG_CUDA_TRY(cudaGraphConditionalHandleCreate(&hB, g, 0, 0));
   std::vector<cudaGraphNode_t> fr;
-  // MAGNUS_EXPAND set-up: X0 = DG (and X1's E0 slot, which with_e0 = 0 keeps)
   IMSRG_TRY(capture(b, g, {}, [&]() -> int {
-    IMSRG_CUDA_TRY(cudaMemcpyAsync(X0->d, DG->d, nb, cudaMemcpyDeviceToDevice, b->stream));
-    IMSRG_CUDA_TRY(cudaMemcpyAsync(X1->d, DG->d, sizeof(double), cudaMemcpyDeviceToDevice, b->stream));
-    IMSRG_TRY(launch_norm(b, X0->d, &F->adv[1]));
-    IMSRG_TRY(launch_norm(b, G->d, &F->fullnorm));
-    k_magnus_init<<<1, 1, 0, b->stream>>>(F, hM);
+    k_magnus_begin<<<b->nchunks, 256, 0, b->stream>>>(DG->d, G->d, X0->d, X1->d, b->d_chunks, b->partials, F,
+                                                      b->d_count, hM);
     return cuda_status(cudaGetLastError());
   }, &fr));
   cudaGraphNode_t wm, wb;
@@ -217,32 +253,28 @@ int build_step_graph(imsrg_basis *b, FlowGraph *fg, imsrg_op *HS, imsrg_op *G, i
   // one Magnus term: X1 = [G, X0]; DG += cof X1; |X1|; X0 = X1
   IMSRG_TRY(capture(b, body, {}, [&]() -> int {
     IMSRG_TRY(commutator_dev(b, G->d, G->herm, X0->d, -1, X1->d, -G->herm * -1, precision, 0));
-    IMSRG_TRY(launch_series_update(b, DG->d, X1->d, &F->cof, X0->d, nullptr));
-    k_norm_next<true><<<1, 256, 0, b->stream>>>(b->partials, b->nchunks, F, hM);
+    k_series_next<true><<<b->nchunks, 256, 0, b->stream>>>(DG->d, X1->d, X0->d, b->d_chunks, b->partials, F,
+                                                           b->d_count, hM);
     return cuda_status(cudaGetLastError());
   }, nullptr));
   // euler_step, then BCH_EXPAND set-up: HS = H0, X0 = H0
   IMSRG_TRY(capture(b, g, {wm}, [&]() -> int {
-    IMSRG_TRY(launch_axpby(b, G->d, 1.0, DG->d, ds, G->d));
-    IMSRG_CUDA_TRY(cudaMemcpyAsync(HS->d, H0->d, nb, cudaMemcpyDeviceToDevice, b->stream));
-    IMSRG_CUDA_TRY(cudaMemcpyAsync(X0->d, H0->d, nb, cudaMemcpyDeviceToDevice, b->stream));
-    k_bch_init<<<1, 1, 0, b->stream>>>(F, hB, ds);
+    k_bch_begin<<<(unsigned)std::min<long>((b->nfull + 255) / 256, 152 * 8), 256, 0, b->stream>>>(
+        G->d, DG->d, ds, H0->d, HS->d, X0->d, b->nfull, F, hB);
     return cuda_status(cudaGetLastError());
   }, &fr));
   IMSRG_TRY(add_while(g, fr, hB, &wb, &body));
   // one BCH term: X1 = [G, X0] (with E0); HS += X1 / n!; |X1|; X0 = X1
   IMSRG_TRY(capture(b, body, {}, [&]() -> int {
     IMSRG_TRY(commutator_dev(b, G->d, G->herm, X0->d, H0->herm, X1->d, -G->herm * H0->herm, precision, 1));
-    IMSRG_TRY(launch_series_update(b, HS->d, X1->d, &F->coef, X0->d, nullptr));
-    k_norm_next<false><<<1, 256, 0, b->stream>>>(b->partials, b->nchunks, F, hB);
+    k_series_next<false><<<b->nchunks, 256, 0, b->stream>>>(HS->d, X1->d, X0->d, b->d_chunks, b->partials, F,
+                                                            b->d_count, hB);
     return cuda_status(cudaGetLastError());
   }, nullptr));
   // next generator and the stop criterion
   IMSRG_TRY(capture(b, g, {wb}, [&]() -> int {
     IMSRG_TRY(launch_white(b, HS->d, HS->herm, DG->d));
-    IMSRG_TRY(launch_mbpt2(b, HS->d, HS->herm, &F->emp2));
-    k_step_end<<<1, 1, 0, b->stream>>>(F, HS->d);
-    return cuda_status(cudaGetLastError());
+    return launch_mbpt2(b, HS->d, HS->herm, &F->emp2, &F->e0);
   }, nullptr));
   IMSRG_CUDA_TRY(cudaGraphInstantiate(&fg->exec, g, 0));
   return IMSRG_OK;
@@ -302,8 +334,7 @@ int flow_graph_begin(imsrg_op *HS, imsrg_op *G, int precision, double ds, double
   IMSRG_TRY(launch_white(b, HS->d, HS->herm, DG->d));
   IMSRG_CUDA_TRY(cudaMemcpyAsync(H0->d, HS->d, b->nfull * sizeof(double), cudaMemcpyDeviceToDevice, b->stream));
   H0->herm = HS->herm;
-  IMSRG_TRY(launch_mbpt2(b, HS->d, HS->herm, &fg->d_state->emp2));
-  k_step_end<<<1, 1, 0, b->stream>>>(fg->d_state, HS->d);
+  IMSRG_TRY(launch_mbpt2(b, HS->d, HS->herm, &fg->d_state->emp2, &fg->d_state->e0));
   IMSRG_CUDA_TRY(cudaMemsetAsync(&fg->d_state->s, 0, sizeof(double), b->stream));
   IMSRG_CUDA_TRY(cudaMemcpyAsync(fg->h_state, fg->d_state, sizeof(FlowDev), cudaMemcpyDeviceToHost, b->stream));
   IMSRG_CUDA_TRY(cudaStreamSynchronize(b->stream));
@@ -601,9 +632,7 @@ int build_batch_graph(BatchFlowGraph *f, imsrg_basis *const *bases, void *oz, cu
     IMSRG_TRY(add_if(g, {wb}, h[2 * n + i], &node, &body));
     IMSRG_TRY(capture(b, body, {}, [&]() -> int {
       IMSRG_TRY(launch_white(b, HS[i]->d, HS[i]->herm, DG[i]->d));
-      IMSRG_TRY(launch_mbpt2(b, HS[i]->d, HS[i]->herm, &F->emp2));
-      k_step_end<<<1, 1, 0, b->stream>>>(F, HS[i]->d);
-      return cuda_status(cudaGetLastError());
+      return launch_mbpt2(b, HS[i]->d, HS[i]->herm, &F->emp2, &F->e0);
     }, nullptr));
   }
   IMSRG_CUDA_TRY(cudaGraphInstantiate(&f->exec, g, 0));
@@ -665,8 +694,7 @@ int batch_flow_run(imsrg_basis *const *bases, int n, void *oz, cudaStream_t st, 
     IMSRG_TRY(launch_white(b, HS[i]->d, HS[i]->herm, DG->d));
     IMSRG_CUDA_TRY(cudaMemcpyAsync(H0->d, HS[i]->d, b->nfull * sizeof(double), cudaMemcpyDeviceToDevice, b->stream));
     H0->herm = HS[i]->herm;
-    IMSRG_TRY(launch_mbpt2(b, HS[i]->d, HS[i]->herm, &f->d_state[i].emp2));
-    k_step_end<<<1, 1, 0, b->stream>>>(f->d_state + i, HS[i]->d);
+    IMSRG_TRY(launch_mbpt2(b, HS[i]->d, HS[i]->herm, &f->d_state[i].emp2, &f->d_state[i].e0));
     IMSRG_CUDA_TRY(cudaMemsetAsync(&f->d_state[i].s, 0, sizeof(double), b->stream));
   }
   for (int i = 0; i < n; i++) IMSRG_CUDA_TRY(cudaStreamSynchronize(bases[i]->stream));

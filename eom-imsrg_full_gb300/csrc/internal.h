@@ -316,6 +316,7 @@ struct imsrg_basis {
   double *partials = nullptr;   // norm/mbpt2 partial sums
   double *h_scal = nullptr;     // pinned host mirror of scal
   int partials_len = 0;
+  unsigned *d_count = nullptr;  // arrivals of a reduction's CTAs on the basis stream; zero between launches
   // grouped GEMM problems
   imsrg::GemmProb *d_probs = nullptr;
   imsrg::GemmTile *d_tiles = nullptr;
@@ -436,13 +437,12 @@ int launch_axpby(imsrg_basis *b, const double *A, double ax, const double *B, do
 int launch_axpby_dev(imsrg_basis *b, const double *A, double ax, const double *B, const double *bx, double *C);
 // S += *coef_dev X1, X0 = X1 (unless X0 is null), *d_norm = mat_frob_norm(X1):
 // one series term's bookkeeping in one pass over X1 (the same values as
-// launch_axpby_dev, a copy and launch_norm).  d_norm null: the norm's
-// partials stay in b->partials (b->nchunks of them) for a kernel that sums
-// them with block_sum_ops in k_final_sum's order
+// launch_axpby_dev, a copy and launch_norm)
 int launch_series_update(imsrg_basis *b, double *S, const double *X1, const double *coef_dev, double *X0,
                          double *d_norm);
 int launch_norm(imsrg_basis *b, const double *op, double *d_out);
-int launch_mbpt2(imsrg_basis *b, const double *H, int herm, double *d_out);
+// (d_e0 set: also H's E0 there)
+int launch_mbpt2(imsrg_basis *b, const double *H, int herm, double *d_out, double *d_e0 = nullptr);
 int launch_white(imsrg_basis *b, const double *H, int hH, double *ETA);
 int launch_generator(imsrg_basis *b, const double *Hden, int hH, const double *Hnum, int use_atan, double *ETA);
 int launch_white_tangent(imsrg_basis *b, const double *H, const double *dH, int hH, double *dETA);

@@ -17,13 +17,6 @@ namespace {
 
 // C = ax A + bx B; bx_dev, when given, supplies bx from device memory (the
 // graph-captured flow), with the same arithmetic as the scalar form.
-// a ax + b bx with its roundings spelled out, shared by every kernel that
-// updates a series sum, so the host-driven and graph-captured flows agree bit
-// for bit whatever the compiler would contract
-__device__ __forceinline__ double axpby_elem(double a, double ax, double b, double bx) {
-  return __fma_rn(b, bx, __dmul_rn(a, ax));
-}
-
 __global__ void k_axpby(const double *__restrict__ A, double ax, const double *__restrict__ B, double bx,
                         const double *bx_dev, double *__restrict__ C, long n) {
   if (bx_dev) bx = *bx_dev;
@@ -46,44 +39,21 @@ __global__ void __launch_bounds__(256) k_norm_partial(const double *__restrict__
   if (threadIdx.x == 0) partials[blockIdx.x] = s * c.weight;
 }
 
-// One Magnus or BCH series term's bookkeeping in one pass over the new term
-// B: C = A + bx B (the sum), X0 = B (the next term's operand, when X0 is set)
-// and B's mat_frob_norm partials, chunk by chunk in k_norm_partial's order
-// (so k_final_sum gives the same norm bit for bit).  E0 (index 0) lies
-// outside the norm chunks and is updated by one thread.
-__global__ void __launch_bounds__(256) k_series_update(const double *A, const double *__restrict__ B,
-                                                       const double *bx_dev, double *C, double *X0,
-                                                       const NormChunk *chunks, double *partials) {
-  __shared__ double sh[32];
-  const double bx = *bx_dev;
-  const NormChunk c = chunks[blockIdx.x];
-  double s = 0.0;
-  for (int i = threadIdx.x; i < c.len; i += blockDim.x) {
-    const long k = c.start + i;
-    const double x = B[k];
-    C[k] = axpby_elem(A[k], 1.0, x, bx);
-    if (X0) X0[k] = x;
-    s = fma(x, x, s);
-  }
-  if (blockIdx.x == 0 && threadIdx.x == 0) {
-    C[0] = axpby_elem(A[0], 1.0, B[0], bx);
-    if (X0) X0[0] = B[0];
-  }
-  s = block_sum_ops(s, sh);
-  if (threadIdx.x == 0) partials[blockIdx.x] = s * c.weight;
+// One Magnus or BCH series term's bookkeeping in one pass (series_chunk).
+__global__ void __launch_bounds__(256) k_series_update(double *C, const double *__restrict__ B, const double *bx_dev,
+                                                       double *X0, const NormChunk *chunks, double *partials) {
+  series_chunk(C, B, *bx_dev, X0, chunks[blockIdx.x], partials);
 }
 
 __global__ void __launch_bounds__(256) k_final_sum(const double *partials, int n, double *out, int take_sqrt) {
-  __shared__ double sh[32];
-  double s = 0.0;
-  for (int i = threadIdx.x; i < n; i += blockDim.x) s += partials[i];
-  s = block_sum_ops(s, sh);
+  const double s = sum_partials(partials, n);
   if (threadIdx.x == 0) *out = take_sqrt ? sqrt(s) : s;
 }
 
 // mbpt2: one CTA per block q; partial = (2J+1) * sum Gamma_pphh^2 / eden
-__global__ void __launch_bounds__(256) k_mbpt2_partial(DevTables T, const double *__restrict__ H, int herm,
-                                                       double *partials) {
+// The last CTA adds the partials to *out, and copies E0 to *e0 if set.
+__global__ void __launch_bounds__(256) k_mbpt2(DevTables T, const double *__restrict__ H, int herm, double *partials,
+                                               double *out, double *e0, unsigned *count) {
   __shared__ double sh[32];
   int q = blockIdx.x;
   int np = T.gam_n1[q * 6 + 2], nh = T.gam_n2[q * 6 + 2];
@@ -102,11 +72,28 @@ __global__ void __launch_bounds__(256) k_mbpt2_partial(DevTables T, const double
   }
   s = block_sum_ops(s, sh);
   if (threadIdx.x == 0) partials[q] = (T.blk_J2[q] + 1.0) * s;
+  if (!last_cta(count)) return;
+  const double sum = sum_partials(partials, gridDim.x);
+  if (threadIdx.x == 0) {
+    *out = sum;
+    if (e0) *e0 = H[0];
+  }
 }
 
-// twobody_monopole(a, b) for every ordered orbit pair
-__global__ void k_monopole(DevTables T, const double *__restrict__ H, int herm, double *mono) {
+constexpr int MONO_THREADS = 128;
+__host__ __device__ constexpr int mono_ctas(int norb) { return (norb * norb + MONO_THREADS - 1) / MONO_THREADS; }
+
+// twobody_monopole(a, b) for every ordered orbit pair by the first CTAs; the
+// rest, where there are any, clear the n doubles at z (the generator to come: a
+// memset ahead of this kernel was one more link of the step's chain)
+__global__ void k_monopole(DevTables T, const double *__restrict__ H, int herm, double *mono, double *z, long n) {
   int t = blockIdx.x * blockDim.x + threadIdx.x;
+  const int own = mono_ctas(T.norb);
+  if ((int)blockIdx.x >= own) {
+    const long stride = (long)(gridDim.x - own) * blockDim.x;
+    for (long i = t - (long)own * blockDim.x; i < n; i += stride) z[i] = 0.0;
+    return;
+  }
   if (t >= T.norb * T.norb) return;
   int a = t / T.norb, b = t % T.norb;
   int ja = T.orb[a].x, jb = T.orb[b].x;
@@ -399,12 +386,9 @@ int launch_axpby_dev(imsrg_basis *b, const double *A, double ax, const double *B
 int launch_series_update(imsrg_basis *b, double *S, const double *X1, const double *coef_dev, double *X0,
                          double *d_norm) {
   ProfScope ps(b, IMSRG_KERNEL_OPS);
-  k_series_update<<<b->nchunks, 256, 0, b->stream>>>(S, X1, coef_dev, S, X0, b->d_chunks, b->partials);
-  b->launches++;
-  if (d_norm) {
-    k_final_sum<<<1, 256, 0, b->stream>>>(b->partials, b->nchunks, d_norm, 1);
-    b->launches++;
-  }
+  k_series_update<<<b->nchunks, 256, 0, b->stream>>>(S, X1, coef_dev, X0, b->d_chunks, b->partials);
+  k_final_sum<<<1, 256, 0, b->stream>>>(b->partials, b->nchunks, d_norm, 1);
+  b->launches += 2;
   return cuda_status(cudaGetLastError());
 }
 
@@ -416,20 +400,19 @@ int launch_norm(imsrg_basis *b, const double *op, double *d_out) {
   return cuda_status(cudaGetLastError());
 }
 
-int launch_mbpt2(imsrg_basis *b, const double *H, int herm, double *d_out) {
+int launch_mbpt2(imsrg_basis *b, const double *H, int herm, double *d_out, double *d_e0) {
   ProfScope ps(b, IMSRG_KERNEL_OPS);
-  k_mbpt2_partial<<<b->nblocks, 256, 0, b->stream>>>(b->T, H, herm, b->partials);
-  k_final_sum<<<1, 256, 0, b->stream>>>(b->partials, b->nblocks, d_out, 0);
-  b->launches += 2;
+  k_mbpt2<<<b->nblocks, 256, 0, b->stream>>>(b->T, H, herm, b->partials, d_out, d_e0, b->d_count);
+  b->launches++;
   return cuda_status(cudaGetLastError());
 }
 
 int launch_generator(imsrg_basis *b, const double *Hden, int hH, const double *Hnum, int use_atan, double *ETA) {
   double *mono = b->mono;
   ProfScope ps(b, IMSRG_KERNEL_OPS);
-  IMSRG_CUDA_TRY(cudaMemsetAsync(ETA + 1, 0, (b->nfull - 1) * sizeof(double), b->stream));
-  int nn = b->norb * b->norb;
-  k_monopole<<<(nn + 127) / 128, 128, 0, b->stream>>>(b->T, Hden, hH, mono);
+  const long nz = b->nfull - 1;
+  const int zero = (int)std::min<long>((nz + 4 * MONO_THREADS - 1) / (4 * MONO_THREADS), 152 * 8);
+  k_monopole<<<mono_ctas(b->norb) + zero, MONO_THREADS, 0, b->stream>>>(b->T, Hden, hH, mono, ETA + 1, nz);
   long n3 = 0;
   for (int q = 0; q < b->nblocks; q++) n3 += (long)b->gam_n1[q * 6 + 2] * b->gam_n2[q * 6 + 2];
   long n = (long)b->P * b->A + n3;
@@ -447,9 +430,8 @@ int launch_white_tangent(imsrg_basis *b, const double *H, const double *dH, int 
   double *mono = b->mono, *dmono = b->mono + (long)b->norb * b->norb;
   ProfScope ps(b, IMSRG_KERNEL_OPS);
   IMSRG_CUDA_TRY(cudaMemsetAsync(dETA, 0, b->nfull * sizeof(double), b->stream));
-  int nn = b->norb * b->norb;
-  k_monopole<<<(nn + 127) / 128, 128, 0, b->stream>>>(b->T, H, hH, mono);
-  k_monopole<<<(nn + 127) / 128, 128, 0, b->stream>>>(b->T, dH, hH, dmono);
+  k_monopole<<<mono_ctas(b->norb), MONO_THREADS, 0, b->stream>>>(b->T, H, hH, mono, nullptr, 0);
+  k_monopole<<<mono_ctas(b->norb), MONO_THREADS, 0, b->stream>>>(b->T, dH, hH, dmono, nullptr, 0);
   long n3 = 0;
   for (int q = 0; q < b->nblocks; q++) n3 += (long)b->gam_n1[q * 6 + 2] * b->gam_n2[q * 6 + 2];
   long n = (long)b->P * b->A + n3;
@@ -464,7 +446,7 @@ int launch_white_adjoint(imsrg_basis *b, const double *H, int hH, const double *
   const int nn = b->norb * b->norb;
   ProfScope ps(b, IMSRG_KERNEL_OPS);
   IMSRG_CUDA_TRY(cudaMemsetAsync(monob, 0, nn * sizeof(double), b->stream));
-  k_monopole<<<(nn + 127) / 128, 128, 0, b->stream>>>(b->T, H, hH, mono);
+  k_monopole<<<mono_ctas(b->norb), MONO_THREADS, 0, b->stream>>>(b->T, H, hH, mono, nullptr, 0);
   long n3 = 0;
   for (int q = 0; q < b->nblocks; q++) n3 += (long)b->gam_n1[q * 6 + 2] * b->gam_n2[q * 6 + 2];
   const long n = (long)b->P * b->A + n3;

@@ -172,7 +172,9 @@ template <bool MAGNUS>
 __global__ void __launch_bounds__(256) k_series_next(double *C, const double *__restrict__ B, double *X0,
                                                      const NormChunk *chunks, double *partials, FlowDev *F,
                                                      unsigned *count, cudaGraphConditionalHandle h) {
-  series_chunk(C, B, MAGNUS ? F->cof : F->coef, X0, chunks[blockIdx.x], partials);
+  const NormChunk c = chunks[blockIdx.x];
+  pdl_wait();
+  series_chunk(C, B, MAGNUS ? F->cof : F->coef, X0, c, partials);
   if (!last_cta(count)) return;
   const double s = sum_partials(partials, gridDim.x);
   if (threadIdx.x == 0) {
@@ -253,9 +255,8 @@ int build_step_graph(imsrg_basis *b, FlowGraph *fg, imsrg_op *HS, imsrg_op *G, i
   // one Magnus term: X1 = [G, X0]; DG += cof X1; |X1|; X0 = X1
   IMSRG_TRY(capture(b, body, {}, [&]() -> int {
     IMSRG_TRY(commutator_dev(b, G->d, G->herm, X0->d, -1, X1->d, -G->herm * -1, precision, 0));
-    k_series_next<true><<<b->nchunks, 256, 0, b->stream>>>(DG->d, X1->d, X0->d, b->d_chunks, b->partials, F,
-                                                           b->d_count, hM);
-    return cuda_status(cudaGetLastError());
+    return cuda_status(launch_after(true, k_series_next<true>, b->nchunks, 256, 0, b->stream, DG->d, X1->d, X0->d,
+                                    b->d_chunks, b->partials, F, b->d_count, hM));
   }, nullptr));
   // euler_step, then BCH_EXPAND set-up: HS = H0, X0 = H0
   IMSRG_TRY(capture(b, g, {wm}, [&]() -> int {
@@ -267,9 +268,8 @@ int build_step_graph(imsrg_basis *b, FlowGraph *fg, imsrg_op *HS, imsrg_op *G, i
   // one BCH term: X1 = [G, X0] (with E0); HS += X1 / n!; |X1|; X0 = X1
   IMSRG_TRY(capture(b, body, {}, [&]() -> int {
     IMSRG_TRY(commutator_dev(b, G->d, G->herm, X0->d, H0->herm, X1->d, -G->herm * H0->herm, precision, 1));
-    k_series_next<false><<<b->nchunks, 256, 0, b->stream>>>(HS->d, X1->d, X0->d, b->d_chunks, b->partials, F,
-                                                            b->d_count, hB);
-    return cuda_status(cudaGetLastError());
+    return cuda_status(launch_after(true, k_series_next<false>, b->nchunks, 256, 0, b->stream, HS->d, X1->d, X0->d,
+                                    b->d_chunks, b->partials, F, b->d_count, hB));
   }, nullptr));
   // next generator and the stop criterion
   IMSRG_TRY(capture(b, g, {wb}, [&]() -> int {

@@ -15,7 +15,7 @@
 #include <new>
 #include <vector>
 
-#include "internal.h"
+#include "front.cuh"
 
 using imsrg::cuda_status;
 
@@ -110,7 +110,7 @@ int commutator_launches(imsrg_basis *b, const double *L, int hL, const double *R
   // same order, so each kernel class's event pair times that kernel alone.
   const bool serial = b->prof.on;
   b->pdl = phases == kPhaseAll;
-  cudaStream_t side = serial ? b->stream : b->side, side2 = serial ? b->stream : b->side2;
+  cudaStream_t side = b->side;
   const size_t bytes = (size_t)b->nfull * sizeof(double);
   const bool oz = precision == IMSRG_PREC_OZAKI;
   // Page-locked host operands (outside profiling): R is copied first, so its
@@ -123,11 +123,16 @@ int commutator_launches(imsrg_basis *b, const double *L, int hL, const double *R
   const size_t pbytes = (size_t)b->neq * sizeof(double);
   // packed page-locked operands the device addresses: no staging copies
   const bool direct = overlap && packed && io->Ldev && io->Rdev && io->RESdev;
-  // the transform also reduces the LCC/RCC block exponents (split precision)
-  int *cc_exps = nullptr, gL = 0, gR = 0;
+  // Split commutators of small bases run one chain of shared launches (front.cuh):
+  // the 122 sums and the one-body part ahead of the products in the slicing's
+  // launch, the rest of the one-body part in the two-body assembly's.  Else the
+  // sums run on side4 and the one-body assembly on side after the products.
+  const bool shared = oz && b->T.ph_terms, merged = shared && !overlap && !serial;
+  const SumsArgs sums{L, R, RES, hL, hR, hRES, merged ? one_body_ctas(b->T) : 0};
+  // the transform also reduces the LCC/RCC block exponents, where it can
+  const bool cc_part = oz && !b->T.ccf_packed;
   if (oz && front) IMSRG_TRY(ozaki_exps_begin(b));
   if (overlap) {
-    if (oz) IMSRG_TRY(ozaki_cc_exponents(b, &cc_exps, &gL, &gR));
     if (direct) {
       // the unpack kernels of R (side2) and L read the host arrays at once
       IMSRG_CUDA_TRY(cudaEventRecord(b->ev_hostR, b->stream));
@@ -149,54 +154,41 @@ int commutator_launches(imsrg_basis *b, const double *L, int hL, const double *R
       IMSRG_CUDA_TRY(cudaMemcpyAsync(const_cast<double *>(L), io->L, bytes, cudaMemcpyHostToDevice, b->stream));
       IMSRG_CUDA_TRY(cudaStreamWaitEvent(b->side2, b->ev_hostR, 0));
     }
+    IMSRG_TRY(launch_front(b, L, hL, R, hR, Front{1, oz ? 2 : 1, 2, oz}, b->side2));
     if (oz) IMSRG_TRY(ozaki_slice(b, L, R, 1, 2, b->side2));
-    IMSRG_TRY(launch_cc_forward(b, L, hL, R, hR, cc_exps, gL, gR, 2, b->side2));
     IMSRG_CUDA_TRY(cudaEventRecord(b->ev_join2, b->side2));
   } else if (io && packed) {  // pageable packed host operands, one after the other
     IMSRG_CUDA_TRY(cudaMemcpyAsync(io->Lst, io->L, pbytes, cudaMemcpyHostToDevice, b->stream));
     IMSRG_TRY(launch_unpack(b, io->Lst, hL, const_cast<double *>(L), b->stream));
-    IMSRG_CUDA_TRY(cudaEventRecord(b->ev_hostL, b->stream));
     IMSRG_CUDA_TRY(cudaMemcpyAsync(io->Rst, io->R, pbytes, cudaMemcpyHostToDevice, b->stream));
     IMSRG_TRY(launch_unpack(b, io->Rst, hR, const_cast<double *>(R), b->stream));
-  } else if (io) {  // pageable host operands: L first, so the digit images of L start while R is in flight
+  } else if (io) {  // pageable host operands
     IMSRG_CUDA_TRY(cudaMemcpyAsync(const_cast<double *>(L), io->L, bytes, cudaMemcpyHostToDevice, b->stream));
-    IMSRG_CUDA_TRY(cudaEventRecord(b->ev_hostL, b->stream));
     IMSRG_CUDA_TRY(cudaMemcpyAsync(const_cast<double *>(R), io->R, bytes, cudaMemcpyHostToDevice, b->stream));
   }
-  auto fork = [&](int k) -> int {
-    if (serial) return IMSRG_OK;
-    IMSRG_CUDA_TRY(cudaEventRecord(b->ev_fork[k], b->stream));
-    IMSRG_CUDA_TRY(cudaStreamWaitEvent(b->side, (io && !overlap && k == 0) ? b->ev_hostL : b->ev_fork[k], 0));
-    return IMSRG_OK;
-  };
-  auto join = [&](int k) -> int {
-    if (serial) return IMSRG_OK;
-    IMSRG_CUDA_TRY(cudaEventRecord(b->ev_join[k], b->side));
-    IMSRG_CUDA_TRY(cudaStreamWaitEvent(b->stream, b->ev_join[k], 0));
-    return IMSRG_OK;
-  };
-  // E0 and the commutator_122 part of the two-body assembly need only L and
-  // R: E0's single CTA runs on side3 and the 122 sums on side4 from where
-  // ev_fork[0] is recorded, beside the Pandya transform, the slicing and the
-  // products.  E0 is joined at the end (after the one-body assembly, where it
-  // ran before, it finished last: the one-body kernel runs slowly beside the
-  // 3,769 CTAs of the two-body assembly), the 122 sums before the rest of the
-  // two-body assembly.
-  auto sums_beside = [&]() -> int {
+  // E0 needs only L and R: its single CTA runs on side3 from where ev_fork[0] is
+  // recorded, and is joined at the end.
+  auto branches = [&]() -> int {
     if (serial) {
       if (with_e0) IMSRG_TRY(launch_e0(b, L, hL, R, hR, RES, b->stream));
-      return launch_asm2_122(b, L, hL, R, hR, RES, hRES, b->stream);
+      return launch_sums_122(b, sums, b->stream);
     }
-    for (cudaStream_t s : {b->side3, b->side4}) {
+    auto on = [&](cudaStream_t s) -> int {
       IMSRG_CUDA_TRY(cudaStreamWaitEvent(s, b->ev_fork[0], 0));
       if (overlap && packed) IMSRG_CUDA_TRY(cudaStreamWaitEvent(s, b->ev_rdev, 0));
-    }
+      return IMSRG_OK;
+    };
     if (with_e0) {
+      IMSRG_TRY(on(b->side3));
       IMSRG_TRY(launch_e0(b, L, hL, R, hR, RES, b->side3));
       IMSRG_CUDA_TRY(cudaEventRecord(b->ev_join3, b->side3));
     }
-    IMSRG_TRY(launch_asm2_122(b, L, hL, R, hR, RES, hRES, b->side4));
-    return cuda_status(cudaEventRecord(b->ev_pre, b->side4));
+    if (!merged) {
+      IMSRG_TRY(on(b->side4));
+      IMSRG_TRY(launch_sums_122(b, sums, b->side4));
+      IMSRG_CUDA_TRY(cudaEventRecord(b->ev_pre, b->side4));
+    }
+    return IMSRG_OK;
   };
   const bool e0_front = (phases & kPhaseJoinE0Front) != 0;
   auto join_e0 = [&]() -> int {
@@ -204,53 +196,61 @@ int commutator_launches(imsrg_basis *b, const double *L, int hL, const double *R
     return IMSRG_OK;
   };
   auto join_pre = [&]() -> int {
-    if (!serial) IMSRG_CUDA_TRY(cudaStreamWaitEvent(b->stream, b->ev_pre, 0));
+    if (!merged && !serial) IMSRG_CUDA_TRY(cudaStreamWaitEvent(b->stream, b->ev_pre, 0));
     return IMSRG_OK;
   };
   if (overlap) {  // R's half is under way on side2; L's half once L is in
-    IMSRG_TRY(fork(0));
-    IMSRG_TRY(sums_beside());
-    if (oz) IMSRG_TRY(ozaki_slice(b, L, R, 0, 1, side));
-    IMSRG_TRY(launch_cc_forward(b, L, hL, R, hR, cc_exps, gL, gR, 1));
+    IMSRG_CUDA_TRY(cudaEventRecord(b->ev_fork[0], b->stream));
+    IMSRG_TRY(branches());
+    IMSRG_TRY(launch_front(b, L, hL, R, hR, Front{0, oz ? 1 : 0, 1, oz}, b->stream));
+    if (oz) {
+      IMSRG_CUDA_TRY(cudaEventRecord(b->ev_fork[1], b->stream));
+      IMSRG_CUDA_TRY(cudaStreamWaitEvent(side, b->ev_fork[1], 0));
+      IMSRG_TRY(ozaki_slice(b, L, R, 0, 1, side));
+      IMSRG_CUDA_TRY(cudaEventRecord(b->ev_join[0], side));
+    }
     IMSRG_CUDA_TRY(cudaStreamWaitEvent(b->stream, b->ev_join2, 0));
     if (oz) {
-      IMSRG_TRY(ozaki_slice(b, L, R, 2, 3, b->stream, cc_exps != nullptr));
-      IMSRG_TRY(join(0));
+      if (cc_part) IMSRG_TRY(launch_front(b, L, hL, R, hR, Front{2, 3, 0}, b->stream));
+      IMSRG_TRY(ozaki_slice(b, L, R, 2, 3, b->stream));
+      IMSRG_CUDA_TRY(cudaStreamWaitEvent(b->stream, b->ev_join[0], 0));
       IMSRG_TRY(ozaki_mma(b, hL, hR));
     } else {
-      IMSRG_TRY(join(0));
       IMSRG_TRY(launch_gemm_fp64(b, L, hL, R, hR));
     }
-  } else if (oz) {
-    // digit images of L and R on a side stream (of R on a second one where the
-    // host's R is still in flight), beside the Pandya transform and the images
-    // of LCC and RCC.  The 122 sums come after them in launch order: a graph
-    // starts its branches in that order, and ahead of them their CTAs took the
-    // warp slots (two emax 6 flow steps: 3,400 us with the sums first, 3,285 so)
-    if (front) {
-      const bool two = io && !serial;
-      IMSRG_TRY(fork(0));
-      if (two) IMSRG_CUDA_TRY(cudaStreamWaitEvent(b->side2, b->ev_fork[0], 0));
-      IMSRG_TRY(ozaki_slice(b, L, R, 0, two ? 1 : 2, side));
-      if (two) IMSRG_TRY(ozaki_slice(b, L, R, 1, 2, side2));
-      IMSRG_TRY(ozaki_cc_exponents(b, &cc_exps, &gL, &gR));
-      IMSRG_TRY(launch_cc_forward(b, L, hL, R, hR, cc_exps, gL, gR));
-      IMSRG_TRY(sums_beside());
-      IMSRG_TRY(ozaki_slice(b, L, R, 2, 3, b->stream, cc_exps != nullptr));
-      IMSRG_TRY(join(0));
-      if (two) {
-        IMSRG_CUDA_TRY(cudaEventRecord(b->ev_join2, b->side2));
-        IMSRG_CUDA_TRY(cudaStreamWaitEvent(b->stream, b->ev_join2, 0));
-      }
-    }
-    if (prods) IMSRG_TRY(ozaki_mma(b, hL, hR));
   } else {
     if (front) {
       if (!serial) IMSRG_CUDA_TRY(cudaEventRecord(b->ev_fork[0], b->stream));
-      IMSRG_TRY(sums_beside());
-      IMSRG_TRY(launch_cc_forward(b, L, hL, R, hR));
+      if (merged) {
+        IMSRG_TRY(launch_front(b, L, hL, R, hR, Front{0, 2, 3, true}, b->stream));
+        IMSRG_TRY(branches());
+        if (cc_part) IMSRG_TRY(launch_front(b, L, hL, R, hR, Front{2, 3, 0}, b->stream));
+        IMSRG_TRY(ozaki_slice(b, L, R, 0, 3, b->stream, &sums));
+      } else {
+        // digit images of L and R on a side stream, beside the Pandya transform
+        // and the images of LCC and RCC.  The 122 sums come after them in launch
+        // order: a graph starts its branches in that order, and ahead of them
+        // their CTAs took the warp slots (two emax 6 flow steps: 3,400 us with the
+        // sums first, 3,285 so)
+        if (oz) {
+          cudaStream_t lr = serial ? b->stream : side;
+          if (!serial) IMSRG_CUDA_TRY(cudaStreamWaitEvent(lr, b->ev_fork[0], 0));
+          IMSRG_TRY(launch_front(b, L, hL, R, hR, Front{0, 2, 0}, lr));
+          IMSRG_TRY(ozaki_slice(b, L, R, 0, 2, lr));
+          if (!serial) IMSRG_CUDA_TRY(cudaEventRecord(b->ev_join[0], lr));
+        } else {
+          IMSRG_TRY(branches());
+        }
+        IMSRG_TRY(launch_front(b, L, hL, R, hR, Front{0, 0, 3, oz}, b->stream));
+        if (oz) {
+          IMSRG_TRY(branches());
+          if (cc_part) IMSRG_TRY(launch_front(b, L, hL, R, hR, Front{2, 3, 0}, b->stream));
+          IMSRG_TRY(ozaki_slice(b, L, R, 2, 3, b->stream));
+          if (!serial) IMSRG_CUDA_TRY(cudaStreamWaitEvent(b->stream, b->ev_join[0], 0));
+        }
+      }
     }
-    if (prods) IMSRG_TRY(launch_gemm_fp64(b, L, hL, R, hR));
+    if (prods) IMSRG_TRY(oz ? ozaki_mma(b, hL, hR) : launch_gemm_fp64(b, L, hL, R, hR));
   }
   if (front && e0_front) {  // phases in separate graphs: join what the front forked
     IMSRG_TRY(join_e0());
@@ -259,9 +259,18 @@ int commutator_launches(imsrg_basis *b, const double *L, int hL, const double *R
   if (!back) return IMSRG_OK;
   int *exps = nullptr, nexps = 0;  // cleared by the two-body assembly
   if (oz) IMSRG_TRY(ozaki_exps_end(b, &exps, &nexps));
-  // one-body assembly beside the two-body assembly
-  IMSRG_TRY(fork(1));
-  IMSRG_TRY(launch_assemble_1body(b, L, hL, R, hR, RES, hRES, side));
+  if (!merged) {  // one-body assembly beside the two-body assembly
+    if (!serial) {
+      IMSRG_CUDA_TRY(cudaEventRecord(b->ev_fork[1], b->stream));
+      IMSRG_CUDA_TRY(cudaStreamWaitEvent(side, b->ev_fork[1], 0));
+    }
+    IMSRG_TRY(launch_one_body(b, sums, !shared, serial ? b->stream : side));
+    if (!serial) IMSRG_CUDA_TRY(cudaEventRecord(b->ev_join[1], side));
+  }
+  auto join_one = [&]() -> int {
+    if (!merged && !serial) IMSRG_CUDA_TRY(cudaStreamWaitEvent(b->stream, b->ev_join[1], 0));
+    return IMSRG_OK;
+  };
   if (overlap && !packed) {
     // two-body elements by output range; each range's copy to the host runs on
     // side2 beside the assembly of the next (see imsrg_basis::asm2_el)
@@ -269,7 +278,7 @@ int commutator_launches(imsrg_basis *b, const double *L, int hL, const double *R
     if (!e0_front) IMSRG_TRY(join_pre());
     for (int c = 0; c < kOutChunks; c++) {
       IMSRG_TRY(launch_asm2_range(b, L, hL, R, hR, RES, hRES, b->asm2_el[c], b->asm2_el[c + 1], true, exps,
-                                  nexps));
+                                  nexps, false));
       IMSRG_CUDA_TRY(cudaEventRecord(b->ev_out[c], b->stream));
       IMSRG_CUDA_TRY(cudaStreamWaitEvent(b->side2, b->ev_out[c], 0));
       const long a0 = b->asm2_addr[c], a1 = b->asm2_addr[c + 1];
@@ -277,7 +286,7 @@ int commutator_launches(imsrg_basis *b, const double *L, int hL, const double *R
         IMSRG_CUDA_TRY(cudaMemcpyAsync(io->RES + a0, RES + a0, (size_t)(a1 - a0) * sizeof(double),
                                        cudaMemcpyDeviceToHost, b->side2));
     }
-    IMSRG_TRY(join(1));
+    IMSRG_TRY(join_one());
     IMSRG_TRY(join_e0());
     // E0 and the one-body part
     IMSRG_CUDA_TRY(cudaMemcpyAsync(io->RES, RES, (size_t)b->asm2_addr[0] * sizeof(double), cudaMemcpyDeviceToHost,
@@ -290,9 +299,9 @@ int commutator_launches(imsrg_basis *b, const double *L, int hL, const double *R
     ProfScope ps(b, IMSRG_KERNEL_ASSEMBLE_2BODY);
     IMSRG_TRY(launch_ph_inputs(b, hL, hR, precision));
     if (!e0_front) IMSRG_TRY(join_pre());
-    IMSRG_TRY(launch_asm2_range(b, L, hL, R, hR, RES, hRES, 0, b->T.n_asm2, false, exps, nexps));
+    IMSRG_TRY(launch_asm2_range(b, L, hL, R, hR, RES, hRES, 0, b->T.n_asm2, false, exps, nexps, merged));
   }
-  IMSRG_TRY(join(1));
+  IMSRG_TRY(join_one());
   if (!e0_front) IMSRG_TRY(join_e0());
   if (direct) {
     IMSRG_TRY(launch_pack(b, RES, io->RESdev, b->stream, true));

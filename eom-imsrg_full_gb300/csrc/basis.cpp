@@ -878,7 +878,7 @@ int build_basis(imsrg_basis *b) {
     };
     std::vector<OneBodyTerm> terms;
     long nel = (long)A * A + (long)P * A + (long)P * P;
-    std::vector<int> ostart(nel), ocount(nel);
+    std::vector<int> ostart(nel), ocount(nel), o121(nel, 0);
     auto same = [&](int x, int y) { return b->jj[x] == b->jj[y] && b->ll[x] == b->ll[y] && b->itzp[x] == b->itzp[y]; };
     for (long e = 0; e < nel; e++) {
       ostart[e] = (int)terms.size();
@@ -922,6 +922,7 @@ int build_basis(imsrg_basis *b) {
           if (idx >= 0) terms.push_back({(int)idx, 1 | (tr << 2) | (ph << 8), (JT + 1.0) * pr});
         }
       }
+      o121[e] = (int)terms.size() - ostart[e];
       // commutator_221 (commutators.f90:470-486)
       int ji = b->jj[pk];
       for (int c = 0; c < N; c++) {
@@ -944,6 +945,7 @@ int build_basis(imsrg_basis *b) {
     IMSRG_TRY(dev_upload(b, terms, &T.obt));
     IMSRG_TRY(dev_upload(b, ostart, &T.obt_start));
     IMSRG_TRY(dev_upload(b, ocount, &T.obt_count));
+    IMSRG_TRY(dev_upload(b, o121, &T.obt_121));
     // work split of the one-body kernel: allowed upper-triangle elements
     // (longest gather list first) and all elements without a gather list
     std::vector<int> heavy, light;

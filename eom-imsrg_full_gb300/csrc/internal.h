@@ -91,8 +91,10 @@ struct DevTables {
   // Gather lists of the one-body assembly (121 and 221 sums), per one-body
   // element in flat order: obt[obt_start[e] .. + obt_count[e]).
   const struct OneBodyTerm *obt;
+  // The first obt_121[e] are 121 terms.
   const int *obt_start;
   const int *obt_count;
+  const int *obt_121;
   // One-body work split: elements with gather lists (a CTA each, longest
   // first) and the rest (a warp each); mirrored lower triangles are in neither.
   const int *asm1_heavy;
@@ -385,11 +387,15 @@ constexpr int ASM2_THREADS = 128;
 inline int asm2_ctas(const imsrg_basis *b) { return (b->T.n_asm2 + ASM2_THREADS - 1) / ASM2_THREADS; }
 
 // launchers (kernels_*.cu); all enqueue on b->stream and bump b->launches
-// Pandya transform into b->lcc, b->rcc; exps != nullptr: also the largest
-// exponent of each LCC block q1 into exps[gL + q1] and RCC block into exps[gR + q1];
-// sides 1 / 2 / 3: LCC only, RCC only, both; st = nullptr: the basis stream
-int launch_cc_forward(imsrg_basis *b, const double *L, int hL, const double *R, int hR, int *exps = nullptr,
-                      int gL = 0, int gR = 0, int sides = 3, cudaStream_t st = nullptr);
+// What a front launch holds: the exponent chunks of the split engine's parts [p0,
+// p1); the Pandya transform of sides 1 / 2 / 3 (LCC only, RCC only, both; 0 none),
+// with the LCC and RCC block exponents if split.
+struct SumsArgs;
+struct Front {
+  int p0 = 0, p1 = 0, sides = 0;
+  bool split = false;
+};
+int launch_front(imsrg_basis *b, const double *L, int hL, const double *R, int hR, const Front &f, cudaStream_t st);
 int launch_gemm_fp64(imsrg_basis *b, const double *L, int hL, const double *R, int hR);
 // The FP64 products of several bases (operators L[i], R[i] of bases[i]) as one
 // problem list with absolute pointers, and its tiles.
@@ -414,7 +420,7 @@ std::vector<GemmTile> gemm_fp64_tiles(const std::vector<GemmProb> &probs);
 int launch_gemm_fp64_merged(const GemmMerged &g, int hL, int hR, const int *act, cudaStream_t st);
 // the two-body assembly: the recoupling inputs of 222_ph, then the elements
 // [w0, w1) of the signature work order or of the order by output range, on
-// top of launch_asm2_122's part in RES
+// top of the 122 sums in RES; one_body: the one-body elements are finished too
 int launch_ph_inputs(imsrg_basis *b, int hL, int hR, int precision);
 // Bases of at most this many two-body elements form the recoupling inputs one
 // thread per input, in the order of Z, larger ones patch by patch.  The line:
@@ -423,15 +429,13 @@ int launch_ph_inputs(imsrg_basis *b, int hL, int hR, int precision);
 // commutators 19.1 / 39.7 us against 20.1 / 41.0, emax 5 / 6 split 52.8 / 115.0
 // against 47.3 / 111.5).
 constexpr long kPhList = 65536;
-// commutator_122 part of every two-body element into RES on stream st (the
-// assembly after the products adds the rest)
-int launch_asm2_122(imsrg_basis *b, const double *L, int hL, const double *R, int hR, double *RES, int hRES,
-                    cudaStream_t st);
 int launch_asm2_range(imsrg_basis *b, const double *L, int hL, const double *R, int hR, double *RES, int hRES,
-                      long w0, long w1, bool by_range, int *exps, int nexps);
-int launch_assemble_1body(imsrg_basis *b, const double *L, int hL, const double *R, int hR, double *RES, int hRES,
-                          cudaStream_t st);
+                      long w0, long w1, bool by_range, int *exps, int nexps, bool one_body);
 // E0 of [L, R] into RES[0] on stream st (independent of the assembly kernels)
+// the one-body elements after the products, in one pass (all) or two
+int launch_one_body(imsrg_basis *b, const SumsArgs &a, bool all, cudaStream_t st);
+// the 122 sums of the two-body elements into RES
+int launch_sums_122(imsrg_basis *b, const SumsArgs &a, cudaStream_t st);
 int launch_e0(imsrg_basis *b, const double *L, int hL, const double *R, int hR, double *RES, cudaStream_t st);
 int launch_axpby(imsrg_basis *b, const double *A, double ax, const double *B, double bx, double *C);
 int launch_axpby_dev(imsrg_basis *b, const double *A, double ax, const double *B, const double *bx, double *C);
@@ -471,12 +475,20 @@ int preload_commutator_fp64_ws();
 
 // Ozaki split-precision contraction engine (ozaki.cu)
 int ozaki_prepare(imsrg_basis *b);  // plans and allocates the engine once; errors if unavailable
-// parts [p0, p1): 0, exponents and digit images of L; 1, of R; 2, of LCC and
-// RCC (after the Pandya transform).  ozaki_mma then runs every contraction.
-// exps_ready: the parts' block exponents are already in place (part 2: the
-// Pandya transform reduced them, see ozaki_cc_exponents).
+// parts [p0, p1): 0, digit images of L; 1, of R; 2, of LCC and RCC (after the
+// Pandya transform), whose block exponents are in place; sums: also the sums of
+// front.cuh.  ozaki_mma then runs every contraction.
 int ozaki_slice(imsrg_basis *b, const double *L, const double *R, int p0, int p1, cudaStream_t st,
-                bool exps_ready = false);
+                const SumsArgs *sums = nullptr);
+// A contiguous chunk of one exponent group's elements (src: 0 L, 1 R, 2 LCC, 3 RCC).
+struct OzChunk {
+  int group, src;
+  long off;
+  int len;
+};
+constexpr int kOzChunk = 1024;
+// the exponent chunks of parts [p0, p1), and where their exponents go
+int ozaki_chunks(imsrg_basis *b, int p0, int p1, const OzChunk **chunks, int *n, int **exps);
 // Where the Pandya transform may leave the LCC/RCC block exponents: exps[gL +
 // q1], exps[gR + q1]; *exps = nullptr if it cannot.
 int ozaki_cc_exponents(imsrg_basis *b, int **exps, int *gL, int *gR);

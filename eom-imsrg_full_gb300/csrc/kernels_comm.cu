@@ -21,6 +21,7 @@
 //                      L and R
 // No float atomics: every reduction has a fixed order, so results are
 // bit-reproducible run to run.
+#include "front.cuh"
 #include "gemm_fp64.cuh"
 
 namespace imsrg {
@@ -37,11 +38,10 @@ namespace {
 // SIDES: 1 = LCC only, 2 = RCC only, 3 = both from one pass over the gather
 // list (the separate passes let the RCC half run while L is still arriving).
 template <int SIDES>
-__global__ void __launch_bounds__(256) k_cc_forward(DevTables T, const double *__restrict__ L, int hL,
-                                                    const double *__restrict__ R, int hR, double *LCC, double *RCC,
-                                                    int *exps, int gL, int gR) {
-  const long t = (long)blockIdx.x * blockDim.x + threadIdx.x;
-  pdl_go();
+__device__ __forceinline__ void cc_forward(const DevTables &T, const double *__restrict__ L, int hL,
+                                           const double *__restrict__ R, int hR, double *LCC, double *RCC, int *exps,
+                                           int gL, int gR, int cta) {
+  const long t = (long)cta * blockDim.x + threadIdx.x;
   int q1 = -1, xL = 0, xR = 0;
   if (t < T.cc_total) {
     const int v = T.ccf_order[t];  // elements grouped by term count
@@ -74,6 +74,51 @@ __global__ void __launch_bounds__(256) k_cc_forward(DevTables T, const double *_
       if (SIDES & 2) atomicMax(exps + gR + q1, mR);
     }
   }
+}
+
+constexpr int CC_THREADS = 256;
+
+// Largest biased exponent of one chunk (at most kOzChunk elements) of an exponent
+// group into out[group]: integer atomicMax, order-independent, so deterministic.
+__device__ __forceinline__ void exponents(const OzChunk &c, const double *L, const double *R, const double *LCC,
+                                          const double *RCC, int *out) {
+  __shared__ int sh[CC_THREADS / 32];
+  const double *src = (c.src == 0 ? L : c.src == 1 ? R : c.src == 2 ? LCC : RCC) + c.off;
+  int m = 0;
+#pragma unroll
+  for (int k = 0; k < kOzChunk / CC_THREADS; k++) {  // independent loads
+    const int i = threadIdx.x + k * CC_THREADS;
+    if (i < c.len) m = max(m, (int)((__double_as_longlong(src[i]) >> 52) & 0x7FF));
+  }
+  m = __reduce_max_sync(0xffffffffu, m);
+  if ((threadIdx.x & 31) == 0) sh[threadIdx.x >> 5] = m;
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    for (int w = 1; w < CC_THREADS / 32; w++) m = max(m, sh[w]);
+    atomicMax(&out[c.group], m);
+  }
+}
+
+// CTAs [0, nexp): exponent chunks; the rest: the Pandya transform.
+struct FrontArgs {
+  const OzChunk *chunks;
+  int *exps;  // of the chunks
+  int nexp;
+};
+template <int SIDES>
+__global__ void __launch_bounds__(CC_THREADS) k_front(DevTables T, const double *__restrict__ L, int hL,
+                                                      const double *__restrict__ R, int hR, double *LCC, double *RCC,
+                                                      int *exps, int gL, int gR, FrontArgs f) {
+  pdl_go();
+  const int cta = blockIdx.x;
+  if (cta < f.nexp) exponents(f.chunks[cta], L, R, LCC, RCC, f.exps);
+  else if (SIDES) cc_forward<SIDES>(T, L, hL, R, hR, LCC, RCC, exps, gL, gR, cta - f.nexp);
+}
+
+// The 122 sums alone (40 registers: beside the one-body part's 54 they took the
+// slicing's and the products' share of an SM, emax 6 104.8 us -> 108.4).
+__global__ void __launch_bounds__(FRONT_THREADS) k_sums_122(DevTables T, SumsArgs a) {
+  sums_122(T, a, blockIdx.x, gridDim.x);
 }
 
 // ---------------------------------------------------------------------------
@@ -231,91 +276,14 @@ __device__ void energy_block(const DevTables &T, const double *L, int hL, const 
   }
 }
 
-// commutator_122 (commutators.f90:283-396) of one element: f_L V_R - f_R V_L
-// over its leg terms (term k at tm[k * STRIDE]), U terms in flight: their gathers
-// and the next U terms are loaded before the first is used
-template <int STRIDE, int U>
-__device__ __forceinline__ double sum122(const unsigned long long *tm, int n122, const double *L, int nL,
-                                         const double *R, int nR) {
-  double t = 0.0;
-  unsigned long long next[U];
-#pragma unroll
-  for (int i = 0; i < U; i++) next[i] = i < n122 ? tm[i * STRIDE] : 0;
-  for (int k = 0; k < n122; k += U) {
-    unsigned long long u[U];
-    double vR[U], vL[U], fL[U], fR[U];
-#pragma unroll
-    for (int i = 0; i < U; i++) {
-      u[i] = next[i];
-      if (k + U + i < n122) next[i] = tm[(k + U + i) * STRIDE];
-      if (i == 0 || k + i < n122) {
-        const long vi = (long)(u[i] & 0xFFFFFFFull), fi = (long)((u[i] >> 28) & 0xFFFFFull);
-        vR[i] = R[vi];
-        vL[i] = L[vi];
-        fL[i] = L[fi];
-        fR[i] = R[fi];
-      }
-    }
-#pragma unroll
-    for (int i = 0; i < U; i++) {
-      if (i > 0 && k + i >= n122) break;
-      const int sg = (int)(u[i] >> 48) & 1, nsq = (int)(u[i] >> 49) & 3, tr = (int)(u[i] >> 51) & 1,
-                ftr = (int)(u[i] >> 52) & 1;
-      double a = dflip(vR[i], tr & nR), b = dflip(vL[i], tr & nL);
-      if (nsq) {
-        const double c = nsq == 1 ? IMSRG_SQRT2 : 2.0000000000000004;
-        a = a * c;
-        b = b * c;
-      }
-      t = fma(dflip(fL[i], (ftr & nL) ^ sg), a, t);
-      t = fma(dflip(fR[i], (ftr & nR) ^ sg ^ 1), b, t);
-    }
-  }
-  return t;
-}
-
-// The commutator_122 part of every two-body element (upper triangles), with
-// the element's 1/sqrt(1 + delta) factors and the diagonal's sign, into RES:
-// it needs only L and R, so it runs ahead of the products, and the assembly
-// after them (k_assemble_2body<true>) starts from it.  One warp per 32
-// elements of equal term count; term k of every lane is one coalesced load.
-// The arithmetic is the assembly's own, so RES is bit-identical either way.
-// (Packing the sqrt(2)-scaled (L, R) pairs first, for one 16-byte gather per
-// term, measured slower here: the pack kernel took more of the shared front
-// than it saved.)  What bounds it: the FP64 pipe (two FMAs a term) and its
-// gathers.  It has time until the products are done, so half of the SMs' warp
-// slots are enough and the kernels before the products find the other half free:
-// with a CTA per four groups it took every slot first (emax = 6, five digits:
-// 112.4 us per commutator, 109.5 with eight CTAs per SM, 111.5 with six or
-// twelve; host call 203 -> 194, two flow steps 3440 -> 3250, FP64 493 -> 487).
-// They gate the products all the same, whose CTAs each want a whole SM (four
-// CTAs per SM 122 us, two 147), with loads as their longest stall: two terms in
-// flight take 108.4 to 106.1 us, three or four 108.8 and 111.2.
-constexpr int kPreCtas = 8;
-__global__ void __launch_bounds__(ASM2_THREADS) k_asm2_122(DevTables T, const double *__restrict__ L, int hL,
-                                                           const double *__restrict__ R, int hR, int hRES,
-                                                           double *RES) {
-  const int lane = threadIdx.x & 31;
-  for (int g = (int)(((long)blockIdx.x * blockDim.x + threadIdx.x) >> 5); g < T.n_pre_warps;
-       g += (int)(gridDim.x * blockDim.x >> 5)) {
-    const unsigned pe = T.pre_el[(long)g * 32 + lane];
-    if (pe >> 31) continue;  // padding
-    const Asm2PreWarp W = T.pre_warp[g];
-    double t = sum122<32, 2>(T.pre_terms + W.base + lane, W.n122, L, hL < 0, R, hR < 0);
-    const int nd = (pe >> 28) & 3;
-    if (nd) t = t * (nd == 1 ? 0.7071067811865476 : 0.5);
-    if ((pe >> 30) & 1) t = dflip(t, hRES < 0);
-    RES[pe & 0x0FFFFFFFu] = t;
-  }
-}
-
 // Every two-body element of RES once (upper triangles of square arrays, the
 // mirror written alongside): the one-body insertions of commutator_122, the
 // antisymmetrised ladder epilogue of 222_pp_hh (:658-764) and the 222_ph
 // recoupling sum over J' of {6j} Z(J').  Thread t takes element w0 + t of the
 // work order `heads` while below w1.  PRE: the 122 part is already in RES
 // (k_asm2_122), and the split engine's nexps block exponents are cleared for the
-// next commutator (nothing reads them any more).  has220 (the allocation-free path, w0 = 0): each CTA leaves
+// next commutator (nothing reads them any more).  The first n1 CTAs finish the
+// one-body elements instead (one_body_221).  has220 (the allocation-free path, w0 = 0): each CTA leaves
 // its commutator_220 partial in e0p for k_energy.
 template <bool PRE>
 __global__ void __launch_bounds__(ASM2_THREADS) k_assemble_2body(DevTables T, const double *__restrict__ L, int hL,
@@ -324,13 +292,21 @@ __global__ void __launch_bounds__(ASM2_THREADS) k_assemble_2body(DevTables T, co
                                                                  const double *__restrict__ W2,
                                                                  const double *__restrict__ Z, double *RES, int hRES,
                                                                  const Asm2Head *__restrict__ heads, long w0, long w1,
-                                                                 int has220, double *e0p, int *exps, int nexps) {
+                                                                 int has220, double *e0p, int *exps, int nexps,
+                                                                 int n1) {
   __shared__ double sh220[ASM2_THREADS / 32];
-  const long w = w0 + (long)blockIdx.x * blockDim.x + threadIdx.x;
+  if ((int)blockIdx.x < n1) {
+    pdl_go();
+    pdl_wait();
+    one_body_221(T, hL, hR, W1, W2, RES, hRES, blockIdx.x);
+    return;
+  }
+  const int cta = (int)blockIdx.x - n1;
+  const long w = w0 + (long)cta * blockDim.x + threadIdx.x;
   const Asm2Head h = w < w1 ? heads[w] : Asm2Head{};
   pdl_go();
   pdl_wait();
-  if (PRE && blockIdx.x == 0)
+  if (PRE && cta == 0)
     for (int i = threadIdx.x; i < nexps; i += ASM2_THREADS) exps[i] = 0;
   double e220 = 0.0;  // this element's commutator_220 term (pphh arrays only)
   if (w < w1) {
@@ -380,7 +356,7 @@ __global__ void __launch_bounds__(ASM2_THREADS) k_assemble_2body(DevTables T, co
     if (threadIdx.x == 0) {
       double t220 = 0.0;
       for (int k = 0; k < (int)(blockDim.x >> 5); k++) t220 += sh220[k];
-      e0p[blockIdx.x] = t220;
+      e0p[cta] = t220;
     }
   }
 }
@@ -433,160 +409,40 @@ __global__ void __launch_bounds__(E0_THREADS) k_e0(DevTables T, const double *__
   }
 }
 
-// One-body assembly.  The (l,j,tz)-allowed upper-triangle elements carry the
-// 121 and 221 gather lists (a few hundred independent terms each) and get a
-// CTA of four warps; every other element only has the four commutator_111 dot
-// products and gets one warp, four elements per CTA.  Each thread folds its
-// partial dot products and gather sums into the element's final linear
-// combination, so one reduction per element remains.
-__global__ void __launch_bounds__(128) k_assemble_1body(DevTables T, const double *L, int hL, const double *R, int hR,
-                                                        const double *W1, const double *W2, double *RES, int hRES) {
-  __shared__ double sh[4][8];
-  const int A = T.A, P = T.P;
-  const double *Lhh = L + T.off_fhh, *Lph = L + T.off_fph, *Lpp = L + T.off_fpp;
-  const double *Rhh = R + T.off_fhh, *Rph = R + T.off_fph, *Rpp = R + T.off_fpp;
-  const int nheavy = T.n_asm1_heavy;
-  const bool whole = (int)blockIdx.x < nheavy;  // block-uniform
-  long e;
-  int tid, nt;
-  if (whole) {
-    e = T.asm1_heavy[blockIdx.x];
-    tid = threadIdx.x;
-    nt = blockDim.x;
-  } else {
-    const int li = ((int)blockIdx.x - nheavy) * 4 + (int)(threadIdx.x >> 5);
-    if (li >= T.n_asm1_light) return;
-    e = T.asm1_light[li];
-    tid = threadIdx.x & 31;
-    nt = 32;
-  }
-  const long nA2 = (long)A * A, nPA = (long)P * A;
-  int type, p, q, pk, qk;
-  if (e < nA2) {
-    type = 0;
-    p = (int)(e % A);
-    q = (int)(e / A);
-    pk = T.hole_orb[p];
-    qk = T.hole_orb[q];
-  } else if (e < nA2 + nPA) {
-    type = 1;
-    p = (int)((e - nA2) % P);
-    q = (int)((e - nA2) / P);
-    pk = T.part_orb[p];
-    qk = T.hole_orb[q];
-  } else {
-    type = 2;
-    p = (int)((e - nA2 - nPA) % P);
-    q = (int)((e - nA2 - nPA) / P);
-    pk = T.part_orb[p];
-    qk = T.part_orb[q];
-  }
-  const bool allowed = T.orb[pk].x == T.orb[qk].x && T.orb[pk].y == T.orb[qk].y && T.orb[pk].z == T.orb[qk].z;
-  // commutator_111 (commutators.f90:36-80): four dot products
-  double v[6] = {0.0, 0.0, 0.0, 0.0, 0.0, 0.0};
-  if (type == 0) {  // th1 = Lhh Rhh, th2 = Lph^T Rph
-    for (int k = tid; k < A; k += nt) {
-      v[0] = fma(Lhh[p + (long)k * A], Rhh[k + (long)q * A], v[0]);
-      v[2] = fma(Lhh[q + (long)k * A], Rhh[k + (long)p * A], v[2]);
-    }
-    for (int k = tid; k < P; k += nt) {
-      v[1] = fma(Lph[k + (long)p * P], Rph[k + (long)q * P], v[1]);
-      v[3] = fma(Lph[k + (long)q * P], Rph[k + (long)p * P], v[3]);
-    }
-  } else if (type == 1) {  // Lph Rhh + Lpp Rph - Rph Lhh - Rpp Lph
-    for (int k = tid; k < A; k += nt) {
-      v[0] = fma(Lph[p + (long)k * P], Rhh[k + (long)q * A], v[0]);
-      v[2] = fma(Rph[p + (long)k * P], Lhh[k + (long)q * A], v[2]);
-    }
-    for (int k = tid; k < P; k += nt) {
-      v[1] = fma(Lpp[p + (long)k * P], Rph[k + (long)q * P], v[1]);
-      v[3] = fma(Rpp[p + (long)k * P], Lph[k + (long)q * P], v[3]);
-    }
-  } else {  // tp1 = Lph Rph^T, tp2 = Lpp Rpp
-    for (int k = tid; k < A; k += nt) {
-      v[0] = fma(Lph[p + (long)k * P], Rph[q + (long)k * P], v[0]);
-      v[2] = fma(Lph[q + (long)k * P], Rph[p + (long)k * P], v[2]);
-    }
-    for (int k = tid; k < P; k += nt) {
-      v[1] = fma(Lpp[p + (long)k * P], Rpp[k + (long)q * P], v[1]);
-      v[3] = fma(Lpp[q + (long)k * P], Rpp[k + (long)p * P], v[3]);
-    }
-  }
-  // commutator_121 and commutator_221 sums from the gather list
-  if (allowed) {
-    const int st = T.obt_start[e], n = T.obt_count[e];
-    const int nL = hL < 0, nR = hR < 0, npm = hL * hR > 0;
-    for (int k = tid; k < n; k += nt) {
-      const OneBodyTerm t = T.obt[st + k];
-      const int kind = t.meta & 3;
-      if (kind < 2) {
-        const int tr = (t.meta >> 2) & 1, ph = t.meta >> 8;
-        const double rv = dflip(R[t.idx], tr & nR) * t.coef;
-        const double lv = dflip(L[t.idx], tr & nL) * t.coef;
-        const double lph = Lph[ph], rph = Rph[ph];
-        if (kind == 0) {  // L_ai (herm_L R) - R_ai (herm_R L) at <a p|i q>
-          v[4] = fma(dflip(lph, nL), rv, v[4]);
-          v[4] = fma(-dflip(rph, nR), lv, v[4]);
-        } else {  // -L_ai R + R_ai L at <i p|a q>
-          v[4] = fma(-lph, rv, v[4]);
-          v[4] = fma(rph, lv, v[4]);
-        }
-      } else {
-        const double *W = (t.meta & 8) ? W2 : W1;
-        const double w = W[t.idx] * t.coef;
-        v[5] += (kind == 3) ? dflip(w, npm) : w;  // the second 221 term enters with -herm_L herm_R
-      }
-    }
-  }
-  // the element is linear in the six sums:
-  //   type 0: v0 + v1 hL - (v2 hL + v3) hR      type 1: v0 + v1 - v2 - v3
-  //   type 2: v0 hR + v1 - (v2 + v3 hR) hL
-  // plus (v4 + v5) / (2j_p + 1) on allowed elements, where a diagonal of fhh
-  // or fpp takes v5 times herm(RES) (((t + s121) hRES + s221) hRES with hRES^2 = 1)
-  double c0 = 1.0, c1 = 1.0, c2 = -1.0, c3 = -1.0;
-  if (type == 0) {
-    c1 = hL;
-    c2 = -(double)(hL * hR);
-    c3 = -hR;
-  } else if (type == 2) {
-    c0 = hR;
-    c2 = -hL;
-    c3 = -(double)(hR * hL);
-  }
-  double x = fma(c3, v[3], fma(c2, v[2], fma(c1, v[1], c0 * v[0])));
-  if (allowed) {
-    const double rj = 1.0 / (T.orb[pk].x + 1.0);
-    const double c5 = (type != 1 && p == q) ? hRES * rj : rj;
-    x = fma(c5, v[5], fma(rj, v[4], x));
-  }
-  x = warp_sum(x);
-  if (whole) {
-    if ((threadIdx.x & 31) == 0) sh[threadIdx.x >> 5][0] = x;
-    __syncthreads();
-    x = ((sh[0][0] + sh[1][0]) + sh[2][0]) + sh[3][0];
-  }
-  if (tid != 0) return;
-  const long base = type == 0 ? T.off_fhh : type == 1 ? T.off_fph : T.off_fpp;
-  const int ld = type == 0 ? A : P;
-  RES[base + p + (long)q * ld] = x;
-  if (allowed && type != 1 && p != q) RES[base + q + (long)p * ld] = x * hRES;
+// The one-body assembly in one launch, after the products.  ALL: in one pass, else
+// in the two of the shared launches (front.cuh), so that every path of one basis
+// and precision gives the same bits.
+template <bool ALL>
+__global__ void __launch_bounds__(FRONT_THREADS, ALL ? 10 : 8) k_one_body(DevTables T, SumsArgs a, const double *__restrict__ W1,
+                                                            const double *__restrict__ W2) {
+  one_body_front<ALL>(T, a, blockIdx.x, W1, W2);
+  if (!ALL && (int)blockIdx.x < T.n_asm1_heavy) one_body_221(T, a.hL, a.hR, W1, W2, a.RES, a.hRES, blockIdx.x);
 }
 
 }  // namespace
 
-int launch_cc_forward(imsrg_basis *b, const double *L, int hL, const double *R, int hR, int *exps, int gL, int gR,
-                      int sides, cudaStream_t st) {
-  long n = b->cc_total;
-  if (n == 0) return IMSRG_OK;
-  if (!st) st = b->stream;
-  ProfScope ps(b, IMSRG_KERNEL_CC_FORWARD, st);
-  const unsigned grid = (unsigned)((n + 255) / 256);
-  if (sides == 1)
-    k_cc_forward<1><<<grid, 256, 0, st>>>(b->T, L, hL, R, hR, b->lcc, b->rcc, exps, gL, gR);
-  else if (sides == 2)
-    k_cc_forward<2><<<grid, 256, 0, st>>>(b->T, L, hL, R, hR, b->lcc, b->rcc, exps, gL, gR);
-  else
-    k_cc_forward<3><<<grid, 256, 0, st>>>(b->T, L, hL, R, hR, b->lcc, b->rcc, exps, gL, gR);
+int launch_front(imsrg_basis *b, const double *L, int hL, const double *R, int hR, const Front &f, cudaStream_t st) {
+  FrontArgs a{};
+  int *exps = nullptr, gL = 0, gR = 0, ncc = 0;
+  if (f.p1 > f.p0) IMSRG_TRY(ozaki_chunks(b, f.p0, f.p1, &a.chunks, &a.nexp, &a.exps));
+  if (f.sides) {
+    ncc = (int)((b->cc_total + CC_THREADS - 1) / CC_THREADS);
+    if (f.split) IMSRG_TRY(ozaki_cc_exponents(b, &exps, &gL, &gR));
+  }
+  const int grid = a.nexp + ncc;
+  if (grid == 0) return IMSRG_OK;
+  ProfScope ps(b, f.sides ? IMSRG_KERNEL_CC_FORWARD : IMSRG_KERNEL_OZAKI_SLICE, st);
+  auto *kernel = f.sides == 0 ? k_front<0> : f.sides == 1 ? k_front<1> : f.sides == 2 ? k_front<2> : k_front<3>;
+  kernel<<<grid, CC_THREADS, 0, st>>>(b->T, L, hL, R, hR, b->lcc, b->rcc, exps, gL, gR, a);
+  b->launches++;
+  return cuda_status(cudaGetLastError());
+}
+
+int launch_sums_122(imsrg_basis *b, const SumsArgs &a, cudaStream_t st) {
+  const int grid = sums_122_ctas(b);
+  if (grid == 0) return IMSRG_OK;
+  ProfScope ps(b, IMSRG_KERNEL_ASSEMBLE_2BODY, st);
+  k_sums_122<<<grid, FRONT_THREADS, 0, st>>>(b->T, a);
   b->launches++;
   return cuda_status(cudaGetLastError());
 }
@@ -686,24 +542,24 @@ int launch_ph_inputs(imsrg_basis *b, int hL, int hR, int precision) {
 }
 
 int launch_asm2_range(imsrg_basis *b, const double *L, int hL, const double *R, int hR, double *RES, int hRES,
-                      long w0, long w1, bool by_range, int *exps, int nexps) {
-  const long n = w1 - w0;
-  if (n > 0) {
-    IMSRG_CUDA_TRY(launch_after(b->pdl, k_assemble_2body<true>, (unsigned)((n + ASM2_THREADS - 1) / ASM2_THREADS),
+                      long w0, long w1, bool by_range, int *exps, int nexps, bool one_body) {
+  const int n1 = one_body ? b->T.n_asm1_heavy : 0;
+  const long grid = n1 + (std::max(w1 - w0, 0L) + ASM2_THREADS - 1) / ASM2_THREADS;
+  if (grid > 0) {
+    IMSRG_CUDA_TRY(launch_after(b->pdl, k_assemble_2body<true>, (unsigned)grid,
                                 ASM2_THREADS, 0, b->stream, b->T, L, hL, R, hR, b->w1, b->w2, b->zph, RES, hRES,
-                                by_range ? b->T.asm2_head_out : b->T.asm2_head, w0, w1, 0, nullptr, exps, nexps));
+                                by_range ? b->T.asm2_head_out : b->T.asm2_head, w0, w1, 0, nullptr, exps, nexps,
+                                n1));
     b->launches++;
   }
   return cuda_status(cudaGetLastError());
 }
 
-int launch_asm2_122(imsrg_basis *b, const double *L, int hL, const double *R, int hR, double *RES, int hRES,
-                    cudaStream_t st) {
-  if (b->T.n_pre_warps == 0) return IMSRG_OK;
-  ProfScope ps(b, IMSRG_KERNEL_ASSEMBLE_2BODY, st);
-  const unsigned grid = (unsigned)std::min(((long)b->T.n_pre_warps * 32 + ASM2_THREADS - 1) / ASM2_THREADS,
-                                           (long)kPreCtas * b->num_sms);
-  k_asm2_122<<<grid, ASM2_THREADS, 0, st>>>(b->T, L, hL, R, hR, hRES, RES);
+int launch_one_body(imsrg_basis *b, const SumsArgs &a, bool all, cudaStream_t st) {
+  const int grid = one_body_ctas(b->T);
+  if (grid == 0) return IMSRG_OK;
+  ProfScope ps(b, IMSRG_KERNEL_ASSEMBLE_1BODY, st);
+  (all ? k_one_body<true> : k_one_body<false>)<<<grid, FRONT_THREADS, 0, st>>>(b->T, a, b->w1, b->w2);
   b->launches++;
   return cuda_status(cudaGetLastError());
 }
@@ -715,26 +571,14 @@ int launch_e0(imsrg_basis *b, const double *L, int hL, const double *R, int hR, 
   return cuda_status(cudaGetLastError());
 }
 
-int launch_assemble_1body(imsrg_basis *b, const double *L, int hL, const double *R, int hR, double *RES, int hRES,
-                          cudaStream_t st) {
-  const int grid = b->T.n_asm1_heavy + (b->T.n_asm1_light + 3) / 4;
-  if (grid == 0) return IMSRG_OK;
-  ProfScope ps(b, IMSRG_KERNEL_ASSEMBLE_1BODY, st);
-  k_assemble_1body<<<grid, 128, 0, st>>>(b->T, L, hL, R, hR, b->w1, b->w2, RES, hRES);
-  b->launches++;
-  return cuda_status(cudaGetLastError());
-}
-
-
 // The four FP64 launches of one commutator with caller-chosen workspace and
 // stream; used by the allocation-free entry point (noalloc.cu).  Allocates
 // nothing and records no profiling events.
 int launch_commutator_fp64_ws(imsrg_basis *b, const Workspace &ws, const double *L, int hL, const double *R, int hR,
                               double *RES, int hRES, int with_e0, cudaStream_t st) {
-  long ncc = b->cc_total;
-  if (ncc > 0) {
-    k_cc_forward<3><<<(unsigned)((ncc + 255) / 256), 256, 0, st>>>(b->T, L, hL, R, hR, ws.lcc, ws.rcc, nullptr, 0,
-                                                                    0);
+  if (b->cc_total > 0) {
+    k_front<3><<<(unsigned)((b->cc_total + CC_THREADS - 1) / CC_THREADS), CC_THREADS, 0, st>>>(
+        b->T, L, hL, R, hR, ws.lcc, ws.rcc, nullptr, 0, 0, FrontArgs{});
     b->launches++;
   }
   if (b->ntiles > 0) {
@@ -756,13 +600,12 @@ int launch_commutator_fp64_ws(imsrg_basis *b, const Workspace &ws, const double 
   const long n2 = b->T.n_asm2;
   if (n2 > 0) {
     const int has220 = with_e0 && hL * hR == -1;
-    k_assemble_2body<false><<<(unsigned)((n2 + ASM2_THREADS - 1) / ASM2_THREADS), ASM2_THREADS, 0, st>>>(
-        b->T, L, hL, R, hR, ws.w1, ws.w2, ws.zph, RES, hRES, b->T.asm2_head, 0, n2, has220, ws.e0p, nullptr, 0);
+    k_assemble_2body<false><<<asm2_ctas(b), ASM2_THREADS, 0, st>>>(b->T, L, hL, R, hR, ws.w1, ws.w2, ws.zph, RES, hRES,
+                                                                  b->T.asm2_head, 0, n2, has220, ws.e0p, nullptr, 0, 0);
     b->launches++;
   }
-  const int grid1 = b->T.n_asm1_heavy + (b->T.n_asm1_light + 3) / 4;
-  if (grid1 > 0) {
-    k_assemble_1body<<<grid1, 128, 0, st>>>(b->T, L, hL, R, hR, ws.w1, ws.w2, RES, hRES);
+  if (const int grid1 = one_body_ctas(b->T)) {
+    k_one_body<true><<<grid1, FRONT_THREADS, 0, st>>>(b->T, SumsArgs{L, R, RES, hL, hR, hRES, 0}, ws.w1, ws.w2);
     b->launches++;
   }
   if (with_e0) {
@@ -775,9 +618,9 @@ int launch_commutator_fp64_ws(imsrg_basis *b, const Workspace &ws, const double 
 
 int preload_commutator_fp64_ws() {
   cudaFuncAttributes a;
-  const void *fns[] = {(const void *)k_cc_forward<3>, (const void *)k_gemm_fp64<false>, (const void *)k_ph_list<false>,
+  const void *fns[] = {(const void *)k_front<3>, (const void *)k_gemm_fp64<false>, (const void *)k_ph_list<false>,
                        (const void *)k_ph_patches<false>,
-                       (const void *)k_assemble_2body<false>, (const void *)k_assemble_1body, (const void *)k_energy};
+                       (const void *)k_assemble_2body<false>, (const void *)k_one_body<true>, (const void *)k_energy};
   for (const void *f : fns) {
     cudaError_t e = cudaFuncGetAttributes(&a, f);
     if (e != cudaSuccess) return cuda_status(e);

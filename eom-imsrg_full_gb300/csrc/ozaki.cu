@@ -5,7 +5,7 @@
 // and WCC = LCC RCC^T of commutator_222_ph, :792-802) with BF16 tensor-core
 // products whose FP32 accumulations are exact integers:
 //
-//   1. k_oz_exponents: one power-of-two scale per block: e with |x| < 2^e for
+//   1. block exponents (k_front): one power-of-two scale per block: e with |x| < 2^e for
 //      every element of the block (all six arrays of a (2J,Tz,parity) block of
 //      L or R; one cross-coupled block of LCC or RCC).  Every product term of
 //      a block multiplies one L array by one R array of that block, so all
@@ -49,7 +49,7 @@
 #include <algorithm>
 #include <map>
 
-#include "device.cuh"
+#include "front.cuh"
 
 namespace imsrg {
 
@@ -87,6 +87,7 @@ constexpr int STAGES = 6;
 // for 47% of the L slicing; 128 took the commutator from 159.6 to 156.5 us,
 // 64 gave 159.5).
 constexpr int SLICE_THREADS = 128;
+static_assert(SLICE_THREADS == FRONT_THREADS, "the sums share the slicing launch");
 constexpr int A_SLICE_BYTES = TM * TK * 2;   // 4096
 __host__ __device__ constexpr int oz_b_slice_bytes(int S) { return oz_tn(S) * TK * 2; }
 __host__ __device__ constexpr int oz_stage_bytes(int S) { return S * (A_SLICE_BYTES + oz_b_slice_bytes(S)); }
@@ -132,13 +133,6 @@ struct OzMatrix {
   int unit_c;      // first unit of the C image (rows n2, K = n1), -1 when no problem reads it
   int rg_r, rg_c;  // row groups (of 8 rows) of each image
   int line_r0, line_c0;  // first line of this matrix in the R / C slicing grids
-};
-
-// A contiguous chunk of one exponent group's elements.
-struct OzChunk {
-  int group, src;
-  long off;
-  int len;
 };
 
 // One 128 x TN output tile, everything its roles need in one contiguous record;
@@ -379,33 +373,6 @@ __device__ __forceinline__ double oz_scale(double d, int k) {
 }
 
 // ---------------------------------------------------------------------------
-// 1. block exponents: max biased exponent of each group (integer atomicMax,
-//    order-independent, so the result is deterministic)
-// ---------------------------------------------------------------------------
-__global__ void __launch_bounds__(256) k_oz_exponents(const OzChunk *chunks, const double *L, const double *R,
-                                                      const double *LCC, const double *RCC, int *exps) {
-  __shared__ int sh[8];
-  pdl_go();  // (the slicing launches meanwhile)
-  OzChunk c = chunks[blockIdx.x];
-  const double *src = (c.src == 0 ? L : c.src == 1 ? R : c.src == 2 ? LCC : RCC) + c.off;
-  // chunks hold at most 4 x 256 elements: four independent loads per thread
-  int m = 0;
-#pragma unroll
-  for (int k = 0; k < 4; k++) {
-    const int i = threadIdx.x + k * 256;
-    if (i < c.len) m = max(m, (int)((__double_as_longlong(src[i]) >> 52) & 0x7FF));
-  }
-#pragma unroll
-  for (int o = 16; o > 0; o >>= 1) m = max(m, __shfl_xor_sync(0xffffffffu, m, o));
-  if ((threadIdx.x & 31) == 0) sh[threadIdx.x >> 5] = m;
-  __syncthreads();
-  if (threadIdx.x == 0) {
-    for (int w = 1; w < (int)(blockDim.x >> 5); w++) m = max(m, sh[w]);
-    atomicMax(&exps[c.group], m);
-  }
-}
-
-// ---------------------------------------------------------------------------
 // 2. digit slicing: one thread per 8-element line of a core matrix
 // ---------------------------------------------------------------------------
 // Digits of x with |x| < 2^e: x = 2^(e-7S) sum_{s} d_s 128^(S-1-s), d_0 first.
@@ -481,14 +448,21 @@ __device__ __forceinline__ uint32_t digit_fp32(int d) {
 // columns of one row).  mat_c / mat_r: the matrix of each line (a walk over the
 // matrices from each CTA's first one took 26 us at emax = 2, where a CTA's lines
 // span dozens).  Padding lines of the images are never written and stay zero.
-template <int S>
-__global__ void __launch_bounds__(SLICE_THREADS) k_oz_slice(const OzMatrix *__restrict__ mats,
+// CTAs from nslice on form the sums of front.cuh, which have time until the
+// assembly: last, where they do not take the slicing's warp slots.
+template <int S, bool SUMS>
+__global__ void __launch_bounds__(SLICE_THREADS) k_oz_slice(DevTables T, SumsArgs sums, int nslice,
+                                                            const OzMatrix *__restrict__ mats,
                                                             const uint16_t *__restrict__ mat_c,
                                                             const uint16_t *__restrict__ mat_r, int cblocks, int c_lo,
                                                             int c_hi, int r_lo, int r_hi, const double *L,
                                                             const double *R, const double *LCC, const double *RCC,
                                                             const int *exps, uint8_t *img, long plane) {
   pdl_wait();
+  if (SUMS && (int)blockIdx.x >= nslice) {
+    sums_cta(T, sums, (int)blockIdx.x - nslice, (int)gridDim.x - nslice);
+    return;
+  }
   const bool cimg = (int)blockIdx.x < cblocks;
   const int t = (cimg ? c_lo : r_lo) + ((int)blockIdx.x - (cimg ? 0 : cblocks)) * blockDim.x + threadIdx.x;
   if (t >= (cimg ? c_hi : r_hi)) return;
@@ -946,7 +920,8 @@ int ozaki_prepare(imsrg_basis *b) {
   int ngroups = 0;
   auto add_group = [&](int src, long off, long len) {
     int g = ngroups++;
-    for (long s0 = 0; s0 < len; s0 += 1024) chunks.push_back({g, src, off + s0, (int)std::min<long>(1024, len - s0)});
+    for (long s0 = 0; s0 < len; s0 += kOzChunk)
+      chunks.push_back({g, src, off + s0, (int)std::min<long>(kOzChunk, len - s0)});
     return g;
   };
   auto add_matrix = [&](int src, int group, long off, int n1, int n2) {
@@ -1207,25 +1182,41 @@ int ozaki_cc_exponents(imsrg_basis *b, int **exps, int *gL, int *gR) {
   return IMSRG_OK;
 }
 
-int ozaki_slice(imsrg_basis *b, const double *L, const double *R, int p0, int p1, cudaStream_t st, bool exps_ready) {
+int ozaki_chunks(imsrg_basis *b, int p0, int p1, const OzChunk **chunks, int *n, int **exps) {
   OzPlan *pl = plan_of(b);
-  if (!pl) return IMSRG_ERR_INVALID;
+  if (!pl || !pl->ok || p0 < 0 || p1 > 3 || p0 >= p1) return IMSRG_ERR_INVALID;
+  *chunks = pl->d_chunks + pl->chunk_lo[p0];
+  *n = pl->chunk_lo[p1] - pl->chunk_lo[p0];
+  *exps = pl->d_exps;
+  return IMSRG_OK;
+}
+
+int ozaki_slice(imsrg_basis *b, const double *L, const double *R, int p0, int p1, cudaStream_t st,
+                const SumsArgs *sums) {
+  OzPlan *pl = plan_of(b);
+  if (!pl || p0 < 0 || p1 > 3 || p0 >= p1) return IMSRG_ERR_INVALID;
   ProfScope ps(b, IMSRG_KERNEL_OZAKI_SLICE, st);
-  if (p0 < 0 || p1 > 3 || p0 >= p1) return IMSRG_ERR_INVALID;
-  const int k0 = pl->chunk_lo[p0], k1 = pl->chunk_lo[p1];
-  if (k1 > k0 && !exps_ready) {
-    k_oz_exponents<<<k1 - k0, 256, 0, st>>>(pl->d_chunks + k0, L, R, b->lcc, b->rcc, pl->d_exps);
-    b->launches++;
-  }
   const int c_lo = pl->linec_lo[p0], c_hi = pl->linec_lo[p1];
   const int r_lo = pl->liner_lo[p0], r_hi = pl->liner_lo[p1];
   const int cblocks = (c_hi - c_lo + SLICE_THREADS - 1) / SLICE_THREADS;
-  const int nblk = cblocks + (r_hi - r_lo + SLICE_THREADS - 1) / SLICE_THREADS;
-  if (nblk) {
-    auto *kernel = pl->S == 4 ? k_oz_slice<4> : pl->S == 5 ? k_oz_slice<5> : pl->S == 6 ? k_oz_slice<6> :
-                   pl->S == 7 ? k_oz_slice<7> : k_oz_slice<8>;
-    IMSRG_CUDA_TRY(launch_after(b->pdl, kernel, nblk, SLICE_THREADS, 0, st, pl->d_mats, pl->d_mat_c, pl->d_mat_r, cblocks, c_lo,
-                                c_hi, r_lo, r_hi, L, R, b->lcc, b->rcc, pl->d_exps, pl->img, pl->units * 256));
+  const int nslice = cblocks + (r_hi - r_lo + SLICE_THREADS - 1) / SLICE_THREADS;
+  SumsArgs a{};
+  int nsums = 0;
+  if (sums) {
+    a = *sums;
+    nsums = sums_122_ctas(b) + a.n1;
+  }
+  if (nslice + nsums) {
+    using Kernel = decltype(&k_oz_slice<4, false>);
+    static constexpr Kernel kernels[5][2] = {{k_oz_slice<4, false>, k_oz_slice<4, true>},
+                                             {k_oz_slice<5, false>, k_oz_slice<5, true>},
+                                             {k_oz_slice<6, false>, k_oz_slice<6, true>},
+                                             {k_oz_slice<7, false>, k_oz_slice<7, true>},
+                                             {k_oz_slice<8, false>, k_oz_slice<8, true>}};
+    const Kernel kernel = kernels[pl->S - 4][sums ? 1 : 0];
+    IMSRG_CUDA_TRY(launch_after(b->pdl, kernel, nslice + nsums, SLICE_THREADS, 0, st, b->T, a, nslice, pl->d_mats,
+                                pl->d_mat_c, pl->d_mat_r, cblocks, c_lo, c_hi, r_lo, r_hi, L, R, b->lcc, b->rcc,
+                                pl->d_exps, pl->img, pl->units * 256));
     b->launches++;
   }
   return cuda_status(cudaGetLastError());

@@ -80,6 +80,7 @@ __global__ void __launch_bounds__(GT_THREADS, GT_CTAS) k_gemm_adj(const AdjProb 
                                                          int hR) {
   const GemmTile t = tiles[blockIdx.x];
   const AdjProb &P = probs[t.prob];
+  pdl_wait();
   gemm_cta_tile<true>(
       t,
       [&](int it, auto add) {
@@ -110,7 +111,10 @@ __global__ void __launch_bounds__(GT_THREADS, GT_CTAS) k_gemm_adj(const AdjProb 
 // first two kernels' CTA ranges: 63.5 -> 53.5 us at emax = 4, where the chain of
 // launches is the time, and 560 -> 548 at emax = 6, where both halves want the
 // FP64 pipe (a high-priority second stream 557, three product CTAs per SM beside
-// it 552).
+// it 552).  On each stream a kernel is launched as the dependent of the one before
+// it, which saves a link's launch latency (53.0 -> 48.4 us, 548 -> 544), but starts
+// as that one ends: started earlier (pdl_go), its CTAs held slots the other stream
+// wanted (51.4 us).
 // ---------------------------------------------------------------------------
 
 // Gather lists of the transposed sums (host-built from the forward's).
@@ -260,6 +264,7 @@ __global__ void __launch_bounds__(ADJ_THREADS) k_adj_122(DevTables T, AdjLists A
                                                          const double *__restrict__ Zb, int first, int n0, int n1,
                                                          double *fpart, double *WCCb, double *Yb) {
   __shared__ double sh[32];
+  pdl_wait();
   const int nL = hL < 0, nR = hR < 0;
   const int blk = blockIdx.x + first;
   if (blk < n0) {
@@ -431,6 +436,7 @@ __global__ void __launch_bounds__(128) k_adj_one(DevTables T, AdjLists A, const 
                                                  const double *__restrict__ Cb, int hRES,
                                                  const double *__restrict__ fpart, int n0, int n1, int n2, double *Yb,
                                                  double *W1b, double *W2b) {
+  pdl_wait();
   const int blk = blockIdx.x;
   if (blk < n0) {
     adj_1body(T, X, hL, hR, Cb, hRES, Yb, W1b, W2b);
@@ -787,6 +793,7 @@ int commutator_adjoint_dev(imsrg_basis *b, const double *X, int hX, const double
   const int p0 = ctas(b->nfull, ADJ_THREADS), p1 = p0 + ctas(T.n_ph, ADJ_THREADS),
             p2 = p1 + ctas(b->cc_total, ADJ_THREADS), p3 = p2 + ctas(b->cc_total, ADJ_ZERO);
   const int v0 = A.n_f_chunks, v1 = v0 + ctas(A.n_v_warps, ADJ_THREADS / 32), v2 = v1 + 4 * T.n_ph_patches;
+  cudaError_t err = cudaSuccess;
   auto prep = [&](int from, int to, cudaStream_t s) {
     if (to == from) return;
     k_adj_prep<<<to - from, ADJ_THREADS, 0, s>>>(T, A, X, hL, hR, Cb, hRES, b->off_2b, from, p0, p1, p2, a->w1b,
@@ -795,7 +802,8 @@ int commutator_adjoint_dev(imsrg_basis *b, const double *X, int hX, const double
   };
   auto sums = [&](int from, int to, cudaStream_t s) {
     if (to == from) return;
-    k_adj_122<<<to - from, ADJ_THREADS, 0, s>>>(T, A, X, hL, hR, a->u, a->zb, from, v0, v1, a->fpart, a->wccb, Yb);
+    err = err ? err : launch_after(true, k_adj_122, to - from, ADJ_THREADS, 0, s, T, A, X, hL, hR, a->u, a->zb, from, v0,
+                                   v1, a->fpart, a->wccb, Yb);
     b->launches++;
   };
   AdjOps ops{};
@@ -808,7 +816,8 @@ int commutator_adjoint_dev(imsrg_basis *b, const double *X, int hX, const double
   ops.dst[AD_RCC] = a->rccb;
   auto products = [&](int from, int to, cudaStream_t s) {
     if (to == from) return;
-    k_gemm_adj<<<to - from, GT_THREADS, 0, s>>>(a->d_probs, a->d_tiles + from, ops, hL, hR);
+    err = err ? err : launch_after(true, k_gemm_adj, to - from, GT_THREADS, 0, s, a->d_probs, a->d_tiles + from, ops, hL,
+                                   hR);
     b->launches++;
   };
   // (while kernel timing is on, one stream; the order below holds there too)
@@ -822,11 +831,13 @@ int commutator_adjoint_dev(imsrg_basis *b, const double *X, int hX, const double
               n2 = n1 + (with_e0 ? ctas((long)b->P * b->A, 128) : 0),
               n3 = n2 + (with_e0 && hL * hR == -1 ? b->nblocks : 0);
     if (n3) {
-      k_adj_one<<<n3, 128, 0, side>>>(T, A, X, hL, hR, Cb, hRES, a->fpart, n0, n1, n2, Yb, a->w1b, a->w2b);
+      err = err ? err : launch_after(true, k_adj_one, n3, 128, 0, side, T, A, X, hL, hR, Cb, hRES, a->fpart, n0, n1, n2,
+                                     Yb, a->w1b, a->w2b);
       b->launches++;
     }
   }
   products(0, a->nladder, side);
+  IMSRG_CUDA_TRY(err);
   if (!serial) {
     IMSRG_CUDA_TRY(cudaEventRecord(a->ev_join, side));
     IMSRG_CUDA_TRY(cudaStreamWaitEvent(st, a->ev_join, 0));

@@ -51,7 +51,9 @@ def _workload_flops(lay):
 
 
 def _cc_flops(orb):
-    """2 * rlen^2 * nph summed over cross-coupled blocks (222_ph product)."""
+    """2 * rlen^2 * nph summed over cross-coupled blocks (222_ph product), the
+    proton-neutron and neutron-proton pairs of a |Tz| = 1 block apart: rows of
+    one vanish against columns of the other."""
     import numpy as np
     nn, ll, jj, tz, con = (np.asarray(orb[k]) for k in ("nn", "ll", "jj", "itzp", "con"))
     N = len(jj)
@@ -61,16 +63,17 @@ def _cc_flops(orb):
         JC = (q1 % (jtm + 1)) * 2
         PAR = q1 // (2 * jtm + 2)
         TZ = (q1 % (2 * jtm + 2)) // (jtm + 1)
-        r = nb = 0
+        r, nb = {}, {}
         for i in range(N):
             for j in range(N):
                 if not (abs(jj[i] - jj[j]) <= JC <= jj[i] + jj[j]):
                     continue
                 if (ll[i] + ll[j]) % 2 != PAR or abs(tz[i] - tz[j]) // 2 != TZ:
                     continue
-                r += 1
-                nb += int(con[i] == 0 and con[j] == 1)
-        f += 2 * r * r * nb
+                d = int(tz[i] - tz[j])
+                r[d] = r.get(d, 0) + 1
+                nb[d] = nb.get(d, 0) + int(con[i] == 0 and con[j] == 1)
+        f += sum(2 * r[d] * r[d] * nb[d] for d in r)
     return f
 
 

@@ -306,7 +306,7 @@ __global__ void __launch_bounds__(ADJ_THREADS) k_adj_122(DevTables T, AdjLists A
 }
 
 // ---------------------------------------------------------------------------
-// 3. One-body assembly^T over k_assemble_1body's work split (an allowed
+// 3. One-body assembly^T over the one-body assembly's work split (an allowed
 //    upper-triangle element per CTA, every other element per warp).  Forward:
 //      x = c0 v0 + c1 v1 + c2 v2 + c3 v3 + [allowed] (rj v4 + c5 v5)
 //    with v0..v3 the commutator_111 dot products, v4 the 121 sums, v5 the 221

@@ -70,7 +70,7 @@ struct DevTables {
   const unsigned char *cc_rowph;  // per cross-coupled row (a, b): (ja + jb) / 2 odd
   int n_ph_patches;
   // The commutator_122 sums again, for the kernel that runs them ahead of the
-  // products (k_asm2_122): warp g takes elements pre_el[32 g .. 32 g + 32),
+  // products (sums_122): warp g takes elements pre_el[32 g .. 32 g + 32),
   // all with pre_warp[g].n122 terms; term k of its lane l is
   // pre_terms[pre_warp[g].base + 32 k + l] (one coalesced load per term).
   // pre_el: bits 0-27 flat index, 28-29 identical orbit pairs, 30 diagonal;

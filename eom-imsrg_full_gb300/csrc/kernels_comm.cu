@@ -1,24 +1,27 @@
 // kernels_comm.cu -- FP64 kernels of one scalar-scalar commutator [L, R].
 //
-// One commutator is these launches on the basis stream (4 on a side stream
-// beside 3; 5 and the commutator_122 sums of 3 (k_asm2_122) on streams of
-// their own from the start, beside 1 and 2):
-//   1. cc_forward      Pandya transform of L and R into LCC, RCC
-//                      (calculate_cross_coupled, cross_coupled.f90:1190-1300)
-//   2. gemm_fp64       every dense contraction as one grouped GEMM: the 12
+// One commutator is these launches:
+//   1. front           Pandya transform of L and R into LCC, RCC
+//                      (calculate_cross_coupled, cross_coupled.f90:1190-1300),
+//                      and in split precision the block exponents
+//   2. sums_122        commutator_122 of every two-body element (commutators.f90:
+//                      283-396), which needs only L and R (front.cuh)
+//   3. gemm_fp64       every dense contraction as one grouped GEMM: the 12
 //                      ladder products per (2J,Tz,parity) block of
 //                      commutator_222_pp_hh (commutators.f90:596-766) and the
 //                      WCC = LCC RCC^T products of commutator_222_ph (:792-802)
-//                      (the split-precision path replaces this launch)
-//   3. ph_inputs +     every two-body element of RES in one pass: the
-//      assemble_2body  one-body insertions of commutator_122 (:283-396), the
-//                      antisymmetrised ladder epilogue of 222_pp_hh
-//                      (:658-764) and the inverse Pandya recoupling of
-//                      222_ph (:804-923); RES is written once
-//   4. assemble_1body  every one-body element: commutator_111 (:36-80),
-//                      121 (:83-280) and 221 (:435-578)
-//   5. e0              E0 from 110 + 220 (:10-33, :399-432), which need only
+//                      (the split-precision path has its slicing and tensor-core
+//                      launches instead)
+//   4. ph_inputs +     every two-body element of RES: the antisymmetrised ladder
+//      assemble_2body  epilogue of 222_pp_hh (:658-764) and the inverse Pandya
+//                      recoupling of 222_ph (:804-923) on top of the 122 sums
+//   5. one_body        every one-body element: commutator_111 (:36-80),
+//                      121 (:83-280) and 221 (:435-578) (front.cuh)
+//   6. e0              E0 from 110 + 220 (:10-33, :399-432), which need only
 //                      L and R
+// 1, 3 and 4 follow one another on the basis stream; the others run on side
+// streams beside them, or in split precision on small bases inside their
+// launches (commutator_launches).
 // No float atomics: every reduction has a fixed order, so results are
 // bit-reproducible run to run.
 #include "front.cuh"
@@ -281,7 +284,7 @@ __device__ void energy_block(const DevTables &T, const double *L, int hL, const 
 // antisymmetrised ladder epilogue of 222_pp_hh (:658-764) and the 222_ph
 // recoupling sum over J' of {6j} Z(J').  Thread t takes element w0 + t of the
 // work order `heads` while below w1.  PRE: the 122 part is already in RES
-// (k_asm2_122), and the split engine's nexps block exponents are cleared for the
+// (sums_122), and the split engine's nexps block exponents are cleared for the
 // next commutator (nothing reads them any more).  The first n1 CTAs finish the
 // one-body elements instead (one_body_221).  has220 (the allocation-free path, w0 = 0): each CTA leaves
 // its commutator_220 partial in e0p for k_energy.

@@ -205,17 +205,32 @@ __device__ __forceinline__ double sum_partials(const double *partials, int n) {
 // A series term's bookkeeping in one pass over the new term B: C += bx B, X0 = B
 // (the next term's operand, when X0 is set) and the CTA's mat_frob_norm partial
 // of B, in k_norm_partial's order (so the norm has its bits).  E0 (index 0) lies
-// outside the norm chunks and is updated by one thread.
+// outside the norm chunks and is updated by one thread.  What bounds it: the
+// latency of its loads, sixteen rounds of them a CTA before four elements of a
+// thread were in flight (three emax 4 flow steps 1,748 -> 1,647 us, two emax 6
+// steps 3,050 -> 3,018; eight no better).
 __device__ __forceinline__ void series_chunk(double *C, const double *__restrict__ B, double bx, double *X0,
                                              const NormChunk &c, double *partials) {
   __shared__ double sh[32];
+  constexpr int U = 4;  // elements of a thread in flight
+  const int nt = blockDim.x;
   double s = 0.0;
-  for (int i = threadIdx.x; i < c.len; i += blockDim.x) {
-    const long k = c.start + i;
-    const double x = B[k];
-    C[k] = axpby_elem(C[k], 1.0, x, bx);
-    if (X0) X0[k] = x;
-    s = fma(x, x, s);
+  for (int i = threadIdx.x; i < c.len; i += U * nt) {
+    double x[U], y[U];
+#pragma unroll
+    for (int u = 0; u < U; u++)
+      if (i + u * nt < c.len) {
+        x[u] = B[c.start + i + u * nt];
+        y[u] = C[c.start + i + u * nt];
+      }
+#pragma unroll
+    for (int u = 0; u < U; u++)
+      if (i + u * nt < c.len) {
+        const long k = c.start + i + u * nt;
+        C[k] = axpby_elem(y[u], 1.0, x[u], bx);
+        if (X0) X0[k] = x[u];
+        s = fma(x[u], x[u], s);
+      }
   }
   if (blockIdx.x == 0 && threadIdx.x == 0) {
     C[0] = axpby_elem(C[0], 1.0, B[0], bx);

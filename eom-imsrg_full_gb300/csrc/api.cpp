@@ -320,7 +320,7 @@ constexpr size_t kCommGraphs = 8;
 
 // One commutator.  Outside profiling and outside a caller's stream capture,
 // the launch sequence of each argument set is captured once into a CUDA graph
-// and replayed (one launch instead of ~12, and no host work per kernel); the
+// and replayed (one launch instead of five to ten, and no host work per kernel); the
 // graph runs the same kernels on the same data, so results are unchanged.
 int commutator_dev(imsrg_basis *b, const double *L, int hL, const double *R, int hR, double *RES, int hRES,
                    int precision, int with_e0, const HostIO *io) {

@@ -445,7 +445,6 @@ int build_basis(imsrg_basis *b) {
   IMSRG_CUDA_TRY(cudaEventCreateWithFlags(&b->ev_pre, cudaEventDisableTiming));
   IMSRG_CUDA_TRY(cudaEventCreateWithFlags(&b->ev_rdev, cudaEventDisableTiming));
   IMSRG_CUDA_TRY(cudaEventCreateWithFlags(&b->ev_join2, cudaEventDisableTiming));
-  IMSRG_CUDA_TRY(cudaEventCreateWithFlags(&b->ev_hostL, cudaEventDisableTiming));
   for (int k = 0; k < 2; k++) {
     IMSRG_CUDA_TRY(cudaEventCreateWithFlags(&b->ev_fork[k], cudaEventDisableTiming));
     IMSRG_CUDA_TRY(cudaEventCreateWithFlags(&b->ev_join[k], cudaEventDisableTiming));
@@ -1096,10 +1095,9 @@ void free_basis_device(imsrg_basis *b) {
   if (b->ev_rdev) cudaEventDestroy(b->ev_rdev);
   b->ev_join3 = b->ev_pre = b->ev_rdev = nullptr;
   if (b->ev_join2) cudaEventDestroy(b->ev_join2);
-  if (b->ev_hostL) cudaEventDestroy(b->ev_hostL);
   if (b->ev_hostR) cudaEventDestroy(b->ev_hostR);
   if (b->ev_outj) cudaEventDestroy(b->ev_outj);
-  b->ev_join2 = b->ev_hostL = b->ev_hostR = b->ev_outj = nullptr;
+  b->ev_join2 = b->ev_hostR = b->ev_outj = nullptr;
   for (cudaEvent_t &ev : b->ev_out) {
     if (ev) cudaEventDestroy(ev);
     ev = nullptr;

@@ -297,7 +297,6 @@ struct imsrg_basis {
   cudaEvent_t ev_rdev = nullptr;   // a packed host operand R is unpacked on the device
   cudaEvent_t ev_fork[2] = {nullptr, nullptr}, ev_join[2] = {nullptr, nullptr}, ev_join2 = nullptr;
   cudaEvent_t ev_join3 = nullptr;
-  cudaEvent_t ev_hostL = nullptr;  // a host operand L has arrived (commutator_host)
   cudaEvent_t ev_hostR = nullptr;  // a host operand R has arrived
   cudaEvent_t ev_out[imsrg::kOutChunks] = {}, ev_outj = nullptr;  // chunked copy of RES to the host
   // Two-body work order by output range: elements asm2_el[c] .. asm2_el[c+1]

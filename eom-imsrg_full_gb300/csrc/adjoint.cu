@@ -38,6 +38,7 @@
 // central finite differences of the flow.
 #include <cmath>
 #include <cstring>
+#include <new>
 #include <vector>
 
 #include "gemm_fp64.cuh"
@@ -500,12 +501,12 @@ __global__ void k_dot_final(const double *__restrict__ part, double *out) {
 
 }  // namespace
 
-// Per-basis state of the adjoint (allocated on first use).
+// Per-basis state of the adjoint (built on first use; imsrg_basis::adjoint is set
+// once all of it stands).
 struct AdjState {
   double *w1b = nullptr, *w2b = nullptr, *rccb = nullptr, *wccb = nullptr, *zb = nullptr, *u = nullptr;
   double *fpart = nullptr;
   AdjLists lists{};
-  double *monob = nullptr, *part = nullptr, *dot = nullptr, *h_dot = nullptr;
   AdjProb *d_probs = nullptr;
   GemmTile *d_tiles = nullptr;
   int ntiles = 0, nladder = 0;  // tiles: the ladder products', then RCCbar's
@@ -719,10 +720,9 @@ int adj_lists(imsrg_basis *b, AdjState *a) {
 
 }  // namespace
 
-int adjoint_prepare(imsrg_basis *b) {
-  if (b->adjoint) return IMSRG_OK;
-  AdjState *a = new AdjState();
-  b->adjoint = a;
+namespace {
+
+int adj_build(imsrg_basis *b, AdjState *a) {
   IMSRG_TRY(adj_alloc(b, b->nfull, &a->w1b));
   IMSRG_TRY(adj_alloc(b, b->nfull, &a->w2b));
   IMSRG_TRY(adj_alloc(b, b->cc_total, &a->rccb));
@@ -731,10 +731,6 @@ int adjoint_prepare(imsrg_basis *b) {
   IMSRG_TRY(adj_lists(b, a));
   IMSRG_TRY(adj_alloc(b, b->nfull, &a->u));
   IMSRG_TRY(adj_alloc(b, a->lists.n_f_chunks, &a->fpart));
-  IMSRG_TRY(adj_alloc(b, (long)b->norb * b->norb, &a->monob));
-  IMSRG_TRY(adj_alloc(b, DOT_CTAS, &a->part));
-  IMSRG_TRY(adj_alloc(b, 1, &a->dot));
-  IMSRG_CUDA_TRY(cudaMallocHost((void **)&a->h_dot, sizeof(double)));
   std::vector<AdjProb> probs = adjoint_problems(b);
   std::vector<GemmShape> shapes;
   for (const AdjProb &p : probs) {
@@ -761,14 +757,39 @@ int adjoint_prepare(imsrg_basis *b) {
   return IMSRG_OK;
 }
 
-void adjoint_free(imsrg_basis *b) {
-  AdjState *a = adj_of(b);
-  if (!a) return;
-  if (a->h_dot) cudaFreeHost(a->h_dot);
+void adj_delete(AdjState *a) {
   if (a->ev_fork) cudaEventDestroy(a->ev_fork);
   if (a->ev_join) cudaEventDestroy(a->ev_join);
   if (a->side) cudaStreamDestroy(a->side);
   delete a;  // device buffers are in b->dev_allocs
+}
+
+}  // namespace
+
+// All or nothing: what a failed attempt allocated is given back, so that the next
+// call fails or succeeds by itself.
+int adjoint_prepare(imsrg_basis *b) {
+  if (b->adjoint) return IMSRG_OK;
+  AdjState *a = new (std::nothrow) AdjState();
+  if (!a) return IMSRG_ERR_OOM;
+  const size_t mark = b->dev_allocs.size();
+  int s = IMSRG_ERR_OOM;
+  try {
+    s = adj_build(b, a);
+  } catch (const std::bad_alloc &) {  // the host's lists
+  }
+  if (s != IMSRG_OK) {
+    cudaGetLastError();  // returned here: not again by the next launch
+    for (; b->dev_allocs.size() > mark; b->dev_allocs.pop_back()) cudaFree(b->dev_allocs.back());
+    adj_delete(a);
+    return s;
+  }
+  b->adjoint = a;
+  return IMSRG_OK;
+}
+
+void adjoint_free(imsrg_basis *b) {
+  if (b->adjoint) adj_delete(adj_of(b));
   b->adjoint = nullptr;
 }
 
@@ -851,17 +872,21 @@ int commutator_adjoint_dev(imsrg_basis *b, const double *X, int hX, const double
 
 // <x, y> over n doubles in a fixed order, into host memory.
 int dot_dev(imsrg_basis *b, const double *x, const double *y, long n, double *out) {
-  IMSRG_TRY(adjoint_prepare(b));
-  AdjState *a = adj_of(b);
-  k_dot_partial<<<DOT_CTAS, DOT_THREADS, 0, b->stream>>>(x, y, n, a->part);
-  k_dot_final<<<1, 1, 0, b->stream>>>(a->part, a->dot);
+  if (!b->dot_part) IMSRG_TRY(adj_alloc(b, DOT_CTAS + 1, &b->dot_part));
+  double *dot = b->dot_part + DOT_CTAS;
+  k_dot_partial<<<DOT_CTAS, DOT_THREADS, 0, b->stream>>>(x, y, n, b->dot_part);
+  k_dot_final<<<1, 1, 0, b->stream>>>(b->dot_part, dot);
   b->launches += 2;
-  IMSRG_CUDA_TRY(cudaMemcpyAsync(a->h_dot, a->dot, sizeof(double), cudaMemcpyDeviceToHost, b->stream));
+  IMSRG_CUDA_TRY(cudaMemcpyAsync(b->h_scal, dot, sizeof(double), cudaMemcpyDeviceToHost, b->stream));
   IMSRG_CUDA_TRY(cudaStreamSynchronize(b->stream));
-  *out = *a->h_dot;
+  *out = b->h_scal[0];
   return IMSRG_OK;
 }
 
-double *adjoint_monob(imsrg_basis *b) { return adj_of(b) ? adj_of(b)->monob : nullptr; }
+int adjoint_monob(imsrg_basis *b, double **out) {
+  if (!b->monob) IMSRG_TRY(adj_alloc(b, (long)b->norb * b->norb, &b->monob));
+  *out = b->monob;
+  return IMSRG_OK;
+}
 
 }  // namespace imsrg

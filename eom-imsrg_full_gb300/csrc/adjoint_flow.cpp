@@ -102,10 +102,11 @@ int imsrg_gpu_white_adjoint(const imsrg_op_t *H, const imsrg_op_t *ETAbar, imsrg
   if (H->b != ETAbar->b || H->b != Hbar->b) return IMSRG_ERR_MISMATCH;
   if (Hbar == H || Hbar == ETAbar) return IMSRG_ERR_INVALID;
   imsrg_basis *b = H->b;
-  IMSRG_TRY(imsrg::adjoint_prepare(b));
+  double *monob = nullptr;
+  IMSRG_TRY(imsrg::adjoint_monob(b, &monob));
   IMSRG_CUDA_TRY(cudaMemsetAsync(Hbar->d, 0, b->nfull * sizeof(double), b->stream));
   Hbar->herm = H->herm;
-  return imsrg::launch_white_adjoint(b, H->d, H->herm, ETAbar->d, Hbar->d, imsrg::adjoint_monob(b));
+  return imsrg::launch_white_adjoint(b, H->d, H->herm, ETAbar->d, Hbar->d, monob);
 }
 
 int imsrg_gpu_op_dot(const imsrg_op_t *A, const imsrg_op_t *B, double *out) {
@@ -135,6 +136,8 @@ int imsrg_gpu_magnus_decouple_adjoint(imsrg_op_t *HS, imsrg_op_t *G, imsrg_op_t 
   if (ds <= 0.0 || max_steps < 0) return IMSRG_ERR_INVALID;
   if (precision != IMSRG_PREC_FP64 && precision != IMSRG_PREC_OZAKI) return IMSRG_ERR_INVALID;
   IMSRG_TRY(imsrg::adjoint_prepare(b));
+  double *monob = nullptr;
+  IMSRG_TRY(imsrg::adjoint_monob(b, &monob));
   const long nf = b->nfull;
   const size_t nb = nf * sizeof(double);
   cudaStream_t st = b->stream;
@@ -265,7 +268,6 @@ int imsrg_gpu_magnus_decouple_adjoint(imsrg_op_t *HS, imsrg_op_t *G, imsrg_op_t 
   IMSRG_TRY(imsrg::work_op(b, 20, &DGb));
   IMSRG_TRY(imsrg::work_op(b, 21, &Sb));
   IMSRG_TRY(imsrg::work_op(b, 22, &T1));
-  double *monob = imsrg::adjoint_monob(b);
   const double one = 1.0;
   IMSRG_CUDA_TRY(cudaMemsetAsync(H0b->d, 0, nb, st));
   IMSRG_CUDA_TRY(cudaMemsetAsync(HSb->d, 0, nb, st));

@@ -339,8 +339,10 @@ struct imsrg_basis {
   void *ozaki = nullptr;
   int split_digits = 6;  // digits per operand of the split engine (4 to 8), fixed once its plan exists
   int split_chunk_steps = 0;  // K steps per exact accumulator chunk (0: the largest exact one)
-  // Reverse-mode (adjoint) workspace (adjoint.cu), allocated on first use
+  // Reverse-mode (adjoint) workspace (adjoint.cu), each allocated on first use:
+  // the commutator's, the partial sums of a dot product, the White generator's
   void *adjoint = nullptr;
+  double *dot_part = nullptr, *monob = nullptr;
   // Graph of one Magnus flow step (graph.cu), built on first use
   void *flowgraph = nullptr;
   // Captured commutator launch sequences, one per argument set (api.cpp)
@@ -526,7 +528,7 @@ void adjoint_free(imsrg_basis *b);
 int commutator_adjoint_dev(imsrg_basis *b, const double *X, int hX, const double *Cb, int hY, int with_e0,
                            double *Yb);
 int dot_dev(imsrg_basis *b, const double *x, const double *y, long n, double *out);  // fixed order
-double *adjoint_monob(imsrg_basis *b);  // norb x norb scratch of the White adjoint
+int adjoint_monob(imsrg_basis *b, double **out);  // norb x norb scratch of the White adjoint
 
 // Magnus flow step as a CUDA graph (graph.cu)
 int flow_tmp_ops(imsrg_basis *b, imsrg_op **H0, imsrg_op **DG, imsrg_op **X0, imsrg_op **X1);  // api.cpp

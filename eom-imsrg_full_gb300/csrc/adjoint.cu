@@ -216,7 +216,7 @@ __global__ void __launch_bounds__(ADJ_THREADS) k_adj_prep(DevTables T, AdjLists 
 // (k_ph_patches): every entry of WCCbar belongs to one (x, y) of the patches, as
 // W(x,y), W(y',x'), W(x',y') or W(y,x), or as several of them at once, so the
 // patches write the whole plane, zeros included, without atomics.
-__device__ __forceinline__ void adj_ph(const DevTables &T, const double *__restrict__ Zb, int hL, int hR, double *WCCb,
+__device__ __forceinline__ void adj_ph(const DevTables &T, const double *Zb, int hL, int hR, double *WCCb,
                                        int quarter) {
   const PhPatch &p = T.ph_patch[quarter >> 2];
   const int lane = threadIdx.x & 31, ty = (threadIdx.x >> 5) + (quarter & 3) * 8, rl = p.rlen;
@@ -261,9 +261,8 @@ __device__ __forceinline__ void adj_ph(const DevTables &T, const double *__restr
 // target's list; [n0, n1): two-body targets, a warp per 32 (sets Ybar there); the rest: the
 // recoupling inputs^T.
 __global__ void __launch_bounds__(ADJ_THREADS) k_adj_122(DevTables T, AdjLists A, const double *__restrict__ X, int hL,
-                                                         int hR, const double *__restrict__ U,
-                                                         const double *__restrict__ Zb, int first, int n0, int n1,
-                                                         double *fpart, double *WCCb, double *Yb) {
+                                                         int hR, const double *U, const double *Zb, int first,
+                                                         int n0, int n1, double *fpart, double *WCCb, double *Yb) {
   __shared__ double sh[32];
   pdl_wait();
   const int nL = hL < 0, nR = hR < 0;
@@ -435,7 +434,7 @@ __device__ __forceinline__ void adj_1body(const DevTables &T, const double *X, i
 // Tz, pi) block: commutator_220^T, E0 -= 2 herm_R (2J+1) L_pphh R_pphh.
 __global__ void __launch_bounds__(128) k_adj_one(DevTables T, AdjLists A, const double *X, int hL, int hR,
                                                  const double *__restrict__ Cb, int hRES,
-                                                 const double *__restrict__ fpart, int n0, int n1, int n2, double *Yb,
+                                                 const double *fpart, int n0, int n1, int n2, double *Yb,
                                                  double *W1b, double *W2b) {
   pdl_wait();
   const int blk = blockIdx.x;

@@ -15,8 +15,13 @@ namespace imsrg {
 // start when every CTA of the kernel before it on the stream has called
 // pdl_go() or ended; all its threads call pdl_wait() before they touch what
 // earlier work wrote (or write what it reads), which waits for that kernel's
-// end.  Only tables that never change are read ahead of it.  A kernel without
-// pdl_go() lets its successor start as it ends.  on: else an ordinary launch.
+// end.  Only tables that never change are read ahead of it.  What the kernel
+// before it writes is read with ordinary loads, neither through __ldg nor through
+// const __restrict__ pointers: both let the compiler take the non-coherent path,
+// which wants its data unchanged from the kernel's start on, and that start now lies
+// before the writer's end.  Tables, and operands that were whole before the writer
+// began, may be read so.  A kernel without pdl_go() lets its successor start as it
+// ends.  on: else an ordinary launch.
 // In a single commutator the launch gaps of the chain are what it gives: emax 2
 // 22.6 -> 22.1 us split, 16.5 -> 16.0 FP64; emax 6 FP64 483 -> 479; Magnus steps
 // emax 4 1,766 -> 1,737, emax 6 3,256 -> 3,173.  Batches keep ordinary launches:
@@ -209,7 +214,7 @@ __device__ __forceinline__ double sum_partials(const double *partials, int n) {
 // latency of its loads, sixteen rounds of them a CTA before four elements of a
 // thread were in flight (three emax 4 flow steps 1,748 -> 1,647 us, two emax 6
 // steps 3,050 -> 3,018; eight no better).
-__device__ __forceinline__ void series_chunk(double *C, const double *__restrict__ B, double bx, double *X0,
+__device__ __forceinline__ void series_chunk(double *C, const double *B, double bx, double *X0,
                                              const NormChunk &c, double *partials) {
   __shared__ double sh[32];
   constexpr int U = 4;  // elements of a thread in flight

@@ -142,8 +142,7 @@ __device__ __forceinline__ void one_body_mirror(const DevTables &T, const OneBod
 }
 
 // One term of a commutator_221 sum; the second kind enters with -herm_L herm_R.
-__device__ __forceinline__ double term_221(const OneBodyTerm &t, int npm, const double *__restrict__ W1,
-                                           const double *__restrict__ W2) {
+__device__ __forceinline__ double term_221(const OneBodyTerm &t, int npm, const double *W1, const double *W2) {
   const double w = ((t.meta & 8) ? W2 : W1)[t.idx] * t.coef;
   return (t.meta & 3) == 3 ? dflip(w, npm) : w;
 }
@@ -278,8 +277,8 @@ inline int sums_122_ctas(const imsrg_basis *b) {
 // Adds commutator_221 to allowed element number cta (see one_body_front), where a
 // diagonal of fhh or fpp takes it times herm(RES) (((t + s121) hRES + s221) hRES
 // with hRES^2 = 1), and mirrors it.
-__device__ __forceinline__ void one_body_221(const DevTables &T, int hL, int hR, const double *__restrict__ W1,
-                                             const double *__restrict__ W2, double *RES, int hRES, int cta) {
+__device__ __forceinline__ void one_body_221(const DevTables &T, int hL, int hR, const double *W1, const double *W2,
+                                             double *RES, int hRES, int cta) {
   __shared__ double sh[4];
   const long e = T.asm1_heavy[cta];
   const OneBody o = one_body(T, e);

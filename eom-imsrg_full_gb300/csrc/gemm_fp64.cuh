@@ -74,9 +74,9 @@ inline std::vector<GemmTile> gemm_tiles(const std::vector<GemmShape> &ps) {
 // repeat the last one (their sums are not stored).  Ascending k: each sum's
 // rounding does not depend on the tile.  The sign flips A on the integer pipe.
 template <int NI, int NJ>
-__device__ __forceinline__ void gemm_mac(const double *__restrict__ A, long sam, long sak,
-                                         const double *__restrict__ B, long sbk, long sbn, int M, int N, int m0,
-                                         int n0, int k0, int k1, int neg, double (&part)[NI][NJ]) {
+__device__ __forceinline__ void gemm_mac(const double *A, long sam, long sak, const double *B, long sbk, long sbn,
+                                         int M, int N, int m0, int n0, int k0, int k1, int neg,
+                                         double (&part)[NI][NJ]) {
   constexpr int KU = 2;  // k per load group: 1 leaves loads exposed (705 us at emax = 6), 4 takes 206 registers (523 us)
   const int r = threadIdx.x & 7, c = (threadIdx.x >> 3) & 3;
   const double *pa[NI], *pb[NJ];
@@ -90,9 +90,9 @@ __device__ __forceinline__ void gemm_mac(const double *__restrict__ A, long sam,
     for (int u = 0; u < KU; u++)
       if (k + u < k1) {
 #pragma unroll
-        for (int i = 0; i < NI; i++) a[u][i] = __ldg(pa[i] + u * sak);
+        for (int i = 0; i < NI; i++) a[u][i] = pa[i][u * sak];
 #pragma unroll
-        for (int j = 0; j < NJ; j++) b[u][j] = __ldg(pb[j] + u * sbk);
+        for (int j = 0; j < NJ; j++) b[u][j] = pb[j][u * sbk];
       }
 #pragma unroll
     for (int i = 0; i < NI; i++) pa[i] += KU * sak;

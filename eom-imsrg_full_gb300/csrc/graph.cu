@@ -169,7 +169,7 @@ __global__ void __launch_bounds__(256) k_bch_begin(double *G, const double *__re
 // A series term: the sum's update (series_chunk), then its norm and the series'
 // stop test by the last CTA (which rewrites the coefficient that every CTA has read).
 template <bool MAGNUS>
-__global__ void __launch_bounds__(256) k_series_next(double *C, const double *__restrict__ B, double *X0,
+__global__ void __launch_bounds__(256) k_series_next(double *C, const double *B, double *X0,
                                                      const NormChunk *chunks, double *partials, FlowDev *F,
                                                      unsigned *count, cudaGraphConditionalHandle h) {
   const NormChunk c = chunks[blockIdx.x];

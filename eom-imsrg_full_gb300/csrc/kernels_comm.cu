@@ -189,9 +189,8 @@ __device__ __forceinline__ double ph_combine(double w1, double w2, double w3, do
 // once the patch is known, and then their sectors (3.5 million at emax = 6
 // against 6.3 million of one thread per input in the order of Z).
 template <bool INT>
-__global__ void __launch_bounds__(256) k_ph_patches(DevTables T, const double *__restrict__ WCC, int hL, int hR,
-                                                    const int *__restrict__ exps, int gL, int gR, int kshift,
-                                                    double *__restrict__ Z) {
+__global__ void __launch_bounds__(256) k_ph_patches(DevTables T, const double *WCC, int hL, int hR,
+                                                    const int *exps, int gL, int gR, int kshift, double *Z) {
   const PhPatch &p = T.ph_patch[blockIdx.x >> 2];
   const int layers = p.layers;
   const int lane = threadIdx.x & 31, ty = (threadIdx.x >> 5) + (blockIdx.x & 3) * 8, rl = p.rlen;
@@ -219,9 +218,8 @@ __global__ void __launch_bounds__(256) k_ph_patches(DevTables T, const double *_
 
 // The same for small bases, one thread per input in the order of Z.
 template <bool INT>
-__global__ void __launch_bounds__(256) k_ph_list(DevTables T, const double *__restrict__ WCC, int hL, int hR,
-                                                 const int *__restrict__ exps, int gL, int gR, int kshift,
-                                                 double *__restrict__ Z) {
+__global__ void __launch_bounds__(256) k_ph_list(DevTables T, const double *WCC, int hL, int hR,
+                                                 const int *exps, int gL, int gR, int kshift, double *Z) {
   const int t = blockIdx.x * blockDim.x + threadIdx.x;
   const PhTerm p = t < T.n_ph ? T.ph_terms[t] : PhTerm{};
   const unsigned m = 0x0FFFFFFFu;
@@ -291,9 +289,8 @@ __device__ void energy_block(const DevTables &T, const double *L, int hL, const 
 template <bool PRE>
 __global__ void __launch_bounds__(ASM2_THREADS) k_assemble_2body(DevTables T, const double *__restrict__ L, int hL,
                                                                  const double *__restrict__ R, int hR,
-                                                                 const double *__restrict__ W1,
-                                                                 const double *__restrict__ W2,
-                                                                 const double *__restrict__ Z, double *RES, int hRES,
+                                                                 const double *W1, const double *W2, const double *Z,
+                                                                 double *RES, int hRES,
                                                                  const Asm2Head *__restrict__ heads, long w0, long w1,
                                                                  int has220, double *e0p, int *exps, int nexps,
                                                                  int n1) {

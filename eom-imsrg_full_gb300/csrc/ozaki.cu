@@ -256,6 +256,14 @@ __device__ __forceinline__ bool mbar_wait(uint64_t *bar, uint32_t parity, volati
   }
 }
 
+// The same by a whole warp, with one outcome for all its lanes: each lane's wait has
+// its own clock and its own look at the flag, and lanes that disagreed at a time
+// limit would part, some at the warp's next instruction for all 32 lanes
+// (__syncwarp, tcgen05.ld), some at the CTA's last barrier, for good.
+__device__ __forceinline__ bool mbar_wait_warp(uint64_t *bar, uint32_t parity, volatile int *abort_flag) {
+  return __all_sync(0xffffffffu, mbar_wait(bar, parity, abort_flag));
+}
+
 // One 3-D TMA tile of a digit image into shared memory (x = 0: the 16-byte
 // rule on the innermost coordinate always holds; rows past the image arrive
 // as zeros).
@@ -643,7 +651,7 @@ __global__ void __launch_bounds__(oz_threads(S), 1) k_oz_mma(const OzTile *__res
             const int buf = nt & 1;
             const uint32_t use = (uint32_t)(nt >> 1);
             nt++;
-            ok = mbar_wait(&acc_empty[buf], (use & 1) ^ 1, abort_flag);
+            ok = mbar_wait_warp(&acc_empty[buf], (use & 1) ^ 1, abort_flag);
             if (!ok) {
               if (leader) atomicExch(err, 2);
               break;
@@ -652,7 +660,7 @@ __global__ void __launch_bounds__(oz_threads(S), 1) k_oz_mma(const OzTile *__res
             first = true;
             left = kchunk;
           }
-          ok = mbar_wait(&full[stage], phase, abort_flag);
+          ok = mbar_wait_warp(&full[stage], phase, abort_flag);
           if (!ok) {
             if (leader) atomicExch(err, 3);
             break;
@@ -694,7 +702,8 @@ __global__ void __launch_bounds__(oz_threads(S), 1) k_oz_mma(const OzTile *__res
     constexpr int EC = oz_ec(S);
     const int n0 = EC * chunk;
     int nt = 0;
-    for (int ti = t_begin; ti < t_end; ti++) {
+    bool ok = true;  // warp-uniform, as the loops' conditions have to be
+    for (int ti = t_begin; ti < t_end && ok; ti++) {
       const OzTile &P = record(ti);
       if (act && !act[P.inst]) continue;  // an instance whose series has stopped: its outputs stay
       const int Mp = P.rows, Np = P.cols, ldc = P.ldc;
@@ -712,9 +721,12 @@ __global__ void __launch_bounds__(oz_threads(S), 1) k_oz_mma(const OzTile *__res
         const int buf = nt & 1;
         const uint32_t use = (uint32_t)(nt >> 1);
         nt++;
-        if (*abort_flag || !mbar_wait(&acc_full[buf], use & 1, abort_flag)) {
-          if (!*abort_flag) atomicExch(err, 4);
-          *abort_flag = 1;
+        ok = mbar_wait_warp(&acc_full[buf], use & 1, abort_flag);
+        if (!ok) {
+          if (lane == 0) {
+            if (!*abort_flag) atomicExch(err, 4);
+            *abort_flag = 1;
+          }
           break;
         }
         tc_fence_after();
@@ -780,7 +792,6 @@ __global__ void __launch_bounds__(oz_threads(S), 1) k_oz_mma(const OzTile *__res
         }
 #undef OZ_LEVEL_SUM
       }
-      if (*abort_flag) break;
     }
   }
   tc_fence_before();

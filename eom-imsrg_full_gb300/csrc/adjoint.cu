@@ -778,7 +778,6 @@ int adjoint_prepare(imsrg_basis *b) {
   } catch (const std::bad_alloc &) {  // the host's lists
   }
   if (s != IMSRG_OK) {
-    cudaGetLastError();  // returned here: not again by the next launch
     for (; b->dev_allocs.size() > mark; b->dev_allocs.pop_back()) cudaFree(b->dev_allocs.back());
     adj_delete(a);
     return s;

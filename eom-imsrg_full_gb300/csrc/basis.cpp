@@ -21,6 +21,7 @@ namespace imsrg {
 
 int cuda_status(cudaError_t e) {
   if (e == cudaSuccess) return IMSRG_OK;
+  cudaGetLastError();  // reported here: not again by the next call's launches
   if (e == cudaErrorMemoryAllocation) return IMSRG_ERR_OOM;
   if (e == cudaErrorNoDevice || e == cudaErrorInsufficientDriver) return IMSRG_ERR_NO_DEVICE;
   return IMSRG_ERR_CUDA;

@@ -110,3 +110,23 @@ def test_a_dot_product_needs_no_adjoint_tables(fake):
     assert not [x for x in fake.log() if x.startswith("malloc")]
     for o in (X, Y, Z, B):
         o.close()
+
+
+@pytest.mark.parametrize("what", ["k_gemm_fp64", "k_assemble_2body", "k_e0", "malloc"])
+def test_an_error_is_reported_once(fake, what):
+    """The runtime keeps the last error until it is asked for; a call that has
+    returned it leaves none for the next one, which may launch in another way."""
+    api = fake.api
+    B = _basis(api)
+    ops = [api.Operator(B, h) for h in (-1, 1, 1)]
+    B.profile(True)  # launches one by one
+    fake.fail(what)
+    with pytest.raises(api.ImsrgError):
+        if what == "malloc":
+            api.Operator(B, 1)
+        else:
+            api.commutator(*ops)
+    api.commutator(*ops)
+    api.mbpt2(ops[1])
+    for o in (*ops, B):
+        o.close()

@@ -102,8 +102,8 @@ int dhds_dev(imsrg_basis *b, const double *HS, int hH, double *DH, int generator
 // transform), the products (kPhaseProducts) and the part after them
 // (kPhaseBack: assemblies, joins); a batch of commutators runs the products
 // of all its bases in one launch between the two (device operands only).
-int commutator_launches(imsrg_basis *b, const double *L, int hL, const double *R, int hR, double *RES, int hRES,
-                        int precision, int with_e0, const HostIO *io, int phases) {
+static int launch_sequence(imsrg_basis *b, const double *L, int hL, const double *R, int hR, double *RES, int hRES,
+                           int precision, int with_e0, const HostIO *io, int phases) {
   const bool front = phases & kPhaseFront, prods = phases & kPhaseProducts, back = phases & kPhaseBack;
   if (io && phases != kPhaseAll) return IMSRG_ERR_INVALID;
   // While kernel timing is on, every launch goes to the basis stream in the
@@ -258,7 +258,7 @@ int commutator_launches(imsrg_basis *b, const double *L, int hL, const double *R
   }
   if (!back) return IMSRG_OK;
   int *exps = nullptr, nexps = 0;  // cleared by the two-body assembly
-  if (oz) IMSRG_TRY(ozaki_exps_end(b, &exps, &nexps));
+  if (oz) IMSRG_TRY(ozaki_exps(b, &exps, &nexps));
   if (!merged) {  // one-body assembly beside the two-body assembly
     if (!serial) {
       IMSRG_CUDA_TRY(cudaEventRecord(b->ev_fork[1], b->stream));
@@ -286,6 +286,7 @@ int commutator_launches(imsrg_basis *b, const double *L, int hL, const double *R
         IMSRG_CUDA_TRY(cudaMemcpyAsync(io->RES + a0, RES + a0, (size_t)(a1 - a0) * sizeof(double),
                                        cudaMemcpyDeviceToHost, b->side2));
     }
+    if (oz) IMSRG_TRY(ozaki_exps_end(b));
     IMSRG_TRY(join_one());
     IMSRG_TRY(join_e0());
     // E0 and the one-body part
@@ -300,6 +301,7 @@ int commutator_launches(imsrg_basis *b, const double *L, int hL, const double *R
     IMSRG_TRY(launch_ph_inputs(b, hL, hR, precision));
     if (!e0_front) IMSRG_TRY(join_pre());
     IMSRG_TRY(launch_asm2_range(b, L, hL, R, hR, RES, hRES, 0, b->T.n_asm2, false, exps, nexps, merged));
+    if (oz) IMSRG_TRY(ozaki_exps_end(b));
   }
   IMSRG_TRY(join_one());
   if (!e0_front) IMSRG_TRY(join_e0());
@@ -312,6 +314,13 @@ int commutator_launches(imsrg_basis *b, const double *L, int hL, const double *R
     IMSRG_CUDA_TRY(cudaMemcpyAsync(io->RES, RES, bytes, cudaMemcpyDeviceToHost, b->stream));
   }
   return IMSRG_OK;
+}
+
+int commutator_launches(imsrg_basis *b, const double *L, int hL, const double *R, int hR, double *RES, int hRES,
+                        int precision, int with_e0, const HostIO *io, int phases) {
+  const int s = launch_sequence(b, L, hL, R, hR, RES, hRES, precision, with_e0, io, phases);
+  if (s != IMSRG_OK) ozaki_exps_clear(b);
+  return s;
 }
 
 namespace {
@@ -356,6 +365,7 @@ int commutator_dev(imsrg_basis *b, const double *L, int hL, const double *R, int
   const bool graphable = !b->prof.on && cs == cudaStreamCaptureStatusNone && pinned &&
                          (precision != IMSRG_PREC_OZAKI || ozaki_tuned(b));
   if (!graphable) return commutator_launches(b, L, hL, R, hR, RES, hRES, precision, with_e0, io, kPhaseAll);
+  IMSRG_TRY(ozaki_exps_clear(b));
   const HostIO none{nullptr, nullptr, nullptr};
   const HostIO &key = io ? *io : none;
   b->comm_calls++;
@@ -802,7 +812,7 @@ int batch_fp64_list(imsrg_batch *bt, imsrg_op_t *const *L, imsrg_op_t *const *R,
 // products on its own streams, the products of all bases in one launch (the
 // split engine's merged plan, or the merged FP64 list), every basis's part
 // after them, joined back into the batch stream.
-int batch_sequence(imsrg_batch *bt, imsrg_op_t *const *L, imsrg_op_t *const *R, imsrg_op_t *const *RES,
+int batch_launches(imsrg_batch *bt, imsrg_op_t *const *L, imsrg_op_t *const *R, imsrg_op_t *const *RES,
                    int precision, int with_e0) {
   const int n = (int)bt->bases.size();
   const bool oz = precision == IMSRG_PREC_OZAKI;
@@ -835,6 +845,22 @@ int batch_sequence(imsrg_batch *bt, imsrg_op_t *const *L, imsrg_op_t *const *R, 
     IMSRG_CUDA_TRY(cudaStreamWaitEvent(bt->st, bt->ev_back[i], 0));
   }
   return IMSRG_OK;
+}
+
+// The bases' block exponents are zero before the sequence and, where it fails
+// between their parts, again after it.
+int batch_exps_clear(imsrg_batch *bt) {
+  int s = IMSRG_OK;
+  for (imsrg_basis *b : bt->bases)
+    if (const int e = imsrg::ozaki_exps_clear(b)) s = e;
+  return s;
+}
+
+int batch_sequence(imsrg_batch *bt, imsrg_op_t *const *L, imsrg_op_t *const *R, imsrg_op_t *const *RES,
+                   int precision, int with_e0) {
+  const int s = batch_launches(bt, L, R, RES, precision, with_e0);
+  if (s != IMSRG_OK) batch_exps_clear(bt);
+  return s;
 }
 
 }  // namespace
@@ -924,6 +950,7 @@ int imsrg_gpu_batch_commutator(imsrg_batch_t *batch, imsrg_op_t *const *L, imsrg
   if (!graphable) {
     IMSRG_TRY(batch_sequence(batch, L, R, RES, precision, with_e0 ? 1 : 0));
   } else {
+    IMSRG_TRY(batch_exps_clear(batch));
     cudaGraphExec_t exec = nullptr;
     for (const imsrg_batch::Graph &g : batch->graphs)
       if (g.key == key) exec = g.exec;

@@ -359,6 +359,7 @@ int flow_graph_set_s(imsrg_basis *b, double s) {
 int flow_graph_launch(imsrg_basis *b) {
   FlowGraph *fg = flow_of(b);
   if (!fg || !fg->exec) return IMSRG_ERR_INVALID;
+  IMSRG_TRY(ozaki_exps_clear(b));
   IMSRG_CUDA_TRY(cudaGraphLaunch(fg->exec, b->stream));
   IMSRG_CUDA_TRY(cudaMemcpyAsync(fg->h_state, fg->d_state, sizeof(FlowDev), cudaMemcpyDeviceToHost, b->stream));
   return IMSRG_OK;
@@ -697,7 +698,10 @@ int batch_flow_run(imsrg_basis *const *bases, int n, void *oz, cudaStream_t st, 
     IMSRG_TRY(launch_mbpt2(b, HS[i]->d, HS[i]->herm, &f->d_state[i].emp2, &f->d_state[i].e0));
     IMSRG_CUDA_TRY(cudaMemsetAsync(&f->d_state[i].s, 0, sizeof(double), b->stream));
   }
-  for (int i = 0; i < n; i++) IMSRG_CUDA_TRY(cudaStreamSynchronize(bases[i]->stream));
+  for (int i = 0; i < n; i++) {
+    IMSRG_TRY(ozaki_exps_clear(bases[i]));
+    IMSRG_CUDA_TRY(cudaStreamSynchronize(bases[i]->stream));
+  }
   IMSRG_CUDA_TRY(cudaMemcpy(f->h_state, f->d_state, n * sizeof(FlowDev), cudaMemcpyDeviceToHost));
   std::vector<double> sv(n, 0.0), crit(n, 0.0);
   std::vector<int> steps(n, 0), nct(n, 0), stat(n, IMSRG_OK);

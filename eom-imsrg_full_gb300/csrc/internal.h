@@ -494,9 +494,13 @@ int ozaki_chunks(imsrg_basis *b, int p0, int p1, const OzChunk **chunks, int *n,
 // q1], exps[gR + q1]; *exps = nullptr if it cannot.
 int ozaki_cc_exponents(imsrg_basis *b, int **exps, int *gL, int *gR);
 // Around a commutator's launches: exponents zero at its start; its two-body
-// assembly clears the n of them at exps.
+// assembly clears the n of them at exps, and has been enqueued at the end.
 int ozaki_exps_begin(imsrg_basis *b);
-int ozaki_exps_end(imsrg_basis *b, int **exps, int *n);
+int ozaki_exps(imsrg_basis *b, int **exps, int *n);
+int ozaki_exps_end(imsrg_basis *b);
+// Ahead of the replay of a graph that holds split commutators of this basis, and
+// where a sequence fails: zero exponents, if one has not come to its end.
+int ozaki_exps_clear(imsrg_basis *b);
 int ozaki_mma(imsrg_basis *b, int hL, int hR);
 int ozaki_check_error(imsrg_basis *b);  // IMSRG_ERR_TIMEOUT if a bounded device wait gave up
 // synchronise the basis stream and then check as ozaki_check_error, with one

@@ -183,7 +183,7 @@ struct OzPlan {
   OzTile *d_tiles = nullptr;   // grouped by CTA
   int *d_sched_off = nullptr;  // [grid + 1] start of each CTA's tiles
   int *d_exps = nullptr;       // per group: max biased exponent (e = value - 1022), zero between commutators
-  bool exps_dirty = false;     // a commutator was enqueued up to its exponents, not to its end
+  bool exps_dirty = false;     // a commutator was enqueued from its exponents on, but not to its end
   int *d_err = nullptr;
   // All digit images in one buffer of S planes, each `units` 256-byte units (8
   // rows x 16 K, two core matrices): one tensor map per box shape serves every
@@ -1163,22 +1163,56 @@ int ozaki_prepare(imsrg_basis *b) {
 // assembly, the last launch of a commutator on its stream and after every
 // reader of them, leaves them zero for the next one (a memset ahead of each
 // part cost three graph nodes, one of them in the chain to the products).
-// ozaki_exps_begin clears them all where a commutator has not come to its end.
+// A call that fails between leaves maxima behind, which would cost the next
+// commutator its digits: exps_dirty says so, and ozaki_exps_clear sets them to
+// zero, as the failing call returns and, should that fail too, ahead of the next
+// sequence and of every replay.  A captured sequence holds no memset and leaves the
+// flag alone, since nothing has run.
+namespace {
+
+int capturing(imsrg_basis *b, bool *yes) {
+  cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
+  IMSRG_CUDA_TRY(cudaStreamIsCapturing(b->stream, &cs));
+  *yes = cs != cudaStreamCaptureStatusNone;
+  return IMSRG_OK;
+}
+
+}  // namespace
+
+int ozaki_exps_clear(imsrg_basis *b) {
+  OzPlan *pl = plan_of(b);
+  if (!pl || !pl->exps_dirty) return IMSRG_OK;
+  // branches of the failed call may still run, and a batch's stream waits for none
+  for (cudaStream_t s : {b->side, b->side2, b->side3, b->side4}) IMSRG_CUDA_TRY(cudaStreamSynchronize(s));
+  IMSRG_CUDA_TRY(cudaMemsetAsync(pl->d_exps, 0, std::max(pl->ngroups, 1) * sizeof(int), b->stream));
+  IMSRG_CUDA_TRY(cudaStreamSynchronize(b->stream));
+  pl->exps_dirty = false;
+  return IMSRG_OK;
+}
+
 int ozaki_exps_begin(imsrg_basis *b) {
   OzPlan *pl = plan_of(b);
   if (!pl || !pl->ok) return IMSRG_ERR_INVALID;
-  if (pl->exps_dirty)
-    IMSRG_CUDA_TRY(cudaMemsetAsync(pl->d_exps, 0, std::max(pl->ngroups, 1) * sizeof(int), b->stream));
+  bool captured = false;
+  IMSRG_TRY(capturing(b, &captured));
+  if (captured) return IMSRG_OK;
+  IMSRG_TRY(ozaki_exps_clear(b));
   pl->exps_dirty = true;
   return IMSRG_OK;
 }
 
-int ozaki_exps_end(imsrg_basis *b, int **exps, int *n) {
+int ozaki_exps(imsrg_basis *b, int **exps, int *n) {
   OzPlan *pl = plan_of(b);
   if (!pl || !pl->ok) return IMSRG_ERR_INVALID;
   *exps = pl->d_exps;
   *n = pl->ngroups;
-  pl->exps_dirty = false;
+  return IMSRG_OK;
+}
+
+int ozaki_exps_end(imsrg_basis *b) {
+  bool captured = false;
+  IMSRG_TRY(capturing(b, &captured));
+  if (!captured) plan_of(b)->exps_dirty = false;
   return IMSRG_OK;
 }
 

@@ -26,8 +26,8 @@ std::map<const void *, void *> symbols;
 std::set<const void *> pinned;
 Graph *capturing = nullptr;
 cudaError_t last_error = cudaSuccess;
-std::string log_text, fail_what;
-long fail_after = 0;
+std::string log_text;
+std::vector<std::pair<std::string, long>> failures;  // armed: part of a log line, calls to go
 struct {
   dim3 grid, block;
   size_t smem;
@@ -39,14 +39,15 @@ cudaError_t done(cudaError_t e) {
   return e;
 }
 
-// A call: logged, and failed if it is the one armed by fake_fail.
+// A call: logged, and failed if fake_fail has armed it.
 cudaError_t call(const std::string &what) {
   log_text += what + "\n";
-  if (fail_after > 0 && what.find(fail_what) != std::string::npos && --fail_after == 0) {
-    log_text += "failed\n";
-    return done(what.compare(0, 6, "malloc") == 0 ? cudaErrorMemoryAllocation : cudaErrorInvalidConfiguration);
-  }
-  return cudaSuccess;
+  bool fails = false;
+  for (auto &f : failures)
+    if (f.second > 0 && what.find(f.first) != std::string::npos && --f.second == 0) fails = true;
+  if (!fails) return cudaSuccess;
+  log_text += "failed\n";
+  return done(what.compare(0, 6, "malloc") == 0 ? cudaErrorMemoryAllocation : cudaErrorInvalidConfiguration);
 }
 
 // Work on a stream: done now, or recorded while a stream is captured.
@@ -79,10 +80,8 @@ int encode_stub() { return 0; }
 extern "C" {
 
 // The nth call from now on whose log line contains `what` fails.
-void fake_fail(const char *what, long nth) {
-  fail_what = what;
-  fail_after = nth;
-}
+void fake_fail(const char *what, long nth) { failures.push_back({what, nth}); }
+void fake_fail_none() { failures.clear(); }
 const char *fake_log() { return log_text.c_str(); }
 void fake_log_clear() { log_text.clear(); }
 

@@ -50,7 +50,7 @@ def fake(fake_lib, monkeypatch):
     monkeypatch.setattr(api, "_lib", None)
     f = Fake(api)
     yield f
-    f.fail("", 0)
+    api.lib().fake_fail_none()
 
 
 def _basis(api, emax=2):
@@ -130,3 +130,134 @@ def test_an_error_is_reported_once(fake, what):
     api.mbpt2(ops[1])
     for o in (*ops, B):
         o.close()
+
+
+# calls of a live split commutator between its exponents and their clearing
+HALFWAY = ["k_oz_slice", "k_oz_mma", "k_ph_list", "k_assemble_2body"]
+
+
+def _split_basis(api, emax=2):
+    """A basis whose split engine is tuned, and operators of it."""
+    B = _basis(api, emax)
+    ops = [api.Operator(B, h) for h in (-1, 1, 1)]
+    api.commutator(*ops, precision="ozaki")
+    return B, ops
+
+
+def _cleared_before_the_next_front(lines):
+    """The block exponents are set to zero ahead of the first kernel that takes
+    their maxima (k_front)."""
+    front = next(k for k, x in enumerate(lines) if "k_front" in x and x.startswith("launch"))
+    return any(x.startswith("memset") and k + 1 < len(lines) and lines[k + 1] != "failed"
+               for k, x in enumerate(lines[:front]))
+
+
+def _fail_a_live_commutator(fake, B, ops, what, clear_fails=False):
+    api = fake.api
+    B.profile(True)  # launches one by one, no graph
+    fake.log()
+    fake.fail(what)
+    if clear_fails:
+        fake.fail("memset")
+    with pytest.raises(api.ImsrgError):
+        api.commutator(*ops, precision="ozaki")
+    B.profile(False)
+    return fake.log()
+
+
+@pytest.mark.parametrize("what", HALFWAY)
+@pytest.mark.parametrize("clear_fails", [False, True])
+@pytest.mark.parametrize("emax", [2, 5])
+def test_cached_commutator_after_a_failed_one(fake, what, clear_fails, emax):
+    """Block exponents are maxima taken from zero, and a commutator's last kernel
+    leaves them zero.  One that fails before it leaves them large, and a cached
+    graph, which holds no memset, would take them over and lose digits."""
+    api = fake.api
+    if emax == 5 and what == "k_ph_list":
+        what = "k_ph_patches"
+    B, ops = _split_basis(api, emax)
+    for _ in range(2):
+        api.commutator(*ops, precision="ozaki")  # captured, then replayed
+    lines = _fail_a_live_commutator(fake, B, ops, what, clear_fails)
+    api.commutator(*ops, precision="ozaki")
+    after = fake.log()
+    assert "replay" in after and "end of capture" not in after
+    start = next(k for k, x in enumerate(lines) if x == "failed")
+    assert _cleared_before_the_next_front(lines[start:] + after)
+    # once, not with every call from then on
+    api.commutator(*ops, precision="ozaki")
+    assert not [x for x in fake.log() if "memset" in x]
+    for o in (*ops, B):
+        o.close()
+
+
+def test_a_capture_holds_no_memset_and_clears_nothing(fake):
+    """Capturing runs nothing: it neither takes a memset in nor, if it fails,
+    leaves the exponents' state changed."""
+    api = fake.api
+    B, ops = _split_basis(api)
+    lines = _fail_a_live_commutator(fake, B, ops, "k_oz_mma", clear_fails=True)
+    fake.fail("instantiate")
+    with pytest.raises(api.ImsrgError):
+        api.commutator(*ops, precision="ozaki")
+    lines += fake.log()
+    api.commutator(*ops, precision="ozaki")
+    lines += fake.log()
+    assert not [x for x in lines if x.startswith("capture memset")]
+    assert _cleared_before_the_next_front(lines[lines.index("failed"):])
+    for o in (*ops, B):
+        o.close()
+
+
+def test_step_graphs_after_a_failed_commutator(fake):
+    """The single flow's step graph and the lockstep flow of a batch."""
+    api = fake.api
+    B, ops = _split_basis(api)
+    HS, G = api.Operator(B, 1), api.Operator(B, -1)
+    launch = api.lib()["_ZN5imsrg17flow_graph_launchEP11imsrg_basis"]
+    # no kernel runs here, so the flow stops before its first step; its graph is built
+    api.magnus_decouple_graph(HS, G, max_steps=1, precision="ozaki")
+    lines = _fail_a_live_commutator(fake, B, ops, "k_ph_list", clear_fails=True)
+    assert launch(B.handle) == 0
+    after = fake.log()
+    assert "replay" in after
+    assert _cleared_before_the_next_front(lines[lines.index("failed"):] + after)
+    bt = api.Batch([B])
+    bt.magnus_decouple([HS], [G], max_steps=1, precision="ozaki")
+    sizes = {x for x in fake.log() if x.startswith("memset")}
+    _fail_a_live_commutator(fake, B, ops, "k_ph_list", clear_fails=True)
+    bt.magnus_decouple([HS], [G], max_steps=1, precision="ozaki")
+    assert {x for x in fake.log() if x.startswith("memset")} - sizes
+    bt.close()
+    for o in (HS, G, *ops, B):
+        o.close()
+
+
+@pytest.mark.parametrize("what", ["k_oz_mma", "k_oz_slice", "k_assemble_2body"])
+def test_batch_after_a_failed_batch(fake, what):
+    api = fake.api
+    made = [_split_basis(api, e) for e in (2, 3)]
+    bt = api.Batch([b for b, _ in made])
+    args = [[ops[k] for _, ops in made] for k in range(3)]
+    for _ in range(2):
+        bt.commutator(*args)
+    for b, _ in made:
+        b.profile(True)
+    fake.log()
+    fake.fail(what)
+    with pytest.raises(api.ImsrgError):
+        bt.commutator(*args)
+    for b, _ in made:
+        b.profile(False)
+    lines = fake.log()
+    bt.commutator(*args)
+    after = fake.log()
+    assert "replay" in after and "end of capture" not in after
+    # every basis whose part before the products was enqueued
+    fronts = len([x for x in lines if "k_front" in x]) if what != "k_oz_slice" else 1
+    both = lines[lines.index("failed"):] + after[:after.index("replay")]
+    assert len([x for x in both if x.startswith("memset")]) >= min(fronts, 2)
+    bt.close()
+    for b, ops in made:
+        for o in (*ops, b):
+            o.close()

@@ -41,6 +41,7 @@
 #include <new>
 #include <vector>
 
+#include "front.cuh"
 #include "gemm_fp64.cuh"
 
 namespace imsrg {
@@ -333,32 +334,12 @@ __device__ __forceinline__ void adj_1body(const DevTables &T, const double *X, i
     tid = threadIdx.x & 31;
     nt = 32;
   }
-  const long nA2 = (long)A * A, nPA = (long)P * A;
-  int type, p, q, pk, qk;
-  if (e < nA2) {
-    type = 0;
-    p = (int)(e % A);
-    q = (int)(e / A);
-    pk = T.hole_orb[p];
-    qk = T.hole_orb[q];
-  } else if (e < nA2 + nPA) {
-    type = 1;
-    p = (int)((e - nA2) % P);
-    q = (int)((e - nA2) / P);
-    pk = T.part_orb[p];
-    qk = T.hole_orb[q];
-  } else {
-    type = 2;
-    p = (int)((e - nA2 - nPA) % P);
-    q = (int)((e - nA2 - nPA) / P);
-    pk = T.part_orb[p];
-    qk = T.part_orb[q];
-  }
-  const bool allowed = T.orb[pk].x == T.orb[qk].x && T.orb[pk].y == T.orb[qk].y && T.orb[pk].z == T.orb[qk].z;
-  const long base = type == 0 ? T.off_fhh : type == 1 ? T.off_fph : T.off_fpp;
-  const int ld = type == 0 ? A : P;
-  double xb = Cb[base + p + (long)q * ld];
-  if (allowed && type != 1 && p != q) xb += hRES * Cb[base + q + (long)p * ld];
+  const OneBody o = one_body(T, e);
+  const int type = o.type, p = o.p, q = o.q;
+  // whole: the (l, j, tz)-allowed elements of the upper triangles
+  const long at = one_body_at(T, o);
+  double xb = Cb[at];
+  if (whole && type != 1 && p != q) xb += hRES * Cb[at + (q - p) + (long)(p - q) * (type == 0 ? A : P)];
   if (xb == 0.0) return;
   double c0 = 1.0, c1 = 1.0, c2 = -1.0, c3 = -1.0;
   if (type == 0) {
@@ -400,9 +381,9 @@ __device__ __forceinline__ void adj_1body(const DevTables &T, const double *X, i
       atomicAdd(Rpp + k + (long)p * P, b3 * Lpp[q + (long)k * P]);
     }
   }
-  if (!allowed) return;
+  if (!whole) return;
   // commutator_121 (:83-280) and 221 (:435-578) terms
-  const double rj = 1.0 / (T.orb[pk].x + 1.0);
+  const double rj = 1.0 / (T.orb[o.pk].x + 1.0);
   const double u4 = rj * xb, u5 = ((type != 1 && p == q) ? hRES * rj : rj) * xb;
   const int st = T.obt_start[e], n = T.obt_count[e];
   const int nL = hL < 0, nR = hR < 0, npm = hL * hR > 0;

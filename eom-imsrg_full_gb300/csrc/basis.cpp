@@ -863,7 +863,6 @@ int build_basis(imsrg_basis *b) {
                      [](const std::pair<long, int> &x, const std::pair<long, int> &y) { return x.first < y.first; });
     std::vector<int> corder(cit.size());
     for (size_t t = 0; t < cit.size(); t++) corder[t] = cit[t].second;
-    T.n_ccf = (int)corder.size();
     IMSRG_TRY(dev_upload(b, corder, &T.ccf_order));
   }
 

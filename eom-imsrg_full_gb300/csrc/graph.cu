@@ -260,7 +260,7 @@ int build_step_graph(imsrg_basis *b, FlowGraph *fg, imsrg_op *HS, imsrg_op *G, i
   }, nullptr));
   // euler_step, then BCH_EXPAND set-up: HS = H0, X0 = H0
   IMSRG_TRY(capture(b, g, {wm}, [&]() -> int {
-    k_bch_begin<<<(unsigned)std::min<long>((b->nfull + 255) / 256, 152 * 8), 256, 0, b->stream>>>(
+    k_bch_begin<<<(unsigned)std::min<long>((b->nfull + 255) / 256, 8 * b->num_sms), 256, 0, b->stream>>>(
         G->d, DG->d, ds, H0->d, HS->d, X0->d, b->nfull, F, hB);
     return cuda_status(cudaGetLastError());
   }, &fr));

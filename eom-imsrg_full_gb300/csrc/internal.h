@@ -80,7 +80,6 @@ struct DevTables {
   const unsigned long long *pre_terms;
   int n_pre_warps;
   const int *ccf_order;    // cross-coupled elements (bits 0-23), with their exponent group in bits 24-30 if ccf_packed
-  int n_ccf;
   int ccf_packed;
   // Gather lists of the Pandya transform: element e of every CC block is
   // sum_k cct_coef[k] * op[cct_idx[k] & 0x7fffffff] (bit 31: read transposed,
@@ -388,10 +387,10 @@ constexpr int ASM2_THREADS = 128;
 inline int asm2_ctas(const imsrg_basis *b) { return (b->T.n_asm2 + ASM2_THREADS - 1) / ASM2_THREADS; }
 
 // launchers (kernels_*.cu); all enqueue on b->stream and bump b->launches
+struct SumsArgs;
 // What a front launch holds: the exponent chunks of the split engine's parts [p0,
 // p1); the Pandya transform of sides 1 / 2 / 3 (LCC only, RCC only, both; 0 none),
 // with the LCC and RCC block exponents if split.
-struct SumsArgs;
 struct Front {
   int p0 = 0, p1 = 0, sides = 0;
   bool split = false;
@@ -432,17 +431,16 @@ int launch_ph_inputs(imsrg_basis *b, int hL, int hR, int precision);
 constexpr long kPhList = 65536;
 int launch_asm2_range(imsrg_basis *b, const double *L, int hL, const double *R, int hR, double *RES, int hRES,
                       long w0, long w1, bool by_range, int *exps, int nexps, bool one_body);
-// E0 of [L, R] into RES[0] on stream st (independent of the assembly kernels)
 // the one-body elements after the products, in one pass (all) or two
 int launch_one_body(imsrg_basis *b, const SumsArgs &a, bool all, cudaStream_t st);
 // the 122 sums of the two-body elements into RES
 int launch_sums_122(imsrg_basis *b, const SumsArgs &a, cudaStream_t st);
+// E0 of [L, R] into RES[0] on stream st (independent of the assembly kernels)
 int launch_e0(imsrg_basis *b, const double *L, int hL, const double *R, int hR, double *RES, cudaStream_t st);
 int launch_axpby(imsrg_basis *b, const double *A, double ax, const double *B, double bx, double *C);
-int launch_axpby_dev(imsrg_basis *b, const double *A, double ax, const double *B, const double *bx, double *C);
 // S += *coef_dev X1, X0 = X1 (unless X0 is null), *d_norm = mat_frob_norm(X1):
 // one series term's bookkeeping in one pass over X1 (the same values as
-// launch_axpby_dev, a copy and launch_norm)
+// launch_axpby with that coefficient, a copy and launch_norm)
 int launch_series_update(imsrg_basis *b, double *S, const double *X1, const double *coef_dev, double *X0,
                          double *d_norm);
 int launch_norm(imsrg_basis *b, const double *op, double *d_out);

@@ -15,11 +15,9 @@ namespace imsrg {
 
 namespace {
 
-// C = ax A + bx B; bx_dev, when given, supplies bx from device memory (the
-// graph-captured flow), with the same arithmetic as the scalar form.
+// C = ax A + bx B
 __global__ void k_axpby(const double *__restrict__ A, double ax, const double *__restrict__ B, double bx,
-                        const double *bx_dev, double *__restrict__ C, long n) {
-  if (bx_dev) bx = *bx_dev;
+                        double *__restrict__ C, long n) {
   long i = (long)blockIdx.x * blockDim.x + threadIdx.x;
   long stride = (long)gridDim.x * blockDim.x;
   for (; i < n; i += stride) C[i] = axpby_elem(A[i], ax, B[i], bx);
@@ -367,18 +365,9 @@ __global__ void k_check_finite(const double *__restrict__ op, long n, int *flag)
 
 int launch_axpby(imsrg_basis *b, const double *A, double ax, const double *B, double bx, double *C) {
   long n = b->nfull;
-  int grid = (int)std::min<long>((n + 255) / 256, 152 * 8);
+  int grid = (int)std::min<long>((n + 255) / 256, 8 * b->num_sms);
   ProfScope ps(b, IMSRG_KERNEL_OPS);
-  k_axpby<<<grid, 256, 0, b->stream>>>(A, ax, B, bx, nullptr, C, n);
-  b->launches++;
-  return cuda_status(cudaGetLastError());
-}
-
-int launch_axpby_dev(imsrg_basis *b, const double *A, double ax, const double *B, const double *bx, double *C) {
-  long n = b->nfull;
-  int grid = (int)std::min<long>((n + 255) / 256, 152 * 8);
-  ProfScope ps(b, IMSRG_KERNEL_OPS);
-  k_axpby<<<grid, 256, 0, b->stream>>>(A, ax, B, 0.0, bx, C, n);
+  k_axpby<<<grid, 256, 0, b->stream>>>(A, ax, B, bx, C, n);
   b->launches++;
   return cuda_status(cudaGetLastError());
 }
@@ -411,7 +400,7 @@ int launch_generator(imsrg_basis *b, const double *Hden, int hH, const double *H
   double *mono = b->mono;
   ProfScope ps(b, IMSRG_KERNEL_OPS);
   const long nz = b->nfull - 1;
-  const int zero = (int)std::min<long>((nz + 4 * MONO_THREADS - 1) / (4 * MONO_THREADS), 152 * 8);
+  const int zero = (int)std::min<long>((nz + 4 * MONO_THREADS - 1) / (4 * MONO_THREADS), 8 * b->num_sms);
   k_monopole<<<mono_ctas(b->norb) + zero, MONO_THREADS, 0, b->stream>>>(b->T, Hden, hH, mono, ETA + 1, nz);
   long n3 = 0;
   for (int q = 0; q < b->nblocks; q++) n3 += (long)b->gam_n1[q * 6 + 2] * b->gam_n2[q * 6 + 2];
@@ -485,7 +474,7 @@ int launch_normal_order(imsrg_basis *b, const double *Tin, int herm, double *H) 
 
 int launch_check_finite(imsrg_basis *b, const double *op, int *d_flag) {
   IMSRG_CUDA_TRY(cudaMemsetAsync(d_flag, 0, sizeof(int), b->stream));
-  k_check_finite<<<152 * 4, 256, 0, b->stream>>>(op, b->nfull, d_flag);
+  k_check_finite<<<4 * b->num_sms, 256, 0, b->stream>>>(op, b->nfull, d_flag);
   b->launches++;
   return cuda_status(cudaGetLastError());
 }

@@ -190,7 +190,7 @@ struct OzPlan {
   // problem, so no tile waits for a descriptor fetch.
   uint8_t *img = nullptr;
   long units = 0;
-  int nmats = 0, ngroups = 0, nchunks = 0;
+  int ngroups = 0, nchunks = 0;
   // The operands fall in three parts that can be sliced separately: part 0 = L,
   // part 1 = R (both available at once), part 2 = LCC and RCC (after the Pandya
   // transform).  Groups, chunks and image lines are numbered part by part; part
@@ -1119,7 +1119,6 @@ int ozaki_prepare(imsrg_basis *b) {
         pl->tiles.push_back(q);
       }
   }
-  pl->nmats = (int)pl->mats.size();
   pl->grid = std::min(nsm, std::max((int)pl->tiles.size(), 1));
 
   std::vector<OzTile> sched;

@@ -392,9 +392,10 @@ int build_basis(imsrg_basis *b) {
   b->nprobs = (int)pb.probs.size();
 
   // norm chunks (mat_frob_norm weights: fph and non-square gam count twice)
-  // Eight rounds of a CTA's 256 threads: three emax 4 / two emax 6 flow steps take
-  // 1,537 / 2,995 us, 1,614 / 3,032 with 4,096 elements, 1,550 / 3,018 with 1,024,
-  // 1,505 / 3,121 with 512.
+  // Eight rounds of a CTA's 256 threads: side by side on one GPU three emax 4 / two
+  // emax 6 flow steps take 1,537 / 2,995 us, 1,614 / 3,032 with 4,096 elements, 1,550 /
+  // 3,018 with 1,024, 1,505 / 3,121 with 512 (other GPUs read 1,562 to 1,628 / 2,966
+  // to 3,031 with the 2,048 kept).
   constexpr long kNormChunk = 2048;
   std::vector<NormChunk> chunks;
   auto add_seg = [&](long start, long len, int w) {

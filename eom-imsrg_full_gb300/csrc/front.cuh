@@ -10,8 +10,9 @@
 // (20.6 -> 18.5 us at emax 2, 31.3 -> 28.8 at emax 4; batch of twelve 438 -> 432).
 // On large ones (more than kPhList two-body elements) and in FP64 the parts run as
 // branches: the 122 sums then gate the products, and one-body work beside them or
-// ahead of the assembly costs more than the links (emax 5 42.8 us, merged 45.1;
-// emax 6 104, merged 106-112; FP64 at emax 2 15.9, merged 16.4).
+// ahead of the assembly costs more than the links (side by side on one GPU: emax 5
+// 42.8 us, merged 45.1; emax 6 104, merged 106-112; FP64 at emax 2 15.9, merged 16.4;
+// from GPU to GPU the branches read 43 to 47, 104 to 109 and 16.0 to 17.8).
 #pragma once
 
 #include "device.cuh"

@@ -25,7 +25,10 @@
 namespace imsrg {
 
 constexpr int GT_THREADS = 128;
-constexpr int GT_CTAS = 4;  // per SM (128 registers): 16 warps hide the operand loads; 5 or 6 spill and are slower
+// CTAs per SM: 16 warps hide the operand loads.  At its 128 registers a build spills
+// 4 bytes of stores and 32 of loads in the plain and the adjoint's kernel, none in
+// the merged one; five or six spill more and are slower.
+constexpr int GT_CTAS = 4;
 
 // Host side: tiles of problems with outputs m x n and contraction work k (the
 // sum of the terms' lengths), longest first.  split[p]: see gemm_split.

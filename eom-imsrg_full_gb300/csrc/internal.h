@@ -427,7 +427,8 @@ int launch_ph_inputs(imsrg_basis *b, int hL, int hR, int precision);
 // below it the inputs' latency counts and few patches fill the GPU badly, above
 // it the four WCC reads of an input (per input against patches: emax 2 / 4 FP64
 // commutators 19.1 / 39.7 us against 20.1 / 41.0, emax 5 / 6 split 52.8 / 115.0
-// against 47.3 / 111.5).
+// against 47.3 / 111.5).  The same line decides whether a split commutator is a
+// chain of shared launches (front.cuh, which gives both sides' times).
 constexpr long kPhList = 65536;
 int launch_asm2_range(imsrg_basis *b, const double *L, int hL, const double *R, int hR, double *RES, int hRES,
                       long w0, long w1, bool by_range, int *exps, int nexps, bool one_body);

@@ -540,7 +540,7 @@ __global__ void __launch_bounds__(oz_threads(S), 1) k_oz_mma(const OzTile *__res
   OzTile *srec = (OzTile *)(smem + STAGES * STAGE_BYTES + 256);
   constexpr int REC_CAP = oz_rec_cap(S);
   int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  // this CTA's tiles (longest first, assigned on the host)
+  // this CTA's tiles (assigned and ordered on the host, see build_sched)
   const int t_begin = sched_off[blockIdx.x], t_end = sched_off[blockIdx.x + 1];
   for (int i = threadIdx.x; i < min(t_end - t_begin, REC_CAP) * (kRecBytes / 16); i += oz_threads(S))
     reinterpret_cast<uint4 *>(srec)[i] = __ldg(reinterpret_cast<const uint4 *>(tiles + t_begin) + i);
@@ -558,7 +558,8 @@ __global__ void __launch_bounds__(oz_threads(S), 1) k_oz_mma(const OzTile *__res
     *abort_flag = 0;
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
-  // (every stage is written whole by its two TMA boxes before the MMAs read it)
+  // (a stage's live rows are written by its two TMA boxes before the MMAs read them;
+  // what smaller A boxes leave of it reaches no stored output, see the producer)
   asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
   if (warp == 1) {
     asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(tmem_slot)),
@@ -1348,7 +1349,7 @@ int ozaki_schedule_info(imsrg_basis *b, int *choice, int *ncand, double *us, int
 // keeps its own output and exponent pointers (a copy of each basis's exponents
 // into a merged array, twelve graph nodes in a row, took 20 us of a batch of
 // twelve); its tensor maps are renumbered into a merged array, and the tiles of
-// all bases are assigned longest first over one grid.  Tiles compute exactly as in a basis's own launch, so results
+// all bases are spread longest first over one grid (build_sched).  Tiles compute exactly as in a basis's own launch, so results
 // are bit-identical.
 namespace {
 struct OzBatch {
